@@ -34,6 +34,21 @@ struct SkinnyParams {
     int M, N, K;
     int act;
 };
+// Rows of the fp16 quantizers: read as they lie, or computed as the kernel of the reference that would have written them in
+// half does (csrc/sd.cu:611-724).
+enum { SDQ_ROWS = 0, SDQ_LN = 1, SDQ_GEGLU = 2, SDQ_UNPAD = 3, SDQ_GN = 4 };
+struct SdSrc {
+    const half* x;
+    int64_t x_stride;   // ROWS, LN: elements between rows
+    const float* w;     // LN, GN: weight and bias
+    const float* b;
+    float eps;          // LN, GN
+    int heads, d, dp;   // UNPAD: heads of d values stored dp wide
+    const double* sums; // GN: per (image, group) sum and sum of squares
+    int groups;         // GN
+    int64_t P;          // GN: pixels per image
+    double cnt;         // GN: values per group, P * C / groups
+};
 // Helpers shared between the translation units (a namespace of their own: the static archive exports them).
 namespace b200q {
 // quant_rows.cu: table of bf16(act(x)) over all bf16 x for Act code `act`, built on first use (on `st`)
@@ -43,8 +58,8 @@ int quant_status_read_clear(int* out);
 // quant_rows.cu: gpu_rotate_rows_f32's prologue + rotation with the rows written as two bf16 terms [M, K] each
 int rotate_rows_split(int prologue, const float* x, int64_t x_stride, int64_t up_offset, const float* norm_w, float eps, void* hi,
                       void* lo, int M, int K, cudaStream_t st);
-// quant_rows.cu: the fp16 row quantizer on the register kernel; false when the shape is outside what it takes
-bool sd_quant_rows_fast(const void* x, int64_t x_stride, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st, int* rc);
+// quant_rows.cu: the fp16 row quantizers on the register kernel; false when the shape is outside what it takes
+bool sd_quant_fast(int src, const SdSrc& s, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st, int* rc);
 bool skinny_gemm_applies(int64_t M, int64_t N, int64_t K);
 int launch_skinny_gemm(int epi, const SkinnyParams& p, int out_dt, int sms, cudaStream_t st);
 // gemm_skinny.cu: the CUDA-core kernel for operands TMA cannot address (K % 16 != 0, bases off a 16-byte boundary)

@@ -561,10 +561,141 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
 // of registers. The division is a reciprocal multiply with one Newton step: the exact quotient of two 11-bit significands
 // is never on a half rounding boundary and at least 2^-23 (relative) away from one, and the refined product is within
 // 2^-24 of it, so both round to the same half (tests/test_quant_division.py enumerates the significand pairs).
-template <int ROT>
-__global__ void __launch_bounds__(512) sd_quant_fast_kernel(const half* __restrict__ x, int64_t x_stride, int8_t* __restrict__ q,
-                                                            float* __restrict__ scales, int M, int K, int tpr, int rows,
-                                                            uint32_t off_amax) {
+//
+// SRC: where a row comes from. SDQ_ROWS reads it as it lies; the other sources compute it as the reference kernel that would
+// have written it in half does (csrc/sd.cu:611-724: LayerNorm, GEGLU, head un-padding, GroupNorm without SiLU). They run as a
+// first phase in which consecutive lanes hold consecutive 16-byte pieces (eight values), so that rows, gates and per-column
+// vectors are read coalesced and each once, and leave the rows in shared memory as half, from where the lanes pick up their
+// 32 values. A row at a time in shared memory as floats, one value per thread and step, was bound by its instruction count:
+// 8192 x 640 LayerNorm 49.2 us, GroupNorm 44.3, GEGLU 8192 x 2560 108 us; this form takes 16.6, 13.8 and 50 us (2048 x 1280:
+// LayerNorm 20.7 -> 9.5).
+// LayerNorm statistics in the reference's order of additions: there 256 threads hold the row, thread t the elements t, t + 256,
+// ... one after the other, then a xor-shuffle tree over the lanes of each warp and another over the eight warps. Here one
+// warp holds a row, lane l the values 8 l .. 8 l + 7 of each run of 256, so the chains over the runs are the lane's own eight
+// accumulators, and the trees run over lane bits 1, 0 and index bits 2, 1, 0 (the lanes of a warp there), then over lane bits
+// 4, 3, 2 (the warps).
+__device__ __forceinline__ float sd_tree256(float (&a)[8]) {
+#pragma unroll
+    for (int o = 2; o >= 1; o >>= 1) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = __fadd_rn(a[i], __shfl_xor_sync(0xffffffffu, a[i], o));
+    }
+    float t = __fadd_rn(__fadd_rn(__fadd_rn(a[0], a[4]), __fadd_rn(a[2], a[6])), __fadd_rn(__fadd_rn(a[1], a[5]), __fadd_rn(a[3], a[7])));
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) t = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+    return t;
+}
+// 16-byte piece c of a row in shared memory sits at piece c ^ ((c >> 2) & 7): pieces in order (phase one) and pieces
+// 4 t + k over lanes t (phase two) are both free of bank conflicts. Rows are padded to whole blocks of eight pieces.
+__device__ __forceinline__ int sd_piece(int c) { return c ^ ((c >> 2) & 7); }
+__device__ __forceinline__ void unpack_half8(const uint4 u, float (&v)[8]) {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+        v[2 * i] = f.x, v[2 * i + 1] = f.y;
+    }
+}
+__device__ __forceinline__ uint4 pack_half8(const float (&v)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 h = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+template <int SRC>
+__device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int pitch, float2* stat, int64_t m0, int live_rows, int K) {
+    const int pieces = K >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    if constexpr (SRC == SDQ_LN) {
+        // the rows as they lie first, all of them in flight together
+        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
+            const int r = i / pieces, c = i - r * pieces;
+            row_s[r * pitch + sd_piece(c)] = __ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * s.x_stride) + c);
+        }
+        __syncthreads();
+        if (warp < nwarps)       // whole warps only
+            for (int r = warp; r < live_rows; r += nwarps) {
+                uint4* row = row_s + r * pitch;
+                float a[8], e[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[i] = 0.f;
+                for (int c = lane; c < pieces; c += 32) {
+                    unpack_half8(row[sd_piece(c)], e);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) a[i] = __fadd_rn(a[i], e[i]);
+                }
+                const float mean = __fdiv_rn(sd_tree256(a), (float)K);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) a[i] = 0.f;
+                for (int c = lane; c < pieces; c += 32) {
+                    unpack_half8(row[sd_piece(c)], e);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float d = __fsub_rn(e[i], mean);
+                        a[i] = __fmaf_rn(d, d, a[i]);
+                    }
+                }
+                const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(sd_tree256(a), (float)K), s.eps));
+                for (int c = lane; c < pieces; c += 32) {
+                    float w[8], b[8];
+                    load8v(s.w + 8 * c, w), load8v(s.b + 8 * c, b);
+                    unpack_half8(row[sd_piece(c)], e);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) e[i] = __fmaf_rn(__fmul_rn(__fsub_rn(e[i], mean), rstd), w[i], b[i]);
+                    row[sd_piece(c)] = pack_half8(e);
+                }
+            }
+    } else if constexpr (SRC == SDQ_GN) {
+        // mean and reciprocal deviation of this image's groups (csrc/sd.cu:198-205), once per CTA
+        const int n = (int)(m0 / s.P);
+        for (int g = threadIdx.x; g < s.groups; g += blockDim.x) {
+            const double su = s.sums[(n * s.groups + g) * 2], sq = s.sums[(n * s.groups + g) * 2 + 1];
+            const double mean = su / s.cnt;
+            const double var = fmax(fma(-mean, mean, sq / s.cnt), 0.0);
+            stat[g] = make_float2((float)mean, (float)(1.0 / sqrt(var + (double)s.eps)));
+        }
+        __syncthreads();
+        const int per = K / s.groups;
+        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
+            const int r = i / pieces, c = i - r * pieces;
+            float e[8], w[8], b[8];
+            unpack_half8(__ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)K) + c), e);
+            load8v(s.w + 8 * c, w), load8v(s.b + 8 * c, b);
+            int g = (8 * c) / per, left = per - (8 * c - g * per);      // values of the group from here on
+            float2 st = stat[g];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (left == 0) st = stat[++g], left = per;
+                --left;
+                e[j] = __fmaf_rn(__fmul_rn(__fsub_rn(e[j], st.x), st.y), w[j], b[j]);
+            }
+            row_s[r * pitch + sd_piece(c)] = pack_half8(e);
+        }
+    } else if constexpr (SRC == SDQ_GEGLU) {
+        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
+            const int r = i / pieces, c = i - r * pieces;
+            const uint4* in = reinterpret_cast<const uint4*>(s.x + (m0 + r) * 2 * (int64_t)K);
+            float e[8], g[8];
+            unpack_half8(__ldg(in + c), e), unpack_half8(__ldg(in + pieces + c), g);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) e[j] = __fmul_rn(e[j], rnd<half>(gelu_f(g[j])));
+            row_s[r * pitch + sd_piece(c)] = pack_half8(e);
+        }
+    } else if constexpr (SRC == SDQ_UNPAD) {
+        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
+            const int r = i / pieces, c = i - r * pieces, h = (8 * c) / s.d;      // d % 8 == 0: a piece lies inside one head
+            row_s[r * pitch + sd_piece(c)] =
+                __ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)s.heads * s.dp + (int64_t)h * s.dp + (8 * c - h * s.d)));
+        }
+    }
+}
+
+template <int ROT, int SRC>
+__global__ void __launch_bounds__(512) sd_quant_fast_kernel(const SdSrc s, int8_t* __restrict__ q, float* __restrict__ scales, int M,
+                                                            int K, int tpr, int rows, uint32_t off_amax, uint32_t off_rows) {
     extern __shared__ __align__(128) uint8_t smem[];
     const unsigned wmask = __activemask();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -573,22 +704,27 @@ __global__ void __launch_bounds__(512) sd_quant_fast_kernel(const half* __restri
     float* tbuf_w = tbuf - 2 * (team >> 1);
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem + off_amax);
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
-    __syncthreads();
+    // rows of this CTA; GroupNorm's belong to one image (blockIdx.y), so that one set of statistics serves the CTA
+    const int64_t limit = SRC == SDQ_GN ? (int64_t)(blockIdx.y + 1) * s.P : M;
+    const int64_t m0 = (SRC == SDQ_GN ? (int64_t)blockIdx.y * s.P : 0) + (int64_t)blockIdx.x * rows;
     const int rloc = threadIdx.x / tpr, tin = threadIdx.x - rloc * tpr;
-    const int64_t m_raw = (int64_t)blockIdx.x * rows + rloc;
-    const bool live = m_raw < M;
-    const int64_t m = live ? m_raw : M - 1;            // idle rows recompute the last row and store nothing
-    const half* r = x + m * x_stride + tin * 32;
+    const int64_t m_raw = m0 + rloc;
+    const bool live = m_raw < limit;
+    const int64_t m = live ? m_raw : limit - 1;        // idle rows recompute the last row and store nothing
     float v[32];
+    if constexpr (SRC == SDQ_ROWS) {
+        __syncthreads();
+        const uint4* r = reinterpret_cast<const uint4*>(s.x + m * s.x_stride) + 4 * tin;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(r) + c);
-        const __half2* h = reinterpret_cast<const __half2*>(&u);
+        for (int c = 0; c < 4; ++c) unpack_half8(__ldg(r + c), *reinterpret_cast<float(*)[8]>(v + 8 * c));
+    } else {
+        uint4* row_s = reinterpret_cast<uint4*>(smem + off_rows);
+        const int pitch = ((K >> 3) + 7) & ~7;
+        sd_source_rows<SRC>(s, row_s, pitch, reinterpret_cast<float2*>(amax_s + ((rows + 1) & ~1)), m0, (int)min((int64_t)rows, limit - m0), K);
+        __syncthreads();
+        const uint4* r = row_s + (int)(m - m0) * pitch;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 f = __half22float2(h[i]);
-            v[8 * c + 2 * i] = f.x, v[8 * c + 2 * i + 1] = f.y;
-        }
+        for (int c = 0; c < 4; ++c) unpack_half8(r[sd_piece(4 * tin + c)], *reinterpret_cast<float(*)[8]>(v + 8 * c));
     }
     float2 P[16];
     if (ROT) {
@@ -757,41 +893,78 @@ int ensure_lut(int which, cudaStream_t st) {
 
 }  // namespace
 
-// gpu_sd_quant_rows through the register kernel above; false when the shape is not one it takes (the caller falls back).
-bool b200q::sd_quant_rows_fast(const void* x, int64_t x_stride, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st,
-                               int* rc) {
-    if (K % 32 || K > 16384 || (rotate == 64 && K % 64) || (rotate == 256 && K % 256) || (rotate != 0 && rotate != 64 && rotate != 256))
-        return false;
-    if ((((uintptr_t)x | (uintptr_t)q) & 15) || (x_stride & 7)) return false;
+namespace {
+template <int ROT, int SRC>
+int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaStream_t st) {
+    auto kern = sd_quant_fast_kernel<ROT, SRC>;
     const int tpr = K / 32;
+    // whole rows and about 256 threads; a whole number of warps where that takes no more than 512
     int rows = 256 / tpr;
     if (rows < 1) rows = 1;
     if (rows * tpr < 32) rows = (32 + tpr - 1) / tpr;
+    if (SRC != SDQ_ROWS) {
+        int even = 32;                                  // rows that make a whole number of warps
+        while (even > 1 && (even / 2 * tpr) % 32 == 0) even /= 2;
+        if (even * tpr <= 512) rows = rows / even > 0 ? rows / even * even : even;
+    }
     const int threads = rows * tpr;
-    const uint32_t off_amax = rotate == 256 ? (uint32_t)((threads + 31) / 32) * kWarpWords * 4 : 0;
-    const size_t smem = off_amax + (size_t)rows * 4;
-    const unsigned grid = (unsigned)((M + rows - 1) / rows);
-    const half* xh = (const half*)x;
-    *rc = 0;
-    if (rotate == 256) {
+    uint32_t off = ROT == 256 ? (uint32_t)((threads + 31) / 32) * kWarpWords * 4 : 0;
+    const uint32_t off_amax = off;
+    off += (uint32_t)((rows + 1) & ~1) * 4 + (SRC == SDQ_GN ? (uint32_t)s.groups * 8 : 0);
+    off = (off + 127) & ~127u;
+    const uint32_t off_rows = off;
+    if (SRC != SDQ_ROWS) off += (uint32_t)rows * (((K >> 3) + 7) & ~7) * 16;
+    if (off > 48 * 1024) {
         static std::atomic<uint64_t> configured{0};
         int dev = 0;
         cudaGetDevice(&dev);
         const uint64_t bit = 1ull << (dev & 63);
-        if (smem > 48 * 1024 && !(configured.load(std::memory_order_acquire) & bit)) {
-            const cudaError_t e = cudaFuncSetAttribute(sd_quant_fast_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-            if (e != cudaSuccess) { *rc = (int)e; return true; }
+        if (!(configured.load(std::memory_order_acquire) & bit)) {
+            const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024);
+            if (e != cudaSuccess) return (int)e;
             configured.fetch_or(bit, std::memory_order_release);
         }
-        sd_quant_fast_kernel<256><<<grid, threads, smem, st>>>(xh, x_stride, q, scales, M, K, tpr, rows, off_amax);
-    } else if (rotate == 64) {
-        sd_quant_fast_kernel<64><<<grid, threads, smem, st>>>(xh, x_stride, q, scales, M, K, tpr, rows, off_amax);
-    } else {
-        sd_quant_fast_kernel<0><<<grid, threads, smem, st>>>(xh, x_stride, q, scales, M, K, tpr, rows, off_amax);
     }
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) *rc = (int)e;
-    return true;
+    const dim3 grid = SRC == SDQ_GN ? dim3((unsigned)((s.P + rows - 1) / rows), (unsigned)(M / s.P)) : dim3((unsigned)((M + rows - 1) / rows));
+    kern<<<grid, threads, off, st>>>(s, q, scales, M, K, tpr, rows, off_amax, off_rows);
+    KCHECK();
+    return 0;
+}
+template <int SRC>
+int launch_sd_fast_rot(const SdSrc& s, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st) {
+    return rotate == 256 ? launch_sd_fast<256, SRC>(s, q, scales, M, K, st)
+           : rotate == 64 ? launch_sd_fast<64, SRC>(s, q, scales, M, K, st) : launch_sd_fast<0, SRC>(s, q, scales, M, K, st);
+}
+}  // namespace
+
+// The fp16 quantizers (gpu_sd_*quant_rows) through the register kernel above; false when the shape is not one it takes (the
+// caller falls back): rows of whole 32-value pieces and rotation groups up to 16384 values, 16-byte aligned.
+bool b200q::sd_quant_fast(int src, const SdSrc& s, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st, int* rc) {
+    if (K % 32 || K > 16384 || (rotate == 64 && K % 64) || (rotate == 256 && K % 256) || (rotate != 0 && rotate != 64 && rotate != 256))
+        return false;
+    if (((uintptr_t)s.x | (uintptr_t)q) & 15) return false;
+    switch (src) {
+        case SDQ_ROWS:
+            if (s.x_stride & 7) return false;
+            *rc = launch_sd_fast_rot<SDQ_ROWS>(s, q, scales, M, K, rotate, st);
+            return true;
+        case SDQ_LN:
+            if ((s.x_stride & 7) || (((uintptr_t)s.w | (uintptr_t)s.b) & 15)) return false;
+            *rc = launch_sd_fast_rot<SDQ_LN>(s, q, scales, M, K, rotate, st);
+            return true;
+        case SDQ_GEGLU:
+            *rc = launch_sd_fast_rot<SDQ_GEGLU>(s, q, scales, M, K, rotate, st);
+            return true;
+        case SDQ_UNPAD:
+            if ((s.d & 7) || (s.dp & 7)) return false;
+            *rc = launch_sd_fast_rot<SDQ_UNPAD>(s, q, scales, M, K, rotate, st);
+            return true;
+        case SDQ_GN:
+            if ((((uintptr_t)s.w | (uintptr_t)s.b) & 15) || M / s.P > 65535) return false;
+            *rc = launch_sd_fast_rot<SDQ_GN>(s, q, scales, M, K, rotate, st);
+            return true;
+        default: return false;
+    }
 }
 
 // Reads and clears the quantizer's status word (a staging wait that ran out); used by gpu_kernels_status.

@@ -166,12 +166,9 @@ __global__ void __launch_bounds__(256) sd_quant_rows_kernel(const half* __restri
     sd_quant_tail(row, red, q + m * (int64_t)K, scales + m, K, rotate, vec);
 }
 
-// The same quantizer for the run-time case (activations of every SD linear): rows in registers instead of shared memory.
-// A thread holds 16 consecutive values: stages 0 and 1 of the rotation are its own; stage 2 (and 3 for groups of 256)
-// pairs it with the three other lanes whose position differs in index bits 4-5 (6-7) through shuffles, each lane
-// computing its own output row of the H4 block with the reference's association ((+-x0 +- x1) +- x2) +- x3. Several rows
-// per CTA, row maximum through a shared-memory atomicMax. Bit-identical to the kernel above.
-template <int ROT>
+// Unrotated rows of an odd number of 16-value pieces (the register kernel of quant_rows.cu takes whole 32-value pieces): a
+// thread holds 16 consecutive values in registers, several rows per CTA, row maximum through a shared-memory atomicMax.
+// Bit-identical to the kernel above.
 __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __restrict__ x, int64_t x_stride,
                                                                 int8_t* __restrict__ q, float* __restrict__ scales, int M, int K,
                                                                 int tpr, int rows_per_cta) {
@@ -191,26 +188,6 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
         for (int i = 0; i < 8; ++i) {
             const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
             v[2 * i] = f.x, v[2 * i + 1] = f.y;
-        }
-    }
-    if (ROT) {
-#pragma unroll
-        for (int i = 0; i < 16; i += 4) h4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) h4(v[i], v[i + 4], v[i + 8], v[i + 12]);
-        const int lane = threadIdx.x & 31;
-#pragma unroll
-        for (int st = 0; st < (ROT == 256 ? 2 : 1); ++st) {
-            const int sh = st ? 4 : 1;                    // lane distance between the block's four inputs
-            const int pos = (tin / sh) & 3;               // this lane's row of the H4 block
-            const int base = lane - pos * sh;
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float x0 = __shfl_sync(0xffffffffu, v[i], base), x1 = __shfl_sync(0xffffffffu, v[i], base + sh);
-                const float x2 = __shfl_sync(0xffffffffu, v[i], base + 2 * sh), x3 = __shfl_sync(0xffffffffu, v[i], base + 3 * sh);
-                const float a = pos == 3 ? -x0 : x0, b = pos == 2 ? -x1 : x1, c = pos == 1 ? -x2 : x2, d = pos == 0 ? -x3 : x3;
-                v[i] = __fmul_rn(0.5f, __fadd_rn(__fadd_rn(__fadd_rn(a, b), c), d));
-            }
         }
     }
     float mx = 0.f;
@@ -235,20 +212,6 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
 // The same quantizer over a row that another of the reference's kernels would have written in half first
 // (csrc/sd.cu:611-724): the row is computed as that kernel computes it, rounded to half, then quantized as above.
 // 256 threads, each adding elements t, t + 256, ... and then the block tree: the reference's order of additions.
-enum { SDQ_LN = 1, SDQ_GEGLU = 2, SDQ_UNPAD = 3, SDQ_GN = 4 };
-struct SdSrc {
-    const half* x;
-    int64_t x_stride;   // LN: elements between rows
-    const float* w;     // LN, GN: weight and bias
-    const float* b;
-    float eps;          // LN, GN
-    int heads, d, dp;   // UNPAD: heads of d values stored dp wide
-    const double* sums; // GN: per (image, group) sum and sum of squares
-    int groups;         // GN
-    int64_t P;          // GN: pixels per image
-    double cnt;         // GN: values per group, P * C / groups
-};
-
 // GroupNorm statistics of x [N, P, C] half: per (image, group) the sum and the sum of squares, accumulated in double
 // from per-block float sums as the reference's sd_group_sums_kernel forms them (csrc/sd.cu:209-233: 256 threads, thread
 // t takes values t, t + 256, ... of the block's pixel range, then the block tree), so the statistics come out the same.
@@ -260,11 +223,29 @@ __global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* __restri
     const int64_t base = (int64_t)n * P * C + g * per;
     const int64_t p0 = P * split / splits, p1 = P * (split + 1) / splits;
     const int64_t count = (p1 - p0) * per;
+    // Value i of the block's range is channel i % per of pixel i / per. The index advances by 256 values with one addition and
+    // one comparison each for pixel and channel (a 64-bit division per value bound this kernel: 2 x 4096 x 640 took 23.0 us, now 11.8), and
+    // eight values are requested before the first is added, which is what hides the memory latency of the serial sums.
     float s = 0.f, ss = 0.f;
-    for (int64_t i = threadIdx.x; i < count; i += blockDim.x) {
-        const float v = __half2float(x[base + (p0 + i / per) * C + (int)(i % per)]);
-        s = __fadd_rn(s, v);
-        ss = __fmaf_rn(v, v, ss);
+    const int dp = 256 / per, dc = 256 - dp * per;
+    int c = (int)threadIdx.x % per;
+    const half* px = x + base + (p0 + (int)threadIdx.x / per) * C;
+    constexpr int kAhead = 8;
+    for (int64_t i = threadIdx.x; i < count; i += 256 * kAhead) {
+        half h[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            h[u] = i + 256 * u < count ? px[c] : __ushort_as_half(0);
+            px += (int64_t)dp * C, c += dc;
+            if (c >= per) c -= per, px += C;
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (i + 256 * u >= count) break;
+            const float v = __half2float(h[u]);
+            s = __fadd_rn(s, v);
+            ss = __fmaf_rn(v, v, ss);
+        }
     }
     s = block_sum(s, red);
     __syncthreads();
@@ -570,11 +551,12 @@ GPU_API int gpu_sd_quant_rows(const void* x, int64_t x_stride, int8_t* q, float*
     if (M <= 0 || K <= 0) return 0;
     {   // rows of whole 32-value pieces: the quantizer's register kernel (transposition through shared memory for R256)
         int rc = 0;
-        if (sd_quant_rows_fast(x, x_stride, q, scales, M, K, rotate, (cudaStream_t)stream, &rc)) return rc;
+        SdSrc src{};
+        src.x = (const half*)x, src.x_stride = x_stride;
+        if (sd_quant_fast(SDQ_ROWS, src, q, scales, M, K, rotate, (cudaStream_t)stream, &rc)) return rc;
     }
-    // register kernel: whole 16-value pieces per thread, rotation groups inside a warp, aligned rows
     const int tpr = K / 16;
-    if (K % 16 == 0 && tpr <= 512 && x_stride % 8 == 0 && (((uintptr_t)x & 15) == 0) && (((uintptr_t)q & 15) == 0)) {
+    if (rotate == 0 && K % 16 == 0 && tpr <= 512 && x_stride % 8 == 0 && (((uintptr_t)x & 15) == 0) && (((uintptr_t)q & 15) == 0)) {
         const int gcd32 = tpr % 32 == 0 ? 32 : tpr % 16 == 0 ? 16 : tpr % 8 == 0 ? 8 : tpr % 4 == 0 ? 4 : tpr % 2 == 0 ? 2 : 1;
         const int r0 = 32 / gcd32;                       // rows that make the CTA a whole number of warps
         int rows = r0 * (256 / (tpr * r0) > 0 ? 256 / (tpr * r0) : 1);
@@ -583,9 +565,7 @@ GPU_API int gpu_sd_quant_rows(const void* x, int64_t x_stride, int8_t* q, float*
             const size_t sm = (size_t)rows * sizeof(unsigned);
             cudaStream_t st = (cudaStream_t)stream;
             const half* xh = (const half*)x;
-            if (rotate == 0) sd_quant_rows_reg_kernel<0><<<grid, threads, sm, st>>>(xh, x_stride, q, scales, M, K, tpr, rows);
-            else if (rotate == 64) sd_quant_rows_reg_kernel<64><<<grid, threads, sm, st>>>(xh, x_stride, q, scales, M, K, tpr, rows);
-            else sd_quant_rows_reg_kernel<256><<<grid, threads, sm, st>>>(xh, x_stride, q, scales, M, K, tpr, rows);
+            sd_quant_rows_reg_kernel<<<grid, threads, sm, st>>>(xh, x_stride, q, scales, M, K, tpr, rows);
             KCHECK();
             return 0;
         }
@@ -604,6 +584,10 @@ template <int MODE>
 int launch_sd_src(const SdSrc& p, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st) {
     if ((rotate != 0 && rotate != 64 && rotate != 256) || (rotate && K % rotate)) return -1;
     if (M <= 0 || K <= 0) return 0;
+    {
+        int rc = 0;
+        if (sd_quant_fast(MODE, p, q, scales, M, K, rotate, st, &rc)) return rc;
+    }
     const size_t smem = (size_t)padded_words(K) * sizeof(float);
     if (int rc = set_smem((const void*)sd_quant_src_kernel<MODE>, smem)) return rc;
     const int vec = (K % 8 == 0) && (((uintptr_t)q & 7) == 0);

@@ -255,3 +255,30 @@ def test_argument_checks_of_the_packers_and_fused_quantizers(pkg, dev):
         L.sd_group_norm_quant_rows(x.view(1, 4, 640), w, w, 48, 1e-5, 0)                       # 640 % 48
     q, s = L.sd_unpad_quant_rows(torch.zeros((0, 10, 72), dtype=torch.float16, device=dev), 64, 64)   # no rows: nothing to do
     assert q.shape == (0, 640)
+
+
+@pytest.mark.parametrize("mode,M,K,rotate", [("ln", 1, 32, 0), ("ln", 37, 96, 0), ("ln", 21, 320, 64), ("ln", 13, 640, 64), ("ln", 3, 1280, 256),
+                                             ("ln", 2, 16384, 256), ("geglu", 5, 320, 64), ("geglu", 3, 5120, 256), ("geglu", 1, 96, 0),
+                                             ("unpad", 19, 320, 64), ("unpad", 7, 1280, 256), ("gn", 77, 320, 64), ("gn", 5, 640, 64), ("gn", 33, 1280, 256)])
+def test_sd_register_kernel_equals_the_shared_memory_kernel(pkg, dev, mode, M, K, rotate):
+    """The register kernel's source phase at partial warps, ragged row blocks and image borders, bit for bit against the
+    shared-memory kernel, which takes the same call when an operand does not start on a 16-byte boundary."""
+    g = torch.Generator(device=dev).manual_seed(M + K)
+    L = pkg.linear
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+
+    def both(t):      # the tensor on a 16-byte boundary, and the same values off it
+        off = torch.empty(t.numel() + 8, dtype=t.dtype, device=dev)[1:1 + t.numel()].view(t.shape)
+        return t, off.copy_(t)
+
+    if mode == "ln":
+        x, b = (rn(M, K) * 2 + 0.5).half(), rn(K) * 0.1
+        got, want = (L.sd_ln_quant_rows(x, w, b, 1e-5, rotate) for w in both(rn(K) * 0.2 + 1))
+    elif mode == "geglu":
+        got, want = (L.sd_geglu_quant_rows(x, rotate) for x in both((rn(M, 2 * K) * 1.5).half()))
+    elif mode == "unpad":
+        got, want = (L.sd_unpad_quant_rows(x, 40, rotate) for x in both(rn(M, K // 40, 64).half()))
+    else:
+        x, b = (rn(3, M, K) * 1.5 + 0.3).half(), rn(K) * 0.1
+        got, want = (L.sd_group_norm_quant_rows(x, w, b, 32, 1e-5, rotate) for w in both(rn(K) * 0.2 + 1))
+    assert_bits_equal(got[1], want[1], "scales"), assert_bits_equal(got[0], want[0], "codes")
