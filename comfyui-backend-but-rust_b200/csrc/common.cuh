@@ -21,6 +21,32 @@ enum DType { DT_F32 = 0, DT_F16 = 1, DT_BF16 = 2 };
 
 typedef __nv_bfloat16 bf16;
 
+// ---- programmatic dependent launch ------------------------------------------------------------------------------------
+// The linears of a block are ten to fifteen short kernels one after the other, and between two of them a stream idles for
+// the drain of the first, the launch of the second and its setup (barriers, tensor memory, tensor maps): 2 to 4 us. So every
+// kernel of a forward pass is launched with `launch_pdl` and begins with
+//   - pdl_trigger(): the stream's next kernel may be brought onto the SMs once every CTA of this one has got here (those
+//     that hold tensor memory trigger after its allocation: a successor that got there first would hold the columns while it
+//     waits for this kernel's end);
+//   - pdl_wait(), before the first access to memory that another kernel reads or writes: everything launched before in the
+//     stream has ended and its writes are visible. Every thread that touches such memory waits, so an order that held
+//     between whole kernels (results, buffers used again, the zeros of the split scratch) holds as before.
+// A successor launched the ordinary way waits for the end of the grid as always.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at, cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return (int)e;
+}
+
 // ---- device status word ---------------------------------------------------------------------------
 // A kernel whose bounded wait runs out records a code here and returns; gpu_kernels_status() reads it.
 enum KernelStatus {

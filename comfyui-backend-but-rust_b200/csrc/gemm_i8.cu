@@ -748,6 +748,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         tmem_relinquish_pair();
     }
     if constexpr (EPI == EPI_ACT_LUT || EPI == EPI_ACT_ROT) {
+        pdl_wait();        // the table may have been built just before
         // the activation table's hot part into shared memory (a gather from the whole table through L1 costs the epilogue
         // one wavefront per distinct line and made it, not the tensor core, the limit)
         if (warp >= 2) {
@@ -760,6 +761,8 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
     cluster_sync_all();   // the peer's barriers exist before anything signals them
     tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
 
     if (warp == 0) {
@@ -1079,6 +1082,8 @@ gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
     const int tm = blockIdx.x % p.tiles_m, tn = blockIdx.x / p.tiles_m;
 
@@ -1277,9 +1282,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap&
         if (e != cudaSuccess) return (int)e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    kern<<<grid, EPI == EPI_ACT_ROT ? kRotThreads : kThreads, kSmemBytes, st>>>(ta, tw, td, p);
-    KCHECK();
-    return 0;
+    return launch_pdl(kern, dim3(grid), EPI == EPI_ACT_ROT ? kRotThreads : kThreads, kSmemBytes, st, ta, tw, td, p);
 }
 template <typename OutT>
 int launch_pair_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, const GemmParams& p,
@@ -1310,9 +1313,7 @@ int launch_small(const CUtensorMap& ta, const CUtensorMap& tw, const GemmParams&
         if (e != cudaSuccess) return (int)e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    kern<<<grid, kSmallThreads, smem, st>>>(ta, tw, p);
-    KCHECK();
-    return 0;
+    return launch_pdl(kern, dim3(grid), kSmallThreads, smem, st, ta, tw, p);
 }
 template <typename OutT>
 int launch_small_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tw, const GemmParams& p, int grid, size_t smem,
@@ -1543,6 +1544,8 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
 // terms (hi + lo = 16 significant bits), one GEMM pass each into f32 accumulators: close to an fp32 product at tensor-core
 // speed. The kernel is the int8 one with kind::f16 MMAs (bf16 operands are addressed as rows of 2 K bytes).
 __global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* __restrict__ q, bf16* __restrict__ out, int64_t n16) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n16) return;
     const uint4 v = __ldg(reinterpret_cast<const uint4*>(q) + i);
@@ -1646,8 +1649,7 @@ GPU_API int gpu_wo8_linear(int prologue, const float* x, int64_t x_stride, int64
     uint8_t* lo = hi + (size_t)M * K * 2;
     if (int rc = rotate_rows_split(prologue, x, x_stride, up_offset, norm_w, eps, hi, lo, M, K, st)) return rc;
     const int64_t n16 = (int64_t)N * K / 16;
-    widen_i8_bf16_kernel<<<(unsigned)((n16 + 255) / 256), 256, 0, st>>>(Wq, reinterpret_cast<bf16*>(w_scratch), n16);
-    KCHECK();
+    if (int rc = launch_pdl(widen_i8_bf16_kernel, dim3((unsigned)((n16 + 255) / 256)), 256, 0, st, Wq, reinterpret_cast<bf16*>(w_scratch), n16)) return rc;
     if (int rc = run_gemm_bf16(beta == 1.f, hi, w_scratch, ws, out, M, N, K, st)) return rc;
     return run_gemm_bf16(true, lo, w_scratch, ws, out, M, N, K, st);
 }

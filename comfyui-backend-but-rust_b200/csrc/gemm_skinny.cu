@@ -14,6 +14,8 @@ constexpr int kRowsPerWarp = 4;
 template <typename OutT, int EPI, int MT>
 __global__ void __launch_bounds__(kWarps * 32) skinny_gemm_kernel(const SkinnyParams p) {
     extern __shared__ __align__(16) int8_t a_s[];   // [M][K]
+    pdl_trigger();
+    pdl_wait();
     const int K = p.K;
     for (int i = threadIdx.x; i < p.M * K / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(a_s)[i] = __ldg(reinterpret_cast<const uint4*>(p.A) + i);
@@ -101,12 +103,9 @@ int launch_mt(const SkinnyParams& p, int grid, size_t smem, cudaStream_t st) {
         cudaFuncSetAttribute(skinny_gemm_kernel<OutT, EPI, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(skinny_gemm_kernel<OutT, EPI, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     }
-    if (p.M == 1) skinny_gemm_kernel<OutT, EPI, 1><<<grid, kWarps * 32, smem, st>>>(p);
-    else if (p.M == 2) skinny_gemm_kernel<OutT, EPI, 2><<<grid, kWarps * 32, smem, st>>>(p);
-    else if (p.M <= 4) skinny_gemm_kernel<OutT, EPI, 4><<<grid, kWarps * 32, smem, st>>>(p);
-    else skinny_gemm_kernel<OutT, EPI, 8><<<grid, kWarps * 32, smem, st>>>(p);
-    KCHECK();
-    return 0;
+    auto kern = p.M == 1 ? skinny_gemm_kernel<OutT, EPI, 1> : p.M == 2 ? skinny_gemm_kernel<OutT, EPI, 2>
+                : p.M <= 4 ? skinny_gemm_kernel<OutT, EPI, 4> : skinny_gemm_kernel<OutT, EPI, 8>;
+    return launch_pdl(kern, dim3(grid), kWarps * 32, smem, st, p);
 }
 
 template <typename OutT>

@@ -109,6 +109,8 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     __syncthreads();
     cluster_sync_all();
     tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
 
     if (warp == 0) {
@@ -381,9 +383,7 @@ int launch_w6_mh(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMa
         if (e != cudaSuccess) return (int)e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    kern<<<grid, kW6Threads, kSmemBytes, st>>>(ta, tlo, thi, td, p, x6);
-    KCHECK();
-    return 0;
+    return launch_pdl(kern, dim3(grid), kW6Threads, kSmemBytes, st, ta, tlo, thi, td, p, x6);
 }
 
 template <typename OutT, int EPI>

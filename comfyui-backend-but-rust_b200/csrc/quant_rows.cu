@@ -263,11 +263,13 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
     uint8_t* stage = smem + p.off_stage;              // [x rows | aux rows], one block of rows
     const uint32_t row_bytes = (uint32_t)p.K * sizeof(T);
 
+    pdl_trigger();
     for (int i = threadIdx.x; i < 3 * p.rows_per_cta; i += blockDim.x) amax_s[i] = 0u;
     if (p.staged && threadIdx.x == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
     }
+    pdl_wait();
     __syncthreads();
 
     // Staging: the rows of block `blk` (and their second stream) -> the staging buffer, one bulk copy each, issued by
@@ -703,7 +705,9 @@ __global__ void __launch_bounds__(512) sd_quant_fast_kernel(const SdSrc s, int8_
     float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
     float* tbuf_w = tbuf - 2 * (team >> 1);
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem + off_amax);
+    pdl_trigger();
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
+    pdl_wait();
     // rows of this CTA; GroupNorm's belong to one image (blockIdx.y), so that one set of statistics serves the CTA
     const int64_t limit = SRC == SDQ_GN ? (int64_t)(blockIdx.y + 1) * s.P : M;
     const int64_t m0 = (SRC == SDQ_GN ? (int64_t)blockIdx.y * s.P : 0) + (int64_t)blockIdx.x * rows;
@@ -926,9 +930,7 @@ int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaS
         }
     }
     const dim3 grid = SRC == SDQ_GN ? dim3((unsigned)((s.P + rows - 1) / rows), (unsigned)(M / s.P)) : dim3((unsigned)((M + rows - 1) / rows));
-    kern<<<grid, threads, off, st>>>(s, q, scales, M, K, tpr, rows, off_amax, off_rows);
-    KCHECK();
-    return 0;
+    return launch_pdl(kern, grid, threads, off, st, s, q, scales, M, K, tpr, rows, off_amax, off_rows);
 }
 template <int SRC>
 int launch_sd_fast_rot(const SdSrc& s, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st) {
@@ -1055,9 +1057,7 @@ int launch_cfg(QuantArgs& p, int threads, size_t smem, bool persistent, cudaStre
         const int resident = per_sm * sm_count_of(dev);
         if (grid > resident) grid = resident;
     }
-    kern<<<grid, threads, smem, st>>>(p);
-    KCHECK();
-    return 0;
+    return launch_pdl(kern, dim3(grid), threads, smem, st, p);
 }
 
 constexpr size_t kMaxSmem = 227 * 1024;
@@ -1225,6 +1225,8 @@ __global__ void __launch_bounds__(512) quant_rotated_kernel(const bf16* __restri
                                                             int8_t* __restrict__ q, float* __restrict__ scales, int M, int K,
                                                             int P, int wpr) {
     __shared__ unsigned s_amax[kRotRows], s_flag[kRotRows];
+    pdl_trigger();
+    pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rloc = warp / wpr, seg = warp - rloc * wpr;
     const int64_t m0 = (int64_t)blockIdx.x * kRotRows, m = m0 + rloc;
@@ -1299,8 +1301,6 @@ GPU_API int gpu_quant_rows_rotated(const void* xr, const float* amax_part, int8_
     // enough warps for every SM to have many loads in flight: two warps share a long row
     const int wpr = K >= 4096 ? 2 : 1;
     const unsigned grid = (unsigned)((M + kRotRows - 1) / kRotRows);
-    quant_rotated_kernel<<<grid, kRotRows * wpr * 32, 0, (cudaStream_t)stream>>>(reinterpret_cast<const bf16*>(xr), amax_part, q,
-                                                                                 scales, M, K, K / 64, wpr);
-    KCHECK();
-    return 0;
+    return launch_pdl(quant_rotated_kernel, dim3(grid), kRotRows * wpr * 32, 0, (cudaStream_t)stream, reinterpret_cast<const bf16*>(xr),
+                      amax_part, q, scales, M, K, K / 64, wpr);
 }

@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
 __global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* __restrict__ x, double* __restrict__ sums, int64_t P,
                                                             int C, int G, int splits) {
     __shared__ float red[33];
+    pdl_trigger();
+    pdl_wait();
     const int ng = blockIdx.x, split = blockIdx.y;
     const int n = ng / G, g = ng % G, per = C / G;
     const int64_t base = (int64_t)n * P * C + g * per;
@@ -512,6 +514,8 @@ __global__ void __launch_bounds__(256) w6_requant_kernel(const bf16* __restrict_
 // (lanes past the end redo the last piece and store nothing).
 __global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ s_rel,
                                                           int8_t* __restrict__ out, int64_t N, int K, int G) {
+    pdl_trigger();
+    pdl_wait();
     const int64_t per = K / 32;
     const int64_t total = N * per;
     const int64_t i_raw = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -630,8 +634,7 @@ GPU_API int gpu_sd_group_norm_quant_rows(const void* x, const float* w, const fl
     if (e != cudaSuccess) return (int)e;
     const int64_t want = P * (C / G) / 4096;
     const int splits = want < 1 ? 1 : want > 64 ? 64 : (int)want;
-    sd_group_sums_kernel<<<dim3(N * G, splits), 256, 0, st>>>((const half*)x, (double*)sums, P, C, G, splits);
-    KCHECK();
+    if (int rc = launch_pdl(sd_group_sums_kernel, dim3(N * G, splits), 256, 0, st, (const half*)x, (double*)sums, P, C, G, splits)) return rc;
     SdSrc p{(const half*)x, 0, w, b, eps, 0, 0, 0, (const double*)sums, G, P, (double)P * (C / G)};
     return launch_sd_src<SDQ_GN>(p, q, scales, (int)(N * P), C, rotate, st);
 }
@@ -710,10 +713,8 @@ GPU_API int gpu_w6_decode(const void* q, const void* s_rel, void* out, int64_t N
     // rows of 3K/4 bytes keep the 16-byte pieces of the nibble plane aligned when K % 64 == 0 (8-byte pieces of the other plane too)
     if (G % 32 == 0 && K % 64 == 0 && (((uintptr_t)q | (uintptr_t)out) & 15) == 0) {
         const int64_t n32 = N * (K / 32);
-        w6_decode32_kernel<<<(unsigned)((n32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const uint8_t*)q, (const uint8_t*)s_rel,
-                                                                                          (int8_t*)out, N, K, G);
-        KCHECK();
-        return 0;
+        return launch_pdl(w6_decode32_kernel, dim3((unsigned)((n32 + 255) / 256)), 256, 0, (cudaStream_t)stream, (const uint8_t*)q,
+                          (const uint8_t*)s_rel, (int8_t*)out, N, K, G);
     }
     const int64_t n = N * (K / 16);
     w6_decode_kernel<<<(unsigned)((n + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const uint8_t*)q, (const uint8_t*)s_rel,
