@@ -35,16 +35,22 @@ typedef __nv_bfloat16 bf16;
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
-inline int launch_pdl(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+inline int launch_pdl_cluster(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, int cluster, const A&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid, cfg.blockDim = dim3(threads), cfg.dynamicSmemBytes = smem, cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at, cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = (unsigned)cluster, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
+    cfg.attrs = at, cfg.numAttrs = cluster > 1 ? 2 : 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
     if (e != cudaSuccess) (void)cudaGetLastError();
     return (int)e;
+}
+template <typename... P, typename... A>
+inline int launch_pdl(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, const A&... args) {
+    return launch_pdl_cluster(kern, grid, threads, smem, st, 1, args...);
 }
 
 // ---- device status word ---------------------------------------------------------------------------

@@ -44,9 +44,10 @@ constexpr int kW6BStages = 4;    // ring of expanded W tiles: only has to span u
 // the unpack warps. Barriers: afull (leader: A bytes of both CTAs), pfull (per CTA: its packed planes), aempty (per
 // CTA: MMAs have read A slot -> its packed slot is free too, the unpack that fed those MMAs being long done),
 // bfull (leader: 16 unpack-warp arrivals), bempty (per CTA: MMAs have read the expanded slot).
-// MH = 256-row halves per tile (1 or 2). With MH = 2 an expanded W tile feeds two sets of MMAs (rows 0-255 and 256-511 of
-// the tile, two accumulators of bn <= 128 columns per buffer), so the unpack work per MMA halves.
-template <typename OutT, int EPI, int MH>
+// A tile has MH = 2 halves of 256 rows and 128 columns: an expanded W tile feeds two sets of MMAs (rows 0-255 and 256-511 of
+// the tile, two accumulators per buffer), so the unpack work per MMA halves. Up to 256 rows take the kernel further down.
+constexpr int MH = 2;
+template <typename OutT, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kW6Threads, 1)
 gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_lo,
                       const __grid_constant__ CUtensorMap tmap_hi, const __grid_constant__ CUtensorMap tmap_d,
@@ -187,11 +188,9 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         // data, so a group pays them once per 128 elements of its rows, and the groups overlap one another's waits.
         const int uw = warp - (2 + kW6EpiWarps);
         const int grp = uw >> 2;
-        // up to 64 rows per CTA (bn <= 128): two threads per row, 64 elements each; else one thread per row
-        const bool two = rows_w <= 64;
-        const int r = two ? 32 * (uw & 1) + lane : 32 * (uw & 3) + lane;      // row of the half tile
-        const int hf = two ? (uw >> 1) & 1 : 0;                               // which 64 elements of the box
-        const bool has_row = r < rows_w;
+        // 64 rows per CTA: two threads per row, 64 elements each
+        const int r = 32 * (uw & 1) + lane;                                   // row of the half tile
+        const int hf = (uw >> 1) & 1;                                         // which 64 elements of the box
         const uint32_t bfull_leader = mapa_shared(bar_bfull, 0);
         const int sw_lo = (r >> 1) & 3, sw_hi = (r >> 2) & 1, sw_out = r & 7;
         const bool wide = (x6.srel_pitch & 15) == 0 && ((uintptr_t)x6.s_rel & 15) == 0;   // scale rows readable 16 bytes at a time
@@ -207,7 +206,6 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = make_uint4(0, 0, 0, 0);
             auto fetch = [&](int kb4) -> uint4 {     // scales of boxes 4*kb4 .. 4*kb4+3
                 uint4 v = make_uint4(0x38383838u, 0x38383838u, 0x38383838u, 0x38383838u);
-                if (!has_row) return v;
                 if (wide && 4 * kb4 + 4 <= p.k_iters) return __ldg(reinterpret_cast<const uint4*>(srow) + kb4);
                 const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
                 const int left = p.k_iters - 4 * kb4;
@@ -232,24 +230,20 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     if (!__all_sync(0xffffffffu, mbar_try_wait(bar_bempty + 8 * sb, pb ^ 1u)) &&
                         !mbar_wait_warp(bar_bempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
                     {
-                        const int rr = has_row ? r : 0;    // lanes beyond the tile's rows redo row 0 (warp votes below) and store nothing
-                        const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + rr * 64;
-                        const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + rr * 32;
-                        uint8_t* out = sm + (sB - base) + sb * b_bytes + rr * 128;
+                        const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
+                        const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
+                        uint8_t* out = sm + (sB - base) + sb * b_bytes + r * 128;
                         const uint4 h0 = *reinterpret_cast<const uint4*>(hi + ((hf ^ sw_hi) << 4));
-                        const uint4 h1 = *reinterpret_cast<const uint4*>(hi + ((1 ^ sw_hi) << 4));
-                        const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                        const uint32_t hw[4] = {h0.x, h0.y, h0.z, h0.w};
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {      // 32 elements = one scale group per 16-byte piece of nibbles
-                            if (two && (c >> 1) != hf) continue;             // the other thread of the row (the same for the whole warp)
-                            const int hi_w = two ? 2 * (c & 1) : 2 * c;
+                            if ((c >> 1) != hf) continue;  // the other thread of the row (the same for the whole warp)
+                            const int hi_w = 2 * (c & 1);
                             const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
                             uint32_t o[8];
                             w6_group(l, hw[hi_w], hw[hi_w + 1], (sr >> (8 * c)) & 0xffu, o);
-                            if (has_row) {
-                                *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                                *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-                            }
+                            *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                            *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
                         }
                     }
                     fence_proxy_async_smem();
@@ -298,7 +292,7 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint32_t ra[32];
 #pragma unroll 1
             for (int hc = 0; hc < MH * nchunks; ++hc) {
-                const int h = MH == 1 ? 0 : hc / nchunks, c = hc - h * nchunks;
+                const int h = hc / nchunks, c = hc - h * nchunks;
                 const int row0 = tm * (2 * BM * MH) + h * 2 * BM + (int)rank * BM + quad * 32;
                 const int row = row0 + lane;
                 const bool row_ok = row < p.M;
@@ -355,6 +349,232 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     }
 }
 
+// ---- few rows: weight rows as the MMA's M, tokens as its N ---------------------------------------------------------------
+// Up to 256 tokens (the block on a short clip, a text prompt) the kernel above is bound by neither memory nor the tensor
+// core but by its chain from the packed tile to the MMA: remote arrivals and commits across the CTA pair for every K box,
+// an accumulator of 256 rows of which a quarter is used, and no way to share a long K between SMs. Here one CTA takes 128
+// weight rows and up to 256 tokens (tcgen05.mma.cta_group::1, M = 128 weight rows, N = tokens rounded up to 16), so every
+// barrier is local and nothing is spent on rows that do not exist; a row tile's K is cut between the CTAs of a cluster
+// (integer sums: any cut gives the same bits), which leave their accumulators in shared memory and finish a share of the
+// outputs each, reading one another's through distributed shared memory: no scratch in global memory, nothing to clear.
+// The four linears of a 5120-wide block with FFN 13824 at 64 rows: 231 us on the pair kernel, 141 here.
+// Warp 0 loads (packed planes and tokens of a K box, one barrier), warp 1 issues the MMAs, warps 2..13 expand: three groups
+// of four warps take K boxes in turn, one thread per weight row. All twelve run the epilogue: a lane owns an output column.
+constexpr int kW6RowsWarps = 12;
+constexpr int kW6RowsThreads = 32 * (2 + kW6RowsWarps);
+constexpr int kW6RowsMaxTokens = 256;
+struct W6RowsParams {
+    const uint8_t* s_rel;   // [N, K / 32] e4m3
+    int srel_pitch;         // K / 32
+    int tokens;             // tokens of the tile: M rounded up to 16
+    int splits, kps;        // CTAs of a cluster share a row tile's K: kps boxes each
+    int sa, sb;             // ring depths: packed planes + tokens, expanded tiles
+};
+__device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
+    int v;
+    asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+template <typename OutT, int EPI>
+__global__ void __launch_bounds__(kW6RowsThreads, 1)
+gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_lo,
+                      const __grid_constant__ CUtensorMap tmap_hi, const GemmParams p, const W6RowsParams x6) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw_addr = smem_u32(smem_raw);
+    const uint32_t base = (raw_addr + 1023u) & ~1023u;     // the same offset in every CTA of the cluster
+    uint8_t* sm = smem_raw + (base - raw_addr);
+    const int SA = x6.sa, SB = x6.sb, T = x6.tokens;
+    const uint32_t w_bytes = BM * BK, lo_bytes = BM * 64, hi_bytes = BM * 32;
+    const uint32_t a_bytes = ((uint32_t)T * BK + 1023u) & ~1023u;      // a tile of 16-row pieces, 1024-byte aligned
+    const uint32_t sW = base, sA = sW + SB * w_bytes, sLo = sA + SA * a_bytes, sHi = sLo + SA * lo_bytes;
+    // barriers sit at the end of the allocation: the accumulators overwrite the rings when these are done with
+    uint8_t* tail = sm + SB * w_bytes + SA * (a_bytes + lo_bytes + hi_bytes);
+    if (tail < sm + (uint32_t)T * 512u) tail = sm + (uint32_t)T * 512u;
+    const uint32_t bar_full = smem_u32(tail), bar_empty = bar_full + 8 * kMaxStages, bar_wfull = bar_empty + 8 * kMaxStages,
+                   bar_wempty = bar_wfull + 8 * kMaxStages, bar_tfull = bar_wempty + 8 * kMaxStages;
+    uint32_t* tmem_ptr_s = reinterpret_cast<uint32_t*>(tail + 8 * (4 * kMaxStages + 1));
+    volatile int* abort_s = reinterpret_cast<volatile int*>(tmem_ptr_s + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t tmem_cols = T <= 32 ? 32u : T <= 64 ? 64u : T <= 128 ? 128u : 256u;
+    const int tn = blockIdx.x / x6.splits, rank = blockIdx.x - tn * x6.splits;     // a cluster = the slices of one row tile
+    const int n0 = tn * BM;
+    const int k0 = rank * x6.kps, k1 = min(k0 + x6.kps, p.k_iters);                // never empty: the host side sees to it
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < SA; ++i) mbar_init(bar_full + 8 * i, 1), mbar_init(bar_empty + 8 * i, 1);
+        for (int i = 0; i < SB; ++i) mbar_init(bar_wfull + 8 * i, 4), mbar_init(bar_wempty + 8 * i, 1);
+        mbar_init(bar_tfull, 1);
+        *abort_s = 0;
+        fence_mbar_init();
+        prefetch_tmap(&tmap_a), prefetch_tmap(&tmap_lo), prefetch_tmap(&tmap_hi);
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_ptr_s), tmem_cols);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    pdl_trigger();
+    pdl_wait();
+    const uint32_t tmem_base = *tmem_ptr_s;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int s = 0;
+            uint32_t ph = 0;
+            for (int kb = k0; kb < k1; ++kb) {
+                if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_s, ST_TIMEOUT_EMPTY)) break;
+                mbar_arrive_expect_tx(bar_full + 8 * s, (uint32_t)T * BK + lo_bytes + hi_bytes);
+                tma_load_2d(sLo + s * lo_bytes, &tmap_lo, kb * 64, n0, bar_full + 8 * s);
+                tma_load_2d(sHi + s * hi_bytes, &tmap_hi, kb * 32, n0, bar_full + 8 * s);
+                tma_load_2d(sA + s * a_bytes, &tmap_a, kb * BK, 0, bar_full + 8 * s);
+                if (++s == SA) s = 0, ph ^= 1u;
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = p.idesc;
+            int sa = 0, sb = 0;
+            uint32_t pa = 0, pb = 0;
+            bool ok = true;
+            for (int kb = k0; kb < k1; ++kb) {
+                if (!mbar_wait(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
+                if (!mbar_wait(bar_wfull + 8 * sb, pb, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
+                tc_fence_after();
+                const uint64_t dw = umma_desc_sw128(sW + sb * w_bytes), da = umma_desc_sw128(sA + sa * a_bytes);
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; ++k) umma_i8(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb - k0) | k);
+                umma_commit(bar_wempty + 8 * sb);
+                umma_commit(bar_empty + 8 * sa);
+                if (++sa == SA) sa = 0, pa ^= 1u;
+                if (++sb == SB) sb = 0, pb ^= 1u;
+            }
+            if (ok) umma_commit(bar_tfull);
+        }
+    } else {
+        const int uw = warp - 2, grp = uw >> 2;
+        const int r = 32 * (uw & 3) + lane;                        // weight row of the tile
+        const uint8_t* srow = x6.s_rel + (size_t)min(n0 + r, p.N - 1) * x6.srel_pitch;
+        const bool wide = (x6.srel_pitch & 15) == 0 && ((uintptr_t)x6.s_rel & 15) == 0;   // scale rows readable 16 bytes at a time
+        auto fetch = [&](int kb4) -> uint4 {                       // scales of boxes 4 kb4 .. 4 kb4 + 3
+            if (wide) return __ldg(reinterpret_cast<const uint4*>(srow) + kb4);
+            uint4 v = make_uint4(0, 0, 0, 0);
+            const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
+            const int left = p.k_iters - 4 * kb4;
+            if (left > 0) v.x = __ldg(s32);
+            if (left > 1) v.y = __ldg(s32 + 1);
+            if (left > 2) v.z = __ldg(s32 + 2);
+            if (left > 3) v.w = __ldg(s32 + 3);
+            return v;
+        };
+        const int sw_lo = (r >> 1) & 3, sw_hi = (r >> 2) & 1, sw_out = r & 7;
+        int sa = 0, sb = 0, turn = 0;
+        uint32_t pa = 0, pb = 0;
+        bool ok = true;
+        uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = fetch(k0 >> 2);
+        for (int kb = k0; kb < k1; ++kb) {
+            if ((kb & 3) == 0 || kb == k0) {
+                sc_cur = sc_next;
+                if ((kb & ~3) + 4 < k1) sc_next = fetch((kb >> 2) + 1);
+            }
+            if (turn == grp) {
+                const int q = kb & 3;
+                const uint32_t sr = q == 0 ? sc_cur.x : q == 1 ? sc_cur.y : q == 2 ? sc_cur.z : sc_cur.w;
+                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
+                    !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
+                    !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
+                const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
+                uint8_t* out = sm + sb * w_bytes + r * 128;
+                const uint4 h0 = *reinterpret_cast<const uint4*>(hi + (sw_hi << 4)), h1 = *reinterpret_cast<const uint4*>(hi + ((1 ^ sw_hi) << 4));
+                const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {                      // 32 codes = one scale group per 16-byte piece of nibbles
+                    const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
+                    uint32_t o[8];
+                    w6_group(l, hw[2 * c], hw[2 * c + 1], (sr >> (8 * c)) & 0xffu, o);
+                    *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
+            }
+            if (++turn == kW6RowsWarps / 4) turn = 0;
+            if (++sa == SA) sa = 0, pa ^= 1u;
+            if (++sb == SB) sb = 0, pb ^= 1u;
+        }
+        // accumulators to shared memory, [token][weight row] int32, over the rings (all copies have landed and all MMAs have
+        // read them when the accumulator is complete)
+        if (ok && mbar_wait_warp(bar_tfull, 0, abort_s, ST_TIMEOUT_TMEM_FULL)) {
+            tc_fence_after();
+            const int quad = warp & 3;                             // TMEM lane quarter this warp may read
+            int* red = reinterpret_cast<int*>(sm) + quad * 32 + lane;
+            for (int c = grp; c < T / 16; c += kW6RowsWarps / 4) {
+                uint32_t v[16];
+                tmem_ld16(tmem_base + ((uint32_t)(quad * 32) << 16) + c * 16, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 16; ++j) red[(c * 16 + j) * BM] = (int)v[j];
+            }
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();
+    if (warp >= 2 && *abort_s == 0) {
+        // eight tokens x 32 columns at a time, dealt out over the cluster's warps
+        const int quads = (p.M + 7) / 8 * 4;
+        for (int u = rank + x6.splits * (warp - 2); u < quads; u += x6.splits * kW6RowsWarps) {
+            const int quad = u & 3, m0 = (u >> 2) * 8;
+            const int n = n0 + quad * 32 + lane;
+            if (n >= p.N) continue;
+            const uint32_t src = base + (uint32_t)(m0 * BM + quad * 32 + lane) * 4u;
+            int acc[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[i] = 0;
+            for (int s = 0; s < x6.splits; ++s) {
+                const uint32_t a = mapa_shared(src, (uint32_t)s);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[i] += ld_shared_cluster(a + i * BM * 4);      // rows up to the next multiple of 16 exist
+            }
+            if constexpr (EPI == EPI_ACC) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (m0 + i < p.M) reinterpret_cast<int*>(p.D)[(int64_t)(m0 + i) * p.N + n] = acc[i];
+            } else {
+                const float ws = p.ws[n], bias = p.bias ? to_f<OutT>(reinterpret_cast<const OutT*>(p.bias)[n]) : 0.f;
+                const float rs = EPI == EPI_RESID ? to_f<OutT>(reinterpret_cast<const OutT*>(p.rscale)[n]) : 0.f;
+                float rr[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    rr[i] = EPI == EPI_RESID && m0 + i < p.M ? to_f<OutT>(reinterpret_cast<const OutT*>(p.resid)[(int64_t)(m0 + i) * p.N + n]) : 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (m0 + i >= p.M) break;
+                    reinterpret_cast<OutT*>(p.D)[(int64_t)(m0 + i) * p.N + n] =
+                        from_f<OutT>(epilogue1<OutT, EPI>(acc[i], p.xs[m0 + i], ws, bias, rs, rr[i], p.act));
+                }
+            }
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();            // nobody leaves while another CTA may read its accumulators
+    if (*abort_s != 0) {
+        for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+        if (threadIdx.x == 0) atomicCAS(&g_kernel_status, 0, *abort_s);
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, tmem_cols);
+    }
+}
+
 // ---- host side ------------------------------------------------------------------------------------------------------
 // Tensor map of one plane of the packed rows: `cols` bytes per row at `pitch` bytes, boxes of box_x bytes x box_rows.
 bool make_plane_tmap(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t cols, int64_t pitch, int box_x, int box_rows,
@@ -370,10 +590,10 @@ bool make_plane_tmap(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t col
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename OutT, int EPI, int MH>
-int launch_w6_mh(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const CUtensorMap& td,
+template <typename OutT, int EPI>
+int launch_w6(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const CUtensorMap& td,
                  const GemmParams& p, const W6Extra& x6, int grid, cudaStream_t st) {
-    auto kern = gemm_w6a8_pair_kernel<OutT, EPI, MH>;
+    auto kern = gemm_w6a8_pair_kernel<OutT, EPI>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -387,10 +607,57 @@ int launch_w6_mh(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMa
 }
 
 template <typename OutT, int EPI>
-int launch_w6(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const CUtensorMap& td,
-              const GemmParams& p, const W6Extra& x6, int mh, int grid, cudaStream_t st) {
-    return mh == 2 ? launch_w6_mh<OutT, EPI, 2>(ta, tlo, thi, td, p, x6, grid, st)
-                   : launch_w6_mh<OutT, EPI, 1>(ta, tlo, thi, td, p, x6, grid, st);
+int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const GemmParams& p, const W6RowsParams& x6,
+                   size_t smem, cudaStream_t st) {
+    auto kern = gemm_w6a8_rows_kernel<OutT, EPI>;
+    static std::atomic<uint64_t> configured{0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+        if (e != cudaSuccess) return (int)e;
+        configured.fetch_or(bit, std::memory_order_release);
+    }
+    return launch_pdl_cluster(kern, dim3(p.tiles_n * x6.splits), kW6RowsThreads, smem, st, x6.splits, ta, tlo, thi, p, x6);
+}
+
+int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, int sms, cudaStream_t st) {
+    const int64_t M = p.M, N = p.N, K = p.K;
+    W6RowsParams x6{s_rel, (int)(K / 32), (int)((M + 15) / 16 * 16), 1, p.k_iters, 0, kW6BStages};
+    p.tiles_n = (int)((N + BM - 1) / BM);
+    p.idesc = umma_idesc_i8(BM, x6.tokens);
+    // K slices: rounds of CTAs times (boxes of a slice + about a dozen boxes' worth of start and end)
+    int64_t best = INT64_MAX;
+    for (int s = 1; s <= 8 && s <= p.k_iters; ++s) {
+        const int kps = (p.k_iters + s - 1) / s;
+        if ((p.k_iters + kps - 1) / kps != s) continue;                      // a slice would be empty
+        const int64_t rounds = ((int64_t)p.tiles_n * s + sms - 1) / sms;
+        const int64_t cost = rounds * (kps + 12) + (s > 1 ? 3 : 0);
+        if (cost < best) best = cost, x6.splits = s, x6.kps = kps;
+    }
+    const int a_bytes = (x6.tokens * BK + 1023) & ~1023;
+    const int stage = a_bytes + BM * (64 + 32);
+    x6.sa = (kSmemBytes - 1024 - kTailBytes - x6.sb * BM * BK) / stage;
+    if (x6.sa > kMaxStages) x6.sa = kMaxStages;
+    if (x6.sa > x6.kps) x6.sa = x6.kps;
+    size_t rings = (size_t)x6.sb * BM * BK + (size_t)x6.sa * stage;
+    if (rings < (size_t)x6.tokens * BM * 4) rings = (size_t)x6.tokens * BM * 4;
+    const size_t smem = 1024 + rings + kTailBytes;
+    const int64_t pitch = 3 * K / 4;
+    CUtensorMap ta, tlo, thi;
+    if (!make_operand_tmap(&ta, A, M, K, x6.tokens)) return -203;
+    if (!make_plane_tmap(&tlo, Wq6, N, K / 2, pitch, 64, BM, CU_TENSOR_MAP_SWIZZLE_64B)) return -203;
+    if (!make_plane_tmap(&thi, Wq6 + K / 2, N, K / 4, pitch, 32, BM, CU_TENSOR_MAP_SWIZZLE_32B)) return -203;
+    if (epi == EPI_ACC) return launch_w6_rows<float, EPI_ACC>(ta, tlo, thi, p, x6, smem, st);
+#define W6_ROWS_DISPATCH(T)                                                                    \
+    (epi == EPI_RESID ? launch_w6_rows<T, EPI_RESID>(ta, tlo, thi, p, x6, smem, st)            \
+     : epi == EPI_ACT ? launch_w6_rows<T, EPI_ACT>(ta, tlo, thi, p, x6, smem, st)              \
+                      : launch_w6_rows<T, EPI_PLAIN>(ta, tlo, thi, p, x6, smem, st))
+    if (out_dt == DT_F32) return W6_ROWS_DISPATCH(float);
+    if (out_dt == DT_F16) return W6_ROWS_DISPATCH(half);
+    return W6_ROWS_DISPATCH(bf16);
+#undef W6_ROWS_DISPATCH
 }
 
 int run_w6_gemm(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, const float* xs, const float* ws,
@@ -412,22 +679,20 @@ int run_w6_gemm(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     p.act = act;
     p.act_lut = nullptr;
     const int esz = epi == EPI_ACC ? 4 : (out_dt == DT_F32 ? 4 : 2);
+    p.k_iters = (int)(K / BK);
+    if (M <= kW6RowsMaxTokens) return run_w6_rows(epi, A, Wq6, s_rel, p, out_dt, device_sm_count(dev), st);
     auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     p.vec_ok = (N % 8 == 0) && al16(D) && al16(ws) && al16(bias) && al16(rscale) && al16(resid);
     p.tma_store = al16(D) && ((N * esz) % 16 == 0);
     p.ksub = 1;
-    p.k_iters = (int)(K / BK);
-    // More than 256 rows: tiles of 512 rows x 128 columns, so that each expanded W tile serves two sets of MMAs and the
-    // unpack work per MMA halves; otherwise one 256-row half and the column width that fills the clusters best.
-    const int mh = M > 256 && N >= 128 ? 2 : 1;
-    const int bn = mh == 2 ? 128 : choose_bn(M, N, clusters);
+    constexpr int bn = 128;
     p.bn = bn;
     p.idesc = umma_idesc_i8(2 * BM, bn);
-    const int stage_bytes = mh * BM * BK + (bn / 2) * (64 + 32);     // A boxes + packed planes; the expanded ring is separate
+    const int stage_bytes = MH * BM * BK + (bn / 2) * (64 + 32);     // A boxes + packed planes; the expanded ring is separate
     const int sbs = kW6BStages;
     const int stages = (kSmemBytes - 1024 - 512 - kW6StagingBytes - sbs * (bn / 2) * BK) / stage_bytes;
     p.stages = stages > kMaxStages ? kMaxStages : stages;
-    p.tiles_m = (int)((M + 2 * BM * mh - 1) / (2 * BM * mh));
+    p.tiles_m = (int)((M + 2 * BM * MH - 1) / (2 * BM * MH));
     p.tiles_n = (int)((N + bn - 1) / bn);
     p.num_tiles = p.tiles_m * p.tiles_n;
     p.whole_tiles = p.num_tiles, p.num_items = p.num_tiles, p.kps = p.k_iters;
@@ -443,11 +708,11 @@ int run_w6_gemm(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     }
     W6Extra x6{s_rel, (int)(K / 32), sbs};
     const int grid = 2 * (p.num_tiles < clusters ? p.num_tiles : clusters);
-    if (epi == EPI_ACC) return launch_w6<float, EPI_ACC>(ta, tlo, thi, td, p, x6, mh, grid, st);
+    if (epi == EPI_ACC) return launch_w6<float, EPI_ACC>(ta, tlo, thi, td, p, x6, grid, st);
 #define W6_DISPATCH(T)                                                                                   \
-    (epi == EPI_RESID ? launch_w6<T, EPI_RESID>(ta, tlo, thi, td, p, x6, mh, grid, st)                      \
-     : epi == EPI_ACT ? launch_w6<T, EPI_ACT>(ta, tlo, thi, td, p, x6, mh, grid, st)                        \
-                      : launch_w6<T, EPI_PLAIN>(ta, tlo, thi, td, p, x6, mh, grid, st))
+    (epi == EPI_RESID ? launch_w6<T, EPI_RESID>(ta, tlo, thi, td, p, x6, grid, st)                      \
+     : epi == EPI_ACT ? launch_w6<T, EPI_ACT>(ta, tlo, thi, td, p, x6, grid, st)                        \
+                      : launch_w6<T, EPI_PLAIN>(ta, tlo, thi, td, p, x6, grid, st))
     if (out_dt == DT_F32) return W6_DISPATCH(float);
     if (out_dt == DT_F16) return W6_DISPATCH(half);
     return W6_DISPATCH(bf16);

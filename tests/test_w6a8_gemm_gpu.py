@@ -91,6 +91,26 @@ def test_full_size_layer_matches_decode_then_gemm(pkg, dev):
     assert L.kernel_status() == 0
 
 
+# up to 256 rows: tokens rounded up to 16 (edges 1, 16 | 17, 128 | 129, 256 | 257), a ragged row tile (N % 128), one K box, a K
+# cut between the CTAs of a cluster (few row tiles, long K) evenly and not, scale rows that 16-byte loads cannot take (K = 640)
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(1, 40, 128), (16, 128, 1024), (17, 1500, 640), (64, 640, 13824), (128, 130, 4224), (129, 384, 2048),
+                                   (256, 5120, 1152), (257, 72, 1024)])
+def test_few_rows_equal_the_two_call_flow(pkg, oracle, dev, dtype, M, N, K):
+    g, packed, s_rel = _packed(oracle, N, K, M + N + K, "fitted")
+    A = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8).to(dev)
+    xs, sc = (torch.rand(M, generator=g) * 0.05 + 1e-3).to(dev), (torch.rand(N, generator=g) * 1e-3 + 1e-4).to(dev)
+    bias, rscale = (torch.randn(N, generator=g).to(dtype).to(dev) for _ in range(2))
+    resid = torch.randn(M, N, generator=g).to(dtype).to(dev)
+    packed, s_rel = packed.to(dev), s_rel.to(dev)
+    L = pkg.linear
+    w8 = L.w6_decode(packed, s_rel, K)
+    for kw in ({}, {"act": 2}, {"rscale": rscale, "resid": resid}):
+        got = L.w6a8_gemm(A, packed, s_rel, xs, sc, bias, out_dtype=dtype, **kw)
+        assert_bits_equal(got, L.int8_gemm(A, w8, xs, sc, bias, out_dtype=dtype, **kw), str(kw.keys()))
+    assert L.kernel_status() == 0
+
+
 @pytest.mark.parametrize("act", [1, 2, 3])
 @pytest.mark.parametrize("M", [96, 1300])
 def test_activation_epilogue_equals_the_int8_form(pkg, dev, act, M):
