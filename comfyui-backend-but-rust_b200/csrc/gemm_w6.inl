@@ -224,24 +224,28 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (turn == grp) {
                     const int q = kb & 3;
                     const uint32_t sr = q == 0 ? sc_cur.x : q == 1 ? sc_cur.y : q == 2 ? sc_cur.z : sc_cur.w;
-                    // usually both are complete already: one probe by every lane, the polling form only when not
-                    if (!__all_sync(0xffffffffu, mbar_try_wait(bar_pfull + 8 * sa, pa)) &&
-                        !mbar_wait_warp(bar_pfull + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                    // usually both are complete already: one probe by every lane, the polling form only when not. The expanded
+                    // slot first: a parity says nothing about a barrier that is two phases behind, and a free slot means that
+                    // every box up to the ring's depth ago has been loaded and multiplied, hence that the packed slot (a ring
+                    // at least as deep) is in the phase awaited or the one before.
                     if (!__all_sync(0xffffffffu, mbar_try_wait(bar_bempty + 8 * sb, pb ^ 1u)) &&
                         !mbar_wait_warp(bar_bempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_try_wait(bar_pfull + 8 * sa, pa)) &&
+                        !mbar_wait_warp(bar_pfull + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
                     {
                         const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
                         const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
                         uint8_t* out = sm + (sB - base) + sb * b_bytes + r * 128;
                         const uint4 h0 = *reinterpret_cast<const uint4*>(hi + ((hf ^ sw_hi) << 4));
                         const uint32_t hw[4] = {h0.x, h0.y, h0.z, h0.w};
+                        const int mode = w6_mode(sr);      // the other thread's half with it: the row's scales of the box
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {      // 32 elements = one scale group per 16-byte piece of nibbles
                             if ((c >> 1) != hf) continue;  // the other thread of the row (the same for the whole warp)
                             const int hi_w = 2 * (c & 1);
                             const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
                             uint32_t o[8];
-                            w6_group(l, hw[hi_w], hw[hi_w + 1], (sr >> (8 * c)) & 0xffu, o);
+                            w6_group(mode, l, hw[hi_w], hw[hi_w + 1], (sr >> (8 * c)) & 0xffu, o);
                             *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                             *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
                         }
@@ -358,9 +362,10 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 // (integer sums: any cut gives the same bits), which leave their accumulators in shared memory and finish a share of the
 // outputs each, reading one another's through distributed shared memory: no scratch in global memory, nothing to clear.
 // The four linears of a 5120-wide block with FFN 13824 at 64 rows: 231 us on the pair kernel, 141 here.
-// Warp 0 loads (packed planes and tokens of a K box, one barrier), warp 1 issues the MMAs, warps 2..13 expand: three groups
-// of four warps take K boxes in turn, one thread per weight row. All twelve run the epilogue: a lane owns an output column.
-constexpr int kW6RowsWarps = 12;
+// Warp 0 loads (packed planes and tokens of a K box, one barrier), warp 1 issues the MMAs, warps 2..21 expand: five groups
+// of four warps take K boxes in turn, one thread per weight row (the expansion is what bounds the kernel, a few instructions per
+// code; three groups left the issue slots idle two cycles in five). All of them run the epilogue: a lane owns an output column.
+constexpr int kW6RowsWarps = 20;
 constexpr int kW6RowsThreads = 32 * (2 + kW6RowsWarps);
 constexpr int kW6RowsMaxTokens = 256;
 struct W6RowsParams {
@@ -369,6 +374,7 @@ struct W6RowsParams {
     int tokens;             // tokens of the tile: M rounded up to 16
     int splits, kps;        // CTAs of a cluster share a row tile's K: kps boxes each
     int sa, sb;             // ring depths: packed planes + tokens, expanded tiles
+    int groups;             // expanding groups of four warps in use
 };
 __device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
     int v;
@@ -474,7 +480,7 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         uint32_t pa = 0, pb = 0;
         bool ok = true;
         uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = fetch(k0 >> 2);
-        for (int kb = k0; kb < k1; ++kb) {
+        for (int kb = grp < x6.groups ? k0 : k1; kb < k1; ++kb) {
             if ((kb & 3) == 0 || kb == k0) {
                 sc_cur = sc_next;
                 if ((kb & ~3) + 4 < k1) sc_next = fetch((kb >> 2) + 1);
@@ -482,28 +488,35 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if (turn == grp) {
                 const int q = kb & 3;
                 const uint32_t sr = q == 0 ? sc_cur.x : q == 1 ? sc_cur.y : q == 2 ? sc_cur.z : sc_cur.w;
-                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
-                    !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                // the expanded slot first, as above: groups <= sb <= sa keeps every awaited phase the current or the last one
                 if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
                     !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
+                    !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
                 const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
                 const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
                 uint8_t* out = sm + sb * w_bytes + r * 128;
                 const uint4 h0 = *reinterpret_cast<const uint4*>(hi + (sw_hi << 4)), h1 = *reinterpret_cast<const uint4*>(hi + ((1 ^ sw_hi) << 4));
                 const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                auto expand = [&](auto mode) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {                      // 32 codes = one scale group per 16-byte piece of nibbles
-                    const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
-                    uint32_t o[8];
-                    w6_group(l, hw[2 * c], hw[2 * c + 1], (sr >> (8 * c)) & 0xffu, o);
-                    *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                    *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-                }
+                    for (int c = 0; c < 4; ++c) {                  // 32 codes = one scale group per 16-byte piece of nibbles
+                        const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
+                        uint32_t o[8];
+                        w6_group<decltype(mode)::value>(l, hw[2 * c], hw[2 * c + 1], (sr >> (8 * c)) & 0xffu, o);
+                        *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                        *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                    }
+                };
+                const int mode = w6_mode(sr);
+                if (mode == W6_SMALL) expand(std::integral_constant<int, W6_SMALL>());
+                else if (mode == W6_UNIT) expand(std::integral_constant<int, W6_UNIT>());
+                else expand(std::integral_constant<int, W6_ANY>());
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
             }
-            if (++turn == kW6RowsWarps / 4) turn = 0;
+            if (++turn == x6.groups) turn = 0;
             if (++sa == SA) sa = 0, pa ^= 1u;
             if (++sb == SB) sb = 0, pb ^= 1u;
         }
@@ -624,7 +637,7 @@ int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensor
 
 int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, int sms, cudaStream_t st) {
     const int64_t M = p.M, N = p.N, K = p.K;
-    W6RowsParams x6{s_rel, (int)(K / 32), (int)((M + 15) / 16 * 16), 1, p.k_iters, 0, kW6BStages};
+    W6RowsParams x6{s_rel, (int)(K / 32), (int)((M + 15) / 16 * 16), 1, p.k_iters, 0, 0, 0};
     p.tiles_n = (int)((N + BM - 1) / BM);
     p.idesc = umma_idesc_i8(BM, x6.tokens);
     // K slices: rounds of CTAs times (boxes of a slice + about a dozen boxes' worth of start and end)
@@ -638,9 +651,14 @@ int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     }
     const int a_bytes = (x6.tokens * BK + 1023) & ~1023;
     const int stage = a_bytes + BM * (64 + 32);
-    x6.sa = (kSmemBytes - 1024 - kTailBytes - x6.sb * BM * BK) / stage;
+    // rings: as many expanded tiles as the packed ring beside them is deep (see the waits of the expanding warps), six at most
+    for (x6.sb = 6; x6.sb > 1; --x6.sb) {
+        x6.sa = (kSmemBytes - 1024 - kTailBytes - x6.sb * BM * BK) / stage;
+        if (x6.sa >= x6.sb) break;
+    }
     if (x6.sa > kMaxStages) x6.sa = kMaxStages;
-    if (x6.sa > x6.kps) x6.sa = x6.kps;
+    x6.groups = x6.sb < kW6RowsWarps / 4 ? x6.sb : kW6RowsWarps / 4;
+    if (x6.sa > x6.kps) x6.sa = x6.kps;      // no slot is used twice then
     size_t rings = (size_t)x6.sb * BM * BK + (size_t)x6.sa * stage;
     if (rings < (size_t)x6.tokens * BM * 4) rings = (size_t)x6.tokens * BM * 4;
     const size_t smem = 1024 + rings + kTailBytes;

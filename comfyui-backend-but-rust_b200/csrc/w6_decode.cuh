@@ -17,12 +17,23 @@
 // (E, F, 0, 1) and the result is final; otherwise it holds code bits 5:4 and the bytes go through half-precision
 // arithmetic two at a time: 1024 + code by setting exponent bits, one fused multiply-add with -1056 * s (exact while
 // that constant is finite), clamp where 32 * |s| can pass 127, rint by adding 1536, low bytes gathered by a permute.
+// The forms are chosen per warp, not per lane: lanes hold different rows with different scales, and a branch that splits the
+// warp costs the sum of its sides. What a packer emits lies in (0, 4]: its largest group has 31 steps for 127, so a scale of
+// 4.0 is common and only the unused code 0 can leave the range there, downwards, by one. That form clamps once, after the rint
+// (12 operations for four pairs where the general form has 20), and a caller with several groups votes once for all of them.
+enum { W6_UNIT = 0, W6_SMALL = 1, W6_ANY = 2 };
+// The form for the four scale bytes of a lane and those of its warp's other lanes (absent ones filled with 0x38, a scale of 1)
+__device__ __forceinline__ int w6_mode(uint32_t sb4) {
+    // bytes up to 0x48 (4.0), sign clear: adding 0x37 carries into bit 7 from 0x49 on
+    const bool small = (((sb4 & 0x7f7f7f7fu) + 0x37373737u) & 0x80808080u) == 0u && (sb4 & 0x80808080u) == 0u;
+    if (!__all_sync(0xffffffffu, small)) return W6_ANY;
+    return __all_sync(0xffffffffu, sb4 == 0x38383838u) ? W6_UNIT : W6_SMALL;
+}
+template <int MODE>
 __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
     const uint32_t lw[4] = {l.x, l.y, l.z, l.w};
     const uint32_t hv[2] = {ha, hb};
-    // The three forms are chosen per warp, not per lane: lanes hold different rows with different scales, and a branch that
-    // splits the warp costs the sum of its sides. The general form is right for every scale, the clamped one too.
-    if (__all_sync(0xffffffffu, sb == 0x38u)) {
+    if constexpr (MODE == W6_UNIT) {
 #pragma unroll
         for (int w = 0; w < 4; ++w) {
             const uint32_t h = hv[w >> 1] >> (16 * (w & 1));
@@ -35,7 +46,6 @@ __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb
     }
     const __half2 s2 = __half2half2(__half(__nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)sb, __NV_E4M3)));
     const __half2 magic = __float2half2_rn(1536.f);
-    const bool clamp = __any_sync(0xffffffffu, (sb & 0x7fu) >= 0x48u);   // some |s| >= 4 (or NaN): 32 * |s| can pass 127
     const __half2 c2 = __hmul2(__float2half2_rn(-1056.f), s2);
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
@@ -47,17 +57,23 @@ __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             __half2 g = *reinterpret_cast<__half2*>(&p[i]);
-            if (!clamp) {
-                g = __hfma2(g, s2, c2);
+            if constexpr (MODE == W6_SMALL) {
+                // (code - 32) * s is in [-128, 124]; the sum with 1536 stays where the spacing is 1
+                g = __hmax2(__hadd2(__hfma2(g, s2, c2), magic), __float2half2_rn(1409.f));
             } else {
                 g = __hmul2(__hsub2(g, __float2half2_rn(1056.f)), s2);
                 g = __hmin2(__hmax2(g, __float2half2_rn(-127.f)), __float2half2_rn(127.f));
+                g = __hadd2(g, magic);
             }
-            g = __hadd2(g, magic);
             p[i] = *reinterpret_cast<uint32_t*>(&g);
         }
         o[2 * w] = __byte_perm(p[0], p[1], 0x6240);
         o[2 * w + 1] = __byte_perm(p[2], p[3], 0x6240);
     }
 }
-
+// with the mode in a variable (the same in the whole warp)
+__device__ __forceinline__ void w6_group(int mode, const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
+    if (mode == W6_SMALL) w6_group<W6_SMALL>(l, ha, hb, sb, o);
+    else if (mode == W6_UNIT) w6_group<W6_UNIT>(l, ha, hb, sb, o);
+    else w6_group<W6_ANY>(l, ha, hb, sb, o);
+}
