@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "epilogue.cuh"
+#include "rotate.cuh"
 
 namespace {
 
@@ -98,20 +99,6 @@ template <int PRO> __host__ __device__ constexpr bool has_aux() {
 // reference's block (ceil(K / 1024) warps), 32 warp sums, the total
 __host__ __device__ inline int norm_words(int K) { return (((K >> 8) + 3) >> 2) * 32 + 33; }
 
-// Transposition buffers: per 8-lane team 256 elements + 4 words of padding per 32 (288 words), laid out so that every
-// shared-memory access of the transposition is free of bank conflicts across the four teams of a warp:
-//   - a lane writes element 32 t8 + i as one 32-bit store per i; over a team's lanes these hit banks 4 t8 + i, i.e. one
-//     residue class modulo 4. The four teams must cover the four classes: teams 1 and 3 store each element pair swapped
-//     (column i ^ 1), teams 2 and 3 start two words later
-//   - a lane reads element pairs (2 t8, 2 t8 + 1) + 16 r as 64-bit loads, 16 consecutive banks per team; a half-warp holds
-//     two teams, which start 16 banks apart
-// Teams 1 and 3 therefore hold their pairs as (odd element, even element) from the transposition on; the codes are
-// swapped back when they are written out.
-constexpr int kGroupWords = 304;          // team pitch inside a warp: 16 banks (mod 32) apart
-constexpr int kWarpWords = 4 * 304 + 32;  // warp pitch: a multiple of 32 words with room for the two-word shift
-
-__device__ __forceinline__ int tpad(int e) { return e + ((e >> 5) << 2); }
-
 template <typename T> __device__ __forceinline__ float finite_max();
 template <> __device__ __forceinline__ float finite_max<float>() { return FLT_MAX; }
 template <> __device__ __forceinline__ float finite_max<bf16>() { return 3.38953139e38f; }
@@ -144,33 +131,6 @@ template <typename T, bool SMEM> __device__ __forceinline__ void load32(const T*
 __device__ __forceinline__ float lut_f(const uint16_t* lut, float x) {   // x holds a bf16 value; whole table, global
     return __uint_as_float((uint32_t)__ldg(lut + (__float_as_uint(x) >> 16)) << 16);
 }
-// Radix-4 butterfly of the regular Hadamard block on packed pairs; outputs in the reference's association:
-//   r0 = .5*(((x0+x1)+x2)-x3)  r1 = .5*(((x0+x1)-x2)+x3)  r2 = .5*(((x0-x1)+x2)+x3)  r3 = .5*(((-x0+x1)+x2)+x3)
-__device__ __forceinline__ void h4x2(float2& x0, float2& x1, float2& x2, float2& x3) {
-    const float2 m1 = make_float2(-1.f, -1.f), hf = make_float2(0.5f, 0.5f);
-    const float2 s = __fadd2_rn(x0, x1);
-    const float2 d = __ffma2_rn(x1, m1, x0);                         // x0 - x1
-    const float2 r0 = __fmul2_rn(hf, __ffma2_rn(x3, m1, __fadd2_rn(s, x2)));
-    const float2 r1 = __fmul2_rn(hf, __fadd2_rn(__ffma2_rn(x2, m1, s), x3));
-    const float2 r2 = __fmul2_rn(hf, __fadd2_rn(__fadd2_rn(d, x2), x3));
-    const float2 r3 = __fmul2_rn(hf, __fadd2_rn(__ffma2_rn(d, m1, x2), x3));   // (-d + x2) + x3
-    x0 = r0, x1 = r1, x2 = r2, x3 = r3;
-}
-// two radix-4 stages over 16 packed values: index bits (0,1) then (2,3) of the position in P
-__device__ __forceinline__ void two_stages(float2 (&P)[16]) {
-#pragma unroll
-    for (int i = 0; i < 16; i += 4) h4x2(P[i], P[i + 1], P[i + 2], P[i + 3]);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h4x2(P[i], P[i + 4], P[i + 8], P[i + 12]);
-}
-
-// max(|a|, |b|, |c|) that is NaN as soon as one input is
-__device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
-    float m;
-    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(m) : "f"(fabsf(a)), "f"(fabsf(b)), "f"(fabsf(c)));
-    return m;
-}
-
 // Codes of two values: q = sat8(rint(T(T(v) / T(scale)))).
 // bf16 fast path. Both operands of the division carry 8 significant bits: a = A 2^i, st = S 2^j with integers
 // A, S < 256. A bf16 rounding boundary is M 2^k with M odd and 256 < M < 512; a quotient equal to one would need

@@ -9,15 +9,17 @@
 //   gpu_dequant_i8         int8 * row scale -> f32                                    csrc/kernels.cu:330-343
 //   gpu_w6_decode          6-bit two-plane codes + e4m3 group scales -> int8          csrc/h3.cu:11-46
 //
-// One CTA per row; the row lives in shared memory as fp32 (padded against bank conflicts). The rotation runs as
-// two register phases: each thread takes 16 consecutive elements (index bits 0-3: radix-4 stages 0 and 1), then 16
-// elements 16 apart (index bits 4-7: stages 2 and 3; groups of 64 have only stage 2), so a row is read and written
-// in shared memory twice whatever its length. Every butterfly adds in the reference's left-to-right order.
+// Rows (or rotation groups) live in registers, K / 32 threads of 32 values each, with the rotation of rotate.cuh. Rows those
+// kernels do not take (longer than 16384 values, buffers off a 16-byte boundary) run one CTA per row with the row in shared
+// memory as fp32 (padded against bank conflicts): the rotation is two register phases there, 16 consecutive elements (index
+// bits 0-3: radix-4 stages 0 and 1), then 16 elements 16 apart (index bits 4-7: stages 2 and 3; groups of 64 have only stage
+// 2). Every butterfly adds in the reference's left-to-right order.
 #include <cstdlib>
 #include <cuda_fp8.h>
 
 #include "common.cuh"
 #include "epilogue.cuh"
+#include "rotate.cuh"
 #include "w6_decode.cuh"
 
 // quant_rows.cu
@@ -357,6 +359,136 @@ __global__ void __launch_bounds__(512) convrot_requant_kernel(const T* __restric
     }
 }
 
+// Stochastic packing with the rows in registers: whole rows of K / 32 threads, 32 values each, the rotation of rotate.cuh, one
+// shared-memory maximum per row. The kernel above walks a row in shared memory one value per thread and step and divides for
+// every value; it took 149 us for 5120 x 5120 bf16 (79 MB moved, a floor of 12 us; the whole load-and-bake pass of such a weight went from 523 to
+// 303 us with this kernel, the inverse and the W6 packer) and stays for rows the loads below cannot take.
+// The bf16 quotient is a reciprocal multiplication (exact: see quant2 in quant_rows.cu), the hash and the noise are as above.
+template <typename T> __device__ __forceinline__ void load_row32(const T* p, float (&v)[32]) {
+#pragma unroll
+    for (int c = 0; c < 32 * (int)sizeof(T) / 16; ++c) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + c);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if constexpr (sizeof(T) == 4) v[4 * c + i] = __uint_as_float(w[i]);
+            else v[8 * c + 2 * i] = __uint_as_float(w[i] << 16), v[8 * c + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+        }
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(512) convrot_requant_regs_kernel(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scales,
+                                                                   int64_t N, int K, int rows, uint64_t seed) {
+    extern __shared__ __align__(128) float smem_f[];
+    const unsigned wmask = __activemask();               // the last warp may be partial
+    const RotLane l = rot_lane(smem_f);
+    unsigned* amax_s = reinterpret_cast<unsigned*>(smem_f + ((blockDim.x + 31) >> 5) * kWarpWords);
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
+    pdl_trigger();
+    pdl_wait();
+    __syncthreads();
+    const int tpr = K >> 5, rloc = threadIdx.x / tpr, tin = threadIdx.x - rloc * tpr;
+    const int64_t m_raw = (int64_t)blockIdx.x * rows + rloc;
+    const bool live = m_raw < N;
+    const int64_t m = live ? m_raw : N - 1;              // idle rows recompute the last row and store nothing
+    float2 P[16];
+    {
+        float v[32];
+        load_row32(x + m * K + tin * 32, v);
+        rotate256_regs(v, P, l, wmask);
+    }
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = max3_abs_nan(amax, P[i].x, P[i].y);
+    const bool has_nan = amax != amax;
+    if (has_nan) {
+        amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fmaxf(fabsf(P[i].x), fabsf(P[i].y)));
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(wmask, amax, o));
+    if (l.t8 == 0) atomicMax(amax_s + rloc, __float_as_uint(amax));       // non-negative floats order as integers
+    __syncthreads();
+    amax = __uint_as_float(amax_s[rloc]);
+    const float scale = fmaxf(fminf(amax, finite_max_t<T>()) * (1.f / 127.f), 1.0e-30f);
+    if (live && tin == 0) scales[m] = scale;
+    const float st = rnd<T>(scale);
+    const bool fast = sizeof(T) == 2 && amax <= FLT_MAX && !has_nan;
+    if (fast) {                                          // one branch for the row, not one per value
+        const float rcp = __frcp_rn(st);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) P[i] = make_float2(rnd<T>(__fmul_rn(rnd<T>(P[i].x), rcp)), rnd<T>(__fmul_rn(rnd<T>(P[i].y), rcp)));
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) P[i] = make_float2(rnd<T>(__fdiv_rn(rnd<T>(P[i].x), st)), rnd<T>(__fdiv_rn(rnd<T>(P[i].y), st)));
+    }
+    const uint64_t key0 = (uint64_t)(m * K + (tin >> 3) * 256 + 2 * l.t8) + seed;
+    uint16_t* cb = reinterpret_cast<uint16_t*>(l.tbuf);
+    uint32_t c16[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const float a[2] = {l.tsw ? P[r].y : P[r].x, l.tsw ? P[r].x : P[r].y};
+        int n[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint64_t key = key0 + (uint64_t)(16 * r + j);
+            const uint32_t folded = (uint32_t)key ^ (uint32_t)(key >> 32);
+            const float f = floorf(noisy_sum(a[j], (float)(pcg_hash(folded) >> 8) * 0x1.0p-24f, (T*)nullptr));
+            n[j] = (int)fminf(127.f, fmaxf(-128.f, f));
+        }
+        c16[r] = (uint32_t)(n[0] & 0xff) | ((uint32_t)(n[1] & 0xff) << 8);
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r) cb[l.t8 + 8 * r] = (uint16_t)c16[r];
+    __syncwarp(wmask);
+    const uint4 lo = reinterpret_cast<const uint4*>(l.tbuf)[2 * l.t8], hi = reinterpret_cast<const uint4*>(l.tbuf)[2 * l.t8 + 1];
+    if (live) {
+        uint4* d = reinterpret_cast<uint4*>(q + m * (int64_t)K + tin * 32);
+        d[0] = lo, d[1] = hi;
+    }
+}
+
+// Back to the original basis with a group of 256 in the registers of eight lanes (rotate.cuh); nothing spans a row, so the
+// groups of all rows are simply dealt out. The kernel below, which walks a row in shared memory, took 53 us for 5120 x 5120 to
+// bf16 (79 MB moved) and stays for buffers that are not 16-byte aligned.
+template <typename T, bool ROUND_BF16>
+__global__ void __launch_bounds__(256) convrot_dequant_regs_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, T* __restrict__ out,
+                                                                   int64_t groups, int groups_per_row) {
+    __shared__ __align__(128) float smem_f[8 * kWarpWords];
+    pdl_trigger();
+    pdl_wait();
+    const RotLane l = rot_lane(smem_f);
+    const int64_t g_raw = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
+    const bool live = g_raw < groups;
+    const int64_t g = live ? g_raw : groups - 1;
+    const float sc = __ldg(s + g / groups_per_row);
+    const uint4* src = reinterpret_cast<const uint4*>(q + g * 256 + 32 * l.t8);
+    float v[32];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const uint4 u = __ldg(src + c);
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t b = w[i] ^ 0x80808080u;       // 2^23 + (code + 128) by setting exponent bits: exact, off the conversion pipe
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                v[16 * c + 4 * i + j] = __fmul_rn(__fsub_rn(__uint_as_float(__byte_perm(b, 0x4B000000u, 0x7440 + j)), 8388736.f), sc);
+        }
+    }
+    float2 P[16];
+    rotate256_regs(v, P, l, 0xffffffffu);
+    if (!live) return;
+    T* o = out + g * 256 + 2 * l.t8;
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const float a = l.tsw ? P[r].y : P[r].x, b = l.tsw ? P[r].x : P[r].y;
+        if constexpr (sizeof(T) == 2) *reinterpret_cast<__nv_bfloat162*>(o + 16 * r) = __floats2bfloat162_rn(a, b);
+        else *reinterpret_cast<float2*>(o + 16 * r) = make_float2(ROUND_BF16 ? rnd<bf16>(a) : a, ROUND_BF16 ? rnd<bf16>(b) : b);
+    }
+}
+
 // OUT_BF16_IN_F32: embed_dequant writes f32 rows holding bf16-rounded values
 template <typename T, bool ROUND_BF16>
 __global__ void __launch_bounds__(512) convrot_dequant_kernel(const int8_t* __restrict__ q, const float* __restrict__ s,
@@ -509,6 +641,105 @@ __global__ void __launch_bounds__(256) w6_requant_kernel(const bf16* __restrict_
     }
 }
 
+// The same packer with rows in registers: after the rotation (rotate.cuh) and the way back through its buffer a thread holds
+// 32 consecutive values, one scale group, so the fit and the codes run without shared memory and on all threads. The kernel
+// above has K / 32 threads of 256 at work on the groups, reads them with eight-way bank conflicts and rounds on the conversion
+// pipe: 241 us for 5120 x 5120. It stays for longer rows (K > 16384) and misaligned weights. Differences in form, not in results:
+//   - rint is an addition of 1.5 * 2^23 after the clamp (integer bounds: the order does not matter; a NaN becomes the lower bound
+//     in both);
+//   - the largest |q gs| of a group is that of its largest value (rounding is monotone; a NaN counts as |q| = 31, as it does there);
+//   - the level search starts at the ceiling of the estimate, which is nearly always the answer, and keeps the two levels that
+//     bracket the value instead of computing them again.
+__device__ __forceinline__ float rint_clamped(float x, float bound) {
+    return __fsub_rn(__fadd_rn(fminf(bound, fmaxf(-bound, x)), 12582912.f), 12582912.f);
+}
+__global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* __restrict__ w, uint8_t* __restrict__ packed, uint8_t* __restrict__ s_rel,
+                                                              float* __restrict__ s_channel, int64_t N, int K, int rows, uint64_t seed) {
+    extern __shared__ __align__(128) float smem_f[];
+    const unsigned wmask = __activemask();               // the last warp may be partial
+    const RotLane l = rot_lane(smem_f);
+    unsigned* amax_s = reinterpret_cast<unsigned*>(smem_f + ((blockDim.x + 31) >> 5) * kWarpWords);
+    for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
+    pdl_trigger();
+    pdl_wait();
+    __syncthreads();
+    const int tpr = K >> 5, rloc = threadIdx.x / tpr, g = threadIdx.x - rloc * tpr;      // thread g of a row has scale group g
+    const int64_t m_raw = (int64_t)blockIdx.x * rows + rloc;
+    const bool live = m_raw < N;
+    const int64_t n = live ? m_raw : N - 1;
+    float v[32];
+    load_row32(w + n * K + g * 32, v);
+    {
+        float2 P[16];
+        rotate256_regs(v, P, l, wmask);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {                   // the rotated weight lives in bf16
+            const __nv_bfloat162 h = __floats2bfloat162_rn(P[i].x, P[i].y);
+            P[i] = __bfloat1622float2(h);
+        }
+        untranspose256(P, v, l, wmask);
+    }
+    float amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) amax = max3_abs_nan(amax, v[i], v[i + 1]);
+    const bool has_nan = amax != amax;
+    if (has_nan) {
+        amax = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    }
+    float gs = fmaxf(__fdiv_rn(amax, 31.f), 1e-8f);
+    float inv = __fdiv_rn(1.f, gs);
+#pragma unroll 1
+    for (int it = 0; it < 2; ++it) {
+        float num = 0.f, den = 0.f;
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            const float q = rint_clamped(__fmul_rn(v[i], inv), 31.f);
+            num = __fmaf_rn(v[i], q, num);
+            den = __fmaf_rn(q, q, den);
+        }
+        gs = fmaxf(__fdiv_rn(num, fmaxf(den, 1e-8f)), 1e-8f);
+        inv = __fdiv_rn(1.f, gs);
+    }
+    const float qmax = has_nan ? 31.f : fabsf(rint_clamped(__fmul_rn(amax, inv), 31.f));
+    atomicMax(amax_s + rloc, __float_as_uint(fmaxf(0.f, __fmul_rn(qmax, gs))));
+    __syncthreads();
+    const float sc = fmaxf(__fdiv_rn(__uint_as_float(amax_s[rloc]), 127.f), 1e-8f);
+    const float inv_sc = __fdiv_rn(1.f, sc);
+    const uint8_t sb = (uint8_t)__nv_cvt_float_to_fp8(__fdiv_rn(gs, sc), __NV_SATFINITE, __NV_E4M3);
+    const float s = e4m3_to_f(sb);
+    const float inv_s = __fdiv_rn(1.f, fmaxf(s, 1e-30f));
+    const uint32_t key = (uint32_t)seed ^ (uint32_t)(seed >> 32);
+    const uint32_t e0 = (uint32_t)(n * (int64_t)K + g * 32);
+    auto level = [&](float f) { return rint_clamped(__fmul_rn(f, s), 127.f); };       // w6_level(i) at f = i - 31
+    uint32_t lo[4] = {0u, 0u, 0u, 0u}, hi[2] = {0u, 0u};
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        const float t = __fmul_rn(v[i], inv_sc);
+        int pos = min(max(__float2int_ru(__fmul_rn(__fsub_rn(ceilf(t), 0.5f), inv_s)), -31), 32) + 31;
+        float f = (float)(pos - 31), below = level(f - 1.f), at = level(f);
+        while (pos > 0 && below >= t) --pos, f -= 1.f, at = below, below = level(f - 1.f);
+        while (pos < 63 && at < t) ++pos, f += 1.f, below = at, at = level(f);
+        int lw = pos - 1;
+        if (pos == 0) lw = 0, below = at, at = level(-30.f);
+        else if (pos == 63) lw = 61, below = level(30.f), at = level(31.f);
+        const uint32_t h = pcg_hash((e0 + (uint32_t)i) ^ key);
+        const float u = __fmul_rn((float)(h >> 8), 1.0f / 16777216.0f);
+        const float thr = __fmaf_rn(u, __fsub_rn(at, below), below);
+        const uint32_t code = (uint32_t)min(lw + (t > thr ? 1 : 0), 62) + 1u;
+        lo[i >> 3] |= (code & 15u) << (4 * (i & 7));
+        hi[i >> 4] |= ((code >> 4) & 3u) << (2 * (i & 15));
+    }
+    if (live) {
+        if (g == 0) s_channel[n] = sc;
+        s_rel[n * tpr + g] = sb;
+        uint8_t* prow = packed + n * (int64_t)(K / 4 * 3);
+        *reinterpret_cast<uint4*>(prow + g * 16) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        *reinterpret_cast<uint2*>(prow + K / 2 + g * 8) = make_uint2(hi[0], hi[1]);
+    }
+}
+
 // The same with 32 codes (one whole scale group when G is a multiple of 32) per thread and the permute-table decode of
 // w6_decode.cuh: 16 + 8 bytes in, 32 bytes out per thread. The decode form is voted per warp, so every lane takes part
 // (lanes past the end redo the last piece and store nothing).
@@ -540,6 +771,18 @@ int set_smem(const void* fn, size_t bytes) {
     if (bytes <= 48 * 1024) return 0;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     return e == cudaSuccess ? 0 : (int)e;
+}
+// Rows in registers, K / 32 threads each: about 256 threads per CTA, at least a warp. Up to 512 threads (K <= 16384), so that a
+// thread may hold its 32 values and what is computed from them.
+struct RegRows { int rows, threads; size_t smem; };
+constexpr int kRegRowsMaxK = 16384;
+RegRows reg_rows(int K) {
+    const int tpr = K / 32;
+    int rows = 256 / tpr;
+    if (rows < 1) rows = 1;
+    if (rows * tpr < 32) rows = (32 + tpr - 1) / tpr;
+    const int threads = rows * tpr;
+    return {rows, threads, (size_t)((threads + 31) / 32) * kWarpWords * 4 + (size_t)rows * 4};
 }
 int row_threads(int work_items, int cap) {
     int t = (work_items + 31) / 32 * 32;
@@ -584,6 +827,15 @@ GPU_API int gpu_sd_quant_rows(const void* x, int64_t x_stride, int8_t* q, float*
 }
 
 namespace {
+// The register kernel where the buffers allow 16-byte accesses; *rc = its launch code.
+template <typename T, bool ROUND_BF16>
+bool dequant_regs(const void* q, const void* s, void* out, int64_t N, int K, cudaStream_t st, int* rc) {
+    const int64_t groups = N * (K / 256), ctas = (groups + 31) / 32;
+    if ((((uintptr_t)q | (uintptr_t)out) & 15) || ctas > INT32_MAX) return false;
+    *rc = launch_pdl(convrot_dequant_regs_kernel<T, ROUND_BF16>, dim3((unsigned)ctas), 256, 0, st, (const int8_t*)q, (const float*)s, (T*)out,
+                     groups, K / 256);
+    return true;
+}
 template <int MODE>
 int launch_sd_src(const SdSrc& p, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st) {
     if ((rotate != 0 && rotate != 64 && rotate != 256) || (rotate && K % rotate)) return -1;
@@ -650,6 +902,15 @@ GPU_API int gpu_convrot_requant(int dtype, const void* x, void* q, void* s, int6
     // the shared-memory kernel below (which stays for the stochastic rounding and for rows the quantizer does not take).
     if (seed == 0 && K <= 32768 && N <= INT32_MAX && ((((uintptr_t)x | (uintptr_t)q) & 15) == 0))
         return gpu_quant_rows(dtype, 0, x, K, nullptr, 0, 0, nullptr, 0.f, nullptr, nullptr, (int8_t*)q, (float*)s, (int)N, K, 1, stream);
+    if (K <= kRegRowsMaxK && ((((uintptr_t)x | (uintptr_t)q) & 15) == 0)) {
+        const RegRows g = reg_rows(K);
+        const dim3 grid((unsigned)((N + g.rows - 1) / g.rows));
+        cudaStream_t st = (cudaStream_t)stream;
+        if (int rc = set_smem(dtype == DT_F32 ? (const void*)convrot_requant_regs_kernel<float> : (const void*)convrot_requant_regs_kernel<bf16>, g.smem)) return rc;
+        if (dtype == DT_F32)
+            return launch_pdl(convrot_requant_regs_kernel<float>, grid, g.threads, g.smem, st, (const float*)x, (int8_t*)q, (float*)s, N, K, g.rows, seed);
+        return launch_pdl(convrot_requant_regs_kernel<bf16>, grid, g.threads, g.smem, st, (const bf16*)x, (int8_t*)q, (float*)s, N, K, g.rows, seed);
+    }
     const size_t smem = (size_t)padded_words(K) * sizeof(float);
     const int threads = row_threads(K / 16, 512);
     if (dtype == DT_F32) {
@@ -669,6 +930,10 @@ GPU_API int gpu_convrot_requant(int dtype, const void* x, void* q, void* s, int6
 GPU_API int gpu_convrot_dequant(int dtype, const void* q, const void* s, void* out, int64_t N, int K, void* stream) {
     if (K % 256) return -1;
     if (N <= 0) return 0;
+    if (dtype != DT_F32 && dtype != DT_BF16) return -4;
+    int rc0 = 0;
+    if (dtype == DT_F32 ? dequant_regs<float, false>(q, s, out, N, K, (cudaStream_t)stream, &rc0)
+                        : dequant_regs<bf16, false>(q, s, out, N, K, (cudaStream_t)stream, &rc0)) return rc0;
     const size_t smem = (size_t)padded_words(K) * sizeof(float);
     const int threads = row_threads(K / 16, 512);
     if (dtype == DT_F32) {
@@ -688,6 +953,8 @@ GPU_API int gpu_convrot_dequant(int dtype, const void* q, const void* s, void* o
 GPU_API int gpu_embed_dequant(const int8_t* q, const float* s, float* out, int M, int K, int rotate, void* stream) {
     if (!rotate || K % 256) return -1;
     if (M <= 0) return 0;
+    int rc0 = 0;
+    if (dequant_regs<float, true>(q, s, out, M, K, (cudaStream_t)stream, &rc0)) return rc0;
     const size_t smem = (size_t)padded_words(K) * sizeof(float);
     if (int rc = set_smem((const void*)convrot_dequant_kernel<float, true>, smem)) return rc;
     convrot_dequant_kernel<float, true><<<M, row_threads(K / 16, 512), smem, (cudaStream_t)stream>>>(q, s, out, K);
@@ -729,6 +996,12 @@ GPU_API int gpu_w6_requant(const void* weight, void* packed, void* s_rel, void* 
                            void* stream) {
     if (K % 256) return -1;
     if (N <= 0) return 0;
+    if (K <= kRegRowsMaxK && (((uintptr_t)weight & 15) == 0)) {
+        const RegRows g = reg_rows(K);
+        if (int rc = set_smem((const void*)w6_requant_regs_kernel, g.smem)) return rc;
+        return launch_pdl(w6_requant_regs_kernel, dim3((unsigned)((N + g.rows - 1) / g.rows)), g.threads, g.smem, (cudaStream_t)stream,
+                          (const bf16*)weight, (uint8_t*)packed, (uint8_t*)s_rel, (float*)s_channel, N, K, g.rows, seed);
+    }
     const size_t smem = (size_t)(padded_words(K) + K / 32) * sizeof(float);
     if (int rc = set_smem((const void*)w6_requant_kernel, smem)) return rc;
     w6_requant_kernel<<<(unsigned)N, 256, smem, (cudaStream_t)stream>>>((const bf16*)weight, (uint8_t*)packed, (uint8_t*)s_rel,

@@ -282,3 +282,38 @@ def test_sd_register_kernel_equals_the_shared_memory_kernel(pkg, dev, mode, M, K
         x, b = (rn(3, M, K) * 1.5 + 0.3).half(), rn(K) * 0.1
         got, want = (L.sd_group_norm_quant_rows(x, w, b, 32, 1e-5, rotate) for w in both(rn(K) * 0.2 + 1))
     assert_bits_equal(got[1], want[1], "scales"), assert_bits_equal(got[0], want[0], "codes")
+
+
+# one group, several rows per CTA with a partial warp, whole warps, the longest row in registers; the buffers one element off a
+# 16-byte boundary take the shared-memory kernels, whose results are pinned to the reference by the tests above
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("N,K", [(33, 256), (7, 768), (5, 5120), (2, 16384)])
+def test_packers_in_registers_equal_the_shared_memory_kernels(pkg, dev, N, K, dtype):
+    """Stochastic packing, its inverse and the W6 packer, infinities, NaN, zero rows and huge and tiny values among the weights:
+    bit-identical in both forms."""
+    L = pkg.linear
+    g = torch.Generator().manual_seed(N + K)
+    w = torch.randn(N, K, generator=g) * 0.02
+    w[0] = 0
+    special = torch.tensor([0.0, -0.0, 1e30, -3e38, 1e-38, float("inf"), float("-inf"), float("nan")])
+    for i in range(1, N, 2):
+        w[i, (97 * i) % K] = special[i // 2 % len(special)]
+    w = w.to(dtype)
+
+    def off(t):                                   # the same values one element past an aligned address
+        buf = torch.empty(t.numel() + 1, dtype=t.dtype, device=dev)
+        buf[1:] = t.to(dev).reshape(-1)
+        return buf[1:].view(t.shape)
+
+    for seed in (1, (7 << 32) + 99):
+        for a, b in zip(L.convrot_requant(w.to(dev), seed), L.convrot_requant(off(w), seed)):
+            assert_bits_equal(a, b, f"requant {seed}")
+        if dtype == torch.bfloat16:
+            for a, b in zip(L.w6_requant(w.to(dev), seed), L.w6_requant(off(w), seed)):
+                assert_bits_equal(a, b, f"w6 {seed}")
+    q = torch.randint(-128, 128, (N, K), generator=g, dtype=torch.int8)
+    s = torch.rand(N, generator=g).to(dev)
+    buf = torch.empty(q.numel() + 4, dtype=torch.int8, device=dev)      # four bytes off: what the other kernel needs
+    buf[4:] = q.to(dev).reshape(-1)
+    assert_bits_equal(L.convrot_dequant(q.to(dev), s, dtype), L.convrot_dequant(buf[4:].view(N, K), s, dtype), "dequant")
+    assert_bits_equal(L.embed_dequant(q.to(dev), s), L.embed_dequant(buf[4:].view(N, K), s), "embed")
