@@ -1,6 +1,7 @@
 """Builds libb200_qlinear.so (the C-ABI library) and libb200_qlinear.a (the same objects as a static archive, for hosts
-that link statically) from csrc/*.cu with nvcc, for sm_100a only. The name differs on purpose from the reference's own
-static library `gpu_kernels`, which keeps supplying every symbol this library does not replace.
+that link statically) from csrc/*.cu with nvcc, for sm_100a only, then _host_ops.so, the CPython extension behind
+linear.py's hot calls. The name differs on purpose from the reference's own static library `gpu_kernels`, which keeps
+supplying every symbol this library does not replace.
 
 The GEMM uses tcgen05.mma kind::i8, which exists on sm_100a and not on sm_103a or sm_120: no other -gencode
 may be added. No fast-math: the rounding points of the quantizer and of the epilogue are part of the contract.
@@ -10,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -17,6 +19,7 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "libb200_qlinear.so")
 ARCHIVE = os.path.join(HERE, "libb200_qlinear.a")
+HOST_OPS = os.path.join(HERE, "_host_ops.so")      # linear.py's hot calls (csrc/host_ops.cpp), linked against LIB and torch
 UNITS = ["quant_rows", "gemm_i8", "gemm_skinny", "weight_pack"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "--expt-relaxed-constexpr",
@@ -28,6 +31,32 @@ def _stale(target: str, deps: list[str]) -> bool:
         return True
     t = os.path.getmtime(target)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _host_ops(force: bool, verbose: bool) -> None:
+    """csrc/host_ops.cpp -> HOST_OPS, against the headers and libraries of the torch that will import it."""
+    src = os.path.join(CSRC, "host_ops.cpp")
+    stamp = os.path.join(OBJ, "host_ops.torch")
+    import torch
+
+    fresh = os.path.exists(stamp) and open(stamp).read() == torch.__version__
+    if not force and fresh and not _stale(HOST_OPS, [src, os.path.abspath(__file__), os.path.join(os.path.dirname(HERE), "include", "gpu_kernels.h")]):
+        return
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(NVCC))
+    dirs = [os.path.join(os.path.dirname(HERE), "include"), os.path.join(root, "include"),
+            os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
+    cmd = ["g++", "-shared", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", src, "-o", HOST_OPS]
+    cmd += [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"] + ["-I" + d for d in dirs]
+    cmd += ["-L" + HERE, "-l:" + os.path.basename(LIB), "-Wl,-rpath,$ORIGIN", "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu",
+            "-lc10", "-lc10_cuda"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if verbose or r.returncode:
+        sys.stderr.write(r.stdout + r.stderr)
+    if r.returncode:
+        raise RuntimeError("g++ failed on host_ops.cpp")
+    with open(stamp, "w") as f:
+        f.write(torch.__version__)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -54,6 +83,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if os.path.exists(ARCHIVE):
             os.remove(ARCHIVE)
         subprocess.check_call(["ar", "rcs", ARCHIVE] + objs)
+    _host_ops(force, verbose)
     return LIB
 
 

@@ -1172,8 +1172,8 @@ bool encode_operand_tmap(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t
 bool encode_output_tmap(CUtensorMap* tm, void* ptr, int64_t M, int64_t N, int esz);
 
 // Encoded tensor maps depend only on address, shape and box, not on the data: an inference loop presents the same
-// buffers again and again, so each thread remembers its last few (a map is 128 bytes; the driver call that encodes
-// one takes about a microsecond of host time, three per GEMM call).
+// buffers again and again, so each thread remembers some (a map is 128 bytes; the driver call that encodes one takes about
+// a microsecond of host time, three per GEMM call).
 struct TmapKey {
     const void* ptr;
     int64_t d0, d1, pitch;
@@ -1182,20 +1182,31 @@ struct TmapKey {
         return ptr == o.ptr && d0 == o.d0 && d1 == o.d1 && pitch == o.pitch && box0 == o.box0 && box1 == o.box1 && kind == o.kind;
     }
 };
-struct TmapCache {
-    static constexpr int kSlots = 16;
-    TmapKey key[kSlots] = {};
-    CUtensorMap map[kSlots];
-    bool used[kSlots] = {};
-    int next = 0;
+struct TmapCache {            // two-way sets: a U-Net block alone presents two dozen maps, which a list of sixteen never finds again
+    static constexpr int kSets = 64;
+    struct Set {
+        TmapKey key[2] = {};
+        CUtensorMap map[2];
+        bool used[2] = {};
+        int next = 0;
+    };
+    Set set[kSets];
+    static int index(const TmapKey& k) {
+        uint64_t h = (uint64_t)(uintptr_t)k.ptr >> 9;
+        h ^= (uint64_t)k.d0 * 0x9E3779B97F4A7C15ull ^ (uint64_t)k.d1 * 0xC2B2AE3D27D4EB4Full ^ (uint64_t)(k.box1 * 4 + k.kind);
+        h *= 0xD6E8FEB86659FD93ull;
+        return (int)(h >> 58);
+    }
     const CUtensorMap* find(const TmapKey& k) const {
-        for (int i = 0; i < kSlots; ++i)
-            if (used[i] && key[i] == k) return &map[i];
+        const Set& s = set[index(k)];
+        for (int i = 0; i < 2; ++i)
+            if (s.used[i] && s.key[i] == k) return &s.map[i];
         return nullptr;
     }
     void put(const TmapKey& k, const CUtensorMap& m) {
-        key[next] = k, map[next] = m, used[next] = true;
-        next = (next + 1) % kSlots;
+        Set& s = set[index(k)];
+        s.key[s.next] = k, s.map[s.next] = m, s.used[s.next] = true;
+        s.next ^= 1;
     }
 };
 thread_local TmapCache g_tmaps;

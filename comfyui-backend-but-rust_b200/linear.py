@@ -12,8 +12,11 @@ from typing import Optional
 
 import torch
 
+from . import _host_ops as _h
 from . import ffi
 from .ffi import ok
+
+_h.ok = ok      # how a call there raises the error of a return code
 
 _DT = {torch.float32: ffi.DT_F32, torch.float16: ffi.DT_F16, torch.bfloat16: ffi.DT_BF16}
 
@@ -44,20 +47,7 @@ def quant_rows(x: torch.Tensor, prologue: int = ffi.PRO_PLAIN, rotate: int = 0, 
                mod_shift: Optional[torch.Tensor] = None):
     """gpu_quant_rows (gpu_quant_rows_b when a LayerNorm bias is given): x [M, >=K] bf16/f32 -> (q int8 [M, K],
     scales f32 [M]). norm_w / norm_b f32 [K]; mod_scale / mod_shift [K] in x's dtype."""
-    _cuda(x)
-    M = x.shape[0]
-    K = K if K is not None else x.shape[1]
-    q = q if q is not None else torch.empty((M, K), dtype=torch.int8, device=x.device)
-    scales = scales if scales is not None else torch.empty((M,), dtype=torch.float32, device=x.device)
-    if norm_b is not None:
-        ok(_lib().gpu_quant_rows_b(_DT[x.dtype], prologue, _ptr(x), x.stride(0), _ptr(norm_w), _ptr(norm_b), eps,
-                                   _ptr(mod_scale), _ptr(mod_shift), _ptr(q), _ptr(scales), M, K, rotate, _stream()),
-           "gpu_quant_rows_b")
-        return q, scales
-    ok(_lib().gpu_quant_rows(_DT[x.dtype], prologue, _ptr(x), x.stride(0), _ptr(g), g.stride(0) if g is not None else 0,
-                             up_offset, _ptr(norm_w), eps, _ptr(mod_scale), _ptr(mod_shift), _ptr(q), _ptr(scales), M, K,
-                             rotate, _stream()), "gpu_quant_rows")
-    return q, scales
+    return _h.quant_rows(x, prologue, rotate, K, g, up_offset, q, scales, norm_w, norm_b, eps, mod_scale, mod_shift)
 
 
 def quant_rows_amax(x: torch.Tensor, prologue: int = ffi.PRO_PLAIN, rotate: int = 0, *, K: Optional[int] = None,
@@ -141,55 +131,27 @@ def wo8_linear(x: torch.Tensor, Wq: torch.Tensor, ws: torch.Tensor, prologue: in
 
 def sd_quant_rows(x: torch.Tensor, rotate: int = 0):
     """gpu_sd_quant_rows: fp16 rows (activations, or weights at load) -> (q int8, scales f32)."""
-    _cuda(x)
-    M, K = x.shape
-    q = torch.empty((M, K), dtype=torch.int8, device=x.device)
-    s = torch.empty((M,), dtype=torch.float32, device=x.device)
-    ok(_lib().gpu_sd_quant_rows(_ptr(x), x.stride(0), _ptr(q), _ptr(s), M, K, rotate, _stream()), "gpu_sd_quant_rows")
-    return q, s
+    return _h.sd_quant_rows(x, rotate)
 
 
 def sd_ln_quant_rows(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, eps: float, rotate: int = 0):
     """gpu_sd_ln_quant_rows: LayerNorm (f32 weight, bias) of half rows, then the fp16 quantizer."""
-    _cuda(x)
-    M, K = x.shape
-    q = torch.empty((M, K), dtype=torch.int8, device=x.device)
-    s = torch.empty((M,), dtype=torch.float32, device=x.device)
-    ok(_lib().gpu_sd_ln_quant_rows(_ptr(x), x.stride(0), _ptr(w), _ptr(b), eps, _ptr(q), _ptr(s), M, K, rotate, _stream()),
-       "gpu_sd_ln_quant_rows")
-    return q, s
+    return _h.sd_ln_quant_rows(x, w, b, eps, rotate)
 
 
 def sd_geglu_quant_rows(x: torch.Tensor, rotate: int = 0):
     """gpu_sd_geglu_quant_rows: x [M, 2 I] half (value, gate) -> codes of value * gelu(gate) [M, I]."""
-    _cuda(x)
-    M, I = x.shape[0], x.shape[1] // 2
-    q = torch.empty((M, I), dtype=torch.int8, device=x.device)
-    s = torch.empty((M,), dtype=torch.float32, device=x.device)
-    ok(_lib().gpu_sd_geglu_quant_rows(_ptr(x), _ptr(q), _ptr(s), M, I, rotate, _stream()), "gpu_sd_geglu_quant_rows")
-    return q, s
+    return _h.sd_geglu_quant_rows(x, rotate)
 
 
 def sd_group_norm_quant_rows(x: torch.Tensor, w: torch.Tensor, b: torch.Tensor, groups: int, eps: float, rotate: int = 0):
     """gpu_sd_group_norm_quant_rows: x [N, P, C] half -> GroupNorm (f32 weight, bias; no SiLU) -> codes [N * P, C]."""
-    _cuda(x)
-    N, P, C = x.shape
-    q = torch.empty((N * P, C), dtype=torch.int8, device=x.device)
-    s = torch.empty((N * P,), dtype=torch.float32, device=x.device)
-    sums = torch.empty((N * groups * 2 + 2,), dtype=torch.float64, device=x.device)
-    ok(_lib().gpu_sd_group_norm_quant_rows(_ptr(x), _ptr(w), _ptr(b), _ptr(sums), N, P, C, groups, eps, _ptr(q), _ptr(s), rotate,
-                                           _stream()), "gpu_sd_group_norm_quant_rows")
-    return q, s
+    return _h.sd_group_norm_quant_rows(x, w, b, groups, eps, rotate)
 
 
 def sd_unpad_quant_rows(x: torch.Tensor, d: int, rotate: int = 0):
     """gpu_sd_unpad_quant_rows: x [M, H, dp] half -> codes of the first d values of every head, [M, H * d]."""
-    _cuda(x)
-    M, H, dp = x.shape
-    q = torch.empty((M, H * d), dtype=torch.int8, device=x.device)
-    s = torch.empty((M,), dtype=torch.float32, device=x.device)
-    ok(_lib().gpu_sd_unpad_quant_rows(_ptr(x), _ptr(q), _ptr(s), M, H, d, dp, rotate, _stream()), "gpu_sd_unpad_quant_rows")
-    return q, s
+    return _h.sd_unpad_quant_rows(x, d, rotate)
 
 
 def convrot_requant(x: torch.Tensor, seed: int = 0):
@@ -242,45 +204,18 @@ def w6_requant(w: torch.Tensor, seed: int = 1):
 
 def int8_gemm(A, W, xs, ws, bias=None, *, out_dtype=torch.bfloat16, act: int = 0, rscale=None, resid=None, out=None):
     """gpu_int8_gemm / gpu_int8_gemm_act / gpu_int8_gemm_residual, chosen by the arguments given."""
-    _cuda(A)
-    M, K = A.shape
-    N = W.shape[0]
-    D = out if out is not None else torch.empty((M, N), dtype=out_dtype, device=A.device)
-    lib = _lib()
-    if resid is not None:
-        ok(lib.gpu_int8_gemm_residual(_ptr(A), _ptr(W), _ptr(xs), _ptr(ws), _ptr(bias), _ptr(rscale), _ptr(resid), _ptr(D),
-                                      M, N, K, _DT[D.dtype], _stream()), "gpu_int8_gemm_residual")
-    elif act:
-        ok(lib.gpu_int8_gemm_act(_ptr(A), _ptr(W), _ptr(xs), _ptr(ws), _ptr(bias), _ptr(D), M, N, K, _DT[D.dtype], act,
-                                 _stream()), "gpu_int8_gemm_act")
-    else:
-        ok(lib.gpu_int8_gemm(_ptr(A), _ptr(W), _ptr(xs), _ptr(ws), _ptr(bias), _ptr(D), M, N, K, _DT[D.dtype], _stream()),
-           "gpu_int8_gemm")
-    return D
+    return _h.int8_gemm(A, W, xs, ws, bias, out_dtype, act, rscale, resid, out)
 
 
 def int8_gemm_act_rot(A, W, xs, ws, bias=None, *, act: int = 1, out=None, amax_part=None):
     """gpu_int8_gemm_act_rot: bf16(R256(act(linear output))) [M, N] and the partial row maxima [N / 64, M] that
     quant_rows_rotated turns into codes and scales."""
-    _cuda(A)
-    M, K = A.shape
-    N = W.shape[0]
-    D = out if out is not None else torch.empty((M, N), dtype=torch.bfloat16, device=A.device)
-    parts = amax_part if amax_part is not None else torch.empty((N // 64, M), dtype=torch.float32, device=A.device)
-    ok(_lib().gpu_int8_gemm_act_rot(_ptr(A), _ptr(W), _ptr(xs), _ptr(ws), _ptr(bias), _ptr(D), _ptr(parts), M, N, K, act,
-                                    _stream()), "gpu_int8_gemm_act_rot")
-    return D, parts
+    return _h.int8_gemm_act_rot(A, W, xs, ws, bias, act, out, amax_part)
 
 
 def quant_rows_rotated(xr, amax_part, *, q=None, scales=None):
     """gpu_quant_rows_rotated: the quantizer's second pass on rows a rotating GEMM epilogue left."""
-    _cuda(xr)
-    M, K = xr.shape
-    q = q if q is not None else torch.empty((M, K), dtype=torch.int8, device=xr.device)
-    scales = scales if scales is not None else torch.empty((M,), dtype=torch.float32, device=xr.device)
-    ok(_lib().gpu_quant_rows_rotated(_ptr(xr), _ptr(amax_part), _ptr(q), _ptr(scales), M, K, _stream()),
-       "gpu_quant_rows_rotated")
-    return q, scales
+    return _h.quant_rows_rotated(xr, amax_part, q, scales)
 
 
 def int8_gemm_acc_i32(A, W, out=None):
@@ -295,21 +230,7 @@ def w6a8_gemm(A, packed, s_rel, xs, s_channel, bias=None, *, out_dtype=torch.bfl
               out=None, G: int = 32):
     """gpu_w6a8_gemm / gpu_w6a8_gemm_act / gpu_w6a8_gemm_residual: the W6A8 linear from the packed weight [N, 3K/4] and
     e4m3 scales [N, K/G]."""
-    _cuda(A)
-    M, K = A.shape
-    N = packed.shape[0]
-    D = out if out is not None else torch.empty((M, N), dtype=out_dtype, device=A.device)
-    lib = _lib()
-    if resid is not None:
-        ok(lib.gpu_w6a8_gemm_residual(_ptr(A), _ptr(packed), _ptr(s_rel), _ptr(xs), _ptr(s_channel), _ptr(bias), _ptr(rscale),
-                                      _ptr(resid), _ptr(D), M, N, K, G, _DT[D.dtype], _stream()), "gpu_w6a8_gemm_residual")
-    elif act:
-        ok(lib.gpu_w6a8_gemm_act(_ptr(A), _ptr(packed), _ptr(s_rel), _ptr(xs), _ptr(s_channel), _ptr(bias), _ptr(D), M, N, K, G,
-                                 _DT[D.dtype], act, _stream()), "gpu_w6a8_gemm_act")
-    else:
-        ok(lib.gpu_w6a8_gemm(_ptr(A), _ptr(packed), _ptr(s_rel), _ptr(xs), _ptr(s_channel), _ptr(bias), _ptr(D), M, N, K, G,
-                             _DT[D.dtype], _stream()), "gpu_w6a8_gemm")
-    return D
+    return _h.w6a8_gemm(A, packed, s_rel, xs, s_channel, bias, out_dtype, act, rscale, resid, out, G)
 
 
 def w6a8_gemm_acc_i32(A, packed, s_rel, G: int = 32):

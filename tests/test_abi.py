@@ -99,3 +99,17 @@ def test_workload_configs(pkg):
     assert len(wl.config(3)) == 12 and all(s.K % s.rotate == 0 for s in wl.config(3))
     block = wl.config(4)
     assert abs(sum(s.ops for s in block) - 3827e9) < 2e9
+
+
+def test_hot_calls_refuse_what_they_refused_through_ctypes(pkg):
+    """linear.py's extension calls raise before any launch: host tensors, what is not a tensor, the wrong number of dimensions."""
+    import torch
+    L = pkg.linear
+    x, s = torch.zeros(4, 256), torch.zeros(4)
+    q = torch.zeros(4, 256, dtype=torch.int8)
+    for call in (lambda: L.quant_rows(x), lambda: L.sd_quant_rows(x.half(), 64), lambda: L.int8_gemm(q, q, s, s),
+                 lambda: L.quant_rows_rotated(x.bfloat16(), s), lambda: L.w6a8_gemm(q, q, q, s, s)):
+        with pytest.raises(ValueError, match="CUDA tensors only"):
+            call()
+    with pytest.raises((TypeError, AttributeError)):
+        L.int8_gemm(None, q, s, s)
