@@ -709,12 +709,16 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int S = p.stages;
     const int BN = p.bn;
     const int KS = p.ksub;
+    const int KA = KIND == 1 ? 2 : KS, KB = KIND == 1 ? 1 : KS;   // boxes of A and W in a stage (KIND 1: both terms of A, one W)
+    // KIND 1 has two accumulators per tile: two tiles' worth fit the tensor memory up to 128 columns, one tile's beyond
+    const bool one_buf = KIND == 1 && BN > 128;
+    const uint32_t lo_acc = one_buf ? 256u : 128u;
     const uint32_t a_bytes = BM * BK;                     // one 128-byte K box of this CTA's A rows
     const uint32_t b_bytes = (uint32_t)(BN / 2) * BK;     // ... and of this CTA's half of the W tile
-    const uint32_t stage_bytes = KS * (a_bytes + b_bytes);
+    const uint32_t stage_bytes = KA * a_bytes + KB * b_bytes;
     uint8_t* staging = sm;                                 // kEpiWarps x 4 KB of output staging
-    const uint32_t sA = base + kStagingBytes;              // S x KS x [128 x 128]
-    const uint32_t sB = sA + S * KS * a_bytes;             // S x KS x [bn/2 x 128]
+    const uint32_t sA = base + kStagingBytes;              // S x KA x [128 x 128]
+    const uint32_t sB = sA + S * KA * a_bytes;             // S x KB x [bn/2 x 128]
     uint8_t* tail = sm + kStagingBytes + S * stage_bytes;
     const uint32_t bar_full = smem_u32(tail);              // kMaxStages barriers (the leader's are used)
     const uint32_t bar_empty = bar_full + 8 * kMaxStages;  // kMaxStages, one set per CTA
@@ -779,9 +783,13 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 const int row_w = tn * BN + (int)rank * (BN / 2);
                 for (int kb = wi.k0; kb < wi.k0 + wi.kn; ++kb) {
                     if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_s, ST_TIMEOUT_EMPTY)) { ok = false; break; }
-                    if (leader) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * KS * (a_bytes + b_bytes));
+                    if (leader) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * stage_bytes);
                     const uint32_t full = mapa_shared(bar_full + 8 * stage, 0);
-                    for (int ks = 0; ks < KS; ++ks) {
+                    if constexpr (KIND == 1) {      // rows of the low terms follow the M rows of the high ones
+                        tma_load_2d_pair(sA + 2 * stage * a_bytes, &tmap_a, kb * BK, row_a, full);
+                        tma_load_2d_pair(sA + (2 * stage + 1) * a_bytes, &tmap_a, kb * BK, p.M + row_a, full);
+                        tma_load_2d_pair(sB + stage * b_bytes, &tmap_w, kb * BK, row_w, full);
+                    } else for (int ks = 0; ks < KS; ++ks) {
                         tma_load_2d_pair(sA + (stage * KS + ks) * a_bytes, &tmap_a, (kb * KS + ks) * BK, row_a, full);
                         tma_load_2d_pair(sB + (stage * KS + ks) * b_bytes, &tmap_w, (kb * KS + ks) * BK, row_w, full);
                     }
@@ -800,7 +808,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (leader && lane == 0) {
             const uint32_t a_lo0 = umma_desc_lo(sA), b_lo0 = umma_desc_lo(sB);
             const uint32_t a_sub = a_bytes >> 4, b_sub = b_bytes >> 4;        // next K box of a stage
-            const uint32_t a_step = KS * a_sub, b_step = KS * b_sub;          // next stage
+            const uint32_t a_step = KA * a_sub, b_step = KB * b_sub;          // next stage
             const uint32_t idesc = p.idesc;
             int stage = 0;
             uint32_t phase = 0;
@@ -822,7 +830,13 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                         umma_pair_lo<KIND>(d_tmem, a_lo + 2, b_lo + 2, idesc, 1);   // +32 bytes inside the swizzle row
                         umma_pair_lo<KIND>(d_tmem, a_lo + 4, b_lo + 4, idesc, 1);
                         umma_pair_lo<KIND>(d_tmem, a_lo + 6, b_lo + 6, idesc, 1);
-                        if (KS == 2) {
+                        if constexpr (KIND == 1) {      // the low terms meet in an accumulator of their own
+                            const uint32_t a2 = a_lo + a_sub, d2 = d_tmem + lo_acc;
+                            umma_pair_lo<KIND>(d2, a2, b_lo, idesc, kb);
+                            umma_pair_lo<KIND>(d2, a2 + 2, b_lo + 2, idesc, 1);
+                            umma_pair_lo<KIND>(d2, a2 + 4, b_lo + 4, idesc, 1);
+                            umma_pair_lo<KIND>(d2, a2 + 6, b_lo + 6, idesc, 1);
+                        } else if (KS == 2) {
                             const uint32_t a2 = a_lo + a_sub, b2 = b_lo + b_sub;
                             umma_pair_lo<KIND>(d_tmem, a2, b2, idesc, 1);
                             umma_pair_lo<KIND>(d_tmem, a2 + 2, b2 + 2, idesc, 1);
@@ -836,7 +850,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
                 if (!ok) break;
                 umma_commit_pair(bar_tfull + 8 * buf);   // accumulator complete: both epilogues may drain it
-                buf ^= 1;
+                if (!one_buf) buf ^= 1;
                 if (buf == 0) tphase ^= 1u;
             }
         }
@@ -966,6 +980,16 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                         }
                     }
                 }
+            } else if (KIND == 1) {
+#pragma unroll 1
+                for (int c = half; c < nchunks; c += 2) {
+                    tmem_ld32(taddr + c * 32, ra);
+                    tmem_ld32(taddr + lo_acc + c * 32, rb);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) ra[e] = __float_as_uint(__fadd_rn(__uint_as_float(ra[e]), __uint_as_float(rb[e])));
+                    emit(ra, c);
+                }
             } else if (!kResidStaged && wi.kind == ITEM_WHOLE) {
                 int c = half;
                 if (c < nchunks) tmem_ld32(taddr + c * 32, ra);
@@ -1014,7 +1038,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_shared(bar_tempty + 8 * buf, 0));
-            buf ^= 1;
+            if (!one_buf) buf ^= 1;
             if (buf == 0) tphase ^= 1u;
         }
         if (p.tma_store && lane == 0) bulk_wait_read<0>();   // staged rows have left shared memory before the CTA exits
@@ -1552,8 +1576,12 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
 
 // ---- weight-only int8 linear (the text encoders' path) ---------------------------------------------------------------
 // int8 codes are exact in bf16, so W goes to the tensor cores as bf16 without loss; the f32 activation goes as two bf16
-// terms (hi + lo = 16 significant bits), one GEMM pass each into f32 accumulators: close to an fp32 product at tensor-core
-// speed. The kernel is the int8 one with kind::f16 MMAs (bf16 operands are addressed as rows of 2 K bytes).
+// terms (hi + lo = 16 significant bits) into two f32 accumulators, added in the epilogue: close to an fp32 product at
+// tensor-core speed. The kernel is the int8 one with kind::f16 MMAs (bf16 operands are addressed as rows of 2 K bytes); a
+// stage holds a K box of both terms and the one box of W that multiplies them. As two launches, the second adding to the
+// output of the first, W was read and D written twice: the MLP of a text encoder layer (512 rows, 2560, FFN 9728) took 301 us,
+// now 252 (271 with tiles of at most 128 columns, whose accumulators fit the tensor memory twice: what the narrower tiles read
+// from L2 costs more than the epilogue that wider ones leave uncovered).
 __global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* __restrict__ q, bf16* __restrict__ out, int64_t n16) {
     pdl_trigger();
     pdl_wait();
@@ -1568,10 +1596,11 @@ __global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* __rest
     reinterpret_cast<uint4*>(out)[2 * i + 1] = *reinterpret_cast<const uint4*>(&o[4]);
 }
 
-// D[M,N] (f32) = [resid +] (A[M,K] . W[N,K]^T) * ws[n], A and W bf16 row-major, K % 8 == 0, 16-byte aligned.
+// D[M,N] (f32) = [D +] ((A[0:M] + A[M:2M]) . W[N,K]^T) * ws[n], A (2 M rows: the high terms, then the low ones) and W bf16
+// row-major, K % 8 == 0, 16-byte aligned.
 int run_gemm_bf16(bool add, const void* A, const void* W, const float* ws, float* D, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
     if (M == 0 || N == 0 || K == 0) return 0;
-    if (M > INT32_MAX || N > INT32_MAX || K > INT32_MAX / 2) return -200;
+    if (M > INT32_MAX / 2 || N > INT32_MAX || K > INT32_MAX / 2) return -200;
     if ((K % 8) != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)D & 15)) return -202;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1584,12 +1613,12 @@ int run_gemm_bf16(bool add, const void* A, const void* W, const float* ws, float
     auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     p.vec_ok = (N % 8 == 0) && al16(ws);
     p.tma_store = (N * 4) % 16 == 0;
-    p.ksub = Kb <= BK ? 1 : 2;
-    p.k_iters = (int)((Kb + p.ksub * BK - 1) / (p.ksub * BK));
+    p.ksub = 1;
+    p.k_iters = (int)((Kb + BK - 1) / BK);
     const int bn = choose_bn(M, N, clusters);
     p.bn = bn;
     p.idesc = umma_idesc_bf16(2 * BM, bn);
-    const int stage_bytes = p.ksub * (BM * BK + (bn / 2) * BK);
+    const int stage_bytes = 2 * BM * BK + (bn / 2) * BK;
     const int stages = (kSmemBytes - 1024 - kTailBytes - kStagingBytes) / stage_bytes;
     p.stages = stages > kMaxStages ? kMaxStages : stages;
     p.tiles_m = (int)((M + 2 * BM - 1) / (2 * BM));
@@ -1597,7 +1626,7 @@ int run_gemm_bf16(bool add, const void* A, const void* W, const float* ws, float
     p.num_tiles = p.tiles_m * p.tiles_n;
     p.whole_tiles = p.num_tiles, p.splits = 0, p.kps = p.k_iters, p.num_items = p.num_tiles;
     CUtensorMap ta, tw, td;
-    if (!make_operand_tmap(&ta, A, M, Kb, BM) || !make_operand_tmap(&tw, W, N, Kb, bn / 2)) return -203;
+    if (!make_operand_tmap(&ta, A, 2 * M, Kb, BM) || !make_operand_tmap(&tw, W, N, Kb, bn / 2)) return -203;
     if (p.tma_store) {
         if (!make_output_tmap(&td, D, M, N, 4)) return -203;
     } else {
@@ -1642,8 +1671,8 @@ GPU_API int gpu_w6a8_gemm_acc_i32(const int8_t* A, const uint8_t* Wq6, const uin
 // New: the weight-only int8 linear of the text encoders in one call. The reference rotates the f32 activation rows
 // (gpu_rotate_rows_f32, csrc/kernels.cu:316-327), dequantizes the whole int8 weight to f32 (gpu_dequant_i8, :330-343) and runs
 // an fp32 GEMM with beta 0 or 1 (src/te.rs:493-511). Here: out[M,N] = beta * out + R256(prologue(x)) . (Wq * ws[n])^T with the
-// product on the bf16 tensor cores: Wq widens to bf16 exactly, the rotated rows go as hi + lo bf16 terms (two passes, f32
-// accumulation), so the result is within about 2^-16 relative of the fp32 product's terms.
+// product on the bf16 tensor cores: Wq widens to bf16 exactly, the rotated rows go as hi + lo bf16 terms (one pass, f32
+// accumulators of their own), so the result is within about 2^-16 relative of the fp32 product's terms.
 //   prologue   PRO_PLAIN, PRO_RMS (norm_w, eps) or PRO_SWIGLU (up_offset) as gpu_rotate_rows_f32 takes them
 //   a_scratch  >= 4 * M * K bytes (the reference's rotated-rows buffer has that size), w_scratch >= 2 * N * K bytes
 //              (half of the reference's dequantized-weight buffer); both 16-byte aligned
@@ -1657,12 +1686,11 @@ GPU_API int gpu_wo8_linear(int prologue, const float* x, int64_t x_stride, int64
     if ((((uintptr_t)a_scratch | (uintptr_t)w_scratch | (uintptr_t)Wq) & 15) || !a_scratch || !w_scratch) return -202;
     cudaStream_t st = (cudaStream_t)stream;
     uint8_t* hi = reinterpret_cast<uint8_t*>(a_scratch);
-    uint8_t* lo = hi + (size_t)M * K * 2;
+    uint8_t* lo = hi + (size_t)M * K * 2;               // one matrix of 2 M rows
     if (int rc = rotate_rows_split(prologue, x, x_stride, up_offset, norm_w, eps, hi, lo, M, K, st)) return rc;
     const int64_t n16 = (int64_t)N * K / 16;
     if (int rc = launch_pdl(widen_i8_bf16_kernel, dim3((unsigned)((n16 + 255) / 256)), 256, 0, st, Wq, reinterpret_cast<bf16*>(w_scratch), n16)) return rc;
-    if (int rc = run_gemm_bf16(beta == 1.f, hi, w_scratch, ws, out, M, N, K, st)) return rc;
-    return run_gemm_bf16(true, lo, w_scratch, ws, out, M, N, K, st);
+    return run_gemm_bf16(beta == 1.f, hi, w_scratch, ws, out, M, N, K, st);
 }
 
 // D[M,N] = (A[M,K] . W[N,K]^T) * xs[m] * ws[n] + bias[n]; replaces the reference's csrc/gemm.cu:123-129.
