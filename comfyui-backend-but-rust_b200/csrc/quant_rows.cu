@@ -568,13 +568,26 @@ __device__ __forceinline__ uint4 pack_half8(const float (&v)[8]) {
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// Piece i = threadIdx.x, threadIdx.x + blockDim.x, ... of the CTA's rows as (row, piece of the row): one division at the start
+// instead of one per piece.
+struct SdPieces {
+    int r, c, dr, dc, pieces;
+    __device__ __forceinline__ explicit SdPieces(int n) : pieces(n) {
+        r = (int)threadIdx.x / n, c = (int)threadIdx.x - r * n;
+        dr = (int)blockDim.x / n, dc = (int)blockDim.x - dr * n;
+    }
+    __device__ __forceinline__ void next() {
+        r += dr, c += dc;
+        if (c >= pieces) c -= pieces, ++r;
+    }
+};
 template <int SRC>
 __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int pitch, float2* stat, int64_t m0, int live_rows, int K) {
     const int pieces = K >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     if constexpr (SRC == SDQ_LN) {
         // the rows as they lie first, all of them in flight together
-        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
-            const int r = i / pieces, c = i - r * pieces;
+        for (SdPieces i(pieces); i.r < live_rows; i.next()) {
+            const int r = i.r, c = i.c;
             row_s[r * pitch + sd_piece(c)] = __ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * s.x_stride) + c);
         }
         __syncthreads();
@@ -621,8 +634,8 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
         }
         __syncthreads();
         const int per = K / s.groups;
-        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
-            const int r = i / pieces, c = i - r * pieces;
+        for (SdPieces i(pieces); i.r < live_rows; i.next()) {
+            const int r = i.r, c = i.c;
             float e[8], w[8], b[8];
             unpack_half8(__ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)K) + c), e);
             load8v(s.w + 8 * c, w), load8v(s.b + 8 * c, b);
@@ -637,8 +650,8 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
             row_s[r * pitch + sd_piece(c)] = pack_half8(e);
         }
     } else if constexpr (SRC == SDQ_GEGLU) {
-        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
-            const int r = i / pieces, c = i - r * pieces;
+        for (SdPieces i(pieces); i.r < live_rows; i.next()) {
+            const int r = i.r, c = i.c;
             const uint4* in = reinterpret_cast<const uint4*>(s.x + (m0 + r) * 2 * (int64_t)K);
             float e[8], g[8];
             unpack_half8(__ldg(in + c), e), unpack_half8(__ldg(in + pieces + c), g);
@@ -647,16 +660,20 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
             row_s[r * pitch + sd_piece(c)] = pack_half8(e);
         }
     } else if constexpr (SRC == SDQ_UNPAD) {
-        for (int i = threadIdx.x; i < live_rows * pieces; i += blockDim.x) {
-            const int r = i / pieces, c = i - r * pieces, h = (8 * c) / s.d;      // d % 8 == 0: a piece lies inside one head
+        for (SdPieces i(pieces); i.r < live_rows; i.next()) {
+            const int r = i.r, c = i.c, h = (8 * c) / s.d;      // d % 8 == 0: a piece lies inside one head
             row_s[r * pitch + sd_piece(c)] =
                 __ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)s.heads * s.dp + (int64_t)h * s.dp + (8 * c - h * s.d)));
         }
     }
 }
 
-template <int ROT, int SRC>
-__global__ void __launch_bounds__(512) sd_quant_fast_kernel(const SdSrc s, int8_t* __restrict__ q, float* __restrict__ scales, int M,
+// Up to 288 threads (rows up to 9216 values) the kernel is held to 56 registers, seven CTAs of 160 threads per SM instead of
+// six: 8192 rows of 640 values are 1024 such CTAs, which six per SM take in two rounds, the second an eighth full.
+// U-Net block of width 640 (eight of these kernels): 328 us with 63 registers, halvings in every stage and a division per piece, 321 now.
+constexpr int kSdThreads = 288;
+template <int ROT, int SRC, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fast_kernel(const SdSrc s, int8_t* __restrict__ q, float* __restrict__ scales, int M,
                                                             int K, int tpr, int rows, uint32_t off_amax, uint32_t off_rows) {
     extern __shared__ __align__(128) uint8_t smem[];
     const unsigned wmask = __activemask();
@@ -694,7 +711,7 @@ __global__ void __launch_bounds__(512) sd_quant_fast_kernel(const SdSrc s, int8_
     if (ROT) {
 #pragma unroll
         for (int i = 0; i < 16; ++i) P[i] = make_float2(v[i], v[i + 16]);
-        two_stages(P);                                  // index bits 0-3
+        two_stages<false>(P);                           // index bits 0-3
     } else {
 #pragma unroll
         for (int i = 0; i < 16; ++i) P[i] = make_float2(v[2 * i], v[2 * i + 1]);
@@ -711,7 +728,7 @@ __global__ void __launch_bounds__(512) sd_quant_fast_kernel(const SdSrc s, int8_
         __syncwarp(wmask);
 #pragma unroll
         for (int rr = 0; rr < 16; ++rr) P[rr] = *reinterpret_cast<const float2*>(tbuf_w + tpad(2 * t8 + 16 * rr));
-        two_stages(P);                                  // index bits 4-7
+        two_stages<false>(P);                           // index bits 4-7
         __syncwarp(wmask);
     } else if (ROT == 64) {
         // third stage, index bits 4 and 5: bit 4 is the pair's half, bit 5 the lane's parity. The even lane holds x0, x1
@@ -725,13 +742,17 @@ __global__ void __launch_bounds__(512) sd_quant_fast_kernel(const SdSrc s, int8_
             const float sd = __fmaf_rn(x1, sg, x0);                                   // x0 + x1 (even) or x0 - x1 (odd)
             const float rx = __fmaf_rn(x3, -sg, __fadd_rn(sd, x2));                   // (sd + x2) - x3   or (sd + x2) + x3
             const float ry = __fadd_rn(__fmaf_rn(even ? x2 : sd, -1.f, even ? sd : x2), x3);   // (sd - x2) + x3 or (-sd + x2) + x3
-            P[i] = make_float2(__fmul_rn(0.5f, rx), __fmul_rn(0.5f, ry));
+            P[i] = make_float2(rx, ry);
         }
     }
+    // The stages' halvings come as one multiplication here. For halves that is exact and the same: the sums stay below 2^16 * 256,
+    // nothing is small enough to underflow, and scaling by a power of two moves no rounding.
+    constexpr float kScale = ROT == 256 ? 0.0625f : 0.125f;
     // round to half; the row maximum is over the rounded values (the NaN-propagating form flags threads that hold one)
     float amax = 0.f;
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
+        if (ROT) P[i] = __fmul2_rn(P[i], make_float2(kScale, kScale));
         P[i] = __half22float2(__floats2half2_rn(P[i].x, P[i].y));
         amax = max3_abs_nan(amax, P[i].x, P[i].y);
     }
@@ -858,27 +879,11 @@ int ensure_lut(int which, cudaStream_t st) {
 }  // namespace
 
 namespace {
-template <int ROT, int SRC>
-int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaStream_t st) {
-    auto kern = sd_quant_fast_kernel<ROT, SRC>;
-    const int tpr = K / 32;
-    // whole rows and about 256 threads; a whole number of warps where that takes no more than 512
-    int rows = 256 / tpr;
-    if (rows < 1) rows = 1;
-    if (rows * tpr < 32) rows = (32 + tpr - 1) / tpr;
-    if (SRC != SDQ_ROWS) {
-        int even = 32;                                  // rows that make a whole number of warps
-        while (even > 1 && (even / 2 * tpr) % 32 == 0) even /= 2;
-        if (even * tpr <= 512) rows = rows / even > 0 ? rows / even * even : even;
-    }
-    const int threads = rows * tpr;
-    uint32_t off = ROT == 256 ? (uint32_t)((threads + 31) / 32) * kWarpWords * 4 : 0;
-    const uint32_t off_amax = off;
-    off += (uint32_t)((rows + 1) & ~1) * 4 + (SRC == SDQ_GN ? (uint32_t)s.groups * 8 : 0);
-    off = (off + 127) & ~127u;
-    const uint32_t off_rows = off;
-    if (SRC != SDQ_ROWS) off += (uint32_t)rows * (((K >> 3) + 7) & ~7) * 16;
-    if (off > 48 * 1024) {
+template <int ROT, int SRC, int MAXT>
+int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 grid, int threads, int rows, uint32_t smem, uint32_t off_amax,
+                  uint32_t off_rows, cudaStream_t st) {
+    auto kern = sd_quant_fast_kernel<ROT, SRC, MAXT>;
+    if (smem > 48 * 1024) {
         static std::atomic<uint64_t> configured{0};
         int dev = 0;
         cudaGetDevice(&dev);
@@ -889,8 +894,28 @@ int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaS
             configured.fetch_or(bit, std::memory_order_release);
         }
     }
+    return launch_pdl(kern, grid, threads, smem, st, s, q, scales, M, K, K / 32, rows, off_amax, off_rows);
+}
+template <int ROT, int SRC>
+int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaStream_t st) {
+    const int tpr = K / 32;
+    // whole rows and about 256 threads; a whole number of warps where that takes no more than 512
+    int rows = 256 / tpr;
+    if (rows < 1) rows = 1;
+    if (rows * tpr < 32) rows = (32 + tpr - 1) / tpr;
+    int even = 32;                                      // rows that make a whole number of warps
+    while (even > 1 && (even / 2 * tpr) % 32 == 0) even /= 2;
+    if (even * tpr <= kSdThreads || (SRC != SDQ_ROWS && even * tpr <= 512)) rows = rows / even > 0 ? rows / even * even : even;
+    const int threads = rows * tpr;
+    uint32_t off = ROT == 256 ? (uint32_t)((threads + 31) / 32) * kWarpWords * 4 : 0;
+    const uint32_t off_amax = off;
+    off += (uint32_t)((rows + 1) & ~1) * 4 + (SRC == SDQ_GN ? (uint32_t)s.groups * 8 : 0);
+    off = (off + 127) & ~127u;
+    const uint32_t off_rows = off;
+    if (SRC != SDQ_ROWS) off += (uint32_t)rows * (((K >> 3) + 7) & ~7) * 16;
     const dim3 grid = SRC == SDQ_GN ? dim3((unsigned)((s.P + rows - 1) / rows), (unsigned)(M / s.P)) : dim3((unsigned)((M + rows - 1) / rows));
-    return launch_pdl(kern, grid, threads, off, st, s, q, scales, M, K, tpr, rows, off_amax, off_rows);
+    if (threads <= kSdThreads) return launch_sd_cfg<ROT, SRC, kSdThreads>(s, q, scales, M, K, grid, threads, rows, off, off_amax, off_rows, st);
+    return launch_sd_cfg<ROT, SRC, 512>(s, q, scales, M, K, grid, threads, rows, off, off_amax, off_rows, st);
 }
 template <int SRC>
 int launch_sd_fast_rot(const SdSrc& s, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st) {

@@ -22,22 +22,26 @@ __device__ __forceinline__ int tpad(int e) { return e + ((e >> 5) << 2); }
 
 // Radix-4 butterfly of the regular Hadamard block on packed pairs; outputs in the reference's association:
 //   r0 = .5*(((x0+x1)+x2)-x3)  r1 = .5*(((x0+x1)-x2)+x3)  r2 = .5*(((x0-x1)+x2)+x3)  r3 = .5*(((-x0+x1)+x2)+x3)
+// HALVE = false leaves the factors 0.5 out.
+template <bool HALVE = true>
 __device__ __forceinline__ void h4x2(float2& x0, float2& x1, float2& x2, float2& x3) {
     const float2 m1 = make_float2(-1.f, -1.f), hf = make_float2(0.5f, 0.5f);
     const float2 s = __fadd2_rn(x0, x1);
     const float2 d = __ffma2_rn(x1, m1, x0);                         // x0 - x1
-    const float2 r0 = __fmul2_rn(hf, __ffma2_rn(x3, m1, __fadd2_rn(s, x2)));
-    const float2 r1 = __fmul2_rn(hf, __fadd2_rn(__ffma2_rn(x2, m1, s), x3));
-    const float2 r2 = __fmul2_rn(hf, __fadd2_rn(__fadd2_rn(d, x2), x3));
-    const float2 r3 = __fmul2_rn(hf, __fadd2_rn(__ffma2_rn(d, m1, x2), x3));   // (-d + x2) + x3
-    x0 = r0, x1 = r1, x2 = r2, x3 = r3;
+    const float2 r0 = __ffma2_rn(x3, m1, __fadd2_rn(s, x2));
+    const float2 r1 = __fadd2_rn(__ffma2_rn(x2, m1, s), x3);
+    const float2 r2 = __fadd2_rn(__fadd2_rn(d, x2), x3);
+    const float2 r3 = __fadd2_rn(__ffma2_rn(d, m1, x2), x3);         // (-d + x2) + x3
+    if (HALVE) x0 = __fmul2_rn(hf, r0), x1 = __fmul2_rn(hf, r1), x2 = __fmul2_rn(hf, r2), x3 = __fmul2_rn(hf, r3);
+    else x0 = r0, x1 = r1, x2 = r2, x3 = r3;
 }
 // two radix-4 stages over 16 packed values: index bits (0,1) then (2,3) of the position in P
+template <bool HALVE = true>
 __device__ __forceinline__ void two_stages(float2 (&P)[16]) {
 #pragma unroll
-    for (int i = 0; i < 16; i += 4) h4x2(P[i], P[i + 1], P[i + 2], P[i + 3]);
+    for (int i = 0; i < 16; i += 4) h4x2<HALVE>(P[i], P[i + 1], P[i + 2], P[i + 3]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) h4x2(P[i], P[i + 4], P[i + 8], P[i + 12]);
+    for (int i = 0; i < 4; ++i) h4x2<HALVE>(P[i], P[i + 4], P[i + 8], P[i + 12]);
 }
 
 // max(|a|, |b|, |c|) that is NaN as soon as one input is
