@@ -207,8 +207,17 @@ __device__ int g_quant_status = 0;   // a staging wait that ran out records ST_T
 
 // MAXT = 384 asks for two CTAs per SM (at most 80 registers: 768 threads with the next block's rows in flight);
 // longer rows take one larger CTA.
-template <typename T, int PRO, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(const QuantArgs p) {
+// DIRECT: the form of a block's linears and of the packers, rotated rows to codes and scales, one row block per CTA. Without the
+// other forms in the same instantiation it fits 56 registers in CTAs of up to 288 threads, 36 warps per SM instead of 24 (RMS,
+// LAYERNORM and SWIGLU: 64 registers, 256 threads, 32 warps); the kernel is bound by issue slots that too few warps fill (59 %
+// busy). DiT block on 4352 x 3072 (three of these kernels) 581 us -> 566, W6A8 block on 2048 x 5120 601 -> 585. f32 rows other than the packers' and SITU would spill and keep the general form.
+template <typename T, int PRO> __host__ __device__ constexpr int direct_threads() {
+    if (sizeof(T) == 4) return PRO == PRO_PLAIN ? 288 : 0;
+    return PRO == PRO_SITU ? 0 : PRO == PRO_RMS || PRO == PRO_LAYERNORM || PRO == PRO_SWIGLU ? 256 : 288;
+}
+template <typename T, int PRO, int MAXT, bool DIRECT = false>
+__global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_rows_kernel(const QuantArgs p) {
+    const bool staged = !DIRECT && p.staged, rotate = DIRECT || p.rotate;
     extern __shared__ __align__(128) uint8_t smem[];
     const uint16_t* lut = g_act_lut[p.lut >= 0 ? p.lut : 0];
     const unsigned wmask = __activemask();            // the last warp of a CTA may be partial (threads = rows * K / 32)
@@ -225,7 +234,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
 
     pdl_trigger();
     for (int i = threadIdx.x; i < 3 * p.rows_per_cta; i += blockDim.x) amax_s[i] = 0u;
-    if (p.staged && threadIdx.x == 0) {
+    if (staged && threadIdx.x == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
     }
@@ -249,7 +258,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
             }
         }
     };
-    if (p.staged && (int)blockIdx.x < p.nblocks) issue_block(blockIdx.x);
+    if (staged && (int)blockIdx.x < p.nblocks) issue_block(blockIdx.x);
 
     const int tpr = p.tpr;
     const int rloc = threadIdx.x / tpr;               // row inside the CTA
@@ -257,13 +266,13 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
     const int grp = tin >> 3, t8 = tin & 7;
     const int col = (grp << 8) + (t8 << 5);
     int it = 0;
-    for (int blk = blockIdx.x; blk < p.nblocks; blk += gridDim.x, ++it) {
+    for (int blk = blockIdx.x; blk < p.nblocks; blk += DIRECT ? p.nblocks : (int)gridDim.x, ++it) {
         const int64_t m_raw = (int64_t)blk * p.rows_per_cta + rloc;
         const bool live = m_raw < p.M;
         const int64_t m = live ? m_raw : p.M - 1;      // idle rows compute on the last row (or on stale staging) and store nothing
 
         float v[32], u[32];
-        if (p.staged) {
+        if (staged) {
             // bounded wait for this block's bytes; on expiry the CTA records the fact and leaves
             bool ok = mbar_try_wait(bar, it & 1);
             if (!ok) {
@@ -403,7 +412,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
         }
 
         float2 P[16];
-        if (p.rotate) {
+        if (rotate) {
             // stages 0, 1 on the lane's two runs of 16, packed as (element i, element i + 16)
 #pragma unroll
             for (int i = 0; i < 16; ++i) P[i] = make_float2(v[i], v[i + 16]);
@@ -427,7 +436,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
             for (int i = 0; i < 16; ++i) P[i] = make_float2(v[2 * i], v[2 * i + 1]);   // natural order
         }
 
-        if (p.out_hi) {  // the weight-only linear's activation side: rotated rows split into two bf16 terms
+        if (!DIRECT && p.out_hi) {  // the weight-only linear's activation side: rotated rows split into two bf16 terms
             if (live) {
                 const int64_t o = m * (int64_t)p.K + (grp << 8) + 2 * t8;
 #pragma unroll
@@ -441,7 +450,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
             }
             continue;
         }
-        if (p.out_f) {   // gpu_rotate_rows_f32: always rotated, so P holds (2 t8, 2 t8 + 1) + 16 r
+        if (!DIRECT && p.out_f) {   // gpu_rotate_rows_f32: always rotated, so P holds (2 t8, 2 t8 + 1) + 16 r
             if (live) {
                 float* o = p.out_f + m * (int64_t)p.K + (grp << 8) + 2 * t8;
 #pragma unroll
@@ -469,12 +478,12 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
         if (t8 == 0) atomicMax(slot, __float_as_uint(amax));
         __syncthreads();
         amax = __uint_as_float(*slot);
-        amax_s[((it + 2) % 3) * p.rows_per_cta + rloc] = 0u;   // next use is two barriers away, last use one barrier back
-        if (p.amax_out) {
+        if (!DIRECT) amax_s[((it + 2) % 3) * p.rows_per_cta + rloc] = 0u;   // next use is two barriers away, last use one barrier back
+        if (!DIRECT && p.amax_out) {
             if (live && tin == 0) p.amax_out[m] = amax;
             continue;
         }
-        if (p.amax_in) amax = p.amax_in[m];
+        if (!DIRECT && p.amax_in) amax = p.amax_in[m];
 
         const float scale = fmaxf(fminf(amax, finite_max<T>()) * (1.f / 127.f), 1.0e-30f);
         if (live && tin == 0) p.scales[m] = scale;
@@ -491,7 +500,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(c
             for (int i = 0; i < 16; ++i) c16[i] = quant2<T>(P[i], st, rcp, false);
         }
         int8_t* q = p.q + m * (int64_t)p.K + col;
-        if (p.rotate) {
+        if (rotate) {
             // codes of (2 t8, 2 t8 + 1) + 16 r back through the group's buffer, so each lane stores 32 contiguous bytes
             uint16_t* cb = reinterpret_cast<uint16_t*>(tbuf);
             const uint32_t order = tsw ? 0x3201u : 0x3210u;   // a swapping team puts its two codes back in element order
@@ -1008,9 +1017,9 @@ struct OccCache {
     size_t smem[8] = {};
 };
 
-template <typename T, int PRO, int MAXT>
+template <typename T, int PRO, int MAXT, bool DIRECT = false>
 int launch_cfg(QuantArgs& p, int threads, size_t smem, bool persistent, cudaStream_t st) {
-    auto kern = quant_rows_kernel<T, PRO, MAXT>;
+    auto kern = quant_rows_kernel<T, PRO, MAXT, DIRECT>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1092,6 +1101,10 @@ int launch_quant(QuantArgs& p, cudaStream_t st) {
     p.staged = !p.rotate && !is_norm<PRO>() && off + stage_bytes <= kMaxSmem;
     const size_t smem = p.staged ? off + stage_bytes : off;
     if (smem > kMaxSmem) return -2;
+    if constexpr (direct_threads<T, PRO>() > 0) {
+        if (p.rotate && threads <= direct_threads<T, PRO>() && !p.out_f && !p.out_hi && !p.amax_in && !p.amax_out)
+            return launch_cfg<T, PRO, direct_threads<T, PRO>(), true>(p, threads, smem, false, st);
+    }
     if (threads > 512) return launch_cfg<T, PRO, 1024>(p, threads, smem, p.staged != 0, st);
     if (threads > 384) return launch_cfg<T, PRO, 512>(p, threads, smem, p.staged != 0, st);
     return launch_cfg<T, PRO, 384>(p, threads, smem, p.staged != 0, st);
