@@ -51,3 +51,17 @@ def test_half_division_by_refined_reciprocal_for_every_significand_pair():
         ieee = (a.astype(np.float32) / S.astype(np.float32)).astype(np.float32)
         assert np.array_equal(t.astype(np.float16), ieee.astype(np.float16)), e
         assert np.array_equal(ieee.astype(np.float16), (a / S).astype(np.float16)), e
+
+
+def test_one_plus_scale_rounds_once_or_twice_to_the_same_bf16():
+    """LayerNorm's modulation factor: bf16(f32(1 + s)), as the reference has it, equals the sum rounded once (a bf16 addition),
+    for every finite bf16 s."""
+    bits = (np.arange(65536, dtype=np.uint32) << 16).view(np.float32)
+    s = bits[np.isfinite(bits)].astype(np.float64)
+
+    def to8(x):                              # nearest-even to eight significant bits
+        m, e = np.frexp(x)
+        return np.ldexp(np.rint(m * 256.0), e - 8)
+
+    exact = 1.0 + s                          # in double: inexact only where s is below 2^-45 or above 2^45, far from any tie
+    assert np.array_equal(to8(exact), to8(exact.astype(np.float32).astype(np.float64)))
