@@ -31,7 +31,10 @@ typedef __nv_bfloat16 bf16;
 //   - pdl_wait(), before the first access to memory that another kernel reads or writes: everything launched before in the
 //     stream has ended and its writes are visible. Every thread that touches such memory waits, so an order that held
 //     between whole kernels (results, buffers used again, the zeros of the split scratch) holds as before.
-// A successor launched the ordinary way waits for the end of the grid as always.
+// A successor launched the ordinary way waits for the end of the grid as always. While a cluster limit keeps SMs free for another
+// stream's kernels (gpu_int8_gemm_set_cluster_limit), every launch is the ordinary way: a successor waiting on the free SMs would
+// take the very room the limit keeps.
+namespace b200q { int gemm_cluster_limit(); }      // gemm_i8.cu
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... P, typename... A>
@@ -43,7 +46,8 @@ inline int launch_pdl_cluster(void (*kern)(P...), dim3 grid, unsigned threads, s
     at[0].val.programmaticStreamSerializationAllowed = 1;
     at[1].id = cudaLaunchAttributeClusterDimension;
     at[1].val.clusterDim.x = (unsigned)cluster, at[1].val.clusterDim.y = 1, at[1].val.clusterDim.z = 1;
-    cfg.attrs = at, cfg.numAttrs = cluster > 1 ? 2 : 1;
+    const int first = b200q::gemm_cluster_limit() > 0 ? 1 : 0;      // 1: without the first attribute
+    cfg.attrs = at + first, cfg.numAttrs = (cluster > 1 ? 2 : 1) - first;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
     if (e != cudaSuccess) (void)cudaGetLastError();
     return (int)e;

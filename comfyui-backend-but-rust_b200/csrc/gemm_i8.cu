@@ -1837,6 +1837,8 @@ GPU_API int gpu_int8_gemm_noalloc(const int8_t* A, const int8_t* W, const float*
 }
 
 
+int b200q::gemm_cluster_limit() { return g_cluster_limit.load(std::memory_order_relaxed); }
+
 // New (tensor parallelism): the persistent GEMM normally takes every SM pair of the device, and a collective's kernels
 // launched beside it on another stream then wait for it to end. A limit of n > 0 makes gpu_int8_gemm* launches that follow
 // (any thread, any device of the process) occupy at most n CTA pairs, leaving the other SMs to concurrent kernels;
