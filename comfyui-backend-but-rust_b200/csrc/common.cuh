@@ -31,12 +31,17 @@ typedef __nv_bfloat16 bf16;
 //   - pdl_wait(), before the first access to memory that another kernel reads or writes: everything launched before in the
 //     stream has ended and its writes are visible. Every thread that touches such memory waits, so an order that held
 //     between whole kernels (results, buffers used again, the zeros of the split scratch) holds as before.
+// Such memory may change while the kernel is resident, so it is not read-only for the kernel's duration: no __ldg and no
+// __restrict__ on what a kernel with a wait reads or writes. Both allow loads through the read-only path, which PTX defines only for
+// memory nothing writes meanwhile and which the compiler may move ahead of the wait; gload() is an ordinary load, which the wait's
+// memory clobber holds back.
 // A successor launched the ordinary way waits for the end of the grid as always. While a cluster limit keeps SMs free for another
 // stream's kernels (gpu_int8_gemm_set_cluster_limit), every launch is the ordinary way: a successor waiting on the free SMs would
 // take the very room the limit keeps.
 namespace b200q { int gemm_cluster_limit(); }      // gemm_i8.cu
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename T> __device__ __forceinline__ T gload(const T* p) { return *p; }
 template <typename... P, typename... A>
 inline int launch_pdl_cluster(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, int cluster, const A&... args) {
     cudaLaunchConfig_t cfg = {};

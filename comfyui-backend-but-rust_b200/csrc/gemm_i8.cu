@@ -248,7 +248,7 @@ __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r
             // (a predicated load; the shared-memory index is masked into range either way)
             const uint32_t bits = __float_as_uint(v) >> 16;
             uint32_t t = lut_sm[act_lut_index(bits)];                                   // sign bit 15 -> the table's second half
-            if (((bits & 0x7fffu) - kActLutLo) >= kActLutHalf) t = __ldg(p.act_lut + bits);
+            if (((bits & 0x7fffu) - kActLutLo) >= kActLutHalf) t = gload(p.act_lut + bits);
             v = __uint_as_float(t << 16);
         } else if (EPI == EPI_ACT) {
             v = p.act == ACT_GELU_TANH ? gelu_tanh_f(v) : p.act == ACT_SILU ? silu_f(v) : gelu_f(v);
@@ -263,11 +263,11 @@ __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r
 // no conversion back and forth. Values outside the shared-memory part (checked once per 8) are read from the whole table.
 // Out of line on purpose: inlined, its eight loads were issued (predicated off) by every group of eight and cost the
 // epilogue a tenth of its instructions.
-__device__ __noinline__ uint4 act_lut_whole8(const uint16_t* __restrict__ lut, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
+__device__ __noinline__ uint4 act_lut_whole8(const uint16_t* lut, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
     const uint32_t w[4] = {w0, w1, w2, w3};
     uint32_t o[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o[i] = (uint32_t)__ldg(lut + (w[i] & 0xffffu)) | ((uint32_t)__ldg(lut + (w[i] >> 16)) << 16);
+    for (int i = 0; i < 4; ++i) o[i] = (uint32_t)gload(lut + (w[i] & 0xffffu)) | ((uint32_t)gload(lut + (w[i] >> 16)) << 16);
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 // t[e] = table entry (16 bits) for column e. Returns false when some entry came from the whole table (values outside the
@@ -532,11 +532,11 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
         int tm, tn;
         tile_coords(w, p.tiles_m, p.tiles_n, tm, tn, p.group_m ? p.group_m : 8);
         const int row = tm * (2 * BM) + rank * BM + quad * 32 + lane;
-        nx_xs = p.xs ? __ldg(p.xs + (row < p.M ? row : p.M - 1)) : 1.f;
+        nx_xs = p.xs ? gload(p.xs + (row < p.M ? row : p.M - 1)) : 1.f;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int n = tn * 256 + (4 * half + k) * 32 + lane;
-            nx_ws[k] = __ldg(p.ws + n);
+            nx_ws[k] = gload(p.ws + n);
             nx_b[k] = bias ? __bfloat162float(bias[n]) : 0.f;
         }
     };
@@ -758,7 +758,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (warp >= 2) {
             uint16_t* dst = reinterpret_cast<uint16_t*>(staging + kVecOffset + kEpiWarps * 1024);
             for (uint32_t i = threadIdx.x - 64; i < 2 * kActLutHalf; i += blockDim.x - 64)
-                dst[i] = __ldg(p.act_lut + act_lut_pattern(i));
+                dst[i] = gload(p.act_lut + act_lut_pattern(i));
         }
     }
     tc_fence_before();
@@ -1582,12 +1582,12 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
 // output of the first, W was read and D written twice: the MLP of a text encoder layer (512 rows, 2560, FFN 9728) took 301 us,
 // now 252 (271 with tiles of at most 128 columns, whose accumulators fit the tensor memory twice: what the narrower tiles read
 // from L2 costs more than the epilogue that wider ones leave uncovered).
-__global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* __restrict__ q, bf16* __restrict__ out, int64_t n16) {
+__global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* q, bf16* out, int64_t n16) {
     pdl_trigger();
     pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n16) return;
-    const uint4 v = __ldg(reinterpret_cast<const uint4*>(q) + i);
+    const uint4 v = gload(reinterpret_cast<const uint4*>(q) + i);
     const int8_t* b = reinterpret_cast<const int8_t*>(&v);
     __nv_bfloat162 o[8];
 #pragma unroll

@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_gemm_kernel(const SkinnyPa
     pdl_wait();
     const int K = p.K;
     for (int i = threadIdx.x; i < p.M * K / 16; i += blockDim.x)
-        reinterpret_cast<uint4*>(a_s)[i] = __ldg(reinterpret_cast<const uint4*>(p.A) + i);
+        reinterpret_cast<uint4*>(a_s)[i] = gload(reinterpret_cast<const uint4*>(p.A) + i);
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nblocks = (p.N + kRowsPerWarp - 1) / kRowsPerWarp;
@@ -40,7 +40,7 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_gemm_kernel(const SkinnyPa
                 for (int r = 0; r < kRowsPerWarp; ++r) {
                     const int n = min(n0 + r, p.N - 1);   // rows past N repeat the last row; their results are dropped
                     const int k0 = kb + 512 * u;
-                    w[u][r] = k0 < K ? __ldg(reinterpret_cast<const uint4*>(p.W + (int64_t)n * K + k0)) : make_uint4(0, 0, 0, 0);
+                    w[u][r] = k0 < K ? gload(reinterpret_cast<const uint4*>(p.W + (int64_t)n * K + k0)) : make_uint4(0, 0, 0, 0);
                 }
 #pragma unroll
             for (int u = 0; u < kAhead; ++u) {

@@ -206,13 +206,13 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = make_uint4(0, 0, 0, 0);
             auto fetch = [&](int kb4) -> uint4 {     // scales of boxes 4*kb4 .. 4*kb4+3
                 uint4 v = make_uint4(0x38383838u, 0x38383838u, 0x38383838u, 0x38383838u);
-                if (wide && 4 * kb4 + 4 <= p.k_iters) return __ldg(reinterpret_cast<const uint4*>(srow) + kb4);
+                if (wide && 4 * kb4 + 4 <= p.k_iters) return gload(reinterpret_cast<const uint4*>(srow) + kb4);
                 const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
                 const int left = p.k_iters - 4 * kb4;
-                if (left > 0) v.x = __ldg(s32);
-                if (left > 1) v.y = __ldg(s32 + 1);
-                if (left > 2) v.z = __ldg(s32 + 2);
-                if (left > 3) v.w = __ldg(s32 + 3);
+                if (left > 0) v.x = gload(s32);
+                if (left > 1) v.y = gload(s32 + 1);
+                if (left > 2) v.z = gload(s32 + 2);
+                if (left > 3) v.w = gload(s32 + 3);
                 return v;
             };
             sc_next = fetch(0);
@@ -465,14 +465,14 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const uint8_t* srow = x6.s_rel + (size_t)min(n0 + r, p.N - 1) * x6.srel_pitch;
         const bool wide = (x6.srel_pitch & 15) == 0 && ((uintptr_t)x6.s_rel & 15) == 0;   // scale rows readable 16 bytes at a time
         auto fetch = [&](int kb4) -> uint4 {                       // scales of boxes 4 kb4 .. 4 kb4 + 3
-            if (wide) return __ldg(reinterpret_cast<const uint4*>(srow) + kb4);
+            if (wide) return gload(reinterpret_cast<const uint4*>(srow) + kb4);
             uint4 v = make_uint4(0, 0, 0, 0);
             const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
             const int left = p.k_iters - 4 * kb4;
-            if (left > 0) v.x = __ldg(s32);
-            if (left > 1) v.y = __ldg(s32 + 1);
-            if (left > 2) v.z = __ldg(s32 + 2);
-            if (left > 3) v.w = __ldg(s32 + 3);
+            if (left > 0) v.x = gload(s32);
+            if (left > 1) v.y = gload(s32 + 1);
+            if (left > 2) v.z = gload(s32 + 2);
+            if (left > 3) v.w = gload(s32 + 3);
             return v;
         };
         const int sw_lo = (r >> 1) & 3, sw_hi = (r >> 2) & 1, sw_out = r & 7;

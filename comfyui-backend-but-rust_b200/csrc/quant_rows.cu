@@ -115,25 +115,25 @@ __device__ __forceinline__ float2 bf16x2_f(const __nv_bfloat162 h) {
     const uint32_t w = *reinterpret_cast<const uint32_t*>(&h);
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
-// 32 consecutive elements -> floats, from global memory (read-only path) or from the staging buffer
+// 32 consecutive elements -> floats, from global memory or from the staging buffer
 template <typename T, bool SMEM> __device__ __forceinline__ void load32(const T* p, float (&v)[32]) {
     if constexpr (sizeof(T) == 2) {
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const uint4 u = SMEM ? reinterpret_cast<const uint4*>(p)[c] : __ldg(reinterpret_cast<const uint4*>(p) + c);
+            const uint4 u = SMEM ? reinterpret_cast<const uint4*>(p)[c] : gload(reinterpret_cast<const uint4*>(p) + c);
             unpack_bf16x8(u, v + 8 * c);
         }
     } else {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
-            const float4 a = SMEM ? reinterpret_cast<const float4*>(p)[c] : __ldg(reinterpret_cast<const float4*>(p) + c);
+            const float4 a = SMEM ? reinterpret_cast<const float4*>(p)[c] : gload(reinterpret_cast<const float4*>(p) + c);
             v[4 * c] = a.x, v[4 * c + 1] = a.y, v[4 * c + 2] = a.z, v[4 * c + 3] = a.w;
         }
     }
 }
 
 __device__ __forceinline__ float lut_f(const uint16_t* lut, float x) {   // x holds a bf16 value; whole table, global
-    return __uint_as_float((uint32_t)__ldg(lut + (__float_as_uint(x) >> 16)) << 16);
+    return __uint_as_float((uint32_t)gload(lut + (__float_as_uint(x) >> 16)) << 16);
 }
 // Codes of two values: q = sat8(rint(T(T(v) / T(scale)))).
 // bf16 fast path. Both operands of the division carry 8 significant bits: a = A 2^i, st = S 2^j with integers
@@ -173,11 +173,11 @@ __device__ __forceinline__ uint32_t quant2(float2 v, float st, float rcp, bool f
 
 // 8 consecutive per-column values as floats
 __device__ __forceinline__ void load8v(const float* p, float (&v)[8]) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    const float4 a = gload(reinterpret_cast<const float4*>(p)), b = gload(reinterpret_cast<const float4*>(p) + 1);
     v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
 }
 __device__ __forceinline__ void load8v(const bf16* p, float (&v)[8]) {
-    unpack_bf16x8(__ldg(reinterpret_cast<const uint4*>(p)), v);
+    unpack_bf16x8(gload(reinterpret_cast<const uint4*>(p)), v);
 }
 
 // The reference's soft-capped gated activation (csrc/common.cuh:73-91), operation for operation.
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
                 for (int c = 0; c < 4; ++c) {
                     uint4 mw = make_uint4(0, 0, 0, 0), sw = mw;
                     float nw[8];
-                    if (PRO == PRO_LN_MOD) mw = __ldg(reinterpret_cast<const uint4*>(ms_p + col + 8 * c)), sw = __ldg(reinterpret_cast<const uint4*>(sh_p + col + 8 * c));
+                    if (PRO == PRO_LN_MOD) mw = gload(reinterpret_cast<const uint4*>(ms_p + col + 8 * c)), sw = gload(reinterpret_cast<const uint4*>(sh_p + col + 8 * c));
                     else if (p.norm_w) load8v(p.norm_w + col + 8 * c, nw);
                     const uint32_t m4[4] = {mw.x, mw.y, mw.z, mw.w}, s4[4] = {sw.x, sw.y, sw.z, sw.w};
 #pragma unroll
@@ -634,7 +634,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
         // the rows as they lie first, all of them in flight together
         for (SdPieces i(pieces); i.r < live_rows; i.next()) {
             const int r = i.r, c = i.c;
-            row_s[r * pitch + sd_piece(c)] = __ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * s.x_stride) + c);
+            row_s[r * pitch + sd_piece(c)] = gload(reinterpret_cast<const uint4*>(s.x + (m0 + r) * s.x_stride) + c);
         }
         __syncthreads();
         if (warp < nwarps)       // whole warps only
@@ -683,7 +683,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
         for (SdPieces i(pieces); i.r < live_rows; i.next()) {
             const int r = i.r, c = i.c;
             float e[8], w[8], b[8];
-            unpack_half8(__ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)K) + c), e);
+            unpack_half8(gload(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)K) + c), e);
             load8v(s.w + 8 * c, w), load8v(s.b + 8 * c, b);
             int g = (8 * c) / per, left = per - (8 * c - g * per);      // values of the group from here on
             float2 st = stat[g];
@@ -700,7 +700,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
             const int r = i.r, c = i.c;
             const uint4* in = reinterpret_cast<const uint4*>(s.x + (m0 + r) * 2 * (int64_t)K);
             float e[8], g[8];
-            unpack_half8(__ldg(in + c), e), unpack_half8(__ldg(in + pieces + c), g);
+            unpack_half8(gload(in + c), e), unpack_half8(gload(in + pieces + c), g);
 #pragma unroll
             for (int j = 0; j < 8; ++j) e[j] = __fmul_rn(e[j], rnd<half>(gelu_f(g[j])));
             row_s[r * pitch + sd_piece(c)] = pack_half8(e);
@@ -709,7 +709,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
         for (SdPieces i(pieces); i.r < live_rows; i.next()) {
             const int r = i.r, c = i.c, h = (8 * c) / s.d;      // d % 8 == 0: a piece lies inside one head
             row_s[r * pitch + sd_piece(c)] =
-                __ldg(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)s.heads * s.dp + (int64_t)h * s.dp + (8 * c - h * s.d)));
+                gload(reinterpret_cast<const uint4*>(s.x + (m0 + r) * (int64_t)s.heads * s.dp + (int64_t)h * s.dp + (8 * c - h * s.d)));
         }
     }
 }
@@ -719,7 +719,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
 // U-Net block of width 640 (eight of these kernels): 328 us with 63 registers, halvings in every stage and a division per piece, 321 now.
 constexpr int kSdThreads = 288;
 template <int ROT, int SRC, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fast_kernel(const SdSrc s, int8_t* __restrict__ q, float* __restrict__ scales, int M,
+__global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fast_kernel(const SdSrc s, int8_t* q, float* scales, int M,
                                                             int K, int tpr, int rows, uint32_t off_amax, uint32_t off_rows) {
     extern __shared__ __align__(128) uint8_t smem[];
     const unsigned wmask = __activemask();
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
         __syncthreads();
         const uint4* r = reinterpret_cast<const uint4*>(s.x + m * s.x_stride) + 4 * tin;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) unpack_half8(__ldg(r + c), *reinterpret_cast<float(*)[8]>(v + 8 * c));
+        for (int c = 0; c < 4; ++c) unpack_half8(gload(r + c), *reinterpret_cast<float(*)[8]>(v + 8 * c));
     } else {
         uint4* row_s = reinterpret_cast<uint4*>(smem + off_rows);
         const int pitch = ((K >> 3) + 7) & ~7;
@@ -1256,8 +1256,8 @@ GPU_API int gpu_quant_rows_scaled(int dtype, int prologue, const void* x, int64_
 // step.
 namespace {
 constexpr int kRotRows = 8;
-__global__ void __launch_bounds__(512) quant_rotated_kernel(const bf16* __restrict__ xr, const float* __restrict__ parts,
-                                                            int8_t* __restrict__ q, float* __restrict__ scales, int M, int K,
+__global__ void __launch_bounds__(512) quant_rotated_kernel(const bf16* xr, const float* parts,
+                                                            int8_t* q, float* scales, int M, int K,
                                                             int P, int wpr) {
     __shared__ unsigned s_amax[kRotRows], s_flag[kRotRows];
     pdl_trigger();
@@ -1275,14 +1275,14 @@ __global__ void __launch_bounds__(512) quant_rotated_kernel(const bf16* __restri
     uint4 a0, b0, a1, b1;
     a0 = b0 = a1 = b1 = make_uint4(0, 0, 0, 0);
     const int e0 = lane * 16;
-    if (live && e0 < per) a0 = __ldg(reinterpret_cast<const uint4*>(src + e0)), b0 = __ldg(reinterpret_cast<const uint4*>(src + e0 + 8));
-    if (live && e0 + 512 < per) a1 = __ldg(reinterpret_cast<const uint4*>(src + e0 + 512)), b1 = __ldg(reinterpret_cast<const uint4*>(src + e0 + 520));
+    if (live && e0 < per) a0 = gload(reinterpret_cast<const uint4*>(src + e0)), b0 = gload(reinterpret_cast<const uint4*>(src + e0 + 8));
+    if (live && e0 + 512 < per) a1 = gload(reinterpret_cast<const uint4*>(src + e0 + 512)), b1 = gload(reinterpret_cast<const uint4*>(src + e0 + 520));
     __syncthreads();
     // the 8 rows' partial maxima, 8 consecutive floats per part; non-negative floats order as integers
     for (int i = threadIdx.x; i < P * kRotRows; i += blockDim.x) {
         const int r = i & (kRotRows - 1);
         if (m0 + r < M) {
-            const uint32_t u = __float_as_uint(__ldg(parts + (int64_t)(i >> 3) * M + m0 + r));
+            const uint32_t u = __float_as_uint(gload(parts + (int64_t)(i >> 3) * M + m0 + r));
             atomicMax(&s_amax[r], u & 0x7fffffffu);
             if (u & 0x80000000u) s_flag[r] = 1u;
         }
@@ -1315,11 +1315,11 @@ __global__ void __launch_bounds__(512) quant_rotated_kernel(const bf16* __restri
 #pragma unroll 1
     for (int e = e0; e < per; e += 1024) {
         uint4 a = a0, b = b0;
-        if (e + 1024 < per) a0 = __ldg(reinterpret_cast<const uint4*>(src + e + 1024)), b0 = __ldg(reinterpret_cast<const uint4*>(src + e + 1032));
+        if (e + 1024 < per) a0 = gload(reinterpret_cast<const uint4*>(src + e + 1024)), b0 = gload(reinterpret_cast<const uint4*>(src + e + 1032));
         convert(a, b, e);
         if (e + 512 < per) {
             a = a1, b = b1;
-            if (e + 1536 < per) a1 = __ldg(reinterpret_cast<const uint4*>(src + e + 1536)), b1 = __ldg(reinterpret_cast<const uint4*>(src + e + 1544));
+            if (e + 1536 < per) a1 = gload(reinterpret_cast<const uint4*>(src + e + 1536)), b1 = gload(reinterpret_cast<const uint4*>(src + e + 1544));
             convert(a, b, e + 512);
         }
     }

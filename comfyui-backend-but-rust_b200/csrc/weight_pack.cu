@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(256) sd_quant_rows_kernel(const half* __restri
     const half* r = x + m * x_stride;
     if (vec) {
         for (int c = threadIdx.x; c < K / 8; c += blockDim.x) {
-            const uint4 u = __ldg(reinterpret_cast<const uint4*>(r) + c);
+            const uint4 u = gload(reinterpret_cast<const uint4*>(r) + c);
             const __half2* h = reinterpret_cast<const __half2*>(&u);
             float* d = row + pad(c * 8);
 #pragma unroll
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
     const half* r = x + m * x_stride + tin * 16;
     float v[16];
     {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(r)), b = __ldg(reinterpret_cast<const uint4*>(r) + 1);
+        const uint4 a = gload(reinterpret_cast<const uint4*>(r)), b = gload(reinterpret_cast<const uint4*>(r) + 1);
         const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
 // GroupNorm statistics of x [N, P, C] half: per (image, group) the sum and the sum of squares, accumulated in double
 // from per-block float sums as the reference's sd_group_sums_kernel forms them (csrc/sd.cu:209-233: 256 threads, thread
 // t takes values t, t + 256, ... of the block's pixel range, then the block tree), so the statistics come out the same.
-__global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* __restrict__ x, double* __restrict__ sums, int64_t P,
+__global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* x, double* sums, int64_t P,
                                                             int C, int G, int splits) {
     __shared__ float red[33];
     pdl_trigger();
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(512) convrot_requant_kernel(const T* __restric
 template <typename T> __device__ __forceinline__ void load_row32(const T* p, float (&v)[32]) {
 #pragma unroll
     for (int c = 0; c < 32 * (int)sizeof(T) / 16; ++c) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + c);
+        const uint4 u = gload(reinterpret_cast<const uint4*>(p) + c);
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -377,7 +377,7 @@ template <typename T> __device__ __forceinline__ void load_row32(const T* p, flo
     }
 }
 template <typename T>
-__global__ void __launch_bounds__(512) convrot_requant_regs_kernel(const T* __restrict__ x, int8_t* __restrict__ q, float* __restrict__ scales,
+__global__ void __launch_bounds__(512) convrot_requant_regs_kernel(const T* x, int8_t* q, float* scales,
                                                                    int64_t N, int K, int rows, uint64_t seed) {
     extern __shared__ __align__(128) float smem_f[];
     const unsigned wmask = __activemask();               // the last warp may be partial
@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(512) convrot_requant_regs_kernel(const T* __re
 // groups of all rows are simply dealt out. The kernel below, which walks a row in shared memory, took 53 us for 5120 x 5120 to
 // bf16 (79 MB moved) and stays for buffers that are not 16-byte aligned.
 template <typename T, bool ROUND_BF16>
-__global__ void __launch_bounds__(256) convrot_dequant_regs_kernel(const int8_t* __restrict__ q, const float* __restrict__ s, T* __restrict__ out,
+__global__ void __launch_bounds__(256) convrot_dequant_regs_kernel(const int8_t* q, const float* s, T* out,
                                                                    int64_t groups, int groups_per_row) {
     __shared__ __align__(128) float smem_f[8 * kWarpWords];
     pdl_trigger();
@@ -462,12 +462,12 @@ __global__ void __launch_bounds__(256) convrot_dequant_regs_kernel(const int8_t*
     const int64_t g_raw = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
     const bool live = g_raw < groups;
     const int64_t g = live ? g_raw : groups - 1;
-    const float sc = __ldg(s + g / groups_per_row);
+    const float sc = gload(s + g / groups_per_row);
     const uint4* src = reinterpret_cast<const uint4*>(q + g * 256 + 32 * l.t8);
     float v[32];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        const uint4 u = __ldg(src + c);
+        const uint4 u = gload(src + c);
         const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -533,8 +533,8 @@ __global__ void __launch_bounds__(256) w6_decode_kernel(const uint8_t* __restric
     const int64_t n = i / per;
     const int c = (int)(i - n * per);
     const uint8_t* row = q + n * (int64_t)(K / 4 * 3);
-    const uint2 lo = __ldg(reinterpret_cast<const uint2*>(row + c * 8));
-    const uint32_t hi = __ldg(reinterpret_cast<const uint32_t*>(row + K / 2 + c * 4));
+    const uint2 lo = gload(reinterpret_cast<const uint2*>(row + c * 8));
+    const uint32_t hi = gload(reinterpret_cast<const uint32_t*>(row + K / 2 + c * 4));
     const float sc = e4m3_to_f(s_rel[n * (K / G) + c * 16 / G]);
     const uint32_t lw[2] = {lo.x, lo.y};
     uint32_t o[4];
@@ -653,8 +653,8 @@ __global__ void __launch_bounds__(256) w6_requant_kernel(const bf16* __restrict_
 __device__ __forceinline__ float rint_clamped(float x, float bound) {
     return __fsub_rn(__fadd_rn(fminf(bound, fmaxf(-bound, x)), 12582912.f), 12582912.f);
 }
-__global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* __restrict__ w, uint8_t* __restrict__ packed, uint8_t* __restrict__ s_rel,
-                                                              float* __restrict__ s_channel, int64_t N, int K, int rows, uint64_t seed) {
+__global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* w, uint8_t* packed, uint8_t* s_rel,
+                                                              float* s_channel, int64_t N, int K, int rows, uint64_t seed) {
     extern __shared__ __align__(128) float smem_f[];
     const unsigned wmask = __activemask();               // the last warp may be partial
     const RotLane l = rot_lane(smem_f);
@@ -743,8 +743,8 @@ __global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* __rest
 // The same with 32 codes (one whole scale group when G is a multiple of 32) per thread and the permute-table decode of
 // w6_decode.cuh: 16 + 8 bytes in, 32 bytes out per thread. The decode form is voted per warp, so every lane takes part
 // (lanes past the end redo the last piece and store nothing).
-__global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* __restrict__ q, const uint8_t* __restrict__ s_rel,
-                                                          int8_t* __restrict__ out, int64_t N, int K, int G) {
+__global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* q, const uint8_t* s_rel,
+                                                          int8_t* out, int64_t N, int K, int G) {
     pdl_trigger();
     pdl_wait();
     const int64_t per = K / 32;
@@ -755,8 +755,8 @@ __global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* __restr
     const int64_t n = i / per;
     const int c = (int)(i - n * per);
     const uint8_t* row = q + n * (int64_t)(K / 4 * 3);
-    const uint4 lo = __ldg(reinterpret_cast<const uint4*>(row + c * 16));
-    const uint2 hi = __ldg(reinterpret_cast<const uint2*>(row + K / 2 + c * 8));
+    const uint4 lo = gload(reinterpret_cast<const uint4*>(row + c * 16));
+    const uint2 hi = gload(reinterpret_cast<const uint2*>(row + K / 2 + c * 8));
     const uint32_t sb = s_rel[n * (K / G) + c * 32 / G];
     uint32_t o[8];
     w6_group(w6_mode(sb | 0x38383800u), lo, hi.x, hi.y, sb, o);
