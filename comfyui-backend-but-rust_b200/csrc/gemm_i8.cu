@@ -765,7 +765,6 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     __syncthreads();
     cluster_sync_all();   // the peer's barriers exist before anything signals them
     tc_fence_after();
-    pdl_trigger();
     pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
 
@@ -1106,7 +1105,6 @@ gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_trigger();
     pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
     const int tm = blockIdx.x % p.tiles_m, tn = blockIdx.x / p.tiles_m;
@@ -1583,11 +1581,11 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
 // now 252 (271 with tiles of at most 128 columns, whose accumulators fit the tensor memory twice: what the narrower tiles read
 // from L2 costs more than the epilogue that wider ones leave uncovered).
 __global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* q, bf16* out, int64_t n16) {
-    pdl_trigger();
     pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n16) return;
     const uint4 v = gload(reinterpret_cast<const uint4*>(q) + i);
+    pdl_trigger();
     const int8_t* b = reinterpret_cast<const int8_t*>(&v);
     __nv_bfloat162 o[8];
 #pragma unroll

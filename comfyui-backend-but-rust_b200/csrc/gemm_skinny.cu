@@ -14,7 +14,6 @@ constexpr int kRowsPerWarp = 4;
 template <typename OutT, int EPI, int MT>
 __global__ void __launch_bounds__(kWarps * 32) skinny_gemm_kernel(const SkinnyParams p) {
     extern __shared__ __align__(16) int8_t a_s[];   // [M][K]
-    pdl_trigger();
     pdl_wait();
     const int K = p.K;
     for (int i = threadIdx.x; i < p.M * K / 16; i += blockDim.x)

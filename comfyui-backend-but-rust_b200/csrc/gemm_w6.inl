@@ -110,7 +110,6 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     __syncthreads();
     cluster_sync_all();
     tc_fence_after();
-    pdl_trigger();
     pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
 
@@ -422,7 +421,6 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    pdl_trigger();
     pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
 

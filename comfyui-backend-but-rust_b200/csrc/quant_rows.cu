@@ -236,7 +236,6 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
     uint8_t* stage = smem + p.off_stage;              // [x rows | aux rows], one block of rows
     const uint32_t row_bytes = (uint32_t)p.K * sizeof(T);
 
-    pdl_trigger();
     for (int i = threadIdx.x; i < 3 * p.rows_per_cta; i += blockDim.x) amax_s[i] = 0u;
     if (staged && threadIdx.x == 0) {
         mbar_init(bar, 1);
@@ -515,6 +514,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
         if (t8 == 0) atomicMax(slot, __float_as_uint(amax));
         __syncthreads();
         amax = __uint_as_float(*slot);
+        if (DIRECT) pdl_trigger();
         if (!DIRECT) amax_s[((it + 2) % 3) * p.rows_per_cta + rloc] = 0u;   // next use is two barriers away, last use one barrier back
         if (!DIRECT && p.amax_out) {
             if (live && tin == 0) p.amax_out[m] = amax;
@@ -728,7 +728,6 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
     float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
     float* tbuf_w = tbuf - 2 * (team >> 1);
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem + off_amax);
-    pdl_trigger();
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
     pdl_wait();
     // rows of this CTA; GroupNorm's belong to one image (blockIdx.y), so that one set of statistics serves the CTA
@@ -817,6 +816,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
         atomicMax(amax_s + rloc, __float_as_uint(amax));
     }
     __syncthreads();
+    pdl_trigger();
     const float mx = __uint_as_float(amax_s[rloc]);
     const float scale = __fdiv_rn(fmaxf(mx, 1e-30f), 127.f);
     if (live && tin == 0) scales[m] = scale;
@@ -1260,7 +1260,6 @@ __global__ void __launch_bounds__(512) quant_rotated_kernel(const bf16* xr, cons
                                                             int8_t* q, float* scales, int M, int K,
                                                             int P, int wpr) {
     __shared__ unsigned s_amax[kRotRows], s_flag[kRotRows];
-    pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rloc = warp / wpr, seg = warp - rloc * wpr;

@@ -220,7 +220,6 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
 __global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* x, double* sums, int64_t P,
                                                             int C, int G, int splits) {
     __shared__ float red[33];
-    pdl_trigger();
     pdl_wait();
     const int ng = blockIdx.x, split = blockIdx.y;
     const int n = ng / G, g = ng % G, per = C / G;
@@ -384,7 +383,6 @@ __global__ void __launch_bounds__(512) convrot_requant_regs_kernel(const T* x, i
     const RotLane l = rot_lane(smem_f);
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem_f + ((blockDim.x + 31) >> 5) * kWarpWords);
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
-    pdl_trigger();
     pdl_wait();
     __syncthreads();
     const int tpr = K >> 5, rloc = threadIdx.x / tpr, tin = threadIdx.x - rloc * tpr;
@@ -456,7 +454,6 @@ template <typename T, bool ROUND_BF16>
 __global__ void __launch_bounds__(256) convrot_dequant_regs_kernel(const int8_t* q, const float* s, T* out,
                                                                    int64_t groups, int groups_per_row) {
     __shared__ __align__(128) float smem_f[8 * kWarpWords];
-    pdl_trigger();
     pdl_wait();
     const RotLane l = rot_lane(smem_f);
     const int64_t g_raw = (int64_t)blockIdx.x * 32 + (threadIdx.x >> 3);
@@ -660,7 +657,6 @@ __global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* w, uin
     const RotLane l = rot_lane(smem_f);
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem_f + ((blockDim.x + 31) >> 5) * kWarpWords);
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
-    pdl_trigger();
     pdl_wait();
     __syncthreads();
     const int tpr = K >> 5, rloc = threadIdx.x / tpr, g = threadIdx.x - rloc * tpr;      // thread g of a row has scale group g
@@ -745,7 +741,6 @@ __global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* w, uin
 // (lanes past the end redo the last piece and store nothing).
 __global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* q, const uint8_t* s_rel,
                                                           int8_t* out, int64_t N, int K, int G) {
-    pdl_trigger();
     pdl_wait();
     const int64_t per = K / 32;
     const int64_t total = N * per;
@@ -758,6 +753,7 @@ __global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* q, cons
     const uint4 lo = gload(reinterpret_cast<const uint4*>(row + c * 16));
     const uint2 hi = gload(reinterpret_cast<const uint2*>(row + K / 2 + c * 8));
     const uint32_t sb = s_rel[n * (K / G) + c * 32 / G];
+    pdl_trigger();
     uint32_t o[8];
     w6_group(w6_mode(sb | 0x38383800u), lo, hi.x, hi.y, sb, o);
     if (live) {

@@ -49,11 +49,21 @@ def _launched_early():
 def test_every_kernel_launched_early_waits():
     kernels, early = _kernels(), _launched_early()
     assert {"quant_rows_kernel", "gemm_i8_pair_kernel", "gemm_w6a8_rows_kernel", "skinny_gemm_kernel", "w6_requant_regs_kernel"} <= early
-    for name in early:
-        body = kernels[name][1]
-        assert "pdl_trigger()" in body and "pdl_wait()" in body, name
     for name, (_, body) in kernels.items():        # and nobody waits for a launch that is not of this kind
         assert ("pdl_wait()" in body) == (name in early), name
+
+
+def test_successors_are_let_in_only_when_a_kernel_is_nearly_done():
+    """A trigger at a kernel's start places the successor's CTAs beside the running kernel, on whatever SMs it leaves idle (a
+    small quantizer after a GEMM: all of it on twenty SMs). GEMMs leave the trigger to the end of their CTAs; where a kernel has
+    one, it comes after its wait and its loads."""
+    for name, (_, body) in _kernels().items():
+        if "pdl_trigger()" not in body:
+            continue
+        assert "gemm" not in name, name
+        at = body.index("pdl_trigger()")
+        assert body.index("pdl_wait()") < at and max(body.find("gload("), body.find("load32<")) < at, name
+        assert "gload(" in body[:at] or "load32<" in body[:at], name
 
 
 def test_no_read_only_loads_in_kernels_that_start_early():
