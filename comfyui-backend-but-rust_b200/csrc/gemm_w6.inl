@@ -633,18 +633,53 @@ int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensor
     return launch_pdl_cluster(kern, dim3(p.tiles_n * x6.splits), kW6RowsThreads, smem, st, x6.splits, ta, tlo, thi, p, x6);
 }
 
-int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, int sms, cudaStream_t st) {
+// Clusters of s CTAs of the kernel above that the current device holds at once: asked of the runtime once per device.
+constexpr int kW6RowsMaxSplits = 8;
+int w6_rows_clusters(int s) {
+    static int count[64][kW6RowsMaxSplits + 1];
+    static std::mutex mu;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    int* c = count[dev & 63];
+    if (c[0] == 0) {
+        auto kern = gemm_w6a8_rows_kernel<bf16, EPI_PLAIN>;
+        c[1] = device_sm_count(dev);
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess) {
+            for (int i = 2; i <= kW6RowsMaxSplits; ++i) {
+                cudaLaunchConfig_t cfg = {};
+                cfg.gridDim = dim3(i), cfg.blockDim = dim3(kW6RowsThreads), cfg.dynamicSmemBytes = kSmemBytes;
+                cudaLaunchAttribute at;
+                at.id = cudaLaunchAttributeClusterDimension;
+                at.val.clusterDim.x = (unsigned)i, at.val.clusterDim.y = 1, at.val.clusterDim.z = 1;
+                cfg.attrs = &at, cfg.numAttrs = 1;
+                if (cudaOccupancyMaxActiveClusters(&c[i], kern, &cfg) != cudaSuccess) c[i] = 0;
+            }
+        }
+        (void)cudaGetLastError();
+        c[0] = 1;
+    }
+    return c[s];
+}
+
+int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, cudaStream_t st) {
     const int64_t M = p.M, N = p.N, K = p.K;
     W6RowsParams x6{s_rel, (int)(K / 32), (int)((M + 15) / 16 * 16), 1, p.k_iters, 0, 0, 0};
     p.tiles_n = (int)((N + BM - 1) / BM);
     p.idesc = umma_idesc_i8(BM, x6.tokens);
-    // K slices: rounds of CTAs times (boxes of a slice + about a dozen boxes' worth of start and end)
+    // K slices: rounds of clusters times the cost of one, in K boxes. A CTA's rings take a whole SM and a cluster has to lie in
+    // one GPC, so the device holds fewer clusters than SMs / s (148, 74, 45, 33, 26, 22, 15, 15 of 1 to 8 CTAs); a second round
+    // costs as much as the first. Start, end and the tokens' share of the epilogue come to 8 + tokens / 32 boxes (a box: 0.56 us
+    // of expansion), the exchange of the accumulators to 3 more, and beyond four slices to tokens / 64: over 25 sizes of N and K
+    // (64 x 1024 to 20480 x 5120) at 16, 64, 128 and 256 tokens the slices chosen are within 3.5 % of the best of all eight.
     int64_t best = INT64_MAX;
-    for (int s = 1; s <= 8 && s <= p.k_iters; ++s) {
+    for (int s = 1; s <= kW6RowsMaxSplits && s <= p.k_iters; ++s) {
         const int kps = (p.k_iters + s - 1) / s;
         if ((p.k_iters + kps - 1) / kps != s) continue;                      // a slice would be empty
-        const int64_t rounds = ((int64_t)p.tiles_n * s + sms - 1) / sms;
-        const int64_t cost = rounds * (kps + 12) + (s > 1 ? 3 : 0);
+        const int room = w6_rows_clusters(s);
+        if (room < 1) continue;
+        const int64_t rounds = ((int64_t)p.tiles_n + room - 1) / room;
+        const int64_t cost = rounds * (64 * (kps + 8) + 2 * x6.tokens + (s > 1 ? 192 : 0) + (s > 4 ? x6.tokens : 0));   // 1/64 boxes
         if (cost < best) best = cost, x6.splits = s, x6.kps = kps;
     }
     const int a_bytes = (x6.tokens * BK + 1023) & ~1023;
@@ -696,7 +731,7 @@ int run_w6_gemm(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     p.act_lut = nullptr;
     const int esz = epi == EPI_ACC ? 4 : (out_dt == DT_F32 ? 4 : 2);
     p.k_iters = (int)(K / BK);
-    if (M <= kW6RowsMaxTokens) return run_w6_rows(epi, A, Wq6, s_rel, p, out_dt, device_sm_count(dev), st);
+    if (M <= kW6RowsMaxTokens) return run_w6_rows(epi, A, Wq6, s_rel, p, out_dt, st);
     auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     p.vec_ok = (N % 8 == 0) && al16(D) && al16(ws) && al16(bias) && al16(rscale) && al16(resid);
     p.tma_store = al16(D) && ((N * esz) % 16 == 0);
