@@ -45,9 +45,9 @@ constexpr int kW6BStages = 4;    // ring of expanded W tiles: only has to span u
 // CTA: MMAs have read A slot -> its packed slot is free too, the unpack that fed those MMAs being long done),
 // bfull (leader: 16 unpack-warp arrivals), bempty (per CTA: MMAs have read the expanded slot).
 // A tile has MH = 2 halves of 256 rows and 128 columns: an expanded W tile feeds two sets of MMAs (rows 0-255 and 256-511 of
-// the tile, two accumulators per buffer), so the unpack work per MMA halves. Up to 256 rows take the kernel further down.
-constexpr int MH = 2;
-template <typename OutT, int EPI>
+// the tile, two accumulators per buffer), so the unpack work per MMA halves. A weight narrower than 128 columns takes one half
+// and up to 128 columns (16896 x 64 x 1024: 11.0 us, 13.0 as two halves). Few rows take the kernel further down.
+template <typename OutT, int EPI, int MH>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kW6Threads, 1)
 gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_lo,
                       const __grid_constant__ CUtensorMap tmap_hi, const __grid_constant__ CUtensorMap tmap_d,
@@ -190,6 +190,7 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         // 64 rows per CTA: two threads per row, 64 elements each
         const int r = 32 * (uw & 1) + lane;                                   // row of the half tile
         const int hf = (uw >> 1) & 1;                                         // which 64 elements of the box
+        const bool has_row = MH == 2 || r < rows_w;                           // one half: tiles of 64 and 96 columns too
         const uint32_t bfull_leader = mapa_shared(bar_bfull, 0);
         const int sw_lo = (r >> 1) & 3, sw_hi = (r >> 2) & 1, sw_out = r & 7;
         const bool wide = (x6.srel_pitch & 15) == 0 && ((uintptr_t)x6.s_rel & 15) == 0;   // scale rows readable 16 bytes at a time
@@ -205,6 +206,7 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = make_uint4(0, 0, 0, 0);
             auto fetch = [&](int kb4) -> uint4 {     // scales of boxes 4*kb4 .. 4*kb4+3
                 uint4 v = make_uint4(0x38383838u, 0x38383838u, 0x38383838u, 0x38383838u);
+                if (!has_row) return v;
                 if (wide && 4 * kb4 + 4 <= p.k_iters) return gload(reinterpret_cast<const uint4*>(srow) + kb4);
                 const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
                 const int left = p.k_iters - 4 * kb4;
@@ -232,9 +234,10 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                     if (!__all_sync(0xffffffffu, mbar_try_wait(bar_pfull + 8 * sa, pa)) &&
                         !mbar_wait_warp(bar_pfull + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
                     {
-                        const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
-                        const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
-                        uint8_t* out = sm + (sB - base) + sb * b_bytes + r * 128;
+                        const int rr = has_row ? r : 0;    // lanes beyond the tile's rows redo row 0 (warp votes below) and store nothing
+                        const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + rr * 64;
+                        const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + rr * 32;
+                        uint8_t* out = sm + (sB - base) + sb * b_bytes + rr * 128;
                         const uint4 h0 = *reinterpret_cast<const uint4*>(hi + ((hf ^ sw_hi) << 4));
                         const uint32_t hw[4] = {h0.x, h0.y, h0.z, h0.w};
                         const int mode = w6_mode(sr);      // the other thread's half with it: the row's scales of the box
@@ -245,8 +248,10 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                             const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
                             uint32_t o[8];
                             w6_group(mode, l, hw[hi_w], hw[hi_w + 1], (sr >> (8 * c)) & 0xffu, o);
-                            *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                            *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                            if (has_row) {
+                                *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                                *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                            }
                         }
                     }
                     fence_proxy_async_smem();
@@ -295,7 +300,7 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint32_t ra[32];
 #pragma unroll 1
             for (int hc = 0; hc < MH * nchunks; ++hc) {
-                const int h = hc / nchunks, c = hc - h * nchunks;
+                const int h = MH == 1 ? 0 : hc / nchunks, c = hc - h * nchunks;
                 const int row0 = tm * (2 * BM * MH) + h * 2 * BM + (int)rank * BM + quad * 32;
                 const int row = row0 + lane;
                 const bool row_ok = row < p.M;
@@ -353,8 +358,8 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 }
 
 // ---- few rows: weight rows as the MMA's M, tokens as its N ---------------------------------------------------------------
-// Up to 256 tokens (the block on a short clip, a text prompt) the kernel above is bound by neither memory nor the tensor
-// core but by its chain from the packed tile to the MMA: remote arrivals and commits across the CTA pair for every K box,
+// Up to 256 tokens (the block on a short clip, a text prompt), or beside a narrow weight, the kernel above is bound by neither
+// memory nor the tensor core but by its chain from the packed tile to the MMA: remote arrivals and commits across the CTA pair for every K box,
 // an accumulator of 256 rows of which a quarter is used, and no way to share a long K between SMs. Here one CTA takes 128
 // weight rows and up to 256 tokens (tcgen05.mma.cta_group::1, M = 128 weight rows, N = tokens rounded up to 16), so every
 // barrier is local and nothing is spent on rows that do not exist; a row tile's K is cut between the CTAs of a cluster
@@ -370,7 +375,7 @@ constexpr int kW6RowsMaxTokens = 256;
 struct W6RowsParams {
     const uint8_t* s_rel;   // [N, K / 32] e4m3
     int srel_pitch;         // K / 32
-    int tokens;             // tokens of the tile: M rounded up to 16
+    int tokens;             // tokens of a tile, a multiple of 16; tiles of tokens lie along the grid's y
     int splits, kps;        // CTAs of a cluster share a row tile's K: kps boxes each
     int sa, sb;             // ring depths: packed planes + tokens, expanded tiles
     int groups;             // expanding groups of four warps in use
@@ -381,7 +386,8 @@ __device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
     return v;
 }
 
-template <typename OutT, int EPI>
+// TILED: several tiles of tokens. With one the offsets are left out: computed, they cost the epilogue of the activation form 0.4 us.
+template <typename OutT, int EPI, bool TILED>
 __global__ void __launch_bounds__(kW6RowsThreads, 1)
 gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_lo,
                       const __grid_constant__ CUtensorMap tmap_hi, const GemmParams p, const W6RowsParams x6) {
@@ -404,6 +410,7 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const uint32_t tmem_cols = T <= 32 ? 32u : T <= 64 ? 64u : T <= 128 ? 128u : 256u;
     const int tn = blockIdx.x / x6.splits, rank = blockIdx.x - tn * x6.splits;     // a cluster = the slices of one row tile
     const int n0 = tn * BM;
+    const int t0 = TILED ? blockIdx.y * T : 0, rows = TILED ? min(p.M - t0, T) : p.M;      // this tile's tokens
     const int k0 = rank * x6.kps, k1 = min(k0 + x6.kps, p.k_iters);                // never empty: the host side sees to it
 
     if (threadIdx.x == 0) {
@@ -433,7 +440,7 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 mbar_arrive_expect_tx(bar_full + 8 * s, (uint32_t)T * BK + lo_bytes + hi_bytes);
                 tma_load_2d(sLo + s * lo_bytes, &tmap_lo, kb * 64, n0, bar_full + 8 * s);
                 tma_load_2d(sHi + s * hi_bytes, &tmap_hi, kb * 32, n0, bar_full + 8 * s);
-                tma_load_2d(sA + s * a_bytes, &tmap_a, kb * BK, 0, bar_full + 8 * s);
+                tma_load_2d(sA + s * a_bytes, &tmap_a, kb * BK, t0, bar_full + 8 * s);
                 if (++s == SA) s = 0, ph ^= 1u;
             }
         }
@@ -539,7 +546,8 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     cluster_sync_all();
     if (warp >= 2 && *abort_s == 0) {
         // eight tokens x 32 columns at a time, dealt out over the cluster's warps
-        const int quads = (p.M + 7) / 8 * 4;
+        const int quads = (rows + 7) / 8 * 4;
+        const int64_t tile = (int64_t)t0 * p.N;                    // the tile's first output
         for (int u = rank + x6.splits * (warp - 2); u < quads; u += x6.splits * kW6RowsWarps) {
             const int quad = u & 3, m0 = (u >> 2) * 8;
             const int n = n0 + quad * 32 + lane;
@@ -556,19 +564,19 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             if constexpr (EPI == EPI_ACC) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    if (m0 + i < p.M) reinterpret_cast<int*>(p.D)[(int64_t)(m0 + i) * p.N + n] = acc[i];
+                    if (m0 + i < rows) reinterpret_cast<int*>(p.D)[tile + (int64_t)(m0 + i) * p.N + n] = acc[i];
             } else {
                 const float ws = p.ws[n], bias = p.bias ? to_f<OutT>(reinterpret_cast<const OutT*>(p.bias)[n]) : 0.f;
                 const float rs = EPI == EPI_RESID ? to_f<OutT>(reinterpret_cast<const OutT*>(p.rscale)[n]) : 0.f;
                 float rr[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i)
-                    rr[i] = EPI == EPI_RESID && m0 + i < p.M ? to_f<OutT>(reinterpret_cast<const OutT*>(p.resid)[(int64_t)(m0 + i) * p.N + n]) : 0.f;
+                    rr[i] = EPI == EPI_RESID && m0 + i < rows ? to_f<OutT>(reinterpret_cast<const OutT*>(p.resid)[tile + (int64_t)(m0 + i) * p.N + n]) : 0.f;
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    if (m0 + i >= p.M) break;
-                    reinterpret_cast<OutT*>(p.D)[(int64_t)(m0 + i) * p.N + n] =
-                        from_f<OutT>(epilogue1<OutT, EPI>(acc[i], p.xs[m0 + i], ws, bias, rs, rr[i], p.act));
+                    if (m0 + i >= rows) break;
+                    reinterpret_cast<OutT*>(p.D)[tile + (int64_t)(m0 + i) * p.N + n] =
+                        from_f<OutT>(epilogue1<OutT, EPI>(acc[i], p.xs[t0 + m0 + i], ws, bias, rs, rr[i], p.act));
                 }
             }
         }
@@ -601,10 +609,10 @@ bool make_plane_tmap(CUtensorMap* tm, const void* ptr, int64_t rows, int64_t col
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename OutT, int EPI>
-int launch_w6(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const CUtensorMap& td,
+template <typename OutT, int EPI, int MH>
+int launch_w6_mh(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const CUtensorMap& td,
                  const GemmParams& p, const W6Extra& x6, int grid, cudaStream_t st) {
-    auto kern = gemm_w6a8_pair_kernel<OutT, EPI>;
+    auto kern = gemm_w6a8_pair_kernel<OutT, EPI, MH>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -618,9 +626,16 @@ int launch_w6(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& 
 }
 
 template <typename OutT, int EPI>
-int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const GemmParams& p, const W6RowsParams& x6,
-                   size_t smem, cudaStream_t st) {
-    auto kern = gemm_w6a8_rows_kernel<OutT, EPI>;
+int launch_w6(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const CUtensorMap& td,
+              const GemmParams& p, const W6Extra& x6, int mh, int grid, cudaStream_t st) {
+    return mh == 2 ? launch_w6_mh<OutT, EPI, 2>(ta, tlo, thi, td, p, x6, grid, st)
+                   : launch_w6_mh<OutT, EPI, 1>(ta, tlo, thi, td, p, x6, grid, st);
+}
+
+template <typename OutT, int EPI, bool TILED>
+int launch_w6_rows_tiled(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const GemmParams& p, const W6RowsParams& x6,
+                         size_t smem, cudaStream_t st) {
+    auto kern = gemm_w6a8_rows_kernel<OutT, EPI, TILED>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -630,12 +645,19 @@ int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensor
         if (e != cudaSuccess) return (int)e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    return launch_pdl_cluster(kern, dim3(p.tiles_n * x6.splits), kW6RowsThreads, smem, st, x6.splits, ta, tlo, thi, p, x6);
+    return launch_pdl_cluster(kern, dim3(p.tiles_n * x6.splits, p.tiles_m), kW6RowsThreads, smem, st, x6.splits, ta, tlo, thi, p, x6);
 }
 
-// Clusters of s CTAs of the kernel above that the current device holds at once: asked of the runtime once per device.
+template <typename OutT, int EPI>
+int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const GemmParams& p, const W6RowsParams& x6,
+                   size_t smem, cudaStream_t st) {
+    return p.tiles_m > 1 ? launch_w6_rows_tiled<OutT, EPI, true>(ta, tlo, thi, p, x6, smem, st)
+                         : launch_w6_rows_tiled<OutT, EPI, false>(ta, tlo, thi, p, x6, smem, st);
+}
+
+// Clusters of 1 .. 8 CTAs of the kernel above that the current device holds at once ([0] unused): asked of the runtime once per device.
 constexpr int kW6RowsMaxSplits = 8;
-int w6_rows_clusters(int s) {
+const int* w6_rows_clusters() {
     static int count[64][kW6RowsMaxSplits + 1];
     static std::mutex mu;
     int dev = 0;
@@ -643,7 +665,7 @@ int w6_rows_clusters(int s) {
     std::lock_guard<std::mutex> lk(mu);
     int* c = count[dev & 63];
     if (c[0] == 0) {
-        auto kern = gemm_w6a8_rows_kernel<bf16, EPI_PLAIN>;
+        auto kern = gemm_w6a8_rows_kernel<bf16, EPI_PLAIN, false>;
         c[1] = device_sm_count(dev);
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess) {
             for (int i = 2; i <= kW6RowsMaxSplits; ++i) {
@@ -659,29 +681,40 @@ int w6_rows_clusters(int s) {
         (void)cudaGetLastError();
         c[0] = 1;
     }
-    return c[s];
+    return c;
 }
 
 int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, cudaStream_t st) {
     const int64_t M = p.M, N = p.N, K = p.K;
-    W6RowsParams x6{s_rel, (int)(K / 32), (int)((M + 15) / 16 * 16), 1, p.k_iters, 0, 0, 0};
+    W6RowsParams x6{s_rel, (int)(K / 32), 0, 1, p.k_iters, 0, 0, 0};
     p.tiles_n = (int)((N + BM - 1) / BM);
-    p.idesc = umma_idesc_i8(BM, x6.tokens);
-    // K slices: rounds of clusters times the cost of one, in K boxes. A CTA's rings take a whole SM and a cluster has to lie in
-    // one GPC, so the device holds fewer clusters than SMs / s (148, 74, 45, 33, 26, 22, 15, 15 of 1 to 8 CTAs); a second round
-    // costs as much as the first. Start, end and the tokens' share of the epilogue come to 8 + tokens / 32 boxes (a box: 0.56 us
-    // of expansion), the exchange of the accumulators to 3 more, and beyond four slices to tokens / 64: over 25 sizes of N and K
-    // (64 x 1024 to 20480 x 5120) at 16, 64, 128 and 256 tokens the slices chosen are within 3.5 % of the best of all eight.
-    int64_t best = INT64_MAX;
-    for (int s = 1; s <= kW6RowsMaxSplits && s <= p.k_iters; ++s) {
-        const int kps = (p.k_iters + s - 1) / s;
-        if ((p.k_iters + kps - 1) / kps != s) continue;                      // a slice would be empty
-        const int room = w6_rows_clusters(s);
-        if (room < 1) continue;
-        const int64_t rounds = ((int64_t)p.tiles_n + room - 1) / room;
-        const int64_t cost = rounds * (64 * (kps + 8) + 2 * x6.tokens + (s > 1 ? 192 : 0) + (s > 4 ? x6.tokens : 0));   // 1/64 boxes
-        if (cost < best) best = cost, x6.splits = s, x6.kps = kps;
+    // Token tiles and K slices: rounds of clusters times the cost of one, in K boxes (0.56 us of expansion each). A CTA's rings take
+    // a whole SM and a cluster has to lie in one GPC, so the device holds fewer clusters than SMs / s (148, 74, 45, 33, 26, 22, 15,
+    // 15 of 1 to 8 CTAs); a second round costs as much as the first. Start, end and the tokens' share of epilogue and exchange as
+    // measured at 16, 64, 128 and 256 tokens for 25 sizes of N and K (64 x 1024 to 20480 x 5120): the slices chosen are within
+    // 3.5 % of the best of all eight. Narrower token tiles expand the weight once more each, which pays where SMs would idle
+    // (256 x 120 x 1024 in four: 7.9 us, 10.9 in one); they have to promise 5 %.
+    const int* clusters = w6_rows_clusters();
+    double best = 1e30;
+    int last = 0;
+    for (const int width : {256, 192, 128, 96, 64}) {
+        const int tiles_m = (int)((M + width - 1) / width);
+        const int tokens = (int)(((M + tiles_m - 1) / tiles_m + 15) / 16 * 16);      // equal shares, at most 256
+        if (tokens == last) continue;
+        last = tokens;
+        double cost = 1e30;
+        int splits = 1, kps = p.k_iters;
+        for (int s = 1; s <= kW6RowsMaxSplits && s <= p.k_iters; ++s) {
+            const int k = (p.k_iters + s - 1) / s, room = clusters[s];
+            if ((p.k_iters + k - 1) / k != s || room < 1) continue;          // a slice would be empty; no such cluster fits
+            const double rounds = (double)(((int64_t)p.tiles_n * tiles_m + room - 1) / room);
+            const double c = rounds * (k + (s == 1 ? 8 + tokens / 28.0 : 10.5 + tokens / (s <= 4 ? 40.0 : 26.0)));
+            if (c < cost) cost = c, splits = s, kps = k;
+        }
+        if (cost < 0.95 * best) best = cost, x6.tokens = tokens, x6.splits = splits, x6.kps = kps;
     }
+    p.tiles_m = (int)((M + x6.tokens - 1) / x6.tokens);
+    p.idesc = umma_idesc_i8(BM, x6.tokens);
     const int a_bytes = (x6.tokens * BK + 1023) & ~1023;
     const int stage = a_bytes + BM * (64 + 32);
     // rings: as many expanded tiles as the packed ring beside them is deep (see the waits of the expanding warps), six at most
@@ -731,19 +764,24 @@ int run_w6_gemm(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     p.act_lut = nullptr;
     const int esz = epi == EPI_ACC ? 4 : (out_dt == DT_F32 ? 4 : 2);
     p.k_iters = (int)(K / BK);
-    if (M <= kW6RowsMaxTokens) return run_w6_rows(epi, A, Wq6, s_rel, p, out_dt, st);
+    // Up to 256 rows, and beside a weight narrower than the pair kernel's 128 columns up to 4 K rows: that kernel gives a cluster
+    // the whole K of 256 rows, the other one spreads K over more SMs but starts and ends once per 256 rows or fewer. 64 columns, the
+    // few-rows kernel | one half: K = 1024, 2048 rows 8.7 | 10.2 us, 4608 10.4 | 10.3, 8448 11.7 | 10.6; K = 2560, 8448 rows 14.8 |
+    // 16.1, 12288 16.4 | 16.2; K = 5120, 300 rows 9.9 | 24.1, 16896 23.9 | 25.9.
+    const bool narrow = N < BM;
+    if (M <= kW6RowsMaxTokens || (narrow && M <= 4 * K && M <= 65535 * 64)) return run_w6_rows(epi, A, Wq6, s_rel, p, out_dt, st);
     auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     p.vec_ok = (N % 8 == 0) && al16(D) && al16(ws) && al16(bias) && al16(rscale) && al16(resid);
     p.tma_store = al16(D) && ((N * esz) % 16 == 0);
     p.ksub = 1;
-    constexpr int bn = 128;
+    const int mh = narrow ? 1 : 2, bn = narrow ? choose_bn(M, N, clusters) : 128;
     p.bn = bn;
     p.idesc = umma_idesc_i8(2 * BM, bn);
-    const int stage_bytes = MH * BM * BK + (bn / 2) * (64 + 32);     // A boxes + packed planes; the expanded ring is separate
+    const int stage_bytes = mh * BM * BK + (bn / 2) * (64 + 32);     // A boxes + packed planes; the expanded ring is separate
     const int sbs = kW6BStages;
     const int stages = (kSmemBytes - 1024 - 512 - kW6StagingBytes - sbs * (bn / 2) * BK) / stage_bytes;
     p.stages = stages > kMaxStages ? kMaxStages : stages;
-    p.tiles_m = (int)((M + 2 * BM * MH - 1) / (2 * BM * MH));
+    p.tiles_m = (int)((M + 2 * BM * mh - 1) / (2 * BM * mh));
     p.tiles_n = (int)((N + bn - 1) / bn);
     p.num_tiles = p.tiles_m * p.tiles_n;
     p.whole_tiles = p.num_tiles, p.num_items = p.num_tiles, p.kps = p.k_iters;
@@ -759,11 +797,11 @@ int run_w6_gemm(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     }
     W6Extra x6{s_rel, (int)(K / 32), sbs};
     const int grid = 2 * (p.num_tiles < clusters ? p.num_tiles : clusters);
-    if (epi == EPI_ACC) return launch_w6<float, EPI_ACC>(ta, tlo, thi, td, p, x6, grid, st);
+    if (epi == EPI_ACC) return launch_w6<float, EPI_ACC>(ta, tlo, thi, td, p, x6, mh, grid, st);
 #define W6_DISPATCH(T)                                                                                   \
-    (epi == EPI_RESID ? launch_w6<T, EPI_RESID>(ta, tlo, thi, td, p, x6, grid, st)                      \
-     : epi == EPI_ACT ? launch_w6<T, EPI_ACT>(ta, tlo, thi, td, p, x6, grid, st)                        \
-                      : launch_w6<T, EPI_PLAIN>(ta, tlo, thi, td, p, x6, grid, st))
+    (epi == EPI_RESID ? launch_w6<T, EPI_RESID>(ta, tlo, thi, td, p, x6, mh, grid, st)                      \
+     : epi == EPI_ACT ? launch_w6<T, EPI_ACT>(ta, tlo, thi, td, p, x6, mh, grid, st)                        \
+                      : launch_w6<T, EPI_PLAIN>(ta, tlo, thi, td, p, x6, mh, grid, st))
     if (out_dt == DT_F32) return W6_DISPATCH(float);
     if (out_dt == DT_F16) return W6_DISPATCH(half);
     return W6_DISPATCH(bf16);

@@ -147,6 +147,39 @@ def test_few_rows_k_slices_fit_the_device_in_one_round(pkg, oracle, dev, M, few,
     assert us[many] < 1.5 * us[few], us
 
 
+# few tokens in several tiles; a weight narrower than 128 rows on more than 256 tokens: whole tiles, ragged last ones, one of a single
+# token, then (more than 4 K rows) the pair kernel with tiles of one half and 64, 96 and 128 columns, ragged too
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,K", [(200, 120, 1024), (256, 200, 1024), (257, 127, 128), (556, 64, 5120), (1024, 8, 640), (9000, 96, 4096), (513, 100, 128), (5000, 127, 1152), (18945, 72, 256), (16897, 100, 256), (40000, 8, 640)])
+def test_narrow_weights_on_many_rows(pkg, oracle, dev, dtype, M, N, K):
+    g, packed, s_rel = _packed(oracle, N, K, M + N + K, "fitted")
+    A = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8).to(dev)
+    xs, sc = (torch.rand(M, generator=g) * 0.05 + 1e-3).to(dev), (torch.rand(N, generator=g) * 1e-3 + 1e-4).to(dev)
+    bias, rscale = (torch.randn(N, generator=g).to(dtype).to(dev) for _ in range(2))
+    resid = torch.randn(M, N, generator=g).to(dtype).to(dev)
+    packed, s_rel = packed.to(dev), s_rel.to(dev)
+    L = pkg.linear
+    w8 = L.w6_decode(packed, s_rel, K)
+    for kw in ({}, {"act": 1}, {"rscale": rscale, "resid": resid}):
+        got = L.w6a8_gemm(A, packed, s_rel, xs, sc, bias, out_dtype=dtype, **kw)
+        assert_bits_equal(got, L.int8_gemm(A, w8, xs, sc, bias, out_dtype=dtype, **kw), str(kw.keys()))
+    assert_bits_equal(L.w6a8_gemm_acc_i32(A, packed, s_rel), L.int8_gemm_acc_i32(A, w8), "accumulators")
+    assert L.kernel_status() == 0
+
+
+def test_narrow_weights_do_not_pay_for_empty_columns(pkg, oracle, dev):
+    """300 x 96 x 5120 beside 256 x 96 x 5120: a second token tile on other SMs, not a tile of 128 columns on one cluster (which
+    took 2.4 times as long)."""
+    us = {}
+    for M in (256, 300):
+        g, packed, s_rel = _packed(oracle, 96, 5120, M, "fitted")
+        A = torch.randint(-128, 128, (M, 5120), generator=g, dtype=torch.int8).to(dev)
+        xs, sc = (torch.rand(M, generator=g) * 0.05).to(dev), (torch.rand(96, generator=g) * 1e-3).to(dev)
+        packed, s_rel, out = packed.to(dev), s_rel.to(dev), torch.empty((M, 96), dtype=torch.bfloat16, device=dev)
+        us[M] = _device_us(dev, lambda: pkg.linear.w6a8_gemm(A, packed, s_rel, xs, sc, None, out=out))
+    assert us[300] < 1.5 * us[256], us
+
+
 @pytest.mark.parametrize("act", [1, 2, 3])
 @pytest.mark.parametrize("M", [96, 1300])
 def test_activation_epilogue_equals_the_int8_form(pkg, dev, act, M):
