@@ -376,8 +376,11 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
                 const float mean = __fdiv_rn(row_sum(false), (float)p.K);
 #pragma unroll
                 for (int i = 0; i < 32; i += 2) {
-                    const float2 d = __fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(-mean, -mean));
-                    v[i] = d.x, v[i + 1] = d.y;
+                    if (PRO == PRO_LAYERNORM) v[i] = __fsub_rn(v[i], mean), v[i + 1] = __fsub_rn(v[i + 1], mean);     // pairs: spills
+                    else {
+                        const float2 d = __fadd2_rn(make_float2(v[i], v[i + 1]), make_float2(-mean, -mean));
+                        v[i] = d.x, v[i + 1] = d.y;
+                    }
                 }
             }
             const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(row_sum(true), (float)p.K), p.eps));
@@ -387,7 +390,8 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
             // rounds once where the other forms round to f32 first, which makes no difference (the f32 sum is inexact only
             // beside a scale below 2^-16 or above 2^16, and neither comes near a tie of bf16). A scalar conversion runs on the
             // narrow conversion pipe; DiT block on 4352 rows (two of these) 566 us before, 560 now, SwiGLU block on 1111 rows 212, 209.
-            constexpr bool kPacked = sizeof(T) == 2 && (PRO == PRO_LN_MOD || PRO == PRO_RMS);
+            // (Not RMS rows beyond 16384 values: 1024 threads leave 64 registers, and both forms in one kernel spilled 268 bytes.)
+            constexpr bool kPacked = sizeof(T) == 2 && (PRO == PRO_LN_MOD || (PRO == PRO_RMS && MAXT < 1024));
             if (kPacked && (PRO == PRO_LN_MOD ? ms_p != nullptr : ms_p == nullptr)) {
                 const float2 rstd2 = make_float2(rstd, rstd);
 #pragma unroll
