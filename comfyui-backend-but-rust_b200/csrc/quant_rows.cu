@@ -737,10 +737,12 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
     // rows of this CTA; GroupNorm's belong to one image (blockIdx.y), so that one set of statistics serves the CTA
     const int64_t limit = SRC == SDQ_GN ? (int64_t)(blockIdx.y + 1) * s.P : M;
     const int64_t m0 = (SRC == SDQ_GN ? (int64_t)blockIdx.y * s.P : 0) + (int64_t)blockIdx.x * rows;
-    const int rloc = threadIdx.x / tpr, tin = threadIdx.x - rloc * tpr;
+    // threads beyond the rows' (they help with the source only) and those of rows past the end recompute the last row and store nothing
+    const int piece = threadIdx.x / tpr, tin = threadIdx.x - piece * tpr, rloc = SRC == SDQ_ROWS ? piece : min(piece, rows - 1);
     const int64_t m_raw = m0 + rloc;
-    const bool live = m_raw < limit;
-    const int64_t m = live ? m_raw : limit - 1;        // idle rows recompute the last row and store nothing
+    const bool live = (SRC == SDQ_ROWS || piece < rows) && m_raw < limit;
+    const int64_t m = SRC == SDQ_ROWS ? (live ? m_raw : limit - 1) : 0;
+    const int rl = (int)min((int64_t)rloc, limit - 1 - m0);      // the row it works on; its own where it has one
     float v[32];
     if constexpr (SRC == SDQ_ROWS) {
         __syncthreads();
@@ -752,7 +754,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
         const int pitch = ((K >> 3) + 7) & ~7;
         sd_source_rows<SRC>(s, row_s, pitch, reinterpret_cast<float2*>(amax_s + ((rows + 1) & ~1)), m0, (int)min((int64_t)rows, limit - m0), K);
         __syncthreads();
-        const uint4* r = row_s + (int)(m - m0) * pitch;
+        const uint4* r = row_s + rl * pitch;
 #pragma unroll
         for (int c = 0; c < 4; ++c) unpack_half8(r[sd_piece(4 * tin + c)], *reinterpret_cast<float(*)[8]>(v + 8 * c));
     }
@@ -823,7 +825,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
     pdl_trigger();
     const float mx = __uint_as_float(amax_s[rloc]);
     const float scale = __fdiv_rn(fmaxf(mx, 1e-30f), 127.f);
-    if (live && tin == 0) scales[m] = scale;
+    if (live && tin == 0) scales[m_raw] = scale;
     const float sh16 = rnd<half>(scale);
     const float st = sh16 > 0.f ? sh16 : scale;          // a scale below half's range divides in float
     const bool fast = sh16 > 0.f && mx <= 65504.f && !has_nan;
@@ -847,7 +849,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
             c16[i] = (uint32_t)(qx & 0xff) | ((uint32_t)(qy & 0xff) << 8);
         }
     }
-    int8_t* qr = q + m * (int64_t)K + tin * 32;
+    int8_t* qr = q + m_raw * K + tin * 32;              // of live rows only
     if (ROT == 256) {
         uint16_t* cb = reinterpret_cast<uint16_t*>(tbuf);
         const uint32_t order = tsw ? 0x3201u : 0x3210u;
@@ -929,6 +931,15 @@ int ensure_lut(int which, cudaStream_t st) {
 }  // namespace
 
 namespace {
+int sm_count_of(int dev) {
+    static int count[64];
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    int& c = count[dev & 63];
+    if (c == 0) cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
+    return c;
+}
+
 template <int ROT, int SRC, int MAXT>
 int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 grid, int threads, int rows, uint32_t smem, uint32_t off_amax,
                   uint32_t off_rows, cudaStream_t st) {
@@ -956,7 +967,22 @@ int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaS
     int even = 32;                                      // rows that make a whole number of warps
     while (even > 1 && (even / 2 * tpr) % 32 == 0) even /= 2;
     if (even * tpr <= kSdThreads || (SRC != SDQ_ROWS && even * tpr <= 512)) rows = rows / even > 0 ? rows / even * even : even;
-    const int threads = rows * tpr;
+    int threads = rows * tpr;
+    if (SRC != SDQ_ROWS) {
+        // Few rows: a row or as few as give every SM a CTA, and up to 256 threads for the source, which has a 16-byte piece of the
+        // row for each (a warp per row for LayerNorm's sums). With the row counts above, 16 rows of 320 values kept one CTA
+        // busy for 6.6 us (LayerNorm; GEGLU 3.8) where a CTA per row had taken 3.4 (2.6).
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const int sms = sm_count_of(dev), share = (M + sms - 1) / sms;
+        if (share < rows) {
+            rows = share;
+            const int work = rows * (SRC == SDQ_LN && 4 * tpr < 32 ? 32 : 4 * tpr);
+            threads = rows * tpr;
+            if (threads < 256) threads = work < 256 ? (work > threads ? work : threads) : 256;
+            threads = (threads + 31) & ~31;
+        }
+    }
     uint32_t off = ROT == 256 ? (uint32_t)((threads + 31) / 32) * kWarpWords * 4 : 0;
     const uint32_t off_amax = off;
     off += (uint32_t)((rows + 1) & ~1) * 4 + (SRC == SDQ_GN ? (uint32_t)s.groups * 8 : 0);
@@ -1041,15 +1067,6 @@ int b200q::act_lut_ptr(int act, cudaStream_t st, const uint16_t** out) {
 }
 
 namespace {
-
-int sm_count_of(int dev) {
-    static int count[64];
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lk(mu);
-    int& c = count[dev & 63];
-    if (c == 0) cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    return c;
-}
 
 // CTAs of one kernel instantiation that fit an SM at a given size: asked of the runtime once per (threads, smem).
 struct OccCache {

@@ -118,3 +118,24 @@ def assert_close_out(got: torch.Tensor, want: torch.Tensor, what: str = "", tiny
     else:
         d = max_ulp_diff(g, w)
         assert d <= 1, f"{what}: {d} ulp apart"
+
+
+def device_us(dev, call, launches=20):
+    """Device time of one call, the launches replayed as a graph (no host time in between), the fastest of five replays."""
+    stream = torch.cuda.Stream(dev)
+    with torch.cuda.stream(stream):
+        call()
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            for _ in range(launches):
+                call()
+        times = []
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            stream.synchronize()
+            times.append(a.elapsed_time(b) * 1e3 / launches)
+    return min(times[1:])

@@ -6,7 +6,7 @@ import importlib
 import pytest
 import torch
 
-from conftest import assert_bits_equal
+from conftest import assert_bits_equal, device_us
 
 pytestmark = pytest.mark.gpu
 
@@ -317,3 +317,43 @@ def test_packers_in_registers_equal_the_shared_memory_kernels(pkg, dev, N, K, dt
     buf[4:] = q.to(dev).reshape(-1)
     assert_bits_equal(L.convrot_dequant(q.to(dev), s, dtype), L.convrot_dequant(buf[4:].view(N, K), s, dtype), "dequant")
     assert_bits_equal(L.embed_dequant(q.to(dev), s), L.embed_dequant(buf[4:].view(N, K), s), "embed")
+
+
+# CTAs of a row or a few with threads that only help with the source (up to a row per SM and one beyond), then of whole rows
+@pytest.mark.parametrize("mode", ["ln", "geglu", "unpad", "gn"])
+@pytest.mark.parametrize("M,K,rotate", [(1, 64, 64), (148, 320, 64), (149, 320, 0), (300, 768, 256), (1500, 96, 0), (2400, 320, 64), (1301, 640, 64),
+                                        (9, 9216, 256), (150, 16384, 0)])
+def test_sd_sources_at_every_split_of_the_rows(pkg, dev, mode, M, K, rotate):
+    """The register kernel against the shared-memory kernel, bit for bit, around the row counts at which its CTAs change."""
+    g = torch.Generator(device=dev).manual_seed(M + K)
+    L = pkg.linear
+    rn = lambda *s: torch.randn(*s, generator=g, device=dev)
+
+    def both(t):      # the tensor on a 16-byte boundary, and the same values off it
+        off = torch.empty(t.numel() + 8, dtype=t.dtype, device=dev)[1:1 + t.numel()].view(t.shape)
+        return t, off.copy_(t)
+
+    if mode == "ln":
+        x, b = (rn(M, K) * 2 + 0.5).half(), rn(K) * 0.1
+        got, want = (L.sd_ln_quant_rows(x, w, b, 1e-5, rotate) for w in both(rn(K) * 0.2 + 1))
+    elif mode == "geglu":
+        got, want = (L.sd_geglu_quant_rows(x, rotate) for x in both((rn(M, 2 * K) * 1.5).half()))
+    elif mode == "unpad":
+        got, want = (L.sd_unpad_quant_rows(x, 32, rotate) for x in both(rn(M, K // 32, 40).half()))
+    else:
+        images = 3 if M % 3 == 0 else 1
+        x, b = (rn(images, M // images, K) * 1.5 + 0.3).half(), rn(K) * 0.1
+        got, want = (L.sd_group_norm_quant_rows(x, w, b, 32, 1e-5, rotate) for w in both(rn(K) * 0.2 + 1))
+    assert_bits_equal(got[1], want[1], "scales"), assert_bits_equal(got[0], want[0], "codes")
+
+
+@pytest.mark.parametrize("mode", ["ln", "geglu"])
+def test_a_few_rows_take_little_longer_than_one(pkg, dev, mode):
+    """Sixteen rows of 320 values go to sixteen SMs; all in one CTA they took twice the time of one row."""
+    L = pkg.linear
+    w, b = torch.ones(320, device=dev), torch.zeros(320, device=dev)
+    us = {}
+    for M in (1, 16):
+        x = torch.randn(M, 640 if mode == "geglu" else 320, device=dev).half()
+        us[M] = device_us(dev, (lambda: L.sd_ln_quant_rows(x, w, b, 1e-5, 64)) if mode == "ln" else (lambda: L.sd_geglu_quant_rows(x, 64)))
+    assert us[16] < 1.4 * us[1], us

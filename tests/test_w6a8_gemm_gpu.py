@@ -7,7 +7,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from conftest import assert_bits_equal
+from conftest import assert_bits_equal, device_us
 
 pytestmark = pytest.mark.gpu
 
@@ -111,27 +111,6 @@ def test_few_rows_equal_the_two_call_flow(pkg, oracle, dev, dtype, M, N, K):
     assert L.kernel_status() == 0
 
 
-def _device_us(dev, call, launches=20):
-    """Device time of one call, the launches replayed as a graph (no host time in between), the fastest of five replays."""
-    stream = torch.cuda.Stream(dev)
-    with torch.cuda.stream(stream):
-        call()
-        stream.synchronize()
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=stream):
-            for _ in range(launches):
-                call()
-        times = []
-        for _ in range(6):
-            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            a.record()
-            graph.replay()
-            b.record()
-            stream.synchronize()
-            times.append(a.elapsed_time(b) * 1e3 / launches)
-    return min(times[1:])
-
-
 @pytest.mark.parametrize("M,few,many,K", [(64, 1920, 2560, 2560), (128, 1920, 2304, 6144), (16, 1920, 2176, 2048)])
 def test_few_rows_k_slices_fit_the_device_in_one_round(pkg, oracle, dev, M, few, many, K):
     """A few row tiles more must not push the clusters that share K into a second round: such a rule counts SMs, while a cluster
@@ -142,7 +121,7 @@ def test_few_rows_k_slices_fit_the_device_in_one_round(pkg, oracle, dev, M, few,
         A = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8).to(dev)
         xs, sc = (torch.rand(M, generator=g) * 0.05).to(dev), (torch.rand(N, generator=g) * 1e-3).to(dev)
         packed, s_rel, out = packed.to(dev), s_rel.to(dev), torch.empty((M, N), dtype=torch.bfloat16, device=dev)
-        us[N] = _device_us(dev, lambda: pkg.linear.w6a8_gemm(A, packed, s_rel, xs, sc, None, out=out))
+        us[N] = device_us(dev, lambda: pkg.linear.w6a8_gemm(A, packed, s_rel, xs, sc, None, out=out))
         assert_bits_equal(out, pkg.linear.int8_gemm(A, pkg.linear.w6_decode(packed, s_rel, K), xs, sc, None))
     assert us[many] < 1.5 * us[few], us
 
@@ -176,7 +155,7 @@ def test_narrow_weights_do_not_pay_for_empty_columns(pkg, oracle, dev):
         A = torch.randint(-128, 128, (M, 5120), generator=g, dtype=torch.int8).to(dev)
         xs, sc = (torch.rand(M, generator=g) * 0.05).to(dev), (torch.rand(96, generator=g) * 1e-3).to(dev)
         packed, s_rel, out = packed.to(dev), s_rel.to(dev), torch.empty((M, 96), dtype=torch.bfloat16, device=dev)
-        us[M] = _device_us(dev, lambda: pkg.linear.w6a8_gemm(A, packed, s_rel, xs, sc, None, out=out))
+        us[M] = device_us(dev, lambda: pkg.linear.w6a8_gemm(A, packed, s_rel, xs, sc, None, out=out))
     assert us[300] < 1.5 * us[256], us
 
 
