@@ -15,6 +15,9 @@
 // bits 0-3: radix-4 stages 0 and 1), then 16 elements 16 apart (index bits 4-7: stages 2 and 3; groups of 64 have only stage
 // 2). Every butterfly adds in the reference's left-to-right order.
 #include <cstdlib>
+#include <mutex>
+#include <vector>
+
 #include <cuda_fp8.h>
 
 #include "common.cuh"
@@ -763,10 +766,25 @@ __global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* q, cons
     }
 }
 
+// Room for `bytes` of dynamic shared memory on the current device. The limit is only ever raised: set to each call's own size, a
+// short row's call on one thread lowered it between a long row's on another and that one's launch, which then failed.
 int set_smem(const void* fn, size_t bytes) {
     if (bytes <= 48 * 1024) return 0;
+    struct Limit { const void* fn; int dev; size_t bytes; };
+    static std::vector<Limit> limits;
+    static std::mutex mu;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    Limit* l = nullptr;
+    for (Limit& e : limits)
+        if (e.fn == fn && e.dev == dev) l = &e;
+    if (l && l->bytes >= bytes) return 0;
     const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return e == cudaSuccess ? 0 : (int)e;
+    if (e != cudaSuccess) return (int)e;
+    if (l) l->bytes = bytes;
+    else limits.push_back({fn, dev, bytes});
+    return 0;
 }
 // Rows in registers, K / 32 threads each: about 256 threads per CTA, at least a warp. Up to 512 threads (K <= 16384), so that a
 // thread may hold its 32 values and what is computed from them.

@@ -357,3 +357,37 @@ def test_a_few_rows_take_little_longer_than_one(pkg, dev, mode):
         x = torch.randn(M, 640 if mode == "geglu" else 320, device=dev).half()
         us[M] = device_us(dev, (lambda: L.sd_ln_quant_rows(x, w, b, 1e-5, 64)) if mode == "ln" else (lambda: L.sd_geglu_quant_rows(x, 64)))
     assert us[16] < 1.4 * us[1], us
+
+
+@pytest.mark.parametrize("call", ["requant", "w6", "sd_rows"])
+def test_loader_threads_with_rows_of_different_length(pkg, dev, call):
+    """Two host threads packing rows of different length at once: the kernel's shared-memory limit belongs to both."""
+    from threading import Thread
+    L = pkg.linear
+    errors = []
+
+    def load(K):
+        w = torch.randn(1, K, device=dev)
+        stream = torch.cuda.Stream(dev)
+        try:
+            with torch.cuda.stream(stream):
+                for i in range(4000):
+                    if call == "requant":
+                        L.convrot_requant(w, 1)
+                    elif call == "w6":
+                        L.w6_requant(w.bfloat16(), 1)
+                    else:
+                        L.sd_quant_rows(w.half(), 0)
+                    if i % 500 == 499:
+                        stream.synchronize()
+        except pkg.GpuKernelError as e:
+            errors.append((K, str(e)))
+
+    lengths = (40960, 20480) if call == "sd_rows" else (16384, 10240)      # sd_rows: rows the register kernel does not take
+    threads = [Thread(target=load, args=(K,)) for K in lengths]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
