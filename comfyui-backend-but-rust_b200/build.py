@@ -1,7 +1,8 @@
 """Builds libb200_qlinear.so (the C-ABI library) and libb200_qlinear.a (the same objects as a static archive, for hosts
 that link statically) from csrc/*.cu with nvcc, for sm_100a only, then _host_ops.so, the CPython extension behind
-linear.py's hot calls. The name differs on purpose from the reference's own static library `gpu_kernels`, which keeps
-supplying every symbol this library does not replace.
+linear.py's hot calls. The libraries need nvcc and nothing else; the extension needs torch and is left out, with a note, where
+torch cannot be imported (a Rust or C host), or with --c-only. The name differs on purpose from the reference's own static
+library `gpu_kernels`, which keeps supplying every symbol this library does not replace.
 
 The GEMM uses tcgen05.mma kind::i8, which exists on sm_100a and not on sm_103a or sm_120: no other -gencode
 may be added. No fast-math: the rounding points of the quantizer and of the epilogue are part of the contract.
@@ -35,10 +36,13 @@ def _stale(target: str, deps: list[str]) -> bool:
 
 def _host_ops(force: bool, verbose: bool) -> None:
     """csrc/host_ops.cpp -> HOST_OPS, against the headers and libraries of the torch that will import it."""
+    try:
+        import torch
+    except ImportError as e:
+        sys.stderr.write(f"{os.path.basename(HOST_OPS)} left out: torch cannot be imported ({e}); {LIB} does not need it\n")
+        return
     src = os.path.join(CSRC, "host_ops.cpp")
     stamp = os.path.join(OBJ, "host_ops.torch")
-    import torch
-
     fresh = os.path.exists(stamp) and open(stamp).read() == torch.__version__
     if not force and fresh and not _stale(HOST_OPS, [src, os.path.abspath(__file__), os.path.join(os.path.dirname(HERE), "include", "gpu_kernels.h")]):
         return
@@ -59,7 +63,7 @@ def _host_ops(force: bool, verbose: bool) -> None:
         f.write(torch.__version__)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
+def build(force: bool = False, verbose: bool = False, c_only: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h", ".inl"))]
     headers.append(os.path.abspath(__file__))
@@ -83,9 +87,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if os.path.exists(ARCHIVE):
             os.remove(ARCHIVE)
         subprocess.check_call(["ar", "rcs", ARCHIVE] + objs)
-    _host_ops(force, verbose)
+    if not c_only:
+        _host_ops(force, verbose)
     return LIB
 
 
 if __name__ == "__main__":
-    print(build(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build(force="--force" in sys.argv, verbose="-v" in sys.argv, c_only="--c-only" in sys.argv))
