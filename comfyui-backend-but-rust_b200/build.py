@@ -34,6 +34,12 @@ def _stale(target: str, deps: list[str]) -> bool:
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _host_ops_stamp(torch) -> str:
+    """What an extension is bound to: the interpreter's ABI and the very torch it was linked against."""
+    return "\n".join([sys.implementation.cache_tag, torch.__version__, os.path.dirname(os.path.abspath(torch.__file__)),
+                      f"cxx11_abi={int(torch.compiled_with_cxx11_abi())}"])
+
+
 def _host_ops(force: bool, verbose: bool) -> None:
     """csrc/host_ops.cpp -> HOST_OPS, against the headers and libraries of the torch that will import it."""
     try:
@@ -43,7 +49,8 @@ def _host_ops(force: bool, verbose: bool) -> None:
         return
     src = os.path.join(CSRC, "host_ops.cpp")
     stamp = os.path.join(OBJ, "host_ops.torch")
-    fresh = os.path.exists(stamp) and open(stamp).read() == torch.__version__
+    bound = _host_ops_stamp(torch)
+    fresh = os.path.exists(stamp) and open(stamp).read() == bound
     if not force and fresh and not _stale(HOST_OPS, [src, os.path.abspath(__file__), os.path.join(os.path.dirname(HERE), "include", "gpu_kernels.h")]):
         return
     root = os.path.dirname(torch.__file__)
@@ -60,7 +67,7 @@ def _host_ops(force: bool, verbose: bool) -> None:
     if r.returncode:
         raise RuntimeError("g++ failed on host_ops.cpp")
     with open(stamp, "w") as f:
-        f.write(torch.__version__)
+        f.write(bound)
 
 
 def build(force: bool = False, verbose: bool = False, c_only: bool = False) -> str:

@@ -12,9 +12,14 @@ from typing import Optional
 
 import torch
 
-from . import _host_ops as _h
 from . import ffi
 from .ffi import ok
+
+try:
+    from . import _host_ops as _h
+except ImportError as e:
+    raise ImportError(f"_host_ops.so is missing or was built for another Python or torch ({e}): build it for this one with "
+                      "`python comfyui-backend-but-rust_b200/build.py`") from e
 
 _h.ok = ok      # how a call there raises the error of a return code
 
