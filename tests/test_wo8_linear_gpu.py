@@ -41,6 +41,38 @@ def test_against_the_fp32_flow(pkg, dev, M, N, K, pro):
     assert L.kernel_status() == 0
 
 
+# The forms of the kernel under it: tiles of more than 128 columns have one accumulator pair (512 x 19456: 192 columns, 204 tiles for
+# at most 74 clusters), narrower ones two; a cluster's second and third tile toggles their phases; ragged rows and columns, columns
+# whose rows of output TMA cannot address (N % 4). `limit` keeps the GEMM to a few clusters, so that each has several tiles.
+@pytest.mark.parametrize("M,N,K,limit", [(512, 19456, 256, 0), (512, 19456, 256, 5), (700, 2560, 512, 3), (300, 1030, 768, 2), (513, 770, 256, 1),
+                                         (257, 1023, 1024, 3)])
+def test_several_tiles_a_cluster_and_ragged_ones(pkg, dev, M, N, K, limit):
+    g = torch.Generator().manual_seed(M + N + K)
+    L = pkg.linear
+    x = (torch.randn(M, K, generator=g) * 1.5).to(dev)
+    Wq, ws = L.convrot_requant((torch.randn(N, K, generator=g) * 0.03).to(dev), 0)
+    xr, wf = L.rotate_rows_f32(x, PLAIN), L.dequant_i8(Wq, ws)
+    exact = xr.double() @ wf.double().t()
+    scale = exact.abs().max().item()
+    # Per output: hi + lo (each rounded to 8 bits) leaves at most 2^-18 of every term; adding K terms in f32 at most K 2^-24 of their
+    # absolute sum. (Not "three times an fp32 product's error": a short sum in fp32 loses less than the 2^-18.)
+    bound = (2.0 ** -18 + K * 2.0 ** -24) * (xr.double().abs() @ wf.double().abs().t())
+    base = torch.randn(M, N, generator=g).to(dev)
+    out = torch.full((M + 1, N), 7.0, device=dev)                  # a row more, which nothing writes
+    acc = base.clone()
+    was = L.set_gemm_cluster_limit(limit)
+    try:
+        L.wo8_linear(x, Wq, ws, PLAIN, out=out[:M])
+        L.wo8_linear(x, Wq, ws, PLAIN, out=acc, beta=1.0)
+    finally:
+        L.set_gemm_cluster_limit(was)
+    err = (out[:M].double() - exact).abs()
+    assert err.max().item() <= 1e-5 * scale and bool((err <= bound).all()), (err.max().item(), scale, (err / bound).max().item())
+    assert bool((out[M] == 7.0).all())
+    assert (acc.double() - (base.double() + exact)).abs().max().item() <= 1e-5 * max(scale, base.abs().max().item())
+    assert L.kernel_status() == 0
+
+
 def test_argument_checks(pkg, dev):
     L = pkg.linear
     x = torch.zeros(4, 300, device=dev)
