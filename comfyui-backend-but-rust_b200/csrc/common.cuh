@@ -28,7 +28,7 @@ typedef __nv_bfloat16 bf16;
 //   - pdl_wait(), before the first access to memory that another kernel reads or writes: everything launched before in the
 //     stream has ended and its writes are visible. Every thread that touches such memory waits, so an order that held
 //     between whole kernels (results, buffers used again, the zeros of the split scratch) holds as before;
-//   - in the quantizers and the decoder pdl_trigger(), when a CTA has its rows and little but the codes and their stores is
+//   - in the quantizers, the W6 decoder and the widening kernel pdl_trigger(), when a CTA has its rows and little but the codes and their stores is
 //     left: the stream's next kernel may be brought onto the SMs once every CTA has got there or ended. The others, the GEMMs
 //     among them, leave it at the end of their CTAs. A trigger at a kernel's start loses more than it hides: the successor's
 //     CTAs then go where there is room beside the running kernel, and a small quantizer after a GEMM on 64 of 74 cluster pairs

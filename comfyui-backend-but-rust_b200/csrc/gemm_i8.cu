@@ -1577,9 +1577,9 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
 // terms (hi + lo = 16 significant bits) into two f32 accumulators, added in the epilogue: close to an fp32 product at
 // tensor-core speed. The kernel is the int8 one with kind::f16 MMAs (bf16 operands are addressed as rows of 2 K bytes); a
 // stage holds a K box of both terms and the one box of W that multiplies them. As two launches, the second adding to the
-// output of the first, W was read and D written twice: the MLP of a text encoder layer (512 rows, 2560, FFN 9728) took 301 us,
-// now 252 (271 with tiles of at most 128 columns, whose accumulators fit the tensor memory twice: what the narrower tiles read
-// from L2 costs more than the epilogue that wider ones leave uncovered).
+// output of the first, W was read and D written twice: 512 x 2560 -> 19456 took 160 us with its
+// rotation and widening, now 127. (Tiles of at most 128 columns, whose accumulators fit the tensor memory twice, were slower, 271
+// against 252 us for the layer's MLP: what they read from L2 costs more than the epilogue that wider ones leave uncovered.)
 __global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* q, bf16* out, int64_t n16) {
     pdl_wait();
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

@@ -214,7 +214,8 @@ __device__ int g_quant_status = 0;   // a staging wait that ran out records ST_T
 // DIRECT: the form of a block's linears and of the packers, rotated rows to codes and scales, one row block per CTA. Without the
 // other forms in the same instantiation it fits 56 registers in CTAs of up to 288 threads, 36 warps per SM instead of 24 (RMS,
 // LAYERNORM and SWIGLU: 64 registers, 256 threads, 32 warps); the kernel is bound by issue slots that too few warps fill (59 %
-// busy). DiT block on 4352 x 3072 (three of these kernels) 581 us -> 566, W6A8 block on 2048 x 5120 601 -> 585. f32 rows other than the packers' and SITU would spill and keep the general form.
+// busy). In a chain of launches: PLAIN 4352 x 3072 17.1 -> 13.6 us, RMS 2048 x 5120 27.9 -> 25.0 (launch order included). f32 rows
+// other than the packers' and SITU would spill and keep the general form.
 template <typename T, int PRO> __host__ __device__ constexpr int direct_threads() {
     if (sizeof(T) == 4) return PRO == PRO_PLAIN ? 288 : 0;
     return PRO == PRO_SITU ? 0 : PRO == PRO_RMS || PRO == PRO_LAYERNORM || PRO == PRO_SWIGLU ? 256 : 288;
@@ -389,7 +390,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
             // The common bf16 forms two values at a time, one packed conversion per rounding. 1 + scale is a bf16 addition: it
             // rounds once where the other forms round to f32 first, which makes no difference (the f32 sum is inexact only
             // beside a scale below 2^-16 or above 2^16, and neither comes near a tie of bf16). A scalar conversion runs on the
-            // narrow conversion pipe; DiT block on 4352 rows (two of these) 566 us before, 560 now, SwiGLU block on 1111 rows 212, 209.
+            // narrow conversion pipe; LN_MOD 4352 x 3072 37.2 us with scalar ones and 80 registers, 30.0 now.
             // (Not RMS rows beyond 16384 values: 1024 threads leave 64 registers, and both forms in one kernel spilled 268 bytes.)
             constexpr bool kPacked = sizeof(T) == 2 && (PRO == PRO_LN_MOD || (PRO == PRO_RMS && MAXT < 1024));
             if (kPacked && (PRO == PRO_LN_MOD ? ms_p != nullptr : ms_p == nullptr)) {
@@ -579,8 +580,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
 // first phase in which consecutive lanes hold consecutive 16-byte pieces (eight values), so that rows, gates and per-column
 // vectors are read coalesced and each once, and leave the rows in shared memory as half, from where the lanes pick up their
 // 32 values. A row at a time in shared memory as floats, one value per thread and step, was bound by its instruction count:
-// 8192 x 640 LayerNorm 49.2 us, GroupNorm 44.3, GEGLU 8192 x 2560 108 us; this form takes 16.6, 13.8 and 50 us (2048 x 1280:
-// LayerNorm 20.7 -> 9.5).
+// 8192 x 640 LayerNorm 46.8 us, GroupNorm 60.9 with its statistics, GEGLU 8192 x 2560 114; this form takes 12.2, 24.7 and 47.7.
 // LayerNorm statistics in the reference's order of additions: there 256 threads hold the row, thread t the elements t, t + 256,
 // ... one after the other, then a xor-shuffle tree over the lanes of each warp and another over the eight warps. Here one
 // warp holds a row, lane l the values 8 l .. 8 l + 7 of each run of 256, so the chains over the runs are the lane's own eight
@@ -720,7 +720,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
 
 // Up to 288 threads (rows up to 9216 values) the kernel is held to 56 registers, seven CTAs of 160 threads per SM instead of
 // six: 8192 rows of 640 values are 1024 such CTAs, which six per SM take in two rounds, the second an eighth full.
-// U-Net block of width 640 (eight of these kernels): 328 us with 63 registers, halvings in every stage and a division per piece, 321 now.
+// In a chain of launches 8192 x 640: rows as they lie 7.6 -> 6.0 us.
 constexpr int kSdThreads = 288;
 template <int ROT, int SRC, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fast_kernel(const SdSrc s, int8_t* q, float* scales, int M,

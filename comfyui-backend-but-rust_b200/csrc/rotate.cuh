@@ -1,4 +1,5 @@
-// The R256 rotation (the reference's csrc/common.cuh:99-126) in registers, shared by the quantizers (quant_rows.cu) and the
+// The R256 rotation (the reference's csrc/common.cuh:99-126) in registers: buffer layout and butterflies for the quantizers
+// (quant_rows.cu, which have the transposition inline, in forms with and without the rotation) and, whole, rotate256_regs for the
 // weight packers (weight_pack.cu). A 256-wide group belongs to 8 consecutive lanes (a team), 32 consecutive values each;
 // stages 0 and 1 run on those, a transposition through the team's padded piece of shared memory hands every lane the pairs
 // (2t, 2t + 1) + 16 r, and stages 2 and 3 run on them.

@@ -214,9 +214,6 @@ __global__ void __launch_bounds__(512) sd_quant_rows_reg_kernel(const half* __re
     if (live) *reinterpret_cast<uint4*>(q + m * (int64_t)K + tin * 16) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// The same quantizer over a row that another of the reference's kernels would have written in half first
-// (csrc/sd.cu:611-724): the row is computed as that kernel computes it, rounded to half, then quantized as above.
-// 256 threads, each adding elements t, t + 256, ... and then the block tree: the reference's order of additions.
 // GroupNorm statistics of x [N, P, C] half: per (image, group) the sum and the sum of squares, accumulated in double
 // from per-block float sums as the reference's sd_group_sums_kernel forms them (csrc/sd.cu:209-233: 256 threads, thread
 // t takes values t, t + 256, ... of the block's pixel range, then the block tree), so the statistics come out the same.
@@ -261,6 +258,9 @@ __global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* x, doubl
         atomicAdd(&sums[ng * 2 + 1], (double)ss);
     }
 }
+// The quantizer over a row that another of the reference's kernels would have written in half first (csrc/sd.cu:611-724), for what
+// the register kernel of quant_rows.cu does not take: the row is computed as that kernel computes it, rounded to half, then
+// quantized as above. 256 threads, each adding elements t, t + 256, ... and then the block tree: the reference's order of additions.
 template <int MODE>
 __global__ void __launch_bounds__(256) sd_quant_src_kernel(const SdSrc p, int8_t* __restrict__ q, float* __restrict__ scales,
                                                            int K, int rotate, int vec) {
@@ -363,8 +363,8 @@ __global__ void __launch_bounds__(512) convrot_requant_kernel(const T* __restric
 
 // Stochastic packing with the rows in registers: whole rows of K / 32 threads, 32 values each, the rotation of rotate.cuh, one
 // shared-memory maximum per row. The kernel above walks a row in shared memory one value per thread and step and divides for
-// every value; it took 149 us for 5120 x 5120 bf16 (79 MB moved, a floor of 12 us; the whole load-and-bake pass of such a weight went from 523 to
-// 303 us with this kernel, the inverse and the W6 packer) and stays for rows the loads below cannot take.
+// every value: 12800 x 6144 bf16 takes it 380 us, this one 129 (236 MB moved, a floor of 36 us). It stays for rows the loads below
+// cannot take.
 // The bf16 quotient is a reciprocal multiplication (exact: see quant2 in quant_rows.cu), the hash and the noise are as above.
 template <typename T> __device__ __forceinline__ void load_row32(const T* p, float (&v)[32]) {
 #pragma unroll
