@@ -28,7 +28,7 @@ typedef __nv_bfloat16 bf16;
 //   - pdl_wait(), before the first access to memory that another kernel reads or writes: everything launched before in the
 //     stream has ended and its writes are visible. Every thread that touches such memory waits, so an order that held
 //     between whole kernels (results, buffers used again, the zeros of the split scratch) holds as before;
-//   - in the quantizers, the W6 decoder and the widening kernel pdl_trigger(), when a CTA has its rows and little but the codes and their stores is
+//   - in the quantizers and the W6 decoder pdl_trigger(), when a CTA has its rows and little but the codes and their stores is
 //     left: the stream's next kernel may be brought onto the SMs once every CTA has got there or ended. The others, the GEMMs
 //     among them, leave it at the end of their CTAs. A trigger at a kernel's start loses more than it hides: the successor's
 //     CTAs then go where there is room beside the running kernel, and a small quantizer after a GEMM on 64 of 74 cluster pairs
@@ -358,6 +358,12 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap,
         ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar_cluster_addr)
         : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* tmap, int x, int y, int z, uint32_t bar_cluster_addr) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+        ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(bar_cluster_addr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_dst, uint32_t ncols) {  // one warp in each CTA of the pair
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_dst), "r"(ncols) : "memory");
 }
@@ -390,31 +396,13 @@ constexpr uint32_t kDescHiSw128 = (uint32_t)(((uint64_t)(1024 >> 4) << 32 | (1ul
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
 // Pair MMA taking the descriptors as (low word, shared high word): the issuing thread's instruction count is
 // what bounds the tensor pipe, so nothing 64-bit is computed per instruction.
-// KIND 0: int8 x int8 -> int32 (kind::i8); KIND 1: bf16 x bf16 -> f32 (kind::f16), 32 bytes of K per instruction either way.
-template <int KIND>
 __device__ __forceinline__ void umma_pair_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
-    if constexpr (KIND == 0) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "mov.b64 da, {%1, %5};\n\t"
-            "mov.b64 db, {%2, %5};\n\t"
-            "tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %3, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128)
-            : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "mov.b64 da, {%1, %5};\n\t"
-            "mov.b64 db, {%2, %5};\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %3, p;\n\t}"
-            ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128)
-            : "memory");
-    }
-}
-// Instruction descriptor for kind::f16 with bf16 operands and f32 accumulators: D f32 (bits 4-5 = 1), A and B bf16
-// (bits 7-9, 10-12 = 1), both K-major, N >> 3 in bits 17-22, M >> 4 in bits 24-28.
-__host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], da, db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128)
+        : "memory");
 }

@@ -186,12 +186,7 @@ __host__ __device__ constexpr uint32_t act_lut_pattern(uint32_t i) {   // bf16 p
 __device__ __forceinline__ uint32_t act_lut_index(uint32_t b) { return (b & 0x7ffu) | ((b >> 4) & 0x800u); }
 constexpr int kActLutBytes = 2 * (int)kActLutHalf * 2;
 
-// Accumulator word -> float: int32 sums of the int8 kernel (KIND 0), or the f32 sums of the bf16 kernel (KIND 1) as they are.
-template <int KIND> __device__ __forceinline__ float acc_f(uint32_t r) {
-    return KIND == 0 ? __int2float_rn((int)r) : __uint_as_float(r);
-}
-
-template <typename OutT, int EPI, int VS = 128, int KIND = 0>
+template <typename OutT, int EPI, int VS = 128>
 __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r, int row, int col, float xs_r, bool vec,
                                           float (&y)[8], const float* vs = nullptr, const uint16_t* lut_sm = nullptr,
                                           bool have_resid8 = false, const uint4 resid8 = uint4{0, 0, 0, 0}) {
@@ -240,7 +235,7 @@ __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r
     }
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-        const float t0 = __fmul_rn(acc_f<KIND>(r[e]), xs_r);
+        const float t0 = __fmul_rn(__int2float_rn((int)r[e]), xs_r);
         float v = rnd<OutT>(__fmaf_rn(t0, w8[e], b8[e]));
         if (EPI == EPI_RESID) v = __fmaf_rn(v, rs8[e], rr[e]);
         else if (EPI == EPI_ACT_LUT) {
@@ -368,7 +363,7 @@ __device__ __forceinline__ float max3_abs_nan_u(float m, uint32_t a, uint32_t b)
 
 // One 32-column chunk of one accumulator row, written straight to global memory (the path for outputs whose row
 // pitch or base TMA cannot address, and for ragged N).
-template <typename OutT, int EPI, int KIND = 0>
+template <typename OutT, int EPI>
 __device__ __forceinline__ void chunk_direct(const GemmParams& p, const uint32_t (&r)[32], int row, int col0, float xs_r) {
     if (EPI == EPI_ACC) {
         int32_t* d = reinterpret_cast<int32_t*>(p.D) + (int64_t)row * p.N + col0;
@@ -388,7 +383,7 @@ __device__ __forceinline__ void chunk_direct(const GemmParams& p, const uint32_t
         if (col0 + j >= p.N) break;
         const bool vec = p.vec_ok && col0 + j + 8 <= p.N;
         float y[8];
-        epilogue8<OutT, EPI, 128, KIND>(p, r + j, row, col0 + j, xs_r, vec, y);
+        epilogue8<OutT, EPI, 128>(p, r + j, row, col0 + j, xs_r, vec, y);
         if (vec) {
             if constexpr (sizeof(OutT) == 2) {
                 *reinterpret_cast<uint4*>(d + j) = pack8<OutT>(y);
@@ -408,7 +403,7 @@ __device__ __forceinline__ void chunk_direct(const GemmParams& p, const uint32_t
 // (2-byte outputs) or 128-byte (4-byte outputs) swizzle expects: row r at r * pitch, its 16-byte piece j at
 // piece j ^ f(r). Eight consecutive lanes then hit eight different bank groups.
 // 2-byte outputs: the chunk's 32 values of this lane's row, computed and packed (no shared-memory traffic yet)
-template <typename OutT, int EPI, int VS = 128, int KIND = 0>
+template <typename OutT, int EPI, int VS = 128>
 __device__ __forceinline__ void chunk_compute16(const GemmParams& p, const uint32_t (&r)[32], int row, int col0, float xs_r,
                                                 const float* vs, uint4 (&pk)[4], const uint16_t* lut_sm = nullptr) {
 #pragma unroll
@@ -417,19 +412,19 @@ __device__ __forceinline__ void chunk_compute16(const GemmParams& p, const uint3
             pk[j] = epilogue8_lut<VS>(p, r + 8 * j, xs_r, vs + 8 * j, lut_sm);
         } else {
             float y[8];
-            epilogue8<OutT, EPI, VS, KIND>(p, r + 8 * j, row, col0 + 8 * j, xs_r, p.vec_ok && col0 + 8 * j + 8 <= p.N, y, vs + 8 * j, lut_sm);
+            epilogue8<OutT, EPI, VS>(p, r + 8 * j, row, col0 + 8 * j, xs_r, p.vec_ok && col0 + 8 * j + 8 <= p.N, y, vs + 8 * j, lut_sm);
             if constexpr (sizeof(OutT) == 2) pk[j] = pack8<OutT>(y);
         }
     }
 }
 // The residual form of the same with the residual's four 16-byte pieces of this row already fetched by the caller
-template <typename OutT, int VS = 128, int KIND = 0>
+template <typename OutT, int VS = 128>
 __device__ __forceinline__ void chunk_compute16_resid(const GemmParams& p, const uint32_t (&r)[32], int row, int col0, float xs_r,
                                                       const float* vs, uint4 (&pk)[4], const uint4 (&rq)[4]) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
         float y[8];
-        epilogue8<OutT, EPI_RESID, VS, KIND>(p, r + 8 * j, row, col0 + 8 * j, xs_r, true, y, vs + 8 * j, nullptr, true, rq[j]);
+        epilogue8<OutT, EPI_RESID, VS>(p, r + 8 * j, row, col0 + 8 * j, xs_r, true, y, vs + 8 * j, nullptr, true, rq[j]);
         if constexpr (sizeof(OutT) == 2) pk[j] = pack8<OutT>(y);
     }
 }
@@ -440,7 +435,7 @@ __device__ __forceinline__ void chunk_write16(const uint4 (&pk)[4], uint8_t* sta
     for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(rowp + ((j ^ sw) << 4)) = pk[j];
 }
 
-template <typename OutT, int EPI, int KIND = 0>
+template <typename OutT, int EPI>
 __device__ __forceinline__ void chunk_to_smem(const GemmParams& p, const uint32_t (&r)[32], int row, int col0, float xs_r,
                                               uint8_t* stage, int lane) {
     constexpr int kEsz = EPI == EPI_ACC ? 4 : (int)sizeof(OutT);
@@ -456,7 +451,7 @@ __device__ __forceinline__ void chunk_to_smem(const GemmParams& p, const uint32_
 #pragma unroll
                 for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(r[8 * j + e]);  // raw int32 bits
             } else {
-                epilogue8<OutT, EPI, 128, KIND>(p, r + 8 * j, row, col0 + 8 * j, xs_r, p.vec_ok && col0 + 8 * j + 8 <= p.N, y);
+                epilogue8<OutT, EPI, 128>(p, r + 8 * j, row, col0 + 8 * j, xs_r, p.vec_ok && col0 + 8 * j + 8 <= p.N, y);
             }
             *reinterpret_cast<float4*>(rowp + (((2 * j) ^ sw) << 4)) = make_float4(y[0], y[1], y[2], y[3]);
             *reinterpret_cast<float4*>(rowp + (((2 * j + 1) ^ sw) << 4)) = make_float4(y[4], y[5], y[6], y[7]);
@@ -698,7 +693,7 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
                                           // themselves are complete when the grid is)
 }
 
-template <typename OutT, int EPI, int KIND = 0>
+template <typename OutT, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EPI == EPI_ACT_ROT ? kRotThreads : kThreads, 1)
 gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                     const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
@@ -709,16 +704,12 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const int S = p.stages;
     const int BN = p.bn;
     const int KS = p.ksub;
-    const int KA = KIND == 1 ? 2 : KS, KB = KIND == 1 ? 1 : KS;   // boxes of A and W in a stage (KIND 1: both terms of A, one W)
-    // KIND 1 has two accumulators per tile: two tiles' worth fit the tensor memory up to 128 columns, one tile's beyond
-    const bool one_buf = KIND == 1 && BN > 128;
-    const uint32_t lo_acc = one_buf ? 256u : 128u;
     const uint32_t a_bytes = BM * BK;                     // one 128-byte K box of this CTA's A rows
     const uint32_t b_bytes = (uint32_t)(BN / 2) * BK;     // ... and of this CTA's half of the W tile
-    const uint32_t stage_bytes = KA * a_bytes + KB * b_bytes;
+    const uint32_t stage_bytes = KS * (a_bytes + b_bytes);
     uint8_t* staging = sm;                                 // kEpiWarps x 4 KB of output staging
-    const uint32_t sA = base + kStagingBytes;              // S x KA x [128 x 128]
-    const uint32_t sB = sA + S * KA * a_bytes;             // S x KB x [bn/2 x 128]
+    const uint32_t sA = base + kStagingBytes;              // S x KS x [128 x 128]
+    const uint32_t sB = sA + S * KS * a_bytes;             // S x KS x [bn/2 x 128]
     uint8_t* tail = sm + kStagingBytes + S * stage_bytes;
     const uint32_t bar_full = smem_u32(tail);              // kMaxStages barriers (the leader's are used)
     const uint32_t bar_empty = bar_full + 8 * kMaxStages;  // kMaxStages, one set per CTA
@@ -784,11 +775,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     if (!mbar_wait(bar_empty + 8 * stage, phase ^ 1u, abort_s, ST_TIMEOUT_EMPTY)) { ok = false; break; }
                     if (leader) mbar_arrive_expect_tx(bar_full + 8 * stage, 2 * stage_bytes);
                     const uint32_t full = mapa_shared(bar_full + 8 * stage, 0);
-                    if constexpr (KIND == 1) {      // rows of the low terms follow the M rows of the high ones
-                        tma_load_2d_pair(sA + 2 * stage * a_bytes, &tmap_a, kb * BK, row_a, full);
-                        tma_load_2d_pair(sA + (2 * stage + 1) * a_bytes, &tmap_a, kb * BK, p.M + row_a, full);
-                        tma_load_2d_pair(sB + stage * b_bytes, &tmap_w, kb * BK, row_w, full);
-                    } else for (int ks = 0; ks < KS; ++ks) {
+                    for (int ks = 0; ks < KS; ++ks) {
                         tma_load_2d_pair(sA + (stage * KS + ks) * a_bytes, &tmap_a, (kb * KS + ks) * BK, row_a, full);
                         tma_load_2d_pair(sB + (stage * KS + ks) * b_bytes, &tmap_w, (kb * KS + ks) * BK, row_w, full);
                     }
@@ -807,7 +794,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if (leader && lane == 0) {
             const uint32_t a_lo0 = umma_desc_lo(sA), b_lo0 = umma_desc_lo(sB);
             const uint32_t a_sub = a_bytes >> 4, b_sub = b_bytes >> 4;        // next K box of a stage
-            const uint32_t a_step = KA * a_sub, b_step = KB * b_sub;          // next stage
+            const uint32_t a_step = KS * a_sub, b_step = KS * b_sub;          // next stage
             const uint32_t idesc = p.idesc;
             int stage = 0;
             uint32_t phase = 0;
@@ -825,22 +812,16 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                         if (!mbar_wait(bar_f, phase, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
                     }
                     {
-                        umma_pair_lo<KIND>(d_tmem, a_lo, b_lo, idesc, kb);
-                        umma_pair_lo<KIND>(d_tmem, a_lo + 2, b_lo + 2, idesc, 1);   // +32 bytes inside the swizzle row
-                        umma_pair_lo<KIND>(d_tmem, a_lo + 4, b_lo + 4, idesc, 1);
-                        umma_pair_lo<KIND>(d_tmem, a_lo + 6, b_lo + 6, idesc, 1);
-                        if constexpr (KIND == 1) {      // the low terms meet in an accumulator of their own
-                            const uint32_t a2 = a_lo + a_sub, d2 = d_tmem + lo_acc;
-                            umma_pair_lo<KIND>(d2, a2, b_lo, idesc, kb);
-                            umma_pair_lo<KIND>(d2, a2 + 2, b_lo + 2, idesc, 1);
-                            umma_pair_lo<KIND>(d2, a2 + 4, b_lo + 4, idesc, 1);
-                            umma_pair_lo<KIND>(d2, a2 + 6, b_lo + 6, idesc, 1);
-                        } else if (KS == 2) {
+                        umma_pair_lo(d_tmem, a_lo, b_lo, idesc, kb);
+                        umma_pair_lo(d_tmem, a_lo + 2, b_lo + 2, idesc, 1);   // +32 bytes inside the swizzle row
+                        umma_pair_lo(d_tmem, a_lo + 4, b_lo + 4, idesc, 1);
+                        umma_pair_lo(d_tmem, a_lo + 6, b_lo + 6, idesc, 1);
+                        if (KS == 2) {
                             const uint32_t a2 = a_lo + a_sub, b2 = b_lo + b_sub;
-                            umma_pair_lo<KIND>(d_tmem, a2, b2, idesc, 1);
-                            umma_pair_lo<KIND>(d_tmem, a2 + 2, b2 + 2, idesc, 1);
-                            umma_pair_lo<KIND>(d_tmem, a2 + 4, b2 + 4, idesc, 1);
-                            umma_pair_lo<KIND>(d_tmem, a2 + 6, b2 + 6, idesc, 1);
+                            umma_pair_lo(d_tmem, a2, b2, idesc, 1);
+                            umma_pair_lo(d_tmem, a2 + 2, b2 + 2, idesc, 1);
+                            umma_pair_lo(d_tmem, a2 + 4, b2 + 4, idesc, 1);
+                            umma_pair_lo(d_tmem, a2 + 6, b2 + 6, idesc, 1);
                         }
                     }
                     umma_commit_pair(bar_e);   // the stage is free in both CTAs once these MMAs have read it
@@ -849,7 +830,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 }
                 if (!ok) break;
                 umma_commit_pair(bar_tfull + 8 * buf);   // accumulator complete: both epilogues may drain it
-                if (!one_buf) buf ^= 1;
+                buf ^= 1;
                 if (buf == 0) tphase ^= 1u;
             }
         }
@@ -908,14 +889,14 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                 if (p.tma_store) {
                     if constexpr (kStageVec) {
                         uint4 pk[4];
-                        chunk_compute16<OutT, EPI, 128, KIND>(p, r, rrow, col0, xs_r, my_vec + 32 * ((c - half) >> 1), pk, lut_sm);
+                        chunk_compute16<OutT, EPI, 128>(p, r, rrow, col0, xs_r, my_vec + 32 * ((c - half) >> 1), pk, lut_sm);
                         if (lane == 0) bulk_wait_read<0>();   // the previous chunk's store has read the buffer
                         __syncwarp();
                         chunk_write16(pk, my_stage, lane);
                     } else {
                         if (lane == 0) bulk_wait_read<0>();
                         __syncwarp();
-                        chunk_to_smem<OutT, EPI, KIND>(p, r, rrow, col0, xs_r, my_stage, lane);
+                        chunk_to_smem<OutT, EPI>(p, r, rrow, col0, xs_r, my_stage, lane);
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
@@ -924,7 +905,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                         bulk_commit();
                     }
                 } else if (row_ok) {
-                    chunk_direct<OutT, EPI, KIND>(p, r, row, col0, xs_r);
+                    chunk_direct<OutT, EPI>(p, r, row, col0, xs_r);
                 }
             };
             constexpr bool kResidStaged = EPI == EPI_RESID && kStageVec;
@@ -941,7 +922,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     };
                     auto finish = [&](const uint32_t (&r)[32], const uint4 (&rq)[4], int c) {
                         uint4 pk[4];
-                        chunk_compute16_resid<OutT, 128, KIND>(p, r, rrow, n0 + c * 32, xs_r, my_vec + 32 * ((c - half) >> 1), pk, rq);
+                        chunk_compute16_resid<OutT, 128>(p, r, rrow, n0 + c * 32, xs_r, my_vec + 32 * ((c - half) >> 1), pk, rq);
                         if (lane == 0) bulk_wait_read<0>();   // the previous chunk's store has read the buffer
                         __syncwarp();
                         chunk_write16(pk, my_stage, lane);
@@ -978,16 +959,6 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                             emit(ra, c);
                         }
                     }
-                }
-            } else if (KIND == 1) {
-#pragma unroll 1
-                for (int c = half; c < nchunks; c += 2) {
-                    tmem_ld32(taddr + c * 32, ra);
-                    tmem_ld32(taddr + lo_acc + c * 32, rb);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) ra[e] = __float_as_uint(__fadd_rn(__uint_as_float(ra[e]), __uint_as_float(rb[e])));
-                    emit(ra, c);
                 }
             } else if (!kResidStaged && wi.kind == ITEM_WHOLE) {
                 int c = half;
@@ -1037,7 +1008,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(mapa_shared(bar_tempty + 8 * buf, 0));
-            if (!one_buf) buf ^= 1;
+            buf ^= 1;
             if (buf == 0) tphase ^= 1u;
         }
         if (p.tma_store && lane == 0) bulk_wait_read<0>();   // staged rows have left shared memory before the CTA exits
@@ -1153,7 +1124,7 @@ gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                 if (col0 >= p.N) break;
                 tmem_ld32(taddr + c * 32, r);
                 tmem_ld_wait();
-                if (row_ok) chunk_direct<OutT, EPI, 0>(p, r, row, col0, xs_r);
+                if (row_ok) chunk_direct<OutT, EPI>(p, r, row, col0, xs_r);
             }
         }
     }
@@ -1302,10 +1273,10 @@ int device_sm_count(int dev) {
     return c;
 }
 
-template <typename OutT, int EPI, int KIND = 0>
+template <typename OutT, int EPI>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, const GemmParams& p, int grid,
                 cudaStream_t st) {
-    auto kern = gemm_i8_pair_kernel<OutT, EPI, KIND>;
+    auto kern = gemm_i8_pair_kernel<OutT, EPI>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1572,68 +1543,7 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
     return rc;
 }
 
-// ---- weight-only int8 linear (the text encoders' path) ---------------------------------------------------------------
-// int8 codes are exact in bf16, so W goes to the tensor cores as bf16 without loss; the f32 activation goes as two bf16
-// terms (hi + lo = 16 significant bits) into two f32 accumulators, added in the epilogue: close to an fp32 product at
-// tensor-core speed. The kernel is the int8 one with kind::f16 MMAs (bf16 operands are addressed as rows of 2 K bytes); a
-// stage holds a K box of both terms and the one box of W that multiplies them. As two launches, the second adding to the
-// output of the first, W was read and D written twice: 512 x 2560 -> 19456 took 160 us with its
-// rotation and widening, now 127. (Tiles of at most 128 columns, whose accumulators fit the tensor memory twice, were slower, 271
-// against 252 us for the layer's MLP: what they read from L2 costs more than the epilogue that wider ones leave uncovered.)
-__global__ void __launch_bounds__(256) widen_i8_bf16_kernel(const int8_t* q, bf16* out, int64_t n16) {
-    pdl_wait();
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n16) return;
-    const uint4 v = gload(reinterpret_cast<const uint4*>(q) + i);
-    pdl_trigger();
-    const int8_t* b = reinterpret_cast<const int8_t*>(&v);
-    __nv_bfloat162 o[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[e] = __floats2bfloat162_rn((float)b[2 * e], (float)b[2 * e + 1]);
-    reinterpret_cast<uint4*>(out)[2 * i] = *reinterpret_cast<const uint4*>(&o[0]);
-    reinterpret_cast<uint4*>(out)[2 * i + 1] = *reinterpret_cast<const uint4*>(&o[4]);
-}
-
-// D[M,N] (f32) = [D +] ((A[0:M] + A[M:2M]) . W[N,K]^T) * ws[n], A (2 M rows: the high terms, then the low ones) and W bf16
-// row-major, K % 8 == 0, 16-byte aligned.
-int run_gemm_bf16(bool add, const void* A, const void* W, const float* ws, float* D, int64_t M, int64_t N, int64_t K, cudaStream_t st) {
-    if (M == 0 || N == 0 || K == 0) return 0;
-    if (M > INT32_MAX / 2 || N > INT32_MAX || K > INT32_MAX / 2) return -200;
-    if ((K % 8) != 0 || ((uintptr_t)A & 15) || ((uintptr_t)W & 15) || ((uintptr_t)D & 15)) return -202;
-    int dev = 0;
-    cudaGetDevice(&dev);
-    int clusters = device_sm_count(dev) / 2;
-    if (const int lim = g_cluster_limit.load(std::memory_order_relaxed); lim > 0 && lim < clusters) clusters = lim;
-    const int64_t Kb = 2 * K;                                   // bytes per row
-    GemmParams p{};
-    p.xs = nullptr, p.ws = ws, p.bias = nullptr, p.rscale = nullptr, p.resid = add ? D : nullptr, p.D = D;
-    p.M = (int)M, p.N = (int)N, p.K = (int)Kb;
-    auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
-    p.vec_ok = (N % 8 == 0) && al16(ws);
-    p.tma_store = (N * 4) % 16 == 0;
-    p.ksub = 1;
-    p.k_iters = (int)((Kb + BK - 1) / BK);
-    const int bn = choose_bn(M, N, clusters);
-    p.bn = bn;
-    p.idesc = umma_idesc_bf16(2 * BM, bn);
-    const int stage_bytes = 2 * BM * BK + (bn / 2) * BK;
-    const int stages = (kSmemBytes - 1024 - kTailBytes - kStagingBytes) / stage_bytes;
-    p.stages = stages > kMaxStages ? kMaxStages : stages;
-    p.tiles_m = (int)((M + 2 * BM - 1) / (2 * BM));
-    p.tiles_n = (int)((N + bn - 1) / bn);
-    p.num_tiles = p.tiles_m * p.tiles_n;
-    p.whole_tiles = p.num_tiles, p.splits = 0, p.kps = p.k_iters, p.num_items = p.num_tiles;
-    CUtensorMap ta, tw, td;
-    if (!make_operand_tmap(&ta, A, 2 * M, Kb, BM) || !make_operand_tmap(&tw, W, N, Kb, bn / 2)) return -203;
-    if (p.tma_store) {
-        if (!make_output_tmap(&td, D, M, N, 4)) return -203;
-    } else {
-        td = ta;
-    }
-    const int grid = 2 * (p.num_items < clusters ? p.num_items : clusters);
-    return add ? launch_pair<float, EPI_RESID, 1>(ta, tw, td, p, grid, st) : launch_pair<float, EPI_PLAIN, 1>(ta, tw, td, p, grid, st);
-}
-
+#include "gemm_wo8.inl"
 #include "gemm_w6.inl"
 
 }  // namespace
@@ -1669,8 +1579,8 @@ GPU_API int gpu_w6a8_gemm_acc_i32(const int8_t* A, const uint8_t* Wq6, const uin
 // New: the weight-only int8 linear of the text encoders in one call. The reference rotates the f32 activation rows
 // (gpu_rotate_rows_f32, csrc/kernels.cu:316-327), dequantizes the whole int8 weight to f32 (gpu_dequant_i8, :330-343) and runs
 // an fp32 GEMM with beta 0 or 1 (src/te.rs:493-511). Here: out[M,N] = beta * out + R256(prologue(x)) . (Wq * ws[n])^T with the
-// product on the bf16 tensor cores: Wq widens to bf16 exactly, the rotated rows go as hi + lo bf16 terms (one pass, f32
-// accumulators of their own), so the result is within about 2^-16 relative of the fp32 product's terms.
+// product on the int8 tensor cores: Wq as it is, the rotated rows as fixed-point numbers of 22 bits and sign in three 8-bit digits, one
+// power of two per row, so a value is within 2^-22 of its row's maximum and the rest is exact up to the f32 roundings at the end.
 //   prologue   PRO_PLAIN, PRO_RMS (norm_w, eps) or PRO_SWIGLU (up_offset) as gpu_rotate_rows_f32 takes them
 //   a_scratch  >= 4 * M * K bytes (the reference's rotated-rows buffer has that size), w_scratch >= 2 * N * K bytes
 //              (half of the reference's dequantized-weight buffer); both 16-byte aligned
@@ -1683,12 +1593,19 @@ GPU_API int gpu_wo8_linear(int prologue, const float* x, int64_t x_stride, int64
     if (M <= 0 || N <= 0) return 0;
     if ((((uintptr_t)a_scratch | (uintptr_t)w_scratch | (uintptr_t)Wq) & 15) || !a_scratch || !w_scratch) return -202;
     cudaStream_t st = (cudaStream_t)stream;
-    uint8_t* hi = reinterpret_cast<uint8_t*>(a_scratch);
-    uint8_t* lo = hi + (size_t)M * K * 2;               // one matrix of 2 M rows
-    if (int rc = rotate_rows_split(prologue, x, x_stride, up_offset, norm_w, eps, hi, lo, M, K, st)) return rc;
-    const int64_t n16 = (int64_t)N * K / 16;
-    if (int rc = launch_pdl(widen_i8_bf16_kernel, dim3((unsigned)((n16 + 255) / 256)), 256, 0, st, Wq, reinterpret_cast<bf16*>(w_scratch), n16)) return rc;
-    return run_gemm_bf16(beta == 1.f, hi, w_scratch, ws, out, M, N, K, st);
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int clusters = device_sm_count(dev) / 2;
+    if (const int lim = g_cluster_limit.load(std::memory_order_relaxed); lim > 0 && lim < clusters) clusters = lim;
+    const Wo8Plan plan = plan_wo8(M, N, K, clusters);
+    int8_t* digits = reinterpret_cast<int8_t*>(a_scratch);
+    float* factors = reinterpret_cast<float*>(digits + (size_t)3 * M * K);
+    if (int rc = rotate_rows_digits(prologue, x, x_stride, up_offset, norm_w, eps, digits, factors, reinterpret_cast<int*>(w_scratch),
+                                    plan.whole ? 0 : plan.clusters * kWo8Counters, M, K, st))
+        return rc;
+    if (M > INT32_MAX / 3 || plan.tiles == 0) return -200;
+    if ((uintptr_t)out & 15) return -202;
+    return run_wo8(beta == 1.f, plan, digits, factors, Wq, ws, out, w_scratch, M, N, K, st);
 }
 
 // D[M,N] = (A[M,K] . W[N,K]^T) * xs[m] * ws[n] + bias[n]; replaces the reference's csrc/gemm.cu:123-129.

@@ -84,10 +84,16 @@ struct QuantArgs {
     // shared-memory plan (byte offsets from the dynamic shared memory base), filled in by launch_quant
     int staged;             // rows arrive through the staging buffer (bulk copies) instead of direct loads
     uint32_t off_amax, off_norm, off_stage, off_bar;
-    // when set (with out_f unset): the rotated fp32 rows leave as two bf16 rows, hi = bf16(v) and lo = bf16(v - hi)
-    bf16* out_hi;
-    bf16* out_lo;
+    // when set (f32 rows, with q and out_f unset): the rotated rows leave as fixed-point numbers in three signed 8-bit digits, planes
+    // [3][M, K], the row's factor in `scales`; the first CTA zeroes nzero words at `zero` for the kernel that follows
+    int8_t* digits;
+    int* zero;
+    int nzero;
 };
+// prologues gpu_rotate_rows_f32 and the weight-only linear take
+template <typename T, int PRO> __host__ __device__ constexpr bool has_digits() {
+    return sizeof(T) == 4 && (PRO == PRO_PLAIN || PRO == PRO_RMS || PRO == PRO_SWIGLU);
+}
 
 template <int PRO> __host__ __device__ constexpr bool is_ln() { return PRO == PRO_LAYERNORM || PRO == PRO_LN_MOD || PRO == PRO_LN_AFFINE; }
 template <int PRO> __host__ __device__ constexpr bool is_norm() { return PRO == PRO_RMS || PRO == PRO_ADALN || is_ln<PRO>(); }
@@ -207,6 +213,53 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                  : "memory");
 }
 
+// The rotated values of a lane ((2 t8, 2 t8 + 1) + 16 r, pairs swapped when tsw) as the weight-only linear takes them:
+// x = (d0 2^16 + d1 2^8 + d2) f with signed 8-bit digits and one power of two f per row, chosen so that the row's maximum lies in
+// [2^21, 2^22): what rounds away is at most 2^-22 of the row's maximum. The product with the power of two is exact and rint comes with the
+// addition of 1.5 * 2^23. A row holding an infinity or a NaN gets the factor NaN.
+__device__ __forceinline__ void store_digits(float2 (&P)[16], float amax, const QuantArgs& p, bool live, int64_t m, int col, int tin, int tsw,
+                                             int t8, float* tbuf, unsigned wmask) {
+    float inv = 0.f, f = 0.f;
+    if (!(amax <= FLT_MAX)) f = __int_as_float(0x7fc00000);
+    else if (amax > 0.f) {
+        float back = 1.f;
+        if (amax < 0x1p-90f) {                      // the power of two would leave f32's range
+            amax *= 0x1p64f, back = 0x1p-64f;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) P[r] = __fmul2_rn(P[r], make_float2(0x1p64f, 0x1p64f));
+        }
+        const int k = (int)(__float_as_uint(amax) >> 23) - 127;
+        inv = __uint_as_float((uint32_t)(127 + 21 - k) << 23);
+        f = __uint_as_float((uint32_t)(127 - 21 + k) << 23) * back;
+    }
+    if (live && tin == 0) p.scales[m] = f;
+    uint32_t w[32];
+    const float2 inv2 = make_float2(inv, inv), magic = make_float2(12582912.f, 12582912.f);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const float2 t = __ffma2_rn(P[r], inv2, magic);
+        // 0x4B400000 + n; with 128 (2^16 + 2^8 + 1) added, the bytes are the digits plus 128
+        w[2 * r] = __float_as_uint(t.x) + (0x808080u - 0x4B400000u), w[2 * r + 1] = __float_as_uint(t.y) + (0x808080u - 0x4B400000u);
+    }
+    uint16_t* cb = reinterpret_cast<uint16_t*>(tbuf);
+    int8_t* q = p.digits + m * (int64_t)p.K + col;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const uint32_t pick = tsw ? (uint32_t)((6 - d) | (2 - d) << 4) : (uint32_t)((2 - d) | (6 - d) << 4);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) cb[t8 + 8 * r] = (uint16_t)__byte_perm(w[2 * r], w[2 * r + 1], pick);
+        __syncwarp(wmask);
+        uint4 lo = reinterpret_cast<const uint4*>(tbuf)[2 * t8], hi = reinterpret_cast<const uint4*>(tbuf)[2 * t8 + 1];
+        __syncwarp(wmask);
+        lo.x ^= 0x80808080u, lo.y ^= 0x80808080u, lo.z ^= 0x80808080u, lo.w ^= 0x80808080u;
+        hi.x ^= 0x80808080u, hi.y ^= 0x80808080u, hi.z ^= 0x80808080u, hi.w ^= 0x80808080u;
+        if (live) {
+            reinterpret_cast<uint4*>(q + d * (int64_t)p.M * p.K)[0] = lo;
+            reinterpret_cast<uint4*>(q + d * (int64_t)p.M * p.K)[1] = hi;
+        }
+    }
+}
+
 __device__ int g_quant_status = 0;   // a staging wait that ran out records ST_TIMEOUT_FULL here
 
 // MAXT = 384 asks for two CTAs per SM (at most 80 registers: 768 threads with the next block's rows in flight);
@@ -243,6 +296,10 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
         fence_mbar_init();
     }
     pdl_wait();
+    if constexpr (!DIRECT && has_digits<T, PRO>()) {
+        if (blockIdx.x == 0)
+            for (int i = threadIdx.x; i < p.nzero; i += blockDim.x) p.zero[i] = 0;
+    }
     __syncthreads();
 
     // Staging: the rows of block `blk` (and their second stream) -> the staging buffer, one bulk copy each, issued by
@@ -477,20 +534,6 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
             for (int i = 0; i < 16; ++i) P[i] = make_float2(v[2 * i], v[2 * i + 1]);   // natural order
         }
 
-        if (!DIRECT && p.out_hi) {  // the weight-only linear's activation side: rotated rows split into two bf16 terms
-            if (live) {
-                const int64_t o = m * (int64_t)p.K + (grp << 8) + 2 * t8;
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const float2 v2 = tsw ? make_float2(P[r].y, P[r].x) : P[r];
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(v2.x, v2.y);
-                    const float2 hf = __bfloat1622float2(h);
-                    *reinterpret_cast<__nv_bfloat162*>(p.out_hi + o + 16 * r) = h;
-                    *reinterpret_cast<__nv_bfloat162*>(p.out_lo + o + 16 * r) = __floats2bfloat162_rn(__fsub_rn(v2.x, hf.x), __fsub_rn(v2.y, hf.y));
-                }
-            }
-            continue;
-        }
         if (!DIRECT && p.out_f) {   // gpu_rotate_rows_f32: always rotated, so P holds (2 t8, 2 t8 + 1) + 16 r
             if (live) {
                 float* o = p.out_f + m * (int64_t)p.K + (grp << 8) + 2 * t8;
@@ -517,6 +560,9 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
         amax = fmaxf(amax, __shfl_xor_sync(wmask, amax, 4));
         unsigned* slot = amax_s + (it % 3) * p.rows_per_cta + rloc;
         if (t8 == 0) atomicMax(slot, __float_as_uint(amax));
+        if constexpr (!DIRECT && has_digits<T, PRO>()) {
+            if (p.digits && has_nan) atomicMax(slot, 0x7fc00000u);      // above every number: the row's factor becomes NaN
+        }
         __syncthreads();
         amax = __uint_as_float(*slot);
         if (DIRECT) pdl_trigger();
@@ -524,6 +570,13 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
         if (!DIRECT && p.amax_out) {
             if (live && tin == 0) p.amax_out[m] = amax;
             continue;
+        }
+        if constexpr (!DIRECT && has_digits<T, PRO>()) {
+            if (p.digits) {
+                pdl_trigger();
+                store_digits(P, amax, p, live, m, col, tin, tsw, t8, tbuf, wmask);
+                continue;
+            }
         }
         if (!DIRECT && p.amax_in) amax = p.amax_in[m];
 
@@ -1124,7 +1177,7 @@ int launch_quant(QuantArgs& p, cudaStream_t st) {
     const uintptr_t mis = (uintptr_t)p.x | (uintptr_t)(p.x_stride * sizeof(T)) |
                           (PRO == PRO_GATE ? (uintptr_t)p.g | (uintptr_t)(p.g_stride * sizeof(T)) : 0) |
                           (has_aux<PRO>() && PRO != PRO_GATE ? (uintptr_t)(p.up_offset * sizeof(T)) : 0) | (uintptr_t)p.q |
-                          (uintptr_t)p.out_f | (uintptr_t)p.out_hi | (uintptr_t)p.out_lo;
+                          (uintptr_t)p.out_f | (uintptr_t)p.digits;
     if (mis & 15) return -5;
     int lut = -1;
     if (sizeof(T) == 2 && (int64_t)p.M * p.K >= (1 << 20)) {
@@ -1160,7 +1213,7 @@ int launch_quant(QuantArgs& p, cudaStream_t st) {
     const size_t smem = p.staged ? off + stage_bytes : off;
     if (smem > kMaxSmem) return -2;
     if constexpr (direct_threads<T, PRO>() > 0) {
-        if (p.rotate && threads <= direct_threads<T, PRO>() && !p.out_f && !p.out_hi && !p.amax_in && !p.amax_out)
+        if (p.rotate && threads <= direct_threads<T, PRO>() && !p.out_f && !p.digits && !p.amax_in && !p.amax_out)
             return launch_cfg<T, PRO, direct_threads<T, PRO>(), true>(p, threads, smem, false, st);
     }
     if (threads > 512) return launch_cfg<T, PRO, 1024>(p, threads, smem, p.staged != 0, st);
@@ -1230,14 +1283,14 @@ GPU_API int gpu_rotate_rows_f32(int prologue, const float* x, int64_t x_stride, 
     }
 }
 
-// The same with the rotated rows written as two bf16 terms (hi + lo carries 16 significant bits of every value): the
-// A operand of the weight-only int8 linear on the bf16 tensor-core kernel.
-int b200q::rotate_rows_split(int prologue, const float* x, int64_t x_stride, int64_t up_offset, const float* norm_w, float eps,
-                             void* hi, void* lo, int M, int K, cudaStream_t st) {
+// The same with the rotated rows written as three 8-bit digits [3][M, K] and a factor per row: the activation side of the
+// weight-only linear on the int8 tensor cores. The first CTA zeroes `nzero` words at `zero`.
+int b200q::rotate_rows_digits(int prologue, const float* x, int64_t x_stride, int64_t up_offset, const float* norm_w, float eps,
+                              int8_t* digits, float* factors, int* zero, int nzero, int M, int K, cudaStream_t st) {
     if ((K % 256) != 0) return -1;
-    QuantArgs p{x, x_stride, nullptr, 0, up_offset, nullptr, nullptr, nullptr, M, K, 1, 0, 0, 0, -1, nullptr, nullptr,
+    QuantArgs p{x, x_stride, nullptr, 0, up_offset, nullptr, factors, nullptr, M, K, 1, 0, 0, 0, -1, nullptr, nullptr,
                 norm_w, nullptr, eps, nullptr, nullptr};
-    p.out_hi = reinterpret_cast<bf16*>(hi), p.out_lo = reinterpret_cast<bf16*>(lo);
+    p.digits = digits, p.zero = zero, p.nzero = nzero;
     switch (prologue) {
         case PRO_PLAIN: return launch_quant<float, PRO_PLAIN>(p, st);
         case PRO_RMS: return launch_quant<float, PRO_RMS>(p, st);

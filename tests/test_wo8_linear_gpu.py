@@ -1,6 +1,6 @@
 """The weight-only int8 linear of the text encoders (gpu_wo8_linear) against the reference's three-call flow: rotate the f32
 rows (gpu_rotate_rows_f32, bit-identical to the reference's kernel), dequantize the weight (gpu_dequant_i8, likewise), fp32
-product. The product here runs on the bf16 tensor cores with the activation split in two bf16 terms, so it is not
+product. The product here runs on the int8 tensor cores with the activation as fixed-point numbers in three 8-bit digits, so it is not
 bit-identical to an fp32 GEMM (which has no canonical summation order either); the tolerance is stated against the exact
 (fp64) product of the same rotated rows and dequantized weights: 1e-5 of the largest output magnitude, and no worse than
 three times the error of an fp32 GEMM of the same operands."""
@@ -71,6 +71,57 @@ def test_several_tiles_a_cluster_and_ragged_ones(pkg, dev, M, N, K, limit):
     assert bool((out[M] == 7.0).all())
     assert (acc.double() - (base.double() + exact)).abs().max().item() <= 1e-5 * max(scale, base.abs().max().item())
     assert L.kernel_status() == 0
+
+
+# Token tiles of 32 to 160, one and several, the last one ragged; columns around the 256 of a tile; tiles whose K boxes one, two or many
+# clusters share (K = 256 is two boxes, 9728 seventy-six), and whole ones where the scratch has no room for that (N = 8).
+@pytest.mark.parametrize("M,N,K", [(1, 8, 256), (20, 520, 9728), (32, 256, 1024), (33, 1000, 2560), (160, 257, 512), (161, 2560, 9728), (330, 255, 4096),
+                                   (513, 5120, 768), (1024, 3584, 1280)])
+def test_digits_keep_a_row_to_22_bits_of_its_maximum(pkg, dev, M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    L = pkg.linear
+    x = torch.randn(M, K, generator=g)
+    x *= torch.exp2(torch.randint(-40, 40, (M, 1), generator=g).float())      # every row has a power of two of its own
+    x[:, 5] *= 40.0
+    x = x.to(dev)
+    Wq, ws = L.convrot_requant((torch.randn(N, K, generator=g) * 0.03).to(dev), 0)
+    xr, wf = L.rotate_rows_f32(x, PLAIN).double(), L.dequant_i8(Wq, ws).double()
+    exact = xr @ wf.t()
+    # a value is off by at most 2^-22 of the row's maximum (half a step of 2^-21 of the power of two below it); the three exact sums are
+    # rounded once each when they become f32, then together, with the row's, the column's factor and, shared between clusters, once
+    # more per cluster
+    bound = xr.abs().amax(1, keepdim=True) * 2.0 ** -22 * wf.abs().sum(1) + exact.abs() * 2.0 ** -20 + xr.abs() @ wf.abs().t() * 2.0 ** -22
+    out = torch.full((M + 1, N), 7.0, device=dev)
+    L.wo8_linear(x, Wq, ws, PLAIN, out=out[:M])
+    assert bool(((out[:M].double() - exact).abs() <= bound).all()) and bool((out[M] == 7.0).all())
+    again = torch.empty(M, N, device=dev)
+    L.wo8_linear(x, Wq, ws, PLAIN, out=again)
+    assert torch.equal(again, out[:M])                             # whoever adds the shares up adds them in the same order
+    base = torch.randn(M, N, generator=g).to(dev)
+    acc = base.clone()
+    L.wo8_linear(x, Wq, ws, PLAIN, out=acc, beta=1.0)
+    assert torch.equal(acc, out[:M] + base)
+    assert L.kernel_status() == 0
+
+
+def test_rows_without_a_maximum(pkg, dev):
+    """Rows holding an infinity or a NaN give NaN, zero rows zero, rows near either end of f32's range their values."""
+    g = torch.Generator().manual_seed(3)
+    L = pkg.linear
+    N, K = 300, 512
+    x = torch.randn(9, K, generator=g)
+    x[1, 7], x[2, 300], x[3, 0] = float("inf"), float("nan"), -float("inf")
+    x[4] = 0.0
+    x[5] *= 2.0 ** 118
+    x[6] *= 2.0 ** -95
+    x[7] *= 2.0 ** -112
+    x = x.to(dev)
+    Wq, ws = L.convrot_requant((torch.randn(N, K, generator=g) * 0.03).to(dev), 0)
+    out = L.wo8_linear(x, Wq, ws, PLAIN)
+    exact = L.rotate_rows_f32(x, PLAIN).double() @ L.dequant_i8(Wq, ws).double().t()
+    assert bool(out[1:4].isnan().all()) and bool((out[4] == 0).all())
+    for m in (0, 5, 6, 7, 8):
+        assert (out[m].double() - exact[m]).abs().max().item() <= 2e-6 * exact[m].abs().max().item(), m
 
 
 def test_argument_checks(pkg, dev):
