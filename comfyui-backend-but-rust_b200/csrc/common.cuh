@@ -254,15 +254,6 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  // whole warp
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// D[tmem] (+)= A[smem desc] * B[smem desc], int8 x int8 -> int32, issued by one thread.
-__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // The mbarrier gets one arrival once every tcgen05.mma this thread issued before has completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -315,10 +306,9 @@ __device__ __forceinline__ void named_bar_sync(int id, int threads) {
 // start address >> 4 in bits [0,14); leading byte offset (unused for this layout) 1 in [16,30);
 // stride byte offset = 1024 B between 8-row groups, >> 4, in [32,46); descriptor version 1 in [46,48);
 // layout type 2 (128-byte swizzle) in [61,64).
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
-    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
+// As (low word, high word): all but the start address is the same for every tile.
+constexpr uint32_t kDescHiSw128 = (uint32_t)(((uint64_t)(1024 >> 4) << 32 | (1ull << 46) | (2ull << 61)) >> 32);
+__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
 // Instruction descriptor for kind::i8: D s32 (bits 4-5 = 2), A and B signed 8-bit (bits 7-9, 10-12 = 1),
 // both K-major (bits 15, 16 = 0), N >> 3 in bits 17-22, M >> 4 in bits 24-28, no saturation.
 __host__ __device__ constexpr uint32_t umma_idesc_i8(int m, int n) {
@@ -373,16 +363,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// One MMA over both SMs of the pair: D rows 0-127 accumulate in the leader's tensor memory, rows 128-255 in the
-// peer's; A comes from each CTA's own tile, B's N columns are split between the two CTAs' tiles.
-__device__ __forceinline__ void umma_i8_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // One arrival on the mbarrier at this shared-memory offset in BOTH CTAs of the pair, once every MMA this thread
 // issued for the pair has completed. (A commit's arrival may be multicast; the TMA loads of this library never are.)
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
@@ -391,11 +371,20 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                  : "memory");
 }
 
-// The high word of umma_desc_sw128(): everything but the start address.
-constexpr uint32_t kDescHiSw128 = (uint32_t)(((uint64_t)(1024 >> 4) << 32 | (1ull << 46) | (2ull << 61)) >> 32);
-__device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
-// Pair MMA taking the descriptors as (low word, shared high word): the issuing thread's instruction count is
-// what bounds the tensor pipe, so nothing 64-bit is computed per instruction.
+// D[tmem] (+)= A[smem desc] * B[smem desc], int8 x int8 -> int32, issued by one thread, which takes the descriptors as (low word, shared
+// high word): its instruction count is what bounds the tensor pipe, so nothing 64-bit is computed per instruction.
+__device__ __forceinline__ void umma_i8_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %5};\n\t"
+        "mov.b64 db, {%2, %5};\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], da, db, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(idesc), "r"(accumulate), "r"(kDescHiSw128)
+        : "memory");
+}
+// The same over both SMs of a pair: D rows 0-127 accumulate in the leader's tensor memory, rows 128-255 in the peer's; A comes from
+// each CTA's own tile, B's N columns are split between the two CTAs' tiles.
 __device__ __forceinline__ void umma_pair_lo(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"

@@ -68,6 +68,7 @@ struct GemmParams {
     int act;
     int vec_ok;          // per-column vectors and rows of D / resid can be read and written 16 bytes at a time
     int tma_store;       // D is written through shared memory with TMA stores
+    int wide;            // 2-byte outputs in whole tiles straight from registers: 2 when rows of D can be written 32 bytes at a time, 1: 16
     int bn;              // columns per tile (multiple of 32, <= 256); each CTA of the pair stages bn/2 rows of W
     int stages;          // shared-memory ring depth
     int ksub;            // 128-byte K boxes per stage (1 or 2): one barrier round trip per 4 or 8 MMAs
@@ -149,22 +150,6 @@ template <> __device__ __forceinline__ void load8<half>(const half* p, float (&y
     }
 }
 
-// 8 two-byte values held in a register quad -> floats (no address is taken: the quad stays in registers)
-template <typename OutT> __device__ __forceinline__ void unpack8(const uint4 u, float (&y)[8]) {
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if constexpr (std::is_same<OutT, bf16>::value) {
-            y[2 * i] = __uint_as_float(w[i] << 16), y[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-        } else if constexpr (std::is_same<OutT, half>::value) {
-            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-            y[2 * i] = f.x, y[2 * i + 1] = f.y;
-        } else {
-            y[2 * i] = 0.f, y[2 * i + 1] = 0.f;
-        }
-    }
-}
-
 // The epilogue arithmetic on 8 consecutive columns of one row (accumulators r[0..7] -> y[0..7], not yet rounded
 // to the output type for the last step; the store rounds).
 //   t0 = float(acc) * xs;  v = out(fma(t0, ws, bias));  RESID: fma(v, rscale, resid);  ACT: act(v)
@@ -188,8 +173,7 @@ constexpr int kActLutBytes = 2 * (int)kActLutHalf * 2;
 
 template <typename OutT, int EPI, int VS = 128>
 __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r, int row, int col, float xs_r, bool vec,
-                                          float (&y)[8], const float* vs = nullptr, const uint16_t* lut_sm = nullptr,
-                                          bool have_resid8 = false, const uint4 resid8 = uint4{0, 0, 0, 0}) {
+                                          float (&y)[8], const float* vs = nullptr, const uint16_t* lut_sm = nullptr) {
     float w8[8], b8[8], rs8[8], rr[8];
     const OutT* rsd = reinterpret_cast<const OutT*>(p.resid) + (int64_t)row * p.N + col;
     if (vs) {
@@ -197,8 +181,7 @@ __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r
         load8<float>(vs + VS, b8);
         if (EPI == EPI_RESID) {
             load8<float>(vs + 2 * VS, rs8);
-            if (have_resid8) unpack8<OutT>(resid8, rr);      // fetched by the caller, 8 two-byte values
-            else if (vec) load8<OutT>(rsd, rr);
+            if (vec) load8<OutT>(rsd, rr);
             else {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) rr[e] = col + e < p.N ? to_f<OutT>(rsd[e]) : 0.f;
@@ -417,17 +400,6 @@ __device__ __forceinline__ void chunk_compute16(const GemmParams& p, const uint3
         }
     }
 }
-// The residual form of the same with the residual's four 16-byte pieces of this row already fetched by the caller
-template <typename OutT, int VS = 128>
-__device__ __forceinline__ void chunk_compute16_resid(const GemmParams& p, const uint32_t (&r)[32], int row, int col0, float xs_r,
-                                                      const float* vs, uint4 (&pk)[4], const uint4 (&rq)[4]) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        float y[8];
-        epilogue8<OutT, EPI_RESID, VS>(p, r + 8 * j, row, col0 + 8 * j, xs_r, true, y, vs + 8 * j, nullptr, true, rq[j]);
-        if constexpr (sizeof(OutT) == 2) pk[j] = pack8<OutT>(y);
-    }
-}
 __device__ __forceinline__ void chunk_write16(const uint4 (&pk)[4], uint8_t* stage, int lane) {
     uint8_t* rowp = stage + lane * 64;
     const int sw = (lane >> 1) & 3;
@@ -468,6 +440,190 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void bulk_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
+
+// ---- draining a tile into 2-byte outputs ------------------------------------------------------------------------------------
+// What a warp does with up to four 32-column chunks of 32 accumulator rows: dequantize, bias, activation or residual, and 32
+// contiguous bytes per lane and store (whole sectors: no staging in shared memory, no fence, nothing to wait for). With a short K
+// this is what sets a tile's pace, so nothing of it is waited for in the drain itself: the per-column vectors, the row scale and
+// the residual of the whole tile are requested before the accumulator is awaited, and the accumulator is handed back as soon as
+// the last chunk is out of tensor memory. %DRAIN%
+__device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+template <typename OutT> __device__ __forceinline__ uint32_t pack2(float2 v) {
+    if constexpr (std::is_same<OutT, bf16>::value) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    } else {
+        const __half2 h = __floats2half2_rn(v.x, v.y);
+        return *reinterpret_cast<const uint32_t*>(&h);
+    }
+}
+template <typename OutT> __device__ __forceinline__ float2 unpack2(uint32_t w) {
+    if constexpr (std::is_same<OutT, bf16>::value) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    else return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+// A warp's per-column vectors of a tile, and the row scale of its lanes: fetched a tile ahead, kept in shared memory while in use
+struct DrainVecs {
+    float ws[4], b[4], rs[4], xs;
+    template <typename OutT, int EPI>
+    __device__ __forceinline__ void fetch(const GemmParams& p, int row, int col0, int chunks, int lane) {
+        xs = p.xs ? gload(p.xs + min(row, p.M - 1)) : 1.f;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int n = col0 + 32 * k + lane;
+            const bool in = k < chunks && n < p.N;
+            ws[k] = in ? gload(p.ws + n) : 0.f;
+            b[k] = in && p.bias ? to_f<OutT>(gload(reinterpret_cast<const OutT*>(p.bias) + n)) : 0.f;
+            if (EPI == EPI_RESID) rs[k] = !in ? 0.f : p.rscale ? to_f<OutT>(gload(reinterpret_cast<const OutT*>(p.rscale) + n)) : 1.f;
+        }
+    }
+    template <int EPI> __device__ __forceinline__ void stage(float* vec, int lane) const {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            vec[32 * k + lane] = ws[k];
+            vec[128 + 32 * k + lane] = b[k];
+            if (EPI == EPI_RESID) vec[256 + 32 * k + lane] = rs[k];
+        }
+        __syncwarp();
+    }
+};
+// The residual's 64 bytes of a lane's row and chunk; nothing beyond the matrix is read (N % 8 == 0)
+template <typename OutT>
+__device__ __forceinline__ void drain_resid(const GemmParams& p, uint4 (&rq)[4], int row, int col) {
+    const uint4* r = reinterpret_cast<const uint4*>(reinterpret_cast<const OutT*>(p.resid) + (int64_t)row * p.N + col);
+    const bool row_ok = row < p.M;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) rq[j] = row_ok && col + 8 * j < p.N ? gload(r + j) : make_uint4(0, 0, 0, 0);
+}
+template <typename OutT, int EPI>
+__device__ __forceinline__ void drain_chunk(const GemmParams& p, const uint32_t (&r)[32], const uint4 (&rq)[4], int row, int col, float xs,
+                                            const float* vs, const uint16_t* lut_sm) {
+    const float2 xs2 = make_float2(xs, xs);
+    OutT* d = reinterpret_cast<OutT*>(p.D) + (int64_t)row * p.N + col;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        uint32_t o[8];
+        if constexpr (EPI == EPI_ACT_LUT) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const uint4 t = epilogue8_lut<128>(p, r + 16 * u + 8 * j, xs, vs + 16 * u + 8 * j, lut_sm);
+                o[4 * j] = t.x, o[4 * j + 1] = t.y, o[4 * j + 2] = t.z, o[4 * j + 3] = t.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int c = 16 * u + 4 * j;
+                const float4 w = *reinterpret_cast<const float4*>(vs + c), b = *reinterpret_cast<const float4*>(vs + 128 + c);
+                float2 v0 = __ffma2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[c]), __int2float_rn((int)r[c + 1])), xs2), make_float2(w.x, w.y),
+                                       make_float2(b.x, b.y));
+                float2 v1 = __ffma2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[c + 2]), __int2float_rn((int)r[c + 3])), xs2),
+                                       make_float2(w.z, w.w), make_float2(b.z, b.w));
+                if constexpr (EPI == EPI_RESID) {
+                    const float4 s = *reinterpret_cast<const float4*>(vs + 256 + c);
+                    const uint4 q = rq[2 * u + (j >> 1)];
+                    v0 = __ffma2_rn(unpack2<OutT>(pack2<OutT>(v0)), make_float2(s.x, s.y), unpack2<OutT>(j & 1 ? q.z : q.x));
+                    v1 = __ffma2_rn(unpack2<OutT>(pack2<OutT>(v1)), make_float2(s.z, s.w), unpack2<OutT>(j & 1 ? q.w : q.y));
+                }
+                o[2 * j] = pack2<OutT>(v0), o[2 * j + 1] = pack2<OutT>(v1);
+            }
+        }
+        if (row < p.M && col + 16 * u < p.N) {
+            if (p.wide == 2) st_global_v8(d + 16 * u, o);
+            else {
+                *reinterpret_cast<uint4*>(d + 16 * u) = make_uint4(o[0], o[1], o[2], o[3]);
+                if (col + 16 * u + 8 < p.N) *reinterpret_cast<uint4*>(d + 16 * u + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+            }
+        }
+    }
+}
+// `chunks` chunks from column `col0` on; `taddr` the first one's tensor-memory address; `done` is called once when the last has been read.
+// rq: the residual of the chunks, already requested.
+template <typename OutT, int EPI, typename Done>
+__device__ __forceinline__ void drain_tile(const GemmParams& p, uint32_t taddr, int row, int col0, int chunks, float xs, const float* vec,
+                                           const uint16_t* lut_sm, const uint4 (&rq)[4][4], Done done) {
+    if constexpr (EPI == EPI_RESID) {      // unrolled: the residual sits in registers
+        uint32_t r[32];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c < chunks) {
+                tmem_ld32(taddr + 32 * c, r);
+                tmem_ld_wait();
+                if (c + 1 == chunks) done();
+                drain_chunk<OutT, EPI>(p, r, rq[c], row, col0 + 32 * c, xs, vec + 32 * c, lut_sm);
+            }
+        }
+    } else {
+        uint32_t ra[32], rb[32];           // the next chunk's load is in flight while one is processed
+        tmem_ld32(taddr, ra);
+#pragma unroll 1
+        for (int c = 0; c < chunks; c += 2) {
+            tmem_ld_wait();
+            if (c + 1 < chunks) tmem_ld32(taddr + 32 * (c + 1), rb);
+            else done();
+            drain_chunk<OutT, EPI>(p, ra, rq[0], row, col0 + 32 * c, xs, vec + 32 * c, lut_sm);
+            if (c + 1 < chunks) {
+                tmem_ld_wait();
+                if (c + 2 < chunks) tmem_ld32(taddr + 32 * (c + 2), ra);
+                else done();
+                drain_chunk<OutT, EPI>(p, rb, rq[0], row, col0 + 32 * (c + 1), xs, vec + 32 * (c + 1), lut_sm);
+            }
+        }
+    }
+}
+// The epilogue warps' loop of the pair kernel over whole tiles (p.wide)
+template <typename OutT, int EPI>
+__device__ __forceinline__ void epilogue_wide(const GemmParams& p, uint8_t* staging, uint32_t bar_tfull, uint32_t bar_tempty, uint32_t tmem_base,
+                                              volatile int* abort_s, int rank, int cluster_id, int nclusters, int warp, int lane) {
+    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;      // half: the tile's first or second half of chunks
+    const int nchunks = p.bn / 32, first = half * ((nchunks + 1) / 2), chunks = min((nchunks + 1) / 2, nchunks - first);
+    float* vec = reinterpret_cast<float*>(staging + kVecOffset + ew * (EPI == EPI_RESID ? 1536 : 1024));
+    const uint16_t* lut_sm = reinterpret_cast<const uint16_t*>(staging + kVecOffset + kEpiWarps * 1024);   // EPI_ACT_LUT only
+    int buf = 0;
+    uint32_t tphase = 0;
+    auto place = [&](int w, int& row, int& col0) {
+        int tm, tn;
+        tile_coords(w, p.tiles_m, p.tiles_n, tm, tn, p.group_m ? p.group_m : 8);
+        row = tm * (2 * BM) + rank * BM + quad * 32 + lane, col0 = tn * p.bn + 32 * first;
+    };
+    DrainVecs next;
+    int row, col0;
+    if (cluster_id < p.num_items) {
+        place(cluster_id, row, col0);
+        next.fetch<OutT, EPI>(p, row, col0, chunks, lane);
+    }
+    for (int w = cluster_id; w < p.num_items; w += nclusters) {
+        place(w, row, col0);
+        const float xs = next.xs;
+        next.stage<EPI>(vec, lane);
+        if (w + nclusters < p.num_items) {
+            int nrow, ncol;
+            place(w + nclusters, nrow, ncol);
+            next.fetch<OutT, EPI>(p, nrow, ncol, chunks, lane);
+        }
+        uint4 rq[4][4];
+        if constexpr (EPI == EPI_RESID) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (c < chunks) drain_resid<OutT>(p, rq[c], row, col0 + 32 * c);
+        }
+        bool ok = true;
+        if (lane == 0) ok = mbar_wait(bar_tfull + 8 * buf, tphase, abort_s, ST_TIMEOUT_TMEM_FULL);
+        if (!__shfl_sync(0xffffffffu, (int)ok, 0)) break;
+        tc_fence_after();
+        drain_tile<OutT, EPI>(p, tmem_base + buf * 256 + ((uint32_t)(quad * 32) << 16) + 32 * first, row, col0, chunks, xs, vec, lut_sm, rq, [&]() {
+            // no cluster-scope release: nothing but tensor memory, ordered by the tcgen05 fences, is handed over
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(mapa_shared(bar_tempty + 8 * buf, 0));
+        });
+        buf ^= 1;
+        if (buf == 0) tphase ^= 1u;
+    }
 }
 
 // ---- the rotating epilogue (EPI_ACT_ROT) --------------------------------------------------------------------------------
@@ -839,6 +995,9 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if constexpr (EPI == EPI_ACT_ROT) {
             epilogue_rot(p, &tmap_d, staging, tail, bar_tfull, bar_tempty, tmem_base, abort_s, (int)rank, cluster_id, nclusters, warp,
                          lane);
+        } else if (EPI != EPI_ACC && sizeof(OutT) == 2 && EPI != EPI_ACT && p.wide) {
+            if constexpr (EPI != EPI_ACC && sizeof(OutT) == 2 && EPI != EPI_ACT)
+                epilogue_wide<OutT, EPI>(p, staging, bar_tfull, bar_tempty, tmem_base, abort_s, (int)rank, cluster_id, nclusters, warp, lane);
         } else {
         constexpr int kEsz = EPI == EPI_ACC ? 4 : (int)sizeof(OutT);
         constexpr bool kStageVec = kEsz == 2;            // 2-byte outputs: 2 KB chunk + 1.5 KB of per-column vectors
@@ -908,59 +1067,7 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                     chunk_direct<OutT, EPI>(p, r, row, col0, xs_r);
                 }
             };
-            constexpr bool kResidStaged = EPI == EPI_RESID && kStageVec;
-            if (kResidStaged && wi.kind == ITEM_WHOLE) {
-                // Residual form. Fetched one by one in front of their eight columns, the residual's 16-byte pieces put four
-                // memory latencies per chunk on the drain of a cluster's last tile (this form was 13 us slower than the
-                // plain one on the down-projection). Here a chunk's four pieces are requested together, one chunk ahead
-                // of their use; the pieces take the place of the second accumulator register set.
-                if constexpr (kResidStaged) {
-                    auto pieces = [&](uint4 (&rq)[4], int c) {
-                        const uint4* rsd = reinterpret_cast<const uint4*>(reinterpret_cast<const OutT*>(p.resid) + (int64_t)rrow * p.N + n0 + c * 32);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) rq[j] = rsd[j];
-                    };
-                    auto finish = [&](const uint32_t (&r)[32], const uint4 (&rq)[4], int c) {
-                        uint4 pk[4];
-                        chunk_compute16_resid<OutT, 128>(p, r, rrow, n0 + c * 32, xs_r, my_vec + 32 * ((c - half) >> 1), pk, rq);
-                        if (lane == 0) bulk_wait_read<0>();   // the previous chunk's store has read the buffer
-                        __syncwarp();
-                        chunk_write16(pk, my_stage, lane);
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            tma_store_2d(&tmap_d, my_stage_u32, n0 + c * 32, row0);
-                            bulk_commit();
-                        }
-                    };
-                    if (staged && p.vec_ok && n0 + BN <= p.N) {
-                        uint4 qa[4], qb[4];
-                        int c = half;
-                        if (c < nchunks) pieces(qa, c);
-#pragma unroll 1
-                        for (; c < nchunks; c += 4) {
-                            tmem_ld32(taddr + c * 32, ra);
-                            if (c + 2 < nchunks) pieces(qb, c + 2);
-                            tmem_ld_wait();
-                            finish(ra, qa, c);
-                            if (c + 2 < nchunks) {
-                                tmem_ld32(taddr + (c + 2) * 32, ra);
-                                if (c + 4 < nchunks) pieces(qa, c + 4);
-                                tmem_ld_wait();
-                                finish(ra, qb, c + 2);
-                            }
-                        }
-                    } else {      // direct stores, unaligned vectors, a tile that reaches past N
-#pragma unroll 1
-                        for (int c = half; c < nchunks; c += 2) {
-                            if (n0 + c * 32 >= p.N) break;
-                            tmem_ld32(taddr + c * 32, ra);
-                            tmem_ld_wait();
-                            emit(ra, c);
-                        }
-                    }
-                }
-            } else if (!kResidStaged && wi.kind == ITEM_WHOLE) {
+            if (wi.kind == ITEM_WHOLE) {
                 int c = half;
                 if (c < nchunks) tmem_ld32(taddr + c * 32, ra);
 #pragma unroll 1
@@ -1042,6 +1149,8 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
 // that store straight to D with the arithmetic of the large kernel. Warp 0 loads, warp 1 issues the MMAs.
 constexpr int kSmallThreads = 192;
 constexpr int kSmallMaxStages = 8;
+constexpr int kSmallTailBytes = 256;          // barriers, tensor-memory pointer, abort flag; the drain's vectors (1536 bytes a warp) behind them
+constexpr int kSmallExtraBytes = 1024 + kSmallTailBytes + 4 * 1536;      // what a CTA needs beside its ring (1024: alignment)
 template <typename OutT, int EPI>
 __global__ void __launch_bounds__(kSmallThreads, 1)
 gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w, const GemmParams p) {
@@ -1101,9 +1210,9 @@ gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
             for (int kb = 0; kb < p.k_iters; ++kb) {
                 if (!mbar_wait(bar_full + 8 * stage, phase, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t da = umma_desc_sw128(sA + stage * a_bytes), db = umma_desc_sw128(sB + stage * b_bytes);
+                const uint32_t da = umma_desc_lo(sA + stage * a_bytes), db = umma_desc_lo(sB + stage * b_bytes);
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k) umma_i8(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);   // +32 bytes per step
+                for (int k = 0; k < BK / UMMA_K; ++k) umma_i8_lo(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);   // +32 bytes per step
                 umma_commit(bar_empty + 8 * stage);
                 if (++stage == S) stage = 0, phase ^= 1u;
             }
@@ -1113,10 +1222,33 @@ gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         const int quad = warp & 3;               // TMEM lane quarter this warp may read (warps 2..5 cover all four)
         const int row = tm * BM + quad * 32 + lane;
         const bool row_ok = row < p.M;
+        const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
+        bool drained = false;
+        if constexpr (EPI != EPI_ACC && EPI != EPI_ACT && sizeof(OutT) == 2) {
+            if (p.wide) {
+                const int col0 = tn * BN, chunks = min(BN / 32, (p.N - col0 + 31) / 32);
+                float* vec = reinterpret_cast<float*>(tail + kSmallTailBytes + (warp - 2) * 1536);
+                DrainVecs v;
+                v.fetch<OutT, EPI>(p, row, col0, chunks, lane);
+                uint4 rq[4][4];
+                if constexpr (EPI == EPI_RESID) {
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+                        if (c < chunks) drain_resid<OutT>(p, rq[c], row, col0 + 32 * c);
+                }
+                v.stage<EPI>(vec, lane);
+                bool ok = true;
+                if (lane == 0) ok = mbar_wait(bar_tfull, 0, abort_s, ST_TIMEOUT_TMEM_FULL);
+                if (__shfl_sync(0xffffffffu, (int)ok, 0)) {
+                    tc_fence_after();
+                    drain_tile<OutT, EPI>(p, taddr, row, col0, chunks, v.xs, vec, nullptr, rq, []() {});
+                }
+                drained = true;
+            }
+        }
         const float xs_r = EPI == EPI_ACC ? 0.f : (p.xs && row_ok) ? p.xs[row] : 1.f;
-        if (mbar_wait_warp_relaxed(bar_tfull, 0, abort_s, ST_TIMEOUT_TMEM_FULL)) {
+        if (!drained && mbar_wait_warp_relaxed(bar_tfull, 0, abort_s, ST_TIMEOUT_TMEM_FULL)) {
             tc_fence_after();
-            const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
             uint32_t r[32];
 #pragma unroll 1
             for (int c = 0; c < BN / 32; ++c) {
@@ -1398,6 +1530,12 @@ int choose_bn(int64_t M, int64_t N, int clusters) {
     return best;
 }
 
+// How the rows of a 2-byte output can be written from registers: 32 or 16 bytes at a time, or not at all (GemmParams::wide)
+int wide_rows(int64_t N, const void* D, const void* resid) {
+    if (N % 8 != 0 || (((uintptr_t)D | (uintptr_t)resid) & 15)) return 0;
+    return N % 16 == 0 && ((uintptr_t)D & 31) == 0 ? 2 : 1;
+}
+
 int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const float* ws, const void* bias,
              const void* rscale, const void* resid, void* D, int64_t M, int64_t N, int64_t K, int out_dt, int act,
              cudaStream_t st, float* amax_part = nullptr) {
@@ -1452,20 +1590,21 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
         auto al16s = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
         p.vec_ok = (N % 8 == 0) && al16s(D) && al16s(ws) && al16s(bias) && al16s(rscale) && al16s(resid);
         p.tma_store = 0;
+        p.wide = wide_rows(N, D, resid);
         p.bn = bn, p.ksub = 1;
         p.k_iters = (int)((K + BK - 1) / BK);
         p.tiles_m = tiles_m, p.tiles_n = (int)((N + bn - 1) / bn), p.num_tiles = p.tiles_m * p.tiles_n;
         // ring depth: the whole K if it fits; half the SM's shared memory when there are more tiles than SMs, so that two
         // CTAs share an SM
         const int stage_bytes = BM * BK + bn * BK;
-        const int budget = (p.num_tiles > device_sm_count(dev) ? kSmemBytes / 2 : kSmemBytes) - 1024 - 256;
+        const int budget = (p.num_tiles > device_sm_count(dev) ? kSmemBytes / 2 : kSmemBytes) - kSmallExtraBytes;
         p.stages = budget / stage_bytes;
         if (p.stages > kSmallMaxStages) p.stages = kSmallMaxStages;
         if (p.stages > p.k_iters) p.stages = p.k_iters;
         p.idesc = umma_idesc_i8(BM, bn);
         CUtensorMap ta, tw;
         if (!make_operand_tmap(&ta, A, M, K, BM) || !make_operand_tmap(&tw, W, N, K, bn)) return -203;
-        const size_t smem = 1024 + (size_t)p.stages * (BM * BK + bn * BK) + 256;
+        const size_t smem = kSmallExtraBytes + (size_t)p.stages * stage_bytes;
         if (epi == EPI_ACC) return launch_small<float, EPI_ACC>(ta, tw, p, p.num_tiles, smem, st);
         if (out_dt == DT_F32) return launch_small_epi<float>(epi, ta, tw, p, p.num_tiles, smem, st);
         if (out_dt == DT_F16) return launch_small_epi<half>(epi, ta, tw, p, p.num_tiles, smem, st);
@@ -1534,6 +1673,7 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
             p.num_items = p.whole_tiles + rem * splits;
         }
     }
+    p.wide = esz == 2 && p.splits == 0 ? wide_rows(N, D, resid) : 0;
     const int grid = 2 * (p.num_items < clusters ? p.num_items : clusters);
     int rc;
     if (epi == EPI_ACC) rc = launch_pair<float, EPI_ACC>(ta, tw, td, p, grid, st);

@@ -454,9 +454,9 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                 if (!mbar_wait(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
                 if (!mbar_wait(bar_wfull + 8 * sb, pb, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
                 tc_fence_after();
-                const uint64_t dw = umma_desc_sw128(sW + sb * w_bytes), da = umma_desc_sw128(sA + sa * a_bytes);
+                const uint32_t dw = umma_desc_lo(sW + sb * w_bytes), da = umma_desc_lo(sA + sa * a_bytes);
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k) umma_i8(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb - k0) | k);
+                for (int k = 0; k < BK / UMMA_K; ++k) umma_i8_lo(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb - k0) | k);
                 umma_commit(bar_wempty + 8 * sb);
                 umma_commit(bar_empty + 8 * sa);
                 if (++sa == SA) sa = 0, pa ^= 1u;

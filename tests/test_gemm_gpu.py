@@ -70,6 +70,38 @@ def test_epilogues_against_the_oracle(pkg, oracle, dev, dtype, M, N, K):
     assert L.kernel_status() == 0
 
 
+# Outputs written from registers: 32 bytes at a time, 16 (N % 16 == 8, or a base 16 bytes off), and not so (N % 8 != 0), for one and for
+# several tiles a cluster, tiles of an odd number of 32-column chunks, ragged rows and columns; nothing outside the matrix is written.
+# Against the epilogue kernel on the exact accumulators.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,limit", [(129, 72, 256, 0), (257, 264, 640, 0), (200, 1000, 128, 0), (2100, 1288, 1280, 0), (2100, 1304, 640, 3), (1500, 2560, 512, 4),
+                                         (1500, 2564, 512, 4), (700, 3080, 1024, 2)])
+def test_outputs_written_from_registers(pkg, dev, dtype, M, N, K, limit):
+    g, A, W, xs, ws = _operands(M, N, K, M + N + K)
+    A, W, xs, ws = A.to(dev), W.to(dev), xs.to(dev), ws.to(dev)
+    bias, rs = (torch.randn(N, generator=g) * 0.1).to(dtype).to(dev), (torch.rand(N, generator=g) + 0.5).to(dtype).to(dev)
+    resid = torch.randn(M, N, generator=g).to(dtype).to(dev)
+    L = pkg.linear
+    acc = L.int8_gemm_acc_i32(A, W)
+    want = {"plain": L.int8_epilogue(acc, xs, ws, bias, out_dtype=dtype), "resid": L.int8_epilogue(acc, xs, ws, bias, out_dtype=dtype, rscale=rs, resid=resid)}
+    was = L.set_gemm_cluster_limit(limit)
+    try:
+        for off in (0, 8, 16):
+            for form in want:
+                buf = torch.full((off + M * N + 32,), 3.0, dtype=dtype, device=dev)
+                out = buf[off:off + M * N].view(M, N)
+                if form == "resid":
+                    out.copy_(resid)                       # in place
+                    L.int8_gemm(A, W, xs, ws, bias, rscale=rs, resid=out, out=out)
+                else:
+                    L.int8_gemm(A, W, xs, ws, bias, out=out)
+                assert_bits_equal(out, want[form], f"{form}, {off}")
+                assert bool((buf[:off] == 3.0).all()) and bool((buf[off + M * N:] == 3.0).all())
+    finally:
+        L.set_gemm_cluster_limit(was)
+    assert L.kernel_status() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_bit_exact_against_the_reference_gemm(pkg, ref, dev, dtype):
     # the last five take the one-CTA-per-tile kernel (small problems; 2048 x 1280 x 1280 by its second rule)
