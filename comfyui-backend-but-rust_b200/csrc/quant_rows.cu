@@ -69,7 +69,7 @@ struct QuantArgs {
     float* out_f;       // when set: write the rotated fp32 rows here instead of quantizing
     int M, K;
     int rotate;
-    int tpr;            // threads per row = K / 32
+    int tpr;            // threads per row = K / 32 (quant_norm_kernel: warps per row)
     int rows_per_cta;
     int nblocks;        // row blocks; CTAs stride over them
     int lut;            // table index of the prologue, or -1
@@ -90,10 +90,6 @@ struct QuantArgs {
     int* zero;
     int nzero;
 };
-// prologues gpu_rotate_rows_f32 and the weight-only linear take
-template <typename T, int PRO> __host__ __device__ constexpr bool has_digits() {
-    return sizeof(T) == 4 && (PRO == PRO_PLAIN || PRO == PRO_RMS || PRO == PRO_SWIGLU);
-}
 
 template <int PRO> __host__ __device__ constexpr bool is_ln() { return PRO == PRO_LAYERNORM || PRO == PRO_LN_MOD || PRO == PRO_LN_AFFINE; }
 template <int PRO> __host__ __device__ constexpr bool is_norm() { return PRO == PRO_RMS || PRO == PRO_ADALN || is_ln<PRO>(); }
@@ -217,14 +213,15 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 // x = (d0 2^16 + d1 2^8 + d2) f with signed 8-bit digits and one power of two f per row, chosen so that the row's maximum lies in
 // [2^21, 2^22): what rounds away is at most 2^-22 of the row's maximum. The product with the power of two is exact and rint comes with the
 // addition of 1.5 * 2^23. A row holding an infinity or a NaN gets the factor NaN.
-__device__ __forceinline__ void store_digits(float2 (&P)[16], float amax, const QuantArgs& p, bool live, int64_t m, int col, int tin, int tsw,
-                                             int t8, float* tbuf, unsigned wmask) {
+// P and amax come in units of `unit` (1/16 without the rotation's halvings).
+__device__ __forceinline__ void store_digits(float2 (&P)[16], float amax, float unit, const QuantArgs& p, bool live, int64_t m, int col, bool first,
+                                             int tsw, int t8, float* tbuf, unsigned wmask) {
     float inv = 0.f, f = 0.f;
     if (!(amax <= FLT_MAX)) f = __int_as_float(0x7fc00000);
     else if (amax > 0.f) {
-        float back = 1.f;
+        float back = unit;
         if (amax < 0x1p-90f) {                      // the power of two would leave f32's range
-            amax *= 0x1p64f, back = 0x1p-64f;
+            amax *= 0x1p64f, back *= 0x1p-64f;
 #pragma unroll
             for (int r = 0; r < 16; ++r) P[r] = __fmul2_rn(P[r], make_float2(0x1p64f, 0x1p64f));
         }
@@ -232,7 +229,7 @@ __device__ __forceinline__ void store_digits(float2 (&P)[16], float amax, const 
         inv = __uint_as_float((uint32_t)(127 + 21 - k) << 23);
         f = __uint_as_float((uint32_t)(127 - 21 + k) << 23) * back;
     }
-    if (live && tin == 0) p.scales[m] = f;
+    if (live && first) p.scales[m] = f;
     uint32_t w[32];
     const float2 inv2 = make_float2(inv, inv), magic = make_float2(12582912.f, 12582912.f);
 #pragma unroll
@@ -262,20 +259,449 @@ __device__ __forceinline__ void store_digits(float2 (&P)[16], float amax, const 
 
 __device__ int g_quant_status = 0;   // a staging wait that ran out records ST_TIMEOUT_FULL here
 
-// MAXT = 384 asks for two CTAs per SM (at most 80 registers: 768 threads with the next block's rows in flight);
-// longer rows take one larger CTA.
-// DIRECT: the form of a block's linears and of the packers, rotated rows to codes and scales, one row block per CTA. Without the
-// other forms in the same instantiation it fits 56 registers in CTAs of up to 288 threads, 36 warps per SM instead of 24 (RMS,
-// LAYERNORM and SWIGLU: 64 registers, 256 threads, 32 warps); the kernel is bound by issue slots that too few warps fill (59 %
-// busy). In a chain of launches: PLAIN 4352 x 3072 17.1 -> 13.6 us, RMS 2048 x 5120 27.9 -> 25.0 (launch order included). f32 rows
-// other than the packers' and SITU would spill and keep the general form.
+// v = T(act(a)) [* b] of the prologues without row statistics: a is the gate logit u (GATE), the row itself otherwise; u the second
+// stream of the others. `lut`: the activation's table, or null.
+template <typename T, int PRO>
+__device__ __forceinline__ void elementwise_prologue(float (&v)[32], float (&u)[32], const uint16_t* lut) {
+    if (PRO == PRO_GATE || PRO == PRO_SWIGLU || PRO == PRO_SILU || PRO == PRO_GELU || PRO == PRO_GELU_TANH) {
+        float* a = PRO == PRO_GATE ? u : v;
+        if (lut) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) a[i] = lut_f(lut, a[i]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                a[i] = rnd<T>(PRO == PRO_GATE ? sigmoid_f(a[i]) : (PRO == PRO_SILU || PRO == PRO_SWIGLU) ? silu_f(a[i])
+                              : PRO == PRO_GELU ? gelu_f(a[i]) : gelu_tanh_f(a[i]));
+        }
+        if (PRO == PRO_GATE || PRO == PRO_SWIGLU) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = rnd<T>(__fmul_rn(v[i], u[i]));
+        }
+    } else if (PRO == PRO_SITU || PRO == PRO_SITU_FAST) {
+        // u = the gate half of the row; the product is not rounded here (csrc/kernels.cu:107-112)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = PRO == PRO_SITU ? situ_f(v[i], u[i]) : situ_fast_f(v[i], u[i]);
+    }
+}
+
+// ---- rotated rows to codes and scales: the form of a block's linears and of the packers ---------------------------------------
+// Kernels of their own beside the general one below: one row block per CTA, no staging, none of the other outputs, which leaves 56 to 64
+// registers and 32 to 36 warps per SM (the general kernel: 80 and 24). What bounds them is instruction issue, so the rotation comes
+// without its sixteen halvings: sums of unhalved values are the reference's times a power of two, whose rounding is the same as long as
+// nothing overflows and nothing that matters is subnormal (values that small become code 0 beside any scale: scales end at
+// 1e-30). An overflow, like an infinity or a NaN in the row, leaves something that is not finite among the rotated values; a CTA that
+// meets one, or a value of 2^127, goes through its rows a second time with the halvings, the IEEE division and the exact clamp.
+
+// The rotation of a lane's 32 consecutive values: P[r] = elements (2 t8, 2 t8 + 1) + 16 r of the group, swapped in a swapping team;
+// 16 times the reference's values without HALVE.
+template <bool HALVE>
+__device__ __forceinline__ void rotate_lane(float2 (&P)[16], const float (&v)[32], float* tbuf_w, int t8, int tsw, unsigned wmask) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) P[i] = make_float2(v[i], v[i + 16]);
+    two_stages<HALVE>(P);
+    float* we = tbuf_w + tpad(t8 << 5) + tsw;
+    float* wo = tbuf_w + tpad(t8 << 5) - tsw;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        float* w = (i & 1) ? wo : we;
+        w[i] = P[i].x;
+        w[16 + i] = P[i].y;
+    }
+    __syncwarp(wmask);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) P[r] = *reinterpret_cast<const float2*>(tbuf_w + tpad(2 * t8 + 16 * r));
+    two_stages<HALVE>(P);
+    __syncwarp(wmask);
+}
+__device__ __forceinline__ float max32_abs_nan(const float2 (&P)[16]) {
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m = max3_abs_nan(m, P[i].x, P[i].y);
+    return m;
+}
+// Code pairs (low 16 bits of c16[r], in element order) -> 32 contiguous bytes per lane of the group's 256
+__device__ __forceinline__ void store_codes(const uint32_t (&c16)[16], int8_t* q, bool live, float* tbuf, int t8, unsigned wmask) {
+    uint16_t* cb = reinterpret_cast<uint16_t*>(tbuf);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) cb[t8 + 8 * r] = (uint16_t)c16[r];
+    __syncwarp(wmask);
+    const uint4 lo = reinterpret_cast<const uint4*>(tbuf)[2 * t8], hi = reinterpret_cast<const uint4*>(tbuf)[2 * t8 + 1];
+    if (live) {
+        reinterpret_cast<uint4*>(q)[0] = lo;
+        reinterpret_cast<uint4*>(q)[1] = hi;
+    }
+}
+// P = 16 x the rotated values, all finite; amax = the row's maximum
+template <typename T>
+__device__ __forceinline__ void codes_fast(float2 (&P)[16], uint32_t (&c16)[16], float amax, float scale, int tsw) {
+    const float2 magic = make_float2(12582912.f, 12582912.f);       // rint: the integer's low byte is the sum's
+    const uint32_t pick = tsw ? 0x0004u : 0x0040u;                   // the two low bytes in element order
+    const float st = rnd<T>(scale);
+    const float rcp = __frcp_rn(st);
+    const float2 rcp2 = make_float2(rcp * 0.0625f, rcp * 0.0625f);
+    if constexpr (sizeof(T) == 2) {
+        auto quotient = [&](float2 v) {      // T(T(v) / T(scale)), see quant2
+            const __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y);
+            const float2 t = __fmul2_rn(bf16x2_f(a), rcp2);
+            return bf16x2_f(__floats2bfloat162_rn(t.x, t.y));
+        };
+        // 128 needs the clamp. Quotients grow with their dividends, so the maximum's tells for the row (about one row in eight).
+        if (rnd<T>(rnd<T>(amax) * rcp) < 127.5f) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float2 u = __fadd2_rn(quotient(P[i]), magic);
+                c16[i] = __byte_perm(__float_as_uint(u.x), __float_as_uint(u.y), pick);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                const float2 u = __fadd2_rn(quotient(P[i]), magic);
+                const int n0 = (int)__float_as_uint(u.x) - 0x4B400000, n1 = (int)__float_as_uint(u.y) - 0x4B400000;
+                c16[i] = __byte_perm((uint32_t)min(n0, 127), (uint32_t)min(n1, 127), pick);
+            }
+        }
+    } else {
+        // The correctly rounded quotient: with the correctly rounded reciprocal y of b, q' = q + (a - b q) y is a / b rounded once q is
+        // one of its two neighbours (Markstein 1990), which a first such step makes of a y. 16 a / (16 b) is the same quotient;
+        // where something underflows on the way the code is 0. The maximum is 127 scales and 2^-22: nothing needs the clamp.
+        const float2 nst2 = make_float2(st * -16.f, st * -16.f);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            float2 t = __fmul2_rn(P[i], rcp2);
+            t = __ffma2_rn(__ffma2_rn(t, nst2, P[i]), rcp2, t);
+            t = __ffma2_rn(__ffma2_rn(t, nst2, P[i]), rcp2, t);
+            const float2 u = __fadd2_rn(t, magic);
+            c16[i] = __byte_perm(__float_as_uint(u.x), __float_as_uint(u.y), pick);
+        }
+    }
+}
+template <typename T> __device__ __forceinline__ float row_scale(float amax) {
+    return fmaxf(fminf(amax, finite_max<T>()) * (1.f / 127.f), 1.0e-30f);
+}
+// A lane's place in both kernels. `bits` in shared memory, zero before: [rows] maxima of the first pass, [rows] of the second, one word that
+// is set when something is not finite or nearly so.
+struct DirectLane {
+    float *tbuf, *tbuf_w;     // the team's transposition buffer, and where the transposition starts in it
+    unsigned* bits;
+    int64_t m;                // the row it works on
+    int rloc, col, t8, tsw;
+    bool live, first;         // whether it stores; whether it stores the row's scale
+    unsigned wmask;
+};
+// From a lane's values to stored codes; false when something in the CTA's rows is not finite.
+template <typename T, bool DIGITS>
+__device__ __forceinline__ bool direct_first(const QuantArgs& p, const DirectLane& l, const float (&v)[32]) {
+    float2 P[16];
+    rotate_lane<false>(P, v, l.tbuf_w, l.t8, l.tsw, l.wmask);
+    unsigned b = __float_as_uint(max32_abs_nan(P));      // non-negative floats order as integers, infinities and NaNs above
+    b = max(b, __shfl_xor_sync(l.wmask, b, 1));
+    b = max(b, __shfl_xor_sync(l.wmask, b, 2));
+    b = max(b, __shfl_xor_sync(l.wmask, b, 4));
+    if (l.t8 == 0) {
+        atomicMax(l.bits + l.rloc, b);
+        if (b >= 0x7f000000u) l.bits[2 * p.rows_per_cta] = 1u;     // 2^127: short of what rounds to an infinity of bf16
+    }
+    __syncthreads();
+    if (l.bits[2 * p.rows_per_cta] != 0u) return false;
+    pdl_trigger();
+    if constexpr (DIGITS) {
+        store_digits(P, __uint_as_float(l.bits[l.rloc]), 0.0625f, p, l.live, l.m, l.col, l.first, l.tsw, l.t8, l.tbuf, l.wmask);
+    } else {
+        const float amax = __uint_as_float(l.bits[l.rloc]) * 0.0625f, scale = row_scale<T>(amax);
+        if (l.live && l.first) p.scales[l.m] = scale;
+        uint32_t c16[16];
+        codes_fast<T>(P, c16, amax, scale, l.tsw);
+        store_codes(c16, p.q + l.m * (int64_t)p.K + l.col, l.live, l.tbuf, l.t8, l.wmask);
+    }
+    return true;
+}
+template <typename T, bool DIGITS>
+__device__ __forceinline__ void direct_second(const QuantArgs& p, const DirectLane& l, const float (&v)[32]) {
+    float2 P[16];
+    rotate_lane<true>(P, v, l.tbuf_w, l.t8, l.tsw, l.wmask);
+    float amax = 0.f;                                    // without NaNs, which the reference's fmaxf drops
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fmaxf(fabsf(P[i].x), fabsf(P[i].y)));
+    if (DIGITS) amax = max32_abs_nan(P);                 // with them: the row's factor becomes one
+    atomicMax(l.bits + p.rows_per_cta + l.rloc, __float_as_uint(amax));
+    __syncthreads();
+    amax = __uint_as_float(l.bits[p.rows_per_cta + l.rloc]);
+    if constexpr (DIGITS) {
+        store_digits(P, amax, 1.f, p, l.live, l.m, l.col, l.first, l.tsw, l.t8, l.tbuf, l.wmask);
+    } else {
+        const float scale = row_scale<T>(amax), st = rnd<T>(scale);
+        if (l.live && l.first) p.scales[l.m] = scale;
+        const uint32_t order = l.tsw ? 0x3201u : 0x3210u;
+        uint32_t c16[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) c16[i] = __byte_perm(quant2<T>(P[i], st, 0.f, false), 0u, order);
+        store_codes(c16, p.q + l.m * (int64_t)p.K + l.col, l.live, l.tbuf, l.t8, l.wmask);
+    }
+}
+__device__ __forceinline__ void direct_clear(const QuantArgs& p, unsigned* bits) {
+    for (int i = threadIdx.x; i <= 2 * p.rows_per_cta; i += blockDim.x) bits[i] = 0u;
+}
+// for the kernel that follows the digits
+__device__ __forceinline__ void clear_counters(const QuantArgs& p) {
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < p.nzero; i += blockDim.x) p.zero[i] = 0;
+}
+
+// Rows as they lie and the prologues without row statistics. f32 rows other than the packers' and SITU would spill and keep the general
+// kernel. In a chain of launches, us, before | now (the halvings kept, the exact form in the same kernel): PLAIN 4352 x 3072 15.9 | 15.7, GATE 1111 x 3072
+// 10.1 | 9.4.
 template <typename T, int PRO> __host__ __device__ constexpr int direct_threads() {
     if (sizeof(T) == 4) return PRO == PRO_PLAIN ? 288 : 0;
-    return PRO == PRO_SITU ? 0 : PRO == PRO_RMS || PRO == PRO_LAYERNORM || PRO == PRO_SWIGLU ? 256 : 288;
+    return is_norm<PRO>() || PRO == PRO_SITU ? 0 : PRO == PRO_SWIGLU ? 256 : 288;
 }
-template <typename T, int PRO, int MAXT, bool DIRECT = false>
-__global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_rows_kernel(const QuantArgs p) {
-    const bool staged = !DIRECT && p.staged, rotate = DIRECT || p.rotate;
+// f32 rows are read in whole lines (lane t8 of a team the 16-byte pieces t8 + 8 j of its group) and pass through the team's buffer, piece c
+// at c ^ (c >> 3), into 32 consecutive values per lane: read as those, a load touched 32 lines for 16 bytes each. 5120 x 5120
+// f32 packed: 46 -> 31 us; the digits of 512 x 9728 with SWIGLU 25 -> 21.
+template <typename T, int PRO>
+__device__ __forceinline__ void direct_values(const QuantArgs& p, const DirectLane& l, float (&v)[32]) {
+    if constexpr (sizeof(T) == 4) {
+        const float4* x = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.x) + l.m * p.x_stride + (l.col & ~255)) + l.t8;
+        const float4* up = PRO == PRO_SWIGLU ? reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + p.up_offset) : x;
+        float4* stage = reinterpret_cast<float4*>(l.tbuf);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            float4 a = gload(x + 8 * j);
+            if constexpr (PRO == PRO_SWIGLU) {
+                const float4 b = gload(up + 8 * j);
+                a.x = __fmul_rn(silu_f(a.x), b.x), a.y = __fmul_rn(silu_f(a.y), b.y);
+                a.z = __fmul_rn(silu_f(a.z), b.z), a.w = __fmul_rn(silu_f(a.w), b.w);
+            }
+            stage[8 * j + (l.t8 ^ j)] = a;
+        }
+        __syncwarp(l.wmask);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const float4 a = stage[8 * l.t8 + (j ^ l.t8)];
+            v[4 * j] = a.x, v[4 * j + 1] = a.y, v[4 * j + 2] = a.z, v[4 * j + 3] = a.w;
+        }
+        __syncwarp(l.wmask);
+    } else {
+        float u[32];
+        const T* x = reinterpret_cast<const T*>(p.x) + l.m * p.x_stride + l.col;
+        load32<T, false>(x, v);
+        if (PRO == PRO_GATE) load32<T, false>(reinterpret_cast<const T*>(p.g) + l.m * p.g_stride + l.col, u);
+        else if (has_aux<PRO>()) load32<T, false>(x + p.up_offset, u);
+        elementwise_prologue<T, PRO>(v, u, p.lut >= 0 ? g_act_lut[p.lut] : nullptr);
+    }
+}
+__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = lane >> 3;
+    const int rloc = threadIdx.x / p.tpr, tin = threadIdx.x - rloc * p.tpr;
+    const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
+    float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
+    // idle rows compute on the last row and store nothing; the last warp of a CTA may be partial (threads = rows * K / 32)
+    return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc, tin << 5, tin & 7, team & 1,
+            m < p.M, tin == 0, __activemask()};
+}
+// The second pass, out of line: what it holds would take registers from the first.
+template <typename T, int PRO, bool DIGITS>
+__device__ __noinline__ void direct_again(const QuantArgs& p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const DirectLane l = direct_lane(p, smem);
+    float v[32];
+    direct_values<T, PRO>(p, l, v);
+    direct_second<T, DIGITS>(p, l, v);
+}
+template <typename T, int PRO, int MAXT, bool DIGITS>
+__global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel(const __grid_constant__ QuantArgs p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const DirectLane l = direct_lane(p, smem);
+    direct_clear(p, l.bits);
+    pdl_wait();
+    if (DIGITS) clear_counters(p);
+    __syncthreads();
+    bool done;
+    {
+        float v[32];
+        direct_values<T, PRO>(p, l, v);
+        done = direct_first<T, DIGITS>(p, l, v);
+    }
+    if (!done) direct_again<T, PRO, DIGITS>(p);
+}
+
+// Normalising prologues on bf16 rows. The row sums are added in the reference's order (csrc/kernels.cu:113-147, csrc/common.cuh:30-55), so
+// that they, and everything after them, come out bit for bit: there a block of nwr = ceil(K / 1024) warps holds the row, warp w the
+// groups w, w + nwr, ..., lane l elements 8 l .. 8 l + 7 of each; a thread adds its elements in that order, then a xor-shuffle tree
+// runs over the lanes and another over the warps. Here the same warps hold the same elements until the row is normalised: the sums are a
+// thread's own, loads (rows, weights, modulation) are whole lines, and a row takes one barrier per sum. The normalised values pass
+// through shared memory as bf16, which they are, into the rotation's layout: warp w' takes the groups 4 w' .. 4 w' + 3 there, from a
+// slice that lies in its own transposition buffer. With the sums in the rotation's layout, running from group to group through
+// shared memory in up to four rounds with a quarter of the lanes at work each, LN_MOD was 50 instructions a value where PLAIN was 22.
+// In a chain of launches: LN_MOD 4352 x 3072 33.3 -> 25.3 us, RMS 1111 x 3072 11.1 -> 8.2.
+__device__ __forceinline__ void row_barrier(int rloc, int warps) {
+    if (warps == 1) __syncwarp();
+    else named_bar_sync(1 + rloc, 32 * warps);
+}
+// f32 rows (RMS without modulation, the weight-only linear's): the same with 1 KB a group.
+template <typename T, int PRO>
+__device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane& l, uint8_t* smem, float (&v)[32]) {
+    static_assert(sizeof(T) == 2 || PRO == PRO_RMS, "f32 rows: RMS only");
+    const int lane = threadIdx.x & 31, nwr = p.tpr, w = (threadIdx.x >> 5) - l.rloc * nwr, ngroups = p.K >> 8, grp = l.col >> 8;
+    float* slice0 = reinterpret_cast<float*>(smem) + l.rloc * nwr * kWarpWords;       // the row's first warp's buffer
+    float* sums = reinterpret_cast<float*>(smem + p.off_norm) + l.rloc * 64;          // [2][32]
+    const T* x = reinterpret_cast<const T*>(p.x) + l.m * p.x_stride + 8 * lane;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int g = w + nwr * i;
+        if constexpr (sizeof(T) == 2) {
+            unpack_bf16x8(g < ngroups ? gload(reinterpret_cast<const uint4*>(x + (g << 8))) : make_uint4(0, 0, 0, 0), v + 8 * i);
+        } else {
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4 a = g < ngroups ? gload(reinterpret_cast<const float4*>(x + (g << 8)) + h) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[8 * i + 4 * h] = a.x, v[8 * i + 4 * h + 1] = a.y, v[8 * i + 4 * h + 2] = a.z, v[8 * i + 4 * h + 3] = a.w;
+            }
+        }
+    }
+    auto row_sum = [&](bool squares, float* slot) -> float {
+        float s = 0.f;                             // the zeros of missing groups come last and change nothing
+#pragma unroll
+        for (int i = 0; i < 32; ++i) s = squares ? __fmaf_rn(v[i], v[i], s) : __fadd_rn(s, v[i]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if (lane == 0) slot[w] = s;
+        row_barrier(l.rloc, nwr);
+        s = lane < nwr ? slot[lane] : 0.f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        return s;
+    };
+    if constexpr (is_ln<PRO>()) {
+        const float mean = __fdiv_rn(row_sum(false, sums), (float)p.K);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float sub = w + nwr * i < ngroups ? mean : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j += 2) {
+                const float2 d = __fadd2_rn(make_float2(v[8 * i + j], v[8 * i + j + 1]), make_float2(-sub, -sub));
+                v[8 * i + j] = d.x, v[8 * i + j + 1] = d.y;
+            }
+        }
+    }
+    const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(row_sum(true, sums + 32), (float)p.K), p.eps));
+    const bf16* ms_p = reinterpret_cast<const bf16*>(p.mod_scale);
+    const bf16* sh_p = reinterpret_cast<const bf16*>(p.mod_shift);
+    const float2 rstd2 = make_float2(rstd, rstd);
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int g = w + nwr * i;
+            if (g >= ngroups) break;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float* e = v + 8 * i + 4 * h;
+                float2 a = __fmul2_rn(make_float2(e[0], e[1]), rstd2), b = __fmul2_rn(make_float2(e[2], e[3]), rstd2);
+                if (p.norm_w) {
+                    const float4 nw = gload(reinterpret_cast<const float4*>(p.norm_w + (g << 8) + 8 * lane) + h);
+                    a = __fmul2_rn(a, make_float2(nw.x, nw.y)), b = __fmul2_rn(b, make_float2(nw.z, nw.w));
+                }
+                const int c = ((g & 3) << 6) + 2 * lane + h;
+                reinterpret_cast<float4*>(slice0 + (g >> 2) * kWarpWords)[c ^ ((c >> 3) & 7)] = make_float4(a.x, a.y, b.x, b.y);
+            }
+        }
+        row_barrier(l.rloc, nwr);
+        const float4* mine = reinterpret_cast<const float4*>(slice0 + w * kWarpWords) + ((grp - 4 * w) << 6);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float4 a = mine[(8 * l.t8 + k) ^ l.t8];
+            v[4 * k] = a.x, v[4 * k + 1] = a.y, v[4 * k + 2] = a.z, v[4 * k + 3] = a.w;
+        }
+        __syncwarp();
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int g = w + nwr * i;
+            if (g >= ngroups) break;
+            const int c0 = (g << 8) + 8 * lane;
+            uint4 mw = make_uint4(0, 0, 0, 0), sw = mw;
+            float nw[8], nb[8];
+            if (ms_p) mw = gload(reinterpret_cast<const uint4*>(ms_p + c0)), sw = gload(reinterpret_cast<const uint4*>(sh_p + c0));
+            const bool has_w = (PRO == PRO_RMS || PRO == PRO_LAYERNORM || PRO == PRO_LN_AFFINE) && p.norm_w;
+            if (has_w) load8v(p.norm_w + c0, nw);
+            if (PRO == PRO_LN_AFFINE) load8v(p.norm_b + c0, nb);
+            const uint32_t m4[4] = {mw.x, mw.y, mw.z, mw.w}, s4[4] = {sw.x, sw.y, sw.z, sw.w};
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                // two values at a time, one packed conversion per rounding (a scalar conversion runs on a narrow pipe)
+                float2 n = __fmul2_rn(make_float2(v[8 * i + 2 * j], v[8 * i + 2 * j + 1]), rstd2);
+                const float2 ms = make_float2(__uint_as_float(m4[j] << 16), __uint_as_float(m4[j] & 0xffff0000u));
+                const float2 sh = make_float2(__uint_as_float(s4[j] << 16), __uint_as_float(s4[j] & 0xffff0000u));
+                auto round2 = [](float2 f) { return bf16x2_f(__floats2bfloat162_rn(f.x, f.y)); };
+                // 1 + scale as a bf16 addition rounds once where the reference rounds to f32 first, which makes no difference (the f32
+                // sum is inexact only beside a scale below 2^-16 or above 2^16, and neither comes near a tie of bf16)
+                auto one_plus = [&]() { return bf16x2_f(__hadd2(__floats2bfloat162_rn(1.f, 1.f), *reinterpret_cast<const __nv_bfloat162*>(&m4[j]))); };
+                if (PRO == PRO_ADALN) {                // one rounding
+                    n = __ffma2_rn(n, __fadd2_rn(make_float2(1.f, 1.f), ms), sh);
+                } else if (PRO == PRO_LN_AFFINE) {
+                    n = __ffma2_rn(n, make_float2(nw[2 * j], nw[2 * j + 1]), make_float2(nb[2 * j], nb[2 * j + 1]));
+                } else {
+                    if (has_w) n = __fmul2_rn(n, make_float2(nw[2 * j], nw[2 * j + 1]));
+                    if (PRO == PRO_LN_MOD) {           // one rounding after the norm, one after the multiply-add
+                        n = ms_p ? __ffma2_rn(round2(n), one_plus(), sh) : __ffma2_rn(round2(n), make_float2(1.f, 1.f), make_float2(0.f, 0.f));
+                    } else if (ms_p) {                 // RMS, LAYERNORM: every step rounded
+                        n = __fadd2_rn(round2(__fmul2_rn(one_plus(), round2(n))), sh);
+                    }
+                }
+                const __nv_bfloat162 h = __floats2bfloat162_rn(n.x, n.y);
+                o[j] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            // piece (g & 3) * 32 + lane of the slice, its low bits mixed with the next ones: free of bank conflicts both ways
+            const int c = ((g & 3) << 5) + lane;
+            reinterpret_cast<uint4*>(slice0 + (g >> 2) * kWarpWords)[c ^ ((c >> 2) & 7)] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        row_barrier(l.rloc, nwr);
+        const uint4* mine = reinterpret_cast<const uint4*>(slice0 + w * kWarpWords);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) unpack_bf16x8(mine[((grp - 4 * w) * 32 + 4 * l.t8 + k) ^ l.t8], v + 8 * k);
+        __syncwarp();                                  // the slice is the transposition buffer from here on
+    }
+}
+__device__ __forceinline__ DirectLane norm_lane(const QuantArgs& p, uint8_t* smem) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = lane >> 3, nwr = p.tpr;      // nwr: warps per row
+    const int rloc = warp / nwr, w = warp - rloc * nwr, ngroups = p.K >> 8, grp = min(4 * w + team, ngroups - 1);
+    const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
+    float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
+    // teams past the row's last group redo it and store nothing, like rows past the last
+    return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc,
+            (grp << 8) + ((lane & 7) << 5), lane & 7, team & 1, m < p.M && 4 * w + team < ngroups, w == 0 && lane == 0, 0xffffffffu};
+}
+template <typename T, int PRO, bool DIGITS>
+__device__ __noinline__ void norm_again(const QuantArgs& p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const DirectLane l = norm_lane(p, smem);
+    float v[32];
+    norm_values<T, PRO>(p, l, smem, v);
+    direct_second<T, DIGITS>(p, l, v);
+}
+template <typename T, int PRO, int MAXT, bool DIGITS>
+__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) quant_norm_kernel(const __grid_constant__ QuantArgs p) {
+    extern __shared__ __align__(128) uint8_t smem[];
+    const DirectLane l = norm_lane(p, smem);
+    direct_clear(p, l.bits);
+    pdl_wait();
+    if (DIGITS) clear_counters(p);
+    __syncthreads();
+    bool done;
+    {
+        float v[32];
+        norm_values<T, PRO>(p, l, smem, v);
+        done = direct_first<T, DIGITS>(p, l, v);
+    }
+    if (!done) norm_again<T, PRO, DIGITS>(p);
+}
+
+// MAXT = 384 asks for two CTAs per SM (at most 80 registers: 768 threads with the next block's rows in flight);
+// longer rows take one larger CTA.
+template <typename T, int PRO, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT <= 384 ? 2 : 1) quant_rows_kernel(const QuantArgs p) {
+    const bool staged = p.staged, rotate = p.rotate;
     extern __shared__ __align__(128) uint8_t smem[];
     const uint16_t* lut = g_act_lut[p.lut >= 0 ? p.lut : 0];
     const unsigned wmask = __activemask();            // the last warp of a CTA may be partial (threads = rows * K / 32)
@@ -296,10 +722,6 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
         fence_mbar_init();
     }
     pdl_wait();
-    if constexpr (!DIRECT && has_digits<T, PRO>()) {
-        if (blockIdx.x == 0)
-            for (int i = threadIdx.x; i < p.nzero; i += blockDim.x) p.zero[i] = 0;
-    }
     __syncthreads();
 
     // Staging: the rows of block `blk` (and their second stream) -> the staging buffer, one bulk copy each, issued by
@@ -327,7 +749,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
     const int grp = tin >> 3, t8 = tin & 7;
     const int col = (grp << 8) + (t8 << 5);
     int it = 0;
-    for (int blk = blockIdx.x; blk < p.nblocks; blk += DIRECT ? p.nblocks : (int)gridDim.x, ++it) {
+    for (int blk = blockIdx.x; blk < p.nblocks; blk += gridDim.x, ++it) {
         const int64_t m_raw = (int64_t)blk * p.rows_per_cta + rloc;
         const bool live = m_raw < p.M;
         const int64_t m = live ? m_raw : p.M - 1;      // idle rows compute on the last row (or on stale staging) and store nothing
@@ -360,27 +782,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
             else if (has_aux<PRO>()) load32<T, false>(x + p.up_offset, u);
         }
 
-        if (PRO == PRO_GATE || PRO == PRO_SWIGLU || PRO == PRO_SILU || PRO == PRO_GELU || PRO == PRO_GELU_TANH) {
-            // v = T(act(a)) [* b]: a is the gate logit (GATE), the row itself otherwise
-            float* a = PRO == PRO_GATE ? u : v;
-            if (use_lut) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) a[i] = lut_f(lut, a[i]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    a[i] = rnd<T>(PRO == PRO_GATE ? sigmoid_f(a[i]) : (PRO == PRO_SILU || PRO == PRO_SWIGLU) ? silu_f(a[i])
-                                  : PRO == PRO_GELU ? gelu_f(a[i]) : gelu_tanh_f(a[i]));
-            }
-            if (PRO == PRO_GATE || PRO == PRO_SWIGLU) {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) v[i] = rnd<T>(__fmul_rn(v[i], u[i]));
-            }
-        } else if (PRO == PRO_SITU || PRO == PRO_SITU_FAST) {
-            // u = the gate half of the row; the product is not rounded here (csrc/kernels.cu:107-112)
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = PRO == PRO_SITU ? situ_f(v[i], u[i]) : situ_fast_f(v[i], u[i]);
-        }
+        elementwise_prologue<T, PRO>(v, u, use_lut ? lut : nullptr);
 
         if constexpr (is_norm<PRO>()) {
             // Row statistics in the reference's order of additions (csrc/kernels.cu:113-147, csrc/common.cuh:30-55), so
@@ -534,7 +936,7 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
             for (int i = 0; i < 16; ++i) P[i] = make_float2(v[2 * i], v[2 * i + 1]);   // natural order
         }
 
-        if (!DIRECT && p.out_f) {   // gpu_rotate_rows_f32: always rotated, so P holds (2 t8, 2 t8 + 1) + 16 r
+        if (p.out_f) {   // gpu_rotate_rows_f32: always rotated, so P holds (2 t8, 2 t8 + 1) + 16 r
             if (live) {
                 float* o = p.out_f + m * (int64_t)p.K + (grp << 8) + 2 * t8;
 #pragma unroll
@@ -560,25 +962,14 @@ __global__ void __launch_bounds__(MAXT, DIRECT ? 4 : MAXT <= 384 ? 2 : 1) quant_
         amax = fmaxf(amax, __shfl_xor_sync(wmask, amax, 4));
         unsigned* slot = amax_s + (it % 3) * p.rows_per_cta + rloc;
         if (t8 == 0) atomicMax(slot, __float_as_uint(amax));
-        if constexpr (!DIRECT && has_digits<T, PRO>()) {
-            if (p.digits && has_nan) atomicMax(slot, 0x7fc00000u);      // above every number: the row's factor becomes NaN
-        }
         __syncthreads();
         amax = __uint_as_float(*slot);
-        if (DIRECT) pdl_trigger();
-        if (!DIRECT) amax_s[((it + 2) % 3) * p.rows_per_cta + rloc] = 0u;   // next use is two barriers away, last use one barrier back
-        if (!DIRECT && p.amax_out) {
+        amax_s[((it + 2) % 3) * p.rows_per_cta + rloc] = 0u;   // next use is two barriers away, last use one barrier back
+        if (p.amax_out) {
             if (live && tin == 0) p.amax_out[m] = amax;
             continue;
         }
-        if constexpr (!DIRECT && has_digits<T, PRO>()) {
-            if (p.digits) {
-                pdl_trigger();
-                store_digits(P, amax, p, live, m, col, tin, tsw, t8, tbuf, wmask);
-                continue;
-            }
-        }
-        if (!DIRECT && p.amax_in) amax = p.amax_in[m];
+        if (p.amax_in) amax = p.amax_in[m];
 
         const float scale = fmaxf(fminf(amax, finite_max<T>()) * (1.f / 127.f), 1.0e-30f);
         if (live && tin == 0) p.scales[m] = scale;
@@ -1128,9 +1519,44 @@ struct OccCache {
     size_t smem[8] = {};
 };
 
-template <typename T, int PRO, int MAXT, bool DIRECT = false>
+// A kernel's limit of dynamic shared memory, raised once per device
+template <typename Kern> int raise_smem(Kern kern, std::atomic<uint64_t>& configured, size_t smem) {
+    if (smem <= 48 * 1024) return 0;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const uint64_t bit = 1ull << (dev & 63);
+    if (configured.load(std::memory_order_acquire) & bit) return 0;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e == cudaSuccess) configured.fetch_or(bit, std::memory_order_release);
+    return (int)e;
+}
+template <typename T, int PRO, int MAXT, bool DIGITS = false>
+int launch_direct(const QuantArgs& p, int threads, size_t smem, cudaStream_t st) {
+    static std::atomic<uint64_t> configured{0};
+    auto kern = quant_direct_kernel<T, PRO, MAXT, DIGITS>;
+    if (int rc = raise_smem(kern, configured, smem)) return rc;
+    return launch_pdl(kern, dim3(p.nblocks), threads, smem, st, p);
+}
+template <typename T, int PRO, int MAXT, bool DIGITS>
+int launch_norm_cfg(const QuantArgs& p, int threads, size_t smem, cudaStream_t st) {
+    static std::atomic<uint64_t> configured{0};
+    auto kern = quant_norm_kernel<T, PRO, MAXT, DIGITS>;
+    if (int rc = raise_smem(kern, configured, smem)) return rc;
+    return launch_pdl(kern, dim3(p.nblocks), threads, smem, st, p);
+}
+// Rows of ceil(K / 1024) warps, about eight warps per CTA
+template <typename T, int PRO, bool DIGITS = false> int launch_norm(QuantArgs p, cudaStream_t st) {
+    const int nwr = ((p.K >> 8) + 3) >> 2, rows = nwr >= 8 ? 1 : 8 / nwr, warps = rows * nwr;
+    p.tpr = nwr, p.rows_per_cta = rows, p.nblocks = (p.M + rows - 1) / rows;
+    p.off_norm = (uint32_t)(warps * kWarpWords * 4);
+    p.off_amax = p.off_norm + rows * 64 * 4;
+    const size_t smem = p.off_amax + (2 * rows + 1) * 4;
+    return warps <= 8 ? launch_norm_cfg<T, PRO, 256, DIGITS>(p, 32 * warps, smem, st) : launch_norm_cfg<T, PRO, 1024, DIGITS>(p, 32 * warps, smem, st);
+}
+
+template <typename T, int PRO, int MAXT>
 int launch_cfg(QuantArgs& p, int threads, size_t smem, bool persistent, cudaStream_t st) {
-    auto kern = quant_rows_kernel<T, PRO, MAXT, DIRECT>;
+    auto kern = quant_rows_kernel<T, PRO, MAXT>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1212,9 +1638,18 @@ int launch_quant(QuantArgs& p, cudaStream_t st) {
     p.staged = !p.rotate && !is_norm<PRO>() && off + stage_bytes <= kMaxSmem;
     const size_t smem = p.staged ? off + stage_bytes : off;
     if (smem > kMaxSmem) return -2;
+    if constexpr (sizeof(T) == 4 && (PRO == PRO_PLAIN || PRO == PRO_SWIGLU)) {
+        if (p.digits) return threads <= 256 ? launch_direct<T, PRO, 256, true>(p, threads, smem, st) : launch_direct<T, PRO, 1024, true>(p, threads, smem, st);
+    }
+    if constexpr (sizeof(T) == 4 && PRO == PRO_RMS) {
+        if (p.digits) return launch_norm<T, PRO, true>(p, st);
+    }
+    const bool codes = p.rotate && !p.out_f && !p.digits && !p.amax_in && !p.amax_out;
     if constexpr (direct_threads<T, PRO>() > 0) {
-        if (p.rotate && threads <= direct_threads<T, PRO>() && !p.out_f && !p.digits && !p.amax_in && !p.amax_out)
-            return launch_cfg<T, PRO, direct_threads<T, PRO>(), true>(p, threads, smem, false, st);
+        if (codes && threads <= direct_threads<T, PRO>()) return launch_direct<T, PRO, direct_threads<T, PRO>()>(p, threads, smem, st);
+    }
+    if constexpr (sizeof(T) == 2 && is_norm<PRO>()) {
+        if (codes) return launch_norm<T, PRO>(p, st);
     }
     if (threads > 512) return launch_cfg<T, PRO, 1024>(p, threads, smem, p.staged != 0, st);
     if (threads > 384) return launch_cfg<T, PRO, 512>(p, threads, smem, p.staged != 0, st);

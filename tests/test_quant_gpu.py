@@ -122,6 +122,27 @@ def test_full_size_properties(pkg, dev):
     assert pkg.linear.kernel_status() == 0
 
 
+@pytest.mark.parametrize("dtype,pro", [(torch.bfloat16, PLAIN), (torch.bfloat16, GATE), (torch.bfloat16, SWIGLU), (torch.bfloat16, GELU_TANH), (torch.float32, PLAIN)])
+@pytest.mark.parametrize("K", [256, 768, 2560, 8192, 9216])
+def test_one_pass_equals_two(pkg, dev, dtype, pro, K):
+    """Rotated rows to codes in one kernel against the row maxima and the quantization as two (which keep the rotation's halvings and the
+    exact division): ordinary rows beside rows with infinities, NaNs and values at both ends of the range, in CTAs of one row and of several."""
+    g = torch.Generator().manual_seed(K + pro)
+    M = 45
+    x = torch.randn(M, 2 * K if pro == SWIGLU else K, generator=g) * torch.exp2(torch.randint(-8, 9, (M, 1), generator=g).float())
+    for m, f in ((3, 2.0 ** 119), (4, 2.0 ** 123), (5, 2.0 ** 126), (6, 2.0 ** -124), (7, 2.0 ** -100), (8, 0.0), (9, 2.0 ** -130)):
+        x[m] *= f
+    x[12, 7], x[13, 100], x[14, 0] = float("inf"), float("nan"), -float("inf")
+    x[20:40, 11] = torch.linspace(3.2e38, 3.4e38, 20)              # alone in its group: around the largest bf16 after the rotation
+    x[20:40] = torch.where(x[20:40].abs() > 1e38, x[20:40], x[20:40] * 2.0 ** -60)
+    x = x.to(dtype).to(dev)
+    kw = dict(g=torch.randn(M, K, generator=g).to(dtype).to(dev)) if pro == GATE else dict(K=K, up_offset=K) if pro == SWIGLU else {}
+    q, s = pkg.linear.quant_rows(x, pro, 1, **kw)
+    q2, s2 = pkg.linear.quant_rows_scaled(x, pkg.linear.quant_rows_amax(x, pro, 1, **kw), pro, 1, **kw)
+    assert_bits_equal(q, q2, "codes")
+    assert_bits_equal(s, s2, "scales")
+
+
 def test_errors(pkg, dev):
     x = torch.zeros(4, 512, device=dev, dtype=torch.bfloat16)
     with pytest.raises(pkg.GpuKernelError, match="-3"):
