@@ -11,16 +11,27 @@ namespace {
 constexpr int kWarps = 8;
 constexpr int kRowsPerWarp = 4;
 
+// size bytes to L2 (both multiples of 16)
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t size) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(size) : "memory");
+}
+
 template <typename OutT, int EPI, int MT>
 __global__ void __launch_bounds__(kWarps * 32) skinny_gemm_kernel(const SkinnyParams p) {
     extern __shared__ __align__(16) int8_t a_s[];   // [M][K]
-    pdl_wait();
     const int K = p.K;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nblocks = (p.N + kRowsPerWarp - 1) / kRowsPerWarp;
+    // This warp's first weight rows on their way to L2 while the predecessor, as a rule the quantizer of these few rows, still runs.
+    // Nothing is read here: whatever the predecessor writes is seen by the loads behind the wait.
+    if (lane == 0) {
+        const int n0 = (blockIdx.x * kWarps + warp) * kRowsPerWarp, rows = min(kRowsPerWarp, p.N - n0);
+        if (rows > 0) prefetch_l2(p.W + (int64_t)n0 * K, (uint32_t)rows * K);
+    }
+    pdl_wait();
     for (int i = threadIdx.x; i < p.M * K / 16; i += blockDim.x)
         reinterpret_cast<uint4*>(a_s)[i] = gload(reinterpret_cast<const uint4*>(p.A) + i);
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nblocks = (p.N + kRowsPerWarp - 1) / kRowsPerWarp;
     for (int nb = blockIdx.x * kWarps + warp; nb < nblocks; nb += gridDim.x * kWarps) {
         const int n0 = nb * kRowsPerWarp;
         int acc[kRowsPerWarp][MT];

@@ -89,6 +89,7 @@ struct QuantArgs {
     int8_t* digits;
     int* zero;
     int nzero;
+    int early;              // the stream's next kernel may start as soon as this one has (see early_trigger)
 };
 
 template <int PRO> __host__ __device__ constexpr bool is_ln() { return PRO == PRO_LAYERNORM || PRO == PRO_LN_MOD || PRO == PRO_LN_AFFINE; }
@@ -514,6 +515,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel
     const DirectLane l = direct_lane(p, smem);
     direct_clear(p, l.bits);
     pdl_wait();
+    if (p.early) pdl_trigger();
     if (DIGITS) clear_counters(p);
     __syncthreads();
     bool done;
@@ -686,6 +688,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) quant_norm_kernel(c
     const DirectLane l = norm_lane(p, smem);
     direct_clear(p, l.bits);
     pdl_wait();
+    if (p.early) pdl_trigger();
     if (DIGITS) clear_counters(p);
     __syncthreads();
     bool done;
@@ -1168,7 +1171,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
 constexpr int kSdThreads = 288;
 template <int ROT, int SRC, int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fast_kernel(const SdSrc s, int8_t* q, float* scales, int M,
-                                                            int K, int tpr, int rows, uint32_t off_amax, uint32_t off_rows) {
+                                                            int K, int tpr, int rows, uint32_t off_amax, uint32_t off_rows, int early) {
     extern __shared__ __align__(128) uint8_t smem[];
     const unsigned wmask = __activemask();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1178,6 +1181,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem + off_amax);
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
     pdl_wait();
+    if (early) pdl_trigger();
     // rows of this CTA; GroupNorm's belong to one image (blockIdx.y), so that one set of statistics serves the CTA
     const int64_t limit = SRC == SDQ_GN ? (int64_t)(blockIdx.y + 1) * s.P : M;
     const int64_t m0 = (SRC == SDQ_GN ? (int64_t)blockIdx.y * s.P : 0) + (int64_t)blockIdx.x * rows;
@@ -1384,6 +1388,14 @@ int sm_count_of(int dev) {
     return c;
 }
 
+// A quantizer of few CTAs, each on an SM of its own, lets its successor in at once: the other SMs are idle, the successor's setup and
+// whatever it may do ahead (the few-rows GEMM brings its weights to L2) run beside it, and no CTA of the quantizer is left that could
+// land badly. The adaLN linear 1 x 3072 -> 18432 with its quantizer: 17.2 us, now 16.3.
+int early_trigger(int64_t ctas) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return ctas <= sm_count_of(dev);
+}
 template <int ROT, int SRC, int MAXT>
 int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 grid, int threads, int rows, uint32_t smem, uint32_t off_amax,
                   uint32_t off_rows, cudaStream_t st) {
@@ -1399,7 +1411,7 @@ int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 g
             configured.fetch_or(bit, std::memory_order_release);
         }
     }
-    return launch_pdl(kern, grid, threads, smem, st, s, q, scales, M, K, K / 32, rows, off_amax, off_rows);
+    return launch_pdl(kern, grid, threads, smem, st, s, q, scales, M, K, K / 32, rows, off_amax, off_rows, early_trigger((int64_t)grid.x * grid.y));
 }
 template <int ROT, int SRC>
 int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaStream_t st) {
@@ -1531,9 +1543,10 @@ template <typename Kern> int raise_smem(Kern kern, std::atomic<uint64_t>& config
     return (int)e;
 }
 template <typename T, int PRO, int MAXT, bool DIGITS = false>
-int launch_direct(const QuantArgs& p, int threads, size_t smem, cudaStream_t st) {
+int launch_direct(QuantArgs& p, int threads, size_t smem, cudaStream_t st) {
     static std::atomic<uint64_t> configured{0};
     auto kern = quant_direct_kernel<T, PRO, MAXT, DIGITS>;
+    p.early = early_trigger(p.nblocks);
     if (int rc = raise_smem(kern, configured, smem)) return rc;
     return launch_pdl(kern, dim3(p.nblocks), threads, smem, st, p);
 }
@@ -1550,6 +1563,7 @@ template <typename T, int PRO, bool DIGITS = false> int launch_norm(QuantArgs p,
     p.tpr = nwr, p.rows_per_cta = rows, p.nblocks = (p.M + rows - 1) / rows;
     p.off_norm = (uint32_t)(warps * kWarpWords * 4);
     p.off_amax = p.off_norm + rows * 64 * 4;
+    p.early = early_trigger(p.nblocks);
     const size_t smem = p.off_amax + (2 * rows + 1) * 4;
     return warps <= 8 ? launch_norm_cfg<T, PRO, 256, DIGITS>(p, 32 * warps, smem, st) : launch_norm_cfg<T, PRO, 1024, DIGITS>(p, 32 * warps, smem, st);
 }
