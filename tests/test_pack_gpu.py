@@ -241,6 +241,21 @@ def test_sd_group_norm_quantizer(pkg, oracle, dev, N, P, C, G, rotate):
         assert_bits_equal(s, sr, "scales vs the reference kernels"), assert_bits_equal(q, qr, "codes vs the reference kernels")
 
 
+# The statistics read a group's runs of C / G values in pieces of four, two or one, 4096 values at a time: runs of 3, 10, 20 and 32, blocks of
+# less than one, of one and a little and of several such portions, a base off an 8-byte boundary.
+@pytest.mark.parametrize("N,P,C,G,off", [(1, 77, 96, 32, 0), (2, 1500, 96, 32, 0), (2, 300, 320, 32, 0), (1, 9001, 640, 32, 0), (1, 500, 320, 32, 2), (1, 40000, 64, 2, 0)])
+def test_group_norm_statistics_in_pieces(pkg, oracle, dev, N, P, C, G, off):
+    g = torch.Generator().manual_seed(N + P + C)
+    x = (torch.randn(N, P, C, generator=g) * 1.5 + 0.25).half()
+    w, b = torch.randn(C, generator=g) * 0.2 + 1.0, torch.randn(C, generator=g) * 0.1
+    base = torch.zeros(x.numel() + off, dtype=torch.half, device=dev)
+    xd = base[off:].view(N, P, C)
+    xd.copy_(x)
+    q, s = pkg.linear.sd_group_norm_quant_rows(xd, w.to(dev), b.to(dev), G, 1e-5, 0)
+    qo, so = oracle.sd_group_norm_quant_rows(x, w, b, G, 1e-5, 0)
+    assert_bits_equal(s, so, "scales"), assert_bits_equal(q, qo, "codes")
+
+
 def test_argument_checks_of_the_packers_and_fused_quantizers(pkg, dev):
     L = pkg.linear
     with pytest.raises(RuntimeError, match="-1"):
