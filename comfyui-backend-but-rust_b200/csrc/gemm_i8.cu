@@ -68,6 +68,8 @@ struct GemmParams {
     int act;
     int vec_ok;          // per-column vectors and rows of D / resid can be read and written 16 bytes at a time
     int tma_store;       // D is written through shared memory with TMA stores
+    int staging;         // bytes of epilogue staging in front of the operand ring
+    int bufs;            // chunk buffers per epilogue warp of the staged drain (epilogue_staged), 0: another form
     int wide;            // 2-byte outputs in whole tiles straight from registers: 2 when rows of D (and of the residual) can be accessed 32 bytes at a time, 1: 16
     int bn;              // columns per tile (multiple of 32, <= 256); each CTA of the pair stages bn/2 rows of W
     int stages;          // shared-memory ring depth
@@ -513,24 +515,21 @@ __device__ __forceinline__ void drain_resid(const GemmParams& p, uint4 (&rq)[4],
 #pragma unroll
     for (int j = 0; j < 4; ++j) rq[j] = row_ok && col + 8 * j < p.N ? gload(r + j) : make_uint4(0, 0, 0, 0);
 }
+// A chunk's 32 values of a lane's row, packed two to a word
 template <typename OutT, int EPI>
-__device__ __forceinline__ void drain_chunk(const GemmParams& p, const uint32_t (&r)[32], const uint4 (&rq)[4], int row, int col, float xs,
-                                            const float* vs, const uint16_t* lut_sm) {
+__device__ __forceinline__ void drain_values(const GemmParams& p, const uint32_t (&r)[32], const uint4 (&rq)[4], float xs, const float* vs,
+                                             const uint16_t* lut_sm, uint32_t (&o)[16]) {
     const float2 xs2 = make_float2(xs, xs);
-    OutT* d = reinterpret_cast<OutT*>(p.D) + (int64_t)row * p.N + col;
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        uint32_t o[8];
+    for (int j = 0; j < 4; ++j) {
         if constexpr (EPI == EPI_ACT_LUT) {
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const uint4 t = epilogue8_lut<128>(p, r + 16 * u + 8 * j, xs, vs + 16 * u + 8 * j, lut_sm);
-                o[4 * j] = t.x, o[4 * j + 1] = t.y, o[4 * j + 2] = t.z, o[4 * j + 3] = t.w;
-            }
+            const uint4 t = epilogue8_lut<128>(p, r + 8 * j, xs, vs + 8 * j, lut_sm);
+            o[4 * j] = t.x, o[4 * j + 1] = t.y, o[4 * j + 2] = t.z, o[4 * j + 3] = t.w;
         } else {
+            const uint32_t q4[4] = {rq[j].x, rq[j].y, rq[j].z, rq[j].w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int c = 16 * u + 4 * j;
+            for (int h = 0; h < 2; ++h) {
+                const int c = 8 * j + 4 * h;
                 const float4 w = *reinterpret_cast<const float4*>(vs + c), b = *reinterpret_cast<const float4*>(vs + 128 + c);
                 float2 v0 = __ffma2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[c]), __int2float_rn((int)r[c + 1])), xs2), make_float2(w.x, w.y),
                                        make_float2(b.x, b.y));
@@ -538,19 +537,28 @@ __device__ __forceinline__ void drain_chunk(const GemmParams& p, const uint32_t 
                                        make_float2(w.z, w.w), make_float2(b.z, b.w));
                 if constexpr (EPI == EPI_RESID) {
                     const float4 s = *reinterpret_cast<const float4*>(vs + 256 + c);
-                    const uint4 q = rq[2 * u + (j >> 1)];
-                    v0 = __ffma2_rn(unpack2<OutT>(pack2<OutT>(v0)), make_float2(s.x, s.y), unpack2<OutT>(j & 1 ? q.z : q.x));
-                    v1 = __ffma2_rn(unpack2<OutT>(pack2<OutT>(v1)), make_float2(s.z, s.w), unpack2<OutT>(j & 1 ? q.w : q.y));
+                    v0 = __ffma2_rn(unpack2<OutT>(pack2<OutT>(v0)), make_float2(s.x, s.y), unpack2<OutT>(q4[2 * h]));
+                    v1 = __ffma2_rn(unpack2<OutT>(pack2<OutT>(v1)), make_float2(s.z, s.w), unpack2<OutT>(q4[2 * h + 1]));
                 }
-                o[2 * j] = pack2<OutT>(v0), o[2 * j + 1] = pack2<OutT>(v1);
+                o[4 * j + 2 * h] = pack2<OutT>(v0), o[4 * j + 2 * h + 1] = pack2<OutT>(v1);
             }
         }
-        if (row < p.M && col + 16 * u < p.N) {
-            if (p.wide == 2) st_global_v8(d + 16 * u, o);
-            else {
-                *reinterpret_cast<uint4*>(d + 16 * u) = make_uint4(o[0], o[1], o[2], o[3]);
-                if (col + 16 * u + 8 < p.N) *reinterpret_cast<uint4*>(d + 16 * u + 8) = make_uint4(o[4], o[5], o[6], o[7]);
-            }
+    }
+}
+template <typename OutT, int EPI>
+__device__ __forceinline__ void drain_chunk(const GemmParams& p, const uint32_t (&r)[32], const uint4 (&rq)[4], int row, int col, float xs,
+                                            const float* vs, const uint16_t* lut_sm) {
+    uint32_t o[16];
+    drain_values<OutT, EPI>(p, r, rq, xs, vs, lut_sm, o);
+    OutT* d = reinterpret_cast<OutT*>(p.D) + (int64_t)row * p.N + col;
+    if (row >= p.M) return;
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        if (col + 16 * u >= p.N) return;
+        if (p.wide == 2) st_global_v8(d + 16 * u, *reinterpret_cast<const uint32_t(*)[8]>(o + 8 * u));
+        else {
+            *reinterpret_cast<uint4*>(d + 16 * u) = make_uint4(o[8 * u], o[8 * u + 1], o[8 * u + 2], o[8 * u + 3]);
+            if (col + 16 * u + 8 < p.N) *reinterpret_cast<uint4*>(d + 16 * u + 8) = make_uint4(o[8 * u + 4], o[8 * u + 5], o[8 * u + 6], o[8 * u + 7]);
         }
     }
 }
@@ -637,6 +645,119 @@ __device__ __forceinline__ void epilogue_wide(const GemmParams& p, uint8_t* stag
         buf ^= 1;
         if (buf == 0) tphase ^= 1u;
     }
+}
+
+// The same through shared memory, for problems whose K is so short that the drain sets the pace. Stores from registers, a row per lane, cost the
+// load-store unit about 53 cycles per kilobyte (32 different lines an instruction): 6900 of a 256 x 256 tile's 7400 at K = 640, where the
+// tile's MMAs take 2560. Written to shared memory and from there by the copy engine they cost 8, but the engine takes its time, so
+// a warp has several chunk buffers and never waits for the chunk just stored. The residual comes the same way, the whole tile of it
+// (four buffers) while the accumulator is awaited. The buffers' room is the ring's: four to five K boxes of operands instead of
+// six, which a tile of few boxes does not miss. Registers -> this, 8192 rows: 640 -> 5120 38.5 -> 31.0 us, with a residual 73.9 -> 45.7;
+// 1280 -> 5120 with a residual 77.7 -> 53.9; 16896 x 640 -> 3072 44.0 -> 36.6 and 81.3 -> 53.6. The lines lie where the longer ring is worth as much as
+// the cheaper drain: 8192 x 1280 -> 5120 42.7 from registers and 43.3 this way, with a residual 2048 -> 5120 83.7 and 72.1, 2560 -> 5120 even.
+constexpr int kStagedMaxK = 1024, kStagedMaxKResid = 2048;
+constexpr int kResidBarOffset = 256;          // in the tail: a barrier per epilogue warp for the residual's copies
+template <typename OutT, int EPI>
+__device__ __forceinline__ void epilogue_staged(const GemmParams& p, const CUtensorMap* tmap_d, const CUtensorMap* tmap_r, uint8_t* staging, uint32_t bar_tail,
+                                                uint32_t bar_tfull, uint32_t bar_tempty, uint32_t tmem_base, volatile int* abort_s, int rank,
+                                                int cluster_id, int nclusters, int warp, int lane) {
+    const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+    const int nchunks = p.bn / 32, first = half * ((nchunks + 1) / 2), chunks = min((nchunks + 1) / 2, nchunks - first);
+    uint8_t* mine = staging + ew * p.bufs * 2048;
+    const uint32_t mine_u32 = smem_u32(mine), bar_r = bar_tail + kResidBarOffset + 8 * ew;
+    float* vec = reinterpret_cast<float*>(staging + kEpiWarps * p.bufs * 2048 + ew * (EPI == EPI_RESID ? 1536 : 1024));
+    const int sw = (lane >> 1) & 3;            // 64-byte rows, 64-byte swizzle
+    int buf = 0, slot = 0;
+    uint32_t tphase = 0, rphase = 0;
+    auto place = [&](int w, int& row, int& col0) {
+        int tm, tn;
+        tile_coords(w, p.tiles_m, p.tiles_n, tm, tn, p.group_m ? p.group_m : 8);
+        row = tm * (2 * BM) + rank * BM + quad * 32 + lane, col0 = tn * p.bn + 32 * first;
+    };
+    auto residual = [&](int row, int col0) {   // lane 0: the tile's residual on its way
+        const int n = min(chunks, (p.N - col0 + 31) / 32);
+        if (n <= 0) return;
+        mbar_arrive_expect_tx(bar_r, (uint32_t)n * 2048u);
+        for (int c = 0; c < n; ++c) tma_load_2d(mine_u32 + 2048 * c, tmap_r, col0 + 32 * c, row, bar_r);
+    };
+    DrainVecs next;
+    int row, col0;
+    if (cluster_id < p.num_items) {
+        place(cluster_id, row, col0);
+        if (EPI == EPI_RESID && lane == 0) residual(row, col0);
+        next.fetch<OutT, EPI>(p, row, col0, chunks, lane);
+    }
+    for (int w = cluster_id; w < p.num_items; w += nclusters) {
+        place(w, row, col0);
+        const float xs = next.xs;
+        next.stage<EPI>(vec, lane);
+        int nrow = 0, ncol = 0;
+        const bool more = w + nclusters < p.num_items;
+        if (more) {
+            place(w + nclusters, nrow, ncol);
+            next.fetch<OutT, EPI>(p, nrow, ncol, chunks, lane);
+        }
+        bool ok = true;
+        if (EPI == EPI_RESID && col0 < p.N) {
+            ok = mbar_wait(bar_r, rphase, abort_s, ST_TIMEOUT_TMEM_FULL);       // every lane reads what has landed
+            rphase ^= 1u;
+        }
+        if (lane == 0) ok = ok && mbar_wait(bar_tfull + 8 * buf, tphase, abort_s, ST_TIMEOUT_TMEM_FULL);
+        if (!__all_sync(0xffffffffu, ok)) break;
+        tc_fence_after();
+        const uint32_t taddr = tmem_base + buf * 256 + ((uint32_t)(quad * 32) << 16) + 32 * first;
+        auto chunk = [&](const uint32_t (&r)[32], int c) {
+            if (col0 + 32 * c >= p.N) return;
+            uint8_t* rowp = mine + 2048 * (EPI == EPI_RESID ? c : slot) + lane * 64;
+            uint4 rq[4];
+            if constexpr (EPI == EPI_RESID) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) rq[j] = *reinterpret_cast<const uint4*>(rowp + ((j ^ sw) << 4));
+            }
+            uint32_t o[16];
+            drain_values<OutT, EPI>(p, r, rq, xs, vec + 32 * c, nullptr, o);
+            if (EPI != EPI_RESID) {
+                if (lane == 0) bulk_wait_read<2>();       // three buffers: the store before the last two has read this one
+                __syncwarp();
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(rowp + ((j ^ sw) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_2d(tmap_d, mine_u32 + 2048 * (EPI == EPI_RESID ? c : slot), col0 + 32 * c, row);
+                bulk_commit();
+            }
+            if (++slot == 3) slot = 0;
+        };
+        auto done = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_remote(mapa_shared(bar_tempty + 8 * buf, 0));
+        };
+        uint32_t ra[32], rb[32];
+        tmem_ld32(taddr, ra);
+#pragma unroll 1
+        for (int c = 0; c < chunks; c += 2) {
+            tmem_ld_wait();
+            if (c + 1 < chunks) tmem_ld32(taddr + 32 * (c + 1), rb);
+            else done();
+            chunk(ra, c);
+            if (c + 1 < chunks) {
+                tmem_ld_wait();
+                if (c + 2 < chunks) tmem_ld32(taddr + 32 * (c + 2), ra);
+                else done();
+                chunk(rb, c + 1);
+            }
+        }
+        if (EPI == EPI_RESID && more && lane == 0) {
+            bulk_wait_read<0>();                          // the buffers are free again
+            residual(nrow, ncol);
+        }
+        buf ^= 1;
+        if (buf == 0) tphase ^= 1u;
+    }
+    if (lane == 0) bulk_wait_read<0>();       // staged rows have left shared memory before the CTA exits (the writes are complete when the grid is)
 }
 
 // ---- the rotating epilogue (EPI_ACT_ROT) --------------------------------------------------------------------------------
@@ -865,7 +986,7 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
 template <typename OutT, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(EPI == EPI_ACT_ROT ? kRotThreads : kThreads, 1)
 gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                    const __grid_constant__ CUtensorMap tmap_d, const GemmParams p) {
+                    const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_r, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw_addr = smem_u32(smem_raw);
     const uint32_t base = (raw_addr + 1023u) & ~1023u;   // same offset in both CTAs of the pair
@@ -876,10 +997,10 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
     const uint32_t a_bytes = BM * BK;                     // one 128-byte K box of this CTA's A rows
     const uint32_t b_bytes = (uint32_t)(BN / 2) * BK;     // ... and of this CTA's half of the W tile
     const uint32_t stage_bytes = KS * (a_bytes + b_bytes);
-    uint8_t* staging = sm;                                 // kEpiWarps x 4 KB of output staging
-    const uint32_t sA = base + kStagingBytes;              // S x KS x [128 x 128]
+    uint8_t* staging = sm;                                 // output staging
+    const uint32_t sA = base + p.staging;                  // S x KS x [128 x 128]
     const uint32_t sB = sA + S * KS * a_bytes;             // S x KS x [bn/2 x 128]
-    uint8_t* tail = sm + kStagingBytes + S * stage_bytes;
+    uint8_t* tail = sm + p.staging + S * stage_bytes;
     const uint32_t bar_full = smem_u32(tail);              // kMaxStages barriers (the leader's are used)
     const uint32_t bar_empty = bar_full + 8 * kMaxStages;  // kMaxStages, one set per CTA
     const uint32_t bar_tfull = bar_empty + 8 * kMaxStages; // 2, per CTA
@@ -901,11 +1022,14 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             mbar_init(bar_tfull + 8 * i, 1);
             mbar_init(bar_tempty + 8 * i, 2 * (EPI == EPI_ACT_ROT ? kRotEpiWarps : kEpiWarps));
         }
+        if (EPI == EPI_RESID)
+            for (int i = 0; i < kEpiWarps; ++i) mbar_init(bar_full + kResidBarOffset + 8 * i, 1);
         *abort_s = 0;
         fence_mbar_init();
         prefetch_tmap(&tmap_a);
         prefetch_tmap(&tmap_w);
         if (p.tma_store) prefetch_tmap(&tmap_d);
+        if (EPI == EPI_RESID && p.bufs) prefetch_tmap(&tmap_r);
     }
     if (warp == 1) {
         tmem_alloc_pair(smem_u32(tmem_ptr_s), 512);
@@ -1008,6 +1132,10 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         if constexpr (EPI == EPI_ACT_ROT) {
             epilogue_rot(p, &tmap_d, staging, tail, bar_tfull, bar_tempty, tmem_base, abort_s, (int)rank, cluster_id, nclusters, warp,
                          lane);
+        } else if ((EPI == EPI_PLAIN || EPI == EPI_RESID) && sizeof(OutT) == 2 && p.bufs) {
+            if constexpr ((EPI == EPI_PLAIN || EPI == EPI_RESID) && sizeof(OutT) == 2)
+                epilogue_staged<OutT, EPI>(p, &tmap_d, &tmap_r, staging, bar_full, bar_tfull, bar_tempty, tmem_base, abort_s, (int)rank, cluster_id,
+                                           nclusters, warp, lane);
         } else if (EPI != EPI_ACC && sizeof(OutT) == 2 && EPI != EPI_ACT && p.wide) {
             if constexpr (EPI != EPI_ACC && sizeof(OutT) == 2 && EPI != EPI_ACT)
                 epilogue_wide<OutT, EPI>(p, staging, bar_tfull, bar_tempty, tmem_base, abort_s, (int)rank, cluster_id, nclusters, warp, lane);
@@ -1423,7 +1551,7 @@ int device_sm_count(int dev) {
 }
 
 template <typename OutT, int EPI>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, const GemmParams& p, int grid,
+int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, const CUtensorMap& tr, const GemmParams& p, int grid,
                 cudaStream_t st) {
     auto kern = gemm_i8_pair_kernel<OutT, EPI>;
     static std::atomic<uint64_t> configured{0};
@@ -1435,20 +1563,20 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap&
         if (e != cudaSuccess) return (int)e;
         configured.fetch_or(bit, std::memory_order_release);
     }
-    return launch_pdl(kern, dim3(grid), EPI == EPI_ACT_ROT ? kRotThreads : kThreads, kSmemBytes, st, ta, tw, td, p);
+    return launch_pdl(kern, dim3(grid), EPI == EPI_ACT_ROT ? kRotThreads : kThreads, kSmemBytes, st, ta, tw, td, tr, p);
 }
 template <typename OutT>
-int launch_pair_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, const GemmParams& p,
+int launch_pair_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, const CUtensorMap& tr, const GemmParams& p,
                     int grid, cudaStream_t st) {
     switch (epi) {
-        case EPI_PLAIN: return launch_pair<OutT, EPI_PLAIN>(ta, tw, td, p, grid, st);
-        case EPI_RESID: return launch_pair<OutT, EPI_RESID>(ta, tw, td, p, grid, st);
-        case EPI_ACT: return launch_pair<OutT, EPI_ACT>(ta, tw, td, p, grid, st);
+        case EPI_PLAIN: return launch_pair<OutT, EPI_PLAIN>(ta, tw, td, tr, p, grid, st);
+        case EPI_RESID: return launch_pair<OutT, EPI_RESID>(ta, tw, td, tr, p, grid, st);
+        case EPI_ACT: return launch_pair<OutT, EPI_ACT>(ta, tw, td, tr, p, grid, st);
         case EPI_ACT_LUT:
-            if constexpr (std::is_same<OutT, bf16>::value) return launch_pair<bf16, EPI_ACT_LUT>(ta, tw, td, p, grid, st);
+            if constexpr (std::is_same<OutT, bf16>::value) return launch_pair<bf16, EPI_ACT_LUT>(ta, tw, td, tr, p, grid, st);
             return -200;
         case EPI_ACT_ROT:
-            if constexpr (std::is_same<OutT, bf16>::value) return launch_pair<bf16, EPI_ACT_ROT>(ta, tw, td, p, grid, st);
+            if constexpr (std::is_same<OutT, bf16>::value) return launch_pair<bf16, EPI_ACT_ROT>(ta, tw, td, tr, p, grid, st);
             return -200;
         default: return -200;
     }
@@ -1638,13 +1766,18 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
     }
     if (rot)
         if (int rc = act_lut_ptr(act, st, &p.act_lut)) return rc;
-    p.ksub = K <= BK ? 1 : 2;
+    if (esz == 2 && p.tma_store) {
+        if (epi == EPI_PLAIN && K <= kStagedMaxK) p.bufs = 3;
+        if (epi == EPI_RESID && K <= kStagedMaxKResid && al16(resid)) p.bufs = 4;
+    }
+    p.staging = p.bufs ? kEpiWarps * (p.bufs * 2048 + (epi == EPI_RESID ? 1536 : 1024)) : kStagingBytes;
+    p.ksub = K <= BK || p.bufs ? 1 : 2;
     p.k_iters = (int)((K + p.ksub * BK - 1) / (p.ksub * BK));
     const int bn = rot ? 256 : choose_bn(M, N, clusters);
     p.bn = bn;
     p.idesc = umma_idesc_i8(2 * BM, bn);
     const int stage_bytes = p.ksub * (BM * BK + (bn / 2) * BK);
-    const int stages = (kSmemBytes - 1024 - kTailBytes - kStagingBytes) / stage_bytes;
+    const int stages = (kSmemBytes - 1024 - kTailBytes - p.staging) / stage_bytes;
     p.stages = stages > kMaxStages ? kMaxStages : stages;
     p.tiles_m = (int)((M + 2 * BM - 1) / (2 * BM));
     p.tiles_n = (int)((N + bn - 1) / bn);
@@ -1656,7 +1789,7 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
         const int gm = (int)((p.tiles_m + bands - 1) / bands);
         p.group_m = (N * K > kResidentOperandBytes / 2 && gm > 12) ? gm : 8;      // a little taller than eight makes no difference
     }
-    CUtensorMap ta, tw, td;
+    CUtensorMap ta, tw, td, tr;
     if (!make_operand_tmap(&ta, A, M, K, BM) || !make_operand_tmap(&tw, W, N, K, bn / 2)) return -203;
     if (rot) {
         if (!make_output_tmap16(&td, D, M, N)) return -203;
@@ -1664,6 +1797,11 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
         if (!make_output_tmap(&td, D, M, N, esz)) return -203;
     } else {
         td = ta;  // unused
+    }
+    if (p.bufs && epi == EPI_RESID) {
+        if (!make_output_tmap(&tr, const_cast<void*>(resid), M, N, esz)) return -203;
+    } else {
+        tr = td;  // unused
     }
     // K split: a problem with fewer tiles than clusters and a long K (few rows, few columns) is cut along K so that
     // more SMs stream it; partial sums meet by atomic adds and the slice that arrives last runs the epilogue. Measured
@@ -1675,7 +1813,7 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
     p.whole_tiles = p.num_tiles, p.splits = 0, p.kps = p.k_iters, p.num_items = p.num_tiles;
     p.scratch = nullptr, p.partials = nullptr;
     const int rem = p.num_tiles % clusters;
-    if (!rot && rem > 0 && p.num_tiles < clusters && 2 * rem <= clusters && p.k_iters >= 16) {
+    if (!rot && !p.bufs && rem > 0 && p.num_tiles < clusters && 2 * rem <= clusters && p.k_iters >= 16) {
         int splits = clusters / rem;
         if (splits > p.k_iters / 8) splits = p.k_iters / 8;
         if (splits > 16) splits = 16;
@@ -1693,10 +1831,10 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
     p.wide = esz == 2 && p.splits == 0 ? wide_rows(N, D, resid) : 0;
     const int grid = 2 * (p.num_items < clusters ? p.num_items : clusters);
     int rc;
-    if (epi == EPI_ACC) rc = launch_pair<float, EPI_ACC>(ta, tw, td, p, grid, st);
-    else if (out_dt == DT_F32) rc = launch_pair_epi<float>(epi, ta, tw, td, p, grid, st);
-    else if (out_dt == DT_F16) rc = launch_pair_epi<half>(epi, ta, tw, td, p, grid, st);
-    else rc = launch_pair_epi<bf16>(epi, ta, tw, td, p, grid, st);
+    if (epi == EPI_ACC) rc = launch_pair<float, EPI_ACC>(ta, tw, td, tr, p, grid, st);
+    else if (out_dt == DT_F32) rc = launch_pair_epi<float>(epi, ta, tw, td, tr, p, grid, st);
+    else if (out_dt == DT_F16) rc = launch_pair_epi<half>(epi, ta, tw, td, tr, p, grid, st);
+    else rc = launch_pair_epi<bf16>(epi, ta, tw, td, tr, p, grid, st);
     return rc;
 }
 
@@ -1864,6 +2002,7 @@ GPU_API int gpu_int8_gemm_noalloc(const int8_t* A, const int8_t* W, const float*
     auto al16 = [](const void* q) { return ((uintptr_t)q & 15) == 0; };
     p.vec_ok = (N % 8 == 0) && al16(D) && al16(ws) && al16(bias);
     p.tma_store = al16(D) && ((N * esz) % 16 == 0);
+    p.staging = kStagingBytes;
     p.ksub = K <= BK ? 1 : 2;
     p.k_iters = (int)((K + p.ksub * BK - 1) / (p.ksub * BK));
     // the width that fills the clusters best, widened while the tiles outnumber the array's 16 slots
@@ -1903,9 +2042,9 @@ GPU_API int gpu_int8_gemm_noalloc(const int8_t* A, const int8_t* W, const float*
         td = ta;
     }
     const int grid = 2 * (p.num_items < clusters ? p.num_items : clusters);
-    if (out_dt == DT_F32) return launch_pair<float, EPI_PLAIN>(ta, tw, td, p, grid, st);
-    if (out_dt == DT_F16) return launch_pair<half, EPI_PLAIN>(ta, tw, td, p, grid, st);
-    return launch_pair<bf16, EPI_PLAIN>(ta, tw, td, p, grid, st);
+    if (out_dt == DT_F32) return launch_pair<float, EPI_PLAIN>(ta, tw, td, td, p, grid, st);
+    if (out_dt == DT_F16) return launch_pair<half, EPI_PLAIN>(ta, tw, td, td, p, grid, st);
+    return launch_pair<bf16, EPI_PLAIN>(ta, tw, td, td, p, grid, st);
 }
 
 

@@ -102,6 +102,14 @@ def test_outputs_written_from_registers(pkg, dev, dtype, M, N, K, limit):
     assert L.kernel_status() == 0
 
 
+# Short K: outputs and residual through shared memory up to K = 1024 and 2048, from registers beyond; rows and columns that end inside a
+# chunk and inside a tile, one tile and many a cluster, a warp whose columns all lie outside the matrix.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,limit", [(2100, 1304, 1024, 2), (2100, 1304, 1152, 2), (1500, 2600, 2048, 3), (1500, 2600, 2176, 3), (4099, 1032, 128, 1)])
+def test_outputs_written_through_shared_memory(pkg, dev, dtype, M, N, K, limit):
+    test_outputs_written_from_registers(pkg, dev, dtype, M, N, K, limit)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 def test_bit_exact_against_the_reference_gemm(pkg, ref, dev, dtype):
     # the last five take the one-CTA-per-tile kernel (small problems; 2048 x 1280 x 1280 by its second rule)
