@@ -1084,7 +1084,8 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
         // stage: descriptor low words advance by adds, nothing 64-bit, one commit (its arrival multicast to both
         // CTAs), no fence between stages (TMA writes and MMA reads are async-proxy accesses ordered by the
         // mbarrier itself), and stages of two K boxes halve the barrier traffic per MMA.
-        if (leader && lane == 0) {
+        if (leader) {
+            const bool one = elect_one();       // the whole warp walks the stages, one lane issues: see the one-CTA kernel
             const uint32_t a_lo0 = umma_desc_lo(sA), b_lo0 = umma_desc_lo(sB);
             const uint32_t a_sub = a_bytes >> 4, b_sub = b_bytes >> 4;        // next K box of a stage
             const uint32_t a_step = KS * a_sub, b_step = KS * b_sub;          // next stage
@@ -1097,14 +1098,12 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
             bool ok = true;
             for (int w = cluster_id; w < p.num_items && ok; w += nclusters) {
                 const int kn = decode_item(p, w).kn;
-                if (!mbar_wait(bar_tempty + 8 * buf, tphase ^ 1u, abort_s, ST_TIMEOUT_TMEM_EMPTY)) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_tempty + 8 * buf, tphase ^ 1u, abort_s, ST_TIMEOUT_TMEM_EMPTY))) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + buf * 256;
                 for (int kb = 0; kb < kn; ++kb) {
-                    if (!mbar_try_wait(bar_f, phase)) {
-                        if (!mbar_wait(bar_f, phase, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
-                    }
-                    {
+                    if (!__all_sync(0xffffffffu, mbar_wait(bar_f, phase, abort_s, ST_TIMEOUT_FULL))) { ok = false; break; }
+                    if (one) {
                         umma_pair_lo(d_tmem, a_lo, b_lo, idesc, kb);
                         umma_pair_lo(d_tmem, a_lo + 2, b_lo + 2, idesc, 1);   // +32 bytes inside the swizzle row
                         umma_pair_lo(d_tmem, a_lo + 4, b_lo + 4, idesc, 1);
@@ -1116,13 +1115,15 @@ gemm_i8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_con
                             umma_pair_lo(d_tmem, a2 + 4, b2 + 4, idesc, 1);
                             umma_pair_lo(d_tmem, a2 + 6, b2 + 6, idesc, 1);
                         }
+                        umma_commit_pair(bar_e);   // the stage is free in both CTAs once these MMAs have read it
                     }
-                    umma_commit_pair(bar_e);   // the stage is free in both CTAs once these MMAs have read it
+                    __syncwarp();
                     ++stage, a_lo += a_step, b_lo += b_step, bar_f += 8, bar_e += 8;
                     if (stage == S) stage = 0, phase ^= 1u, a_lo = a_lo0, b_lo = b_lo0, bar_f = bar_full, bar_e = bar_empty;
                 }
                 if (!ok) break;
-                umma_commit_pair(bar_tfull + 8 * buf);   // accumulator complete: both epilogues may drain it
+                if (one) umma_commit_pair(bar_tfull + 8 * buf);   // accumulator complete: both epilogues may drain it
+                __syncwarp();
                 buf ^= 1;
                 if (buf == 0) tphase ^= 1u;
             }

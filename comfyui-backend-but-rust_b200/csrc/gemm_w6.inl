@@ -445,25 +445,27 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = p.idesc;
-            int sa = 0, sb = 0;
-            uint32_t pa = 0, pb = 0;
-            bool ok = true;
-            for (int kb = k0; kb < k1; ++kb) {
-                if (!mbar_wait(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
-                if (!mbar_wait(bar_wfull + 8 * sb, pb, abort_s, ST_TIMEOUT_FULL)) { ok = false; break; }
-                tc_fence_after();
-                const uint32_t dw = umma_desc_lo(sW + sb * w_bytes), da = umma_desc_lo(sA + sa * a_bytes);
+        const bool one = elect_one();          // the whole warp walks the boxes, one lane issues: see the one-CTA int8 kernel
+        const uint32_t idesc = p.idesc;
+        int sa = 0, sb = 0;
+        uint32_t pa = 0, pb = 0;
+        bool ok = true;
+        for (int kb = k0; kb < k1; ++kb) {
+            if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_FULL) &&
+                                             mbar_wait(bar_wfull + 8 * sb, pb, abort_s, ST_TIMEOUT_FULL))) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t dw = umma_desc_lo(sW + sb * w_bytes), da = umma_desc_lo(sA + sa * a_bytes);
+            if (one) {
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k) umma_i8_lo(tmem_base, dw + 2 * k, da + 2 * k, idesc, (kb - k0) | k);
                 umma_commit(bar_wempty + 8 * sb);
                 umma_commit(bar_empty + 8 * sa);
-                if (++sa == SA) sa = 0, pa ^= 1u;
-                if (++sb == SB) sb = 0, pb ^= 1u;
             }
-            if (ok) umma_commit(bar_tfull);
+            __syncwarp();
+            if (++sa == SA) sa = 0, pa ^= 1u;
+            if (++sb == SB) sb = 0, pb ^= 1u;
         }
+        if (ok && one) umma_commit(bar_tfull);
     } else {
         const int uw = warp - 2, grp = uw >> 2;
         const int r = 32 * (uw & 3) + lane;                        // weight row of the tile

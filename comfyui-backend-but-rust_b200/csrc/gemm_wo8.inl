@@ -97,26 +97,31 @@ gemm_wo8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             }
         }
     } else if (warp == 1) {
-        if (leader && lane == 0) {
+        if (leader) {
+            const bool one = elect_one();
             int stage = 0;
             uint32_t phase = 0, tphase = 0;
             int kb = (int)(u0 % p.k_iters);
             bool fresh = true;
             for (int64_t u = u0; u < u1; ++u) {
-                if (fresh && !mbar_wait(bar_tempty, tphase ^ 1u, abort_s, ST_TIMEOUT_TMEM_EMPTY)) break;
+                if (fresh && !__all_sync(0xffffffffu, mbar_wait(bar_tempty, tphase ^ 1u, abort_s, ST_TIMEOUT_TMEM_EMPTY))) break;
                 if (fresh) tc_fence_after();
-                if (!mbar_wait(bar_full + 8 * stage, phase, abort_s, ST_TIMEOUT_FULL)) break;
+                if (!__all_sync(0xffffffffu, mbar_wait(bar_full + 8 * stage, phase, abort_s, ST_TIMEOUT_FULL))) break;
                 const uint32_t w_lo = umma_desc_lo(base + stage * stage_bytes), x_lo = w_lo + (w_bytes >> 4);
+                if (one) {
 #pragma unroll
-                for (int k = 0; k < BK / UMMA_K; ++k) {
-                    umma_pair_lo(tmem_base, w_lo + 2 * k, x_lo + 2 * k, umma_idesc_i8(2 * BM, 2 * r0), !fresh || k != 0);
-                    if (r1 > 0) umma_pair_lo(tmem_base + 2 * r0, w_lo + 2 * k, x_lo + 8 * r0 + 2 * k, umma_idesc_i8(2 * BM, 2 * r1), !fresh || k != 0);
+                    for (int k = 0; k < BK / UMMA_K; ++k) {
+                        umma_pair_lo(tmem_base, w_lo + 2 * k, x_lo + 2 * k, umma_idesc_i8(2 * BM, 2 * r0), !fresh || k != 0);
+                        if (r1 > 0) umma_pair_lo(tmem_base + 2 * r0, w_lo + 2 * k, x_lo + 8 * r0 + 2 * k, umma_idesc_i8(2 * BM, 2 * r1), !fresh || k != 0);
+                    }
+                    umma_commit_pair(bar_empty + 8 * stage);
                 }
-                umma_commit_pair(bar_empty + 8 * stage);
+                __syncwarp();
                 if (++stage == S) stage = 0, phase ^= 1u;
                 fresh = ++kb == p.k_iters || u + 1 == u1;
                 if (fresh) {
-                    umma_commit_pair(bar_tfull);
+                    if (one) umma_commit_pair(bar_tfull);
+                    __syncwarp();
                     tphase ^= 1u;
                     if (kb == p.k_iters) kb = 0;
                 }
