@@ -367,8 +367,12 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 // outputs each, reading one another's through distributed shared memory: no scratch in global memory, nothing to clear.
 // The four linears of a 5120-wide block with FFN 13824 at 64 rows, under ncu: 231 us on the pair kernel, 128 here.
 // Warp 0 loads (packed planes and tokens of a K box, one barrier), warp 1 issues the MMAs, warps 2..21 expand: five groups
-// of four warps take K boxes in turn, one thread per weight row (the expansion is what bounds the kernel, a few instructions per
-// code; three groups left the issue slots idle two cycles in five). All of them run the epilogue: a lane owns an output column.
+// of four warps take K boxes in turn (the expansion is what bounds the kernel, a few instructions per code; three groups left the
+// issue slots idle two cycles in five). A lane expands one scale group of one row at a time, eight rows of a box to a warp's step, so
+// that a tile need not have 128 rows: the host side picks the height (a multiple of eight; the MMA's other rows are never read) that
+// spreads the weight's rows evenly over the SMs. 15360 rows are 120 tiles of 128 for 148 SMs, or 148 of 104. All of them run the epilogue:
+// a lane owns an output column. Tiles of 128 rows and one row a lane -> this, at 64 tokens: 5120 -> 15360 34.0 -> 31.8 us, 5120 -> 13824 34.4 -> 30.4;
+// 5120 -> 5120 (40 tiles in either form) 18.6 -> 18.9, 13824 -> 5120 30.8 -> 31.4.
 constexpr int kW6RowsWarps = 20;
 constexpr int kW6RowsThreads = 32 * (2 + kW6RowsWarps);
 constexpr int kW6RowsMaxTokens = 256;
@@ -379,6 +383,7 @@ struct W6RowsParams {
     int splits, kps;        // CTAs of a cluster share a row tile's K: kps boxes each
     int sa, sb;             // ring depths: packed planes + tokens, expanded tiles
     int groups;             // expanding groups of four warps in use
+    int height;             // weight rows of a tile, a multiple of 8, at most 128
 };
 __device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
     int v;
@@ -396,7 +401,8 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const uint32_t base = (raw_addr + 1023u) & ~1023u;     // the same offset in every CTA of the cluster
     uint8_t* sm = smem_raw + (base - raw_addr);
     const int SA = x6.sa, SB = x6.sb, T = x6.tokens;
-    const uint32_t w_bytes = BM * BK, lo_bytes = BM * 64, hi_bytes = BM * 32;
+    const int R = x6.height;
+    const uint32_t w_bytes = BM * BK, lo_bytes = (uint32_t)(R * 64 + 1023) & ~1023u, hi_bytes = (uint32_t)R * 32;
     const uint32_t a_bytes = ((uint32_t)T * BK + 1023u) & ~1023u;      // a tile of 16-row pieces, 1024-byte aligned
     const uint32_t sW = base, sA = sW + SB * w_bytes, sLo = sA + SA * a_bytes, sHi = sLo + SA * lo_bytes;
     // barriers sit at the end of the allocation: the accumulators overwrite the rings when these are done with
@@ -409,7 +415,7 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t tmem_cols = T <= 32 ? 32u : T <= 64 ? 64u : T <= 128 ? 128u : 256u;
     const int tn = blockIdx.x / x6.splits, rank = blockIdx.x - tn * x6.splits;     // a cluster = the slices of one row tile
-    const int n0 = tn * BM;
+    const int n0 = tn * R;
     const int t0 = TILED ? blockIdx.y * T : 0, rows = TILED ? min(p.M - t0, T) : p.M;      // this tile's tokens
     const int k0 = rank * x6.kps, k1 = min(k0 + x6.kps, p.k_iters);                // never empty: the host side sees to it
 
@@ -437,7 +443,7 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             uint32_t ph = 0;
             for (int kb = k0; kb < k1; ++kb) {
                 if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_s, ST_TIMEOUT_EMPTY)) break;
-                mbar_arrive_expect_tx(bar_full + 8 * s, (uint32_t)T * BK + lo_bytes + hi_bytes);
+                mbar_arrive_expect_tx(bar_full + 8 * s, (uint32_t)(T * BK + R * 96));
                 tma_load_2d(sLo + s * lo_bytes, &tmap_lo, kb * 64, n0, bar_full + 8 * s);
                 tma_load_2d(sHi + s * hi_bytes, &tmap_hi, kb * 32, n0, bar_full + 8 * s);
                 tma_load_2d(sA + s * a_bytes, &tmap_a, kb * BK, t0, bar_full + 8 * s);
@@ -468,64 +474,60 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (ok && one) umma_commit(bar_tfull);
     } else {
         const int uw = warp - 2, grp = uw >> 2;
-        const int r = 32 * (uw & 3) + lane;                        // weight row of the tile
-        const uint8_t* srow = x6.s_rel + (size_t)min(n0 + r, p.N - 1) * x6.srel_pitch;
-        const bool wide = (x6.srel_pitch & 15) == 0 && ((uintptr_t)x6.s_rel & 15) == 0;   // scale rows readable 16 bytes at a time
-        auto fetch = [&](int kb4) -> uint4 {                       // scales of boxes 4 kb4 .. 4 kb4 + 3
-            if (wide) return gload(reinterpret_cast<const uint4*>(srow) + kb4);
-            uint4 v = make_uint4(0, 0, 0, 0);
-            const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
-            const int left = p.k_iters - 4 * kb4;
-            if (left > 0) v.x = gload(s32);
-            if (left > 1) v.y = gload(s32 + 1);
-            if (left > 2) v.z = gload(s32 + 2);
-            if (left > 3) v.w = gload(s32 + 3);
-            return v;
+        // Step i of a box: its rows 8 i .. 8 i + 7; lane = (row, scale group). Warp j of a group takes every fourth step, counted from
+        // where its last box left off, so that all four do as much.
+        const int steps = R / 8, c = lane & 3;
+        auto row_of = [&](int i) { return 8 * i + (lane >> 2); };
+        auto first = [&](int kb) { return ((uw & 3) + 4 - (kb / x6.groups * steps & 3)) & 3; };
+        auto fetch = [&](int kb) -> uint32_t {                     // the steps' scale bytes of box kb, a turn ahead of their use
+            uint32_t b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = first(kb) + 4 * j;
+                b[j] = i < steps && kb < k1 ? gload(x6.s_rel + (size_t)min(n0 + row_of(i), p.N - 1) * x6.srel_pitch + 4 * kb + c) : 0x38u;
+            }
+            return b[0] | b[1] << 8 | b[2] << 16 | b[3] << 24;
         };
-        const int sw_lo = (r >> 1) & 3, sw_hi = (r >> 2) & 1, sw_out = r & 7;
-        int sa = 0, sb = 0, turn = 0;
+        const int g = x6.groups;
+        int sa = grp, sb = grp;                                    // a group beyond the boxes has none
         uint32_t pa = 0, pb = 0;
         bool ok = true;
-        uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = fetch(k0 >> 2);
-        for (int kb = grp < x6.groups ? k0 : k1; kb < k1; ++kb) {
-            if ((kb & 3) == 0 || kb == k0) {
-                sc_cur = sc_next;
-                if ((kb & ~3) + 4 < k1) sc_next = fetch((kb >> 2) + 1);
-            }
-            if (turn == grp) {
-                const int q = kb & 3;
-                const uint32_t sr = q == 0 ? sc_cur.x : q == 1 ? sc_cur.y : q == 2 ? sc_cur.z : sc_cur.w;
-                // the expanded slot first, as above: groups <= sb <= sa keeps every awaited phase the current or the last one
-                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
-                    !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
-                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
-                    !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
-                const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
-                const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
-                uint8_t* out = sm + sb * w_bytes + r * 128;
-                const uint4 h0 = *reinterpret_cast<const uint4*>(hi + (sw_hi << 4)), h1 = *reinterpret_cast<const uint4*>(hi + ((1 ^ sw_hi) << 4));
-                const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                auto expand = [&](auto mode) {
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {                  // 32 codes = one scale group per 16-byte piece of nibbles
-                        const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
-                        uint32_t o[8];
-                        w6_group<decltype(mode)::value>(l, hw[2 * c], hw[2 * c + 1], (sr >> (8 * c)) & 0xffu, o);
-                        *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                        *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
-                    }
-                };
-                const int mode = w6_mode(sr);
-                if (mode == W6_SMALL) expand(std::integral_constant<int, W6_SMALL>());
-                else if (mode == W6_UNIT) expand(std::integral_constant<int, W6_UNIT>());
-                else expand(std::integral_constant<int, W6_ANY>());
-                fence_proxy_async_smem();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
-            }
-            if (++turn == x6.groups) turn = 0;
-            if (++sa == SA) sa = 0, pa ^= 1u;
-            if (++sb == SB) sb = 0, pb ^= 1u;
+        uint32_t sc_next = fetch(k0 + grp);
+        for (int kb = grp < g ? k0 + grp : k1; kb < k1; kb += g) {
+            const uint32_t sc = sc_next;
+            sc_next = fetch(kb + g);
+            // the expanded slot first, as above: groups <= sb <= sa keeps every awaited phase the current or the last one
+            if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
+                !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
+                !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+            const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes;
+            const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes;
+            uint8_t* out = sm + sb * w_bytes;
+            auto expand = [&](auto mode) {
+#pragma unroll 1
+                for (int i = first(kb), s4 = (int)sc; i < steps; i += 4, s4 = (int)((uint32_t)s4 >> 8)) {
+                    const int r = row_of(i);
+                    const uint4 l = *reinterpret_cast<const uint4*>(lo + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
+                    const uint2 h = *reinterpret_cast<const uint2*>(hi + r * 32 + (((c >> 1) ^ ((r >> 2) & 1)) << 4) + ((c & 1) << 3));
+                    uint32_t o[8];
+                    w6_group<decltype(mode)::value>(l, h.x, h.y, (uint32_t)s4 & 0xffu, o);
+                    uint8_t* row = out + r * 128;
+                    *reinterpret_cast<uint4*>(row + (((2 * c) ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                    *reinterpret_cast<uint4*>(row + (((2 * c + 1) ^ (r & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                }
+            };
+            const int mode = w6_mode(sc);
+            if (mode == W6_MID) expand(std::integral_constant<int, W6_MID>());
+            else if (mode == W6_SMALL) expand(std::integral_constant<int, W6_SMALL>());
+            else if (mode == W6_UNIT) expand(std::integral_constant<int, W6_UNIT>());
+            else expand(std::integral_constant<int, W6_ANY>());
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
+            sa += g, sb += g;
+            if (sa >= SA) sa -= SA, pa ^= 1u;
+            if (sb >= SB) sb -= SB, pb ^= 1u;
         }
         // accumulators to shared memory, [token][weight row] int32, over the rings (all copies have landed and all MMAs have
         // read them when the accumulator is complete)
@@ -553,7 +555,7 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         for (int u = rank + x6.splits * (warp - 2); u < quads; u += x6.splits * kW6RowsWarps) {
             const int quad = u & 3, m0 = (u >> 2) * 8;
             const int n = n0 + quad * 32 + lane;
-            if (n >= p.N) continue;
+            if (n >= p.N || quad * 32 + lane >= R) continue;
             const uint32_t src = base + (uint32_t)(m0 * BM + quad * 32 + lane) * 4u;
             int acc[8];
 #pragma unroll
@@ -688,8 +690,7 @@ const int* w6_rows_clusters() {
 
 int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, cudaStream_t st) {
     const int64_t M = p.M, N = p.N, K = p.K;
-    W6RowsParams x6{s_rel, (int)(K / 32), 0, 1, p.k_iters, 0, 0, 0};
-    p.tiles_n = (int)((N + BM - 1) / BM);
+    W6RowsParams x6{s_rel, (int)(K / 32), 0, 1, p.k_iters, 0, 0, 0, BM};
     // Token tiles and K slices: rounds of clusters times the cost of one, in K boxes (0.56 us of expansion each). A CTA's rings take
     // a whole SM and a cluster has to lie in one GPC, so the device holds fewer clusters than SMs / s (148, 74, 45, 33, 26, 22, 15,
     // 15 of 1 to 8 CTAs); a second round costs as much as the first. Start, end and the tokens' share of epilogue and exchange as
@@ -706,19 +707,22 @@ int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
         last = tokens;
         double cost = 1e30;
         int splits = 1, kps = p.k_iters;
-        for (int s = 1; s <= kW6RowsMaxSplits && s <= p.k_iters; ++s) {
-            const int k = (p.k_iters + s - 1) / s, room = clusters[s];
-            if ((p.k_iters + k - 1) / k != s || room < 1) continue;          // a slice would be empty; no such cluster fits
-            const double rounds = (double)(((int64_t)p.tiles_n * tiles_m + room - 1) / room);
-            const double c = rounds * (k + (s == 1 ? 8 + tokens / 28.0 : 10.5 + tokens / (s <= 4 ? 40.0 : 26.0)));
-            if (c < cost) cost = c, splits = s, kps = k;
-        }
-        if (cost < 0.95 * best) best = cost, x6.tokens = tokens, x6.splits = splits, x6.kps = kps;
+        int height = BM;
+        for (int h = BM; h >= 64; h -= 8)
+            for (int s = 1; s <= kW6RowsMaxSplits && s <= p.k_iters; ++s) {
+                const int k = (p.k_iters + s - 1) / s, room = clusters[s];
+                if ((p.k_iters + k - 1) / k != s || room < 1) continue;          // a slice would be empty; no such cluster fits
+                const double rounds = (double)(((N + h - 1) / h * tiles_m + room - 1) / room);
+                const double c = rounds * (k * (h / 8 + 2) / 18.0 + (s == 1 ? 8 + tokens / 28.0 : 10.5 + tokens / (s <= 4 ? 40.0 : 26.0)));
+                if (c < cost) cost = c, splits = s, kps = k, height = h;
+            }
+        if (cost < 0.95 * best) best = cost, x6.tokens = tokens, x6.splits = splits, x6.kps = kps, x6.height = height;
     }
     p.tiles_m = (int)((M + x6.tokens - 1) / x6.tokens);
+    p.tiles_n = (int)((N + x6.height - 1) / x6.height);
     p.idesc = umma_idesc_i8(BM, x6.tokens);
     const int a_bytes = (x6.tokens * BK + 1023) & ~1023;
-    const int stage = a_bytes + BM * (64 + 32);
+    const int stage = a_bytes + ((x6.height * 64 + 1023) & ~1023) + x6.height * 32;
     // rings: as many expanded tiles as the packed ring beside them is deep (see the waits of the expanding warps), six at most
     for (x6.sb = 6; x6.sb > 1; --x6.sb) {
         x6.sa = (kSmemBytes - 1024 - kTailBytes - x6.sb * BM * BK) / stage;
@@ -733,8 +737,8 @@ int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_r
     const int64_t pitch = 3 * K / 4;
     CUtensorMap ta, tlo, thi;
     if (!make_operand_tmap(&ta, A, M, K, x6.tokens)) return -203;
-    if (!make_plane_tmap(&tlo, Wq6, N, K / 2, pitch, 64, BM, CU_TENSOR_MAP_SWIZZLE_64B)) return -203;
-    if (!make_plane_tmap(&thi, Wq6 + K / 2, N, K / 4, pitch, 32, BM, CU_TENSOR_MAP_SWIZZLE_32B)) return -203;
+    if (!make_plane_tmap(&tlo, Wq6, N, K / 2, pitch, 64, x6.height, CU_TENSOR_MAP_SWIZZLE_64B)) return -203;
+    if (!make_plane_tmap(&thi, Wq6 + K / 2, N, K / 4, pitch, 32, x6.height, CU_TENSOR_MAP_SWIZZLE_32B)) return -203;
     if (epi == EPI_ACC) return launch_w6_rows<float, EPI_ACC>(ta, tlo, thi, p, x6, smem, st);
 #define W6_ROWS_DISPATCH(T)                                                                    \
     (epi == EPI_RESID ? launch_w6_rows<T, EPI_RESID>(ta, tlo, thi, p, x6, smem, st)            \

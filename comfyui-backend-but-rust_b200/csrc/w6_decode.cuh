@@ -21,13 +21,17 @@
 // warp costs the sum of its sides. What a packer emits lies in (0, 4]: its largest group has 31 steps for 127, so a scale of
 // 4.0 is common and only the unused code 0 can leave the range there, downwards, by one. That form clamps once, after the rint
 // (12 operations for four pairs where the general form has 20), and a caller with several groups votes once for all of them.
-enum { W6_UNIT = 0, W6_SMALL = 1, W6_ANY = 2 };
+// With scales of at least 1/4 besides (W6_MID), 32 s is a whole number and so is 1536 - 96 s, exact in half: (64 + code) s + that is the
+// rounded code in one fused multiply-add. 64 + code is two bytes side by side, the nibble shifted up and 0x54 + the top bits, so nothing is
+// merged before the permute that pairs them.
+enum { W6_UNIT = 0, W6_SMALL = 1, W6_ANY = 2, W6_MID = 3 };
 // The form for the four scale bytes of a lane and those of its warp's other lanes (absent ones filled with 0x38, a scale of 1)
 __device__ __forceinline__ int w6_mode(uint32_t sb4) {
     // bytes up to 0x48 (4.0), sign clear: adding 0x37 carries into bit 7 from 0x49 on
     const bool small = (((sb4 & 0x7f7f7f7fu) + 0x37373737u) & 0x80808080u) == 0u && (sb4 & 0x80808080u) == 0u;
     if (!__all_sync(0xffffffffu, small)) return W6_ANY;
-    return __all_sync(0xffffffffu, sb4 == 0x38383838u) ? W6_UNIT : W6_SMALL;
+    if (!__all_sync(0xffffffffu, (((sb4 | 0x80808080u) - 0x28282828u) & 0x80808080u) == 0x80808080u)) return W6_SMALL;      // from 0x28 (1/4) on
+    return __all_sync(0xffffffffu, sb4 == 0x38383838u) ? W6_UNIT : W6_MID;
 }
 template <int MODE>
 __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
@@ -41,6 +45,26 @@ __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb
             const uint32_t de = (lw[w] & 0x0F0F0F0Fu) | te, dd = ((lw[w] >> 4) & 0x0F0F0F0Fu) | to;
             o[2 * w] = __byte_perm(de, dd, 0x5140);        // e0 o0 e1 o1
             o[2 * w + 1] = __byte_perm(de, dd, 0x7362);    // e2 o2 e3 o3
+        }
+        return;
+    }
+    if constexpr (MODE == W6_MID) {
+        const __half2 s2 = __half2half2(__half(__nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)sb, __NV_E4M3)));
+        const __half2 c2 = __hfma2(__float2half2_rn(-96.f), s2, __float2half2_rn(1536.f));
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            const uint32_t h = hv[w >> 1] >> (16 * (w & 1));
+            const uint32_t te = __byte_perm(0x57565554u, 0u, h & 0x3333u), to = __byte_perm(0x57565554u, 0u, (h >> 2) & 0x3333u);
+            const uint32_t ne = (lw[w] << 4) & 0xF0F0F0F0u, no = lw[w] & 0xF0F0F0F0u;
+            uint32_t p[4] = {__byte_perm(ne, te, 0x5140), __byte_perm(no, to, 0x5140),       // (e0,e2) (e1,e3)
+                             __byte_perm(ne, te, 0x7362), __byte_perm(no, to, 0x7362)};      // (e4,e6) (e5,e7)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const __half2 g = __hmax2(__hfma2(*reinterpret_cast<__half2*>(&p[i]), s2, c2), __float2half2_rn(1409.f));
+                p[i] = *reinterpret_cast<const uint32_t*>(&g);
+            }
+            o[2 * w] = __byte_perm(p[0], p[1], 0x6240);
+            o[2 * w + 1] = __byte_perm(p[2], p[3], 0x6240);
         }
         return;
     }
@@ -73,7 +97,8 @@ __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb
 }
 // with the mode in a variable (the same in the whole warp)
 __device__ __forceinline__ void w6_group(int mode, const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
-    if (mode == W6_SMALL) w6_group<W6_SMALL>(l, ha, hb, sb, o);
+    if (mode == W6_MID) w6_group<W6_MID>(l, ha, hb, sb, o);
+    else if (mode == W6_SMALL) w6_group<W6_SMALL>(l, ha, hb, sb, o);
     else if (mode == W6_UNIT) w6_group<W6_UNIT>(l, ha, hb, sb, o);
     else w6_group<W6_ANY>(l, ha, hb, sb, o);
 }

@@ -111,6 +111,23 @@ def test_few_rows_equal_the_two_call_flow(pkg, oracle, dev, dtype, M, N, K):
     assert L.kernel_status() == 0
 
 
+# Few rows, tiles lower than 128 weight rows: N just below, at and above a round of 148 tiles of 64 and of 104 rows, K boxes that leave the
+# expanding warps' turns ragged, and scales of 1/4 to 4 throughout (the expansion in one multiply-add) with every code in each.
+@pytest.mark.parametrize("M", [5, 64, 256])
+@pytest.mark.parametrize("N,K", [(9472, 640), (9480, 128), (15385, 896), (15392, 256), (15400, 384)])
+def test_few_rows_tiles_of_every_height(pkg, oracle, dev, M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    n, k = torch.arange(N)[:, None], torch.arange(K)[None, :]
+    codes = ((k + 32 * (n % 2) + n // 128) % 64).to(torch.uint8)
+    s_rel = (0x28 + (n + torch.arange(K // 32)[None, :]) % 33).to(torch.uint8)
+    A = torch.randint(-128, 128, (M, K), generator=g, dtype=torch.int8).to(dev)
+    packed = oracle.w6_pack_codes(codes)
+    w8 = oracle.w6_decode(packed, s_rel, K).to(dev)
+    L = pkg.linear
+    assert_bits_equal(L.w6a8_gemm_acc_i32(A, packed.to(dev), s_rel.to(dev)), L.int8_gemm_acc_i32(A, w8), "accumulators")
+    assert L.kernel_status() == 0
+
+
 @pytest.mark.parametrize("M,few,many,K", [(64, 1920, 2560, 2560), (128, 1920, 2304, 6144), (16, 1920, 2176, 2048)])
 def test_few_rows_k_slices_fit_the_device_in_one_round(pkg, oracle, dev, M, few, many, K):
     """A few row tiles more must not push the clusters that share K into a second round: such a rule counts SMs, while a cluster
