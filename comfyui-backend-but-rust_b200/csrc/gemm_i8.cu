@@ -237,10 +237,9 @@ __device__ __forceinline__ void epilogue8(const GemmParams& p, const uint32_t* r
     }
 }
 
-// The table-driven activation epilogue on 8 consecutive columns of one row, for bf16 outputs through the staged path:
-// y = bf16(fma(float(acc) * xs, ws, bias)) is formed two at a time (one packed conversion), its 16 bits index the table
-// (hot part in shared memory, sign in the index's top bit), and the table's 16-bit entries are the output as they are:
-// no conversion back and forth. Values outside the shared-memory part (checked once per 8) are read from the whole table.
+// The table-driven activation epilogue, for bf16 outputs: y = bf16(fma(float(acc) * xs, ws, bias)) is formed two at a time (one packed
+// conversion), its 16 bits index the table (hot part in shared memory, sign in the index's top bit), and the table's 16-bit entries are
+// the output as they are: no conversion back and forth. Values outside the shared-memory part are read from the whole table, eight columns at a time.
 // Out of line on purpose: inlined, its eight loads were issued (predicated off) by every group of eight and cost the
 // epilogue a tenth of its instructions.
 __device__ __noinline__ uint4 act_lut_whole8(const uint16_t* lut, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
@@ -250,47 +249,55 @@ __device__ __noinline__ uint4 act_lut_whole8(const uint16_t* lut, uint32_t w0, u
     for (int i = 0; i < 4; ++i) o[i] = (uint32_t)gload(lut + (w[i] & 0xffffu)) | ((uint32_t)gload(lut + (w[i] >> 16)) << 16);
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
-// t[e] = table entry (16 bits) for column e. Returns false when some entry came from the whole table (values outside the
-// shared-memory part: the caller may want to look at their size).
+// 32 columns of one row: r[e] = accumulator in, table entry (16 bits) out. Returns false when some entry came from the whole table (values
+// outside the shared-memory part: the caller may want to look at their size). The 32 look-ups are in flight together and one vote
+// covers them all; with a vote and a branch for every eight, a warp waited for each eight in turn (the rotating epilogue on
+// 4352 x 3072 -> 12288: 138.5 us, now 133; 16896 rows 492, now 470).
 template <int VS>
-__device__ __forceinline__ bool epilogue8_lut_bits(const GemmParams& p, const uint32_t* r, float xs_r, const float* vs,
-                                                   const uint16_t* lut_sm, uint32_t (&t)[8]) {
-    float w8[8], b8[8], v[8];
-    load8<float>(vs, w8);
-    load8<float>(vs + VS, b8);
+__device__ __forceinline__ bool epilogue32_lut_bits(const GemmParams& p, uint32_t (&r)[32], float xs_r, const float* vs, const uint16_t* lut_sm) {
+    const float2 xs2 = make_float2(xs_r, xs_r);
+    uint32_t w[16];
+    bool in[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = __fmaf_rn(__fmul_rn(__int2float_rn((int)r[e]), xs_r), w8[e], b8[e]);
-    // inside the shared-memory part when 2^-11 <= |v| < 31.875 for all eight (rounding to bf16 then stays below 32); a NaN
-    // fails the comparison
-    float lo = fabsf(v[0]), hi = lo;
+    for (int j = 0; j < 4; ++j) {
+        float lo = 0.f, hi = 0.f;
 #pragma unroll
-    for (int e = 1; e < 7; e += 2) {
-        asm("min.f32 %0, %1, %2, %3;" : "=f"(lo) : "f"(lo), "f"(fabsf(v[e])), "f"(fabsf(v[e + 1])));
-        asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(hi) : "f"(hi), "f"(fabsf(v[e])), "f"(fabsf(v[e + 1])));
+        for (int h = 0; h < 2; ++h) {
+            const int c = 8 * j + 4 * h;
+            const float4 w4 = *reinterpret_cast<const float4*>(vs + c), b4 = *reinterpret_cast<const float4*>(vs + VS + c);
+            const float2 v0 = __ffma2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[c]), __int2float_rn((int)r[c + 1])), xs2), make_float2(w4.x, w4.y),
+                                         make_float2(b4.x, b4.y));
+            const float2 v1 = __ffma2_rn(__fmul2_rn(make_float2(__int2float_rn((int)r[c + 2]), __int2float_rn((int)r[c + 3])), xs2),
+                                         make_float2(w4.z, w4.w), make_float2(b4.z, b4.w));
+            // inside the shared-memory part when 2^-11 <= |v| < 31.875 for all eight (rounding to bf16 then stays below 32); a NaN
+            // fails the comparison
+            if (h == 0) {
+                asm("min.f32 %0, %1, %2, %3;" : "=f"(lo) : "f"(fabsf(v0.x)), "f"(fabsf(v0.y)), "f"(fabsf(v1.x)));
+                asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(hi) : "f"(fabsf(v0.x)), "f"(fabsf(v0.y)), "f"(fabsf(v1.x)));
+                lo = fminf(lo, fabsf(v1.y));
+                asm("max.NaN.f32 %0, %1, %2;" : "=f"(hi) : "f"(hi), "f"(fabsf(v1.y)));
+            } else {
+                asm("min.f32 %0, %1, %2, %3;" : "=f"(lo) : "f"(lo), "f"(fabsf(v0.x)), "f"(fabsf(v0.y)));
+                asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(hi) : "f"(hi), "f"(fabsf(v0.x)), "f"(fabsf(v0.y)));
+                asm("min.f32 %0, %1, %2, %3;" : "=f"(lo) : "f"(lo), "f"(fabsf(v1.x)), "f"(fabsf(v1.y)));
+                asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(hi) : "f"(hi), "f"(fabsf(v1.x)), "f"(fabsf(v1.y)));
+            }
+            const __nv_bfloat162 h0 = __floats2bfloat162_rn(v0.x, v0.y), h1 = __floats2bfloat162_rn(v1.x, v1.y);
+            w[4 * j + 2 * h] = *reinterpret_cast<const uint32_t*>(&h0), w[4 * j + 2 * h + 1] = *reinterpret_cast<const uint32_t*>(&h1);
+        }
+        in[j] = lo >= kActLutMinAbs && hi < kActLutMaxAbs;
     }
-    lo = fminf(lo, fabsf(v[7]));
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(hi) : "f"(hi), "f"(fabsf(v[7])));
-    uint32_t w[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-        w[i] = *reinterpret_cast<const uint32_t*>(&h);
-        t[2 * i] = lut_sm[act_lut_index(w[i])];
-        t[2 * i + 1] = lut_sm[act_lut_index(w[i] >> 16)];
+    for (int i = 0; i < 16; ++i) r[2 * i] = lut_sm[act_lut_index(w[i])], r[2 * i + 1] = lut_sm[act_lut_index(w[i] >> 16)];
+    if (__all_sync(0xffffffffu, in[0] && in[1] && in[2] && in[3])) return true;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (__all_sync(0xffffffffu, in[j])) continue;
+        const uint4 o = act_lut_whole8(p.act_lut, w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+        r[8 * j] = o.x & 0xffffu, r[8 * j + 1] = o.x >> 16, r[8 * j + 2] = o.y & 0xffffu, r[8 * j + 3] = o.y >> 16;
+        r[8 * j + 4] = o.z & 0xffffu, r[8 * j + 5] = o.z >> 16, r[8 * j + 6] = o.w & 0xffffu, r[8 * j + 7] = o.w >> 16;
     }
-    const bool inside = lo >= kActLutMinAbs && hi < kActLutMaxAbs;
-    if (__all_sync(0xffffffffu, inside)) return true;
-    const uint4 o = act_lut_whole8(p.act_lut, w[0], w[1], w[2], w[3]);
-    t[0] = o.x & 0xffffu, t[1] = o.x >> 16, t[2] = o.y & 0xffffu, t[3] = o.y >> 16;
-    t[4] = o.z & 0xffffu, t[5] = o.z >> 16, t[6] = o.w & 0xffffu, t[7] = o.w >> 16;
     return false;
-}
-template <int VS>
-__device__ __forceinline__ uint4 epilogue8_lut(const GemmParams& p, const uint32_t* r, float xs_r, const float* vs,
-                                               const uint16_t* lut_sm) {
-    uint32_t t[8];
-    epilogue8_lut_bits<VS>(p, r, xs_r, vs, lut_sm, t);
-    return make_uint4(t[0] | (t[1] << 16), t[2] | (t[3] << 16), t[4] | (t[5] << 16), t[6] | (t[7] << 16));
 }
 
 // Radix-4 butterfly of the regular Hadamard block on f32 bit patterns, outputs in the reference's association
@@ -391,11 +398,18 @@ __device__ __forceinline__ void chunk_direct(const GemmParams& p, const uint32_t
 template <typename OutT, int EPI, int VS = 128>
 __device__ __forceinline__ void chunk_compute16(const GemmParams& p, const uint32_t (&r)[32], int row, int col0, float xs_r,
                                                 const float* vs, uint4 (&pk)[4], const uint16_t* lut_sm = nullptr) {
+    if constexpr (EPI == EPI_ACT_LUT) {
+        uint32_t t[32];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if constexpr (EPI == EPI_ACT_LUT) {
-            pk[j] = epilogue8_lut<VS>(p, r + 8 * j, xs_r, vs + 8 * j, lut_sm);
-        } else {
+        for (int e = 0; e < 32; ++e) t[e] = r[e];
+        epilogue32_lut_bits<VS>(p, t, xs_r, vs, lut_sm);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            pk[j] = make_uint4(t[8 * j] | (t[8 * j + 1] << 16), t[8 * j + 2] | (t[8 * j + 3] << 16), t[8 * j + 4] | (t[8 * j + 5] << 16),
+                               t[8 * j + 6] | (t[8 * j + 7] << 16));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
             float y[8];
             epilogue8<OutT, EPI, VS>(p, r + 8 * j, row, col0 + 8 * j, xs_r, p.vec_ok && col0 + 8 * j + 8 <= p.N, y, vs + 8 * j, lut_sm);
             if constexpr (sizeof(OutT) == 2) pk[j] = pack8<OutT>(y);
@@ -520,12 +534,16 @@ template <typename OutT, int EPI>
 __device__ __forceinline__ void drain_values(const GemmParams& p, const uint32_t (&r)[32], const uint4 (&rq)[4], float xs, const float* vs,
                                              const uint16_t* lut_sm, uint32_t (&o)[16]) {
     const float2 xs2 = make_float2(xs, xs);
+    if constexpr (EPI == EPI_ACT_LUT) {
+        uint32_t t[32];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if constexpr (EPI == EPI_ACT_LUT) {
-            const uint4 t = epilogue8_lut<128>(p, r + 8 * j, xs, vs + 8 * j, lut_sm);
-            o[4 * j] = t.x, o[4 * j + 1] = t.y, o[4 * j + 2] = t.z, o[4 * j + 3] = t.w;
-        } else {
+        for (int e = 0; e < 32; ++e) t[e] = r[e];
+        epilogue32_lut_bits<128>(p, t, xs, vs, lut_sm);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = t[2 * i] | (t[2 * i + 1] << 16);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
             const uint32_t q4[4] = {rq[j].x, rq[j].y, rq[j].z, rq[j].w};
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -861,22 +879,16 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
                 tmem_ld_wait();
                 bool wide = false;
                 const float* vs = my_vec + 64 * blk;
+                if (!epilogue32_lut_bits<128>(p, a, xs_r, vs, lut_sm)) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    uint32_t t[8];
-                    if (!epilogue8_lut_bits<128>(p, a + 8 * j, xs_r, vs + 8 * j, lut_sm, t)) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) wide |= (t[e] & 0x7fffu) >= 0x7B80u;
-                    }
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) a[8 * j + e] = t[e] << 16;
-                    if (!epilogue8_lut_bits<128>(p, b + 8 * j, xs_r, vs + 32 + 8 * j, lut_sm, t)) {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) wide |= (t[e] & 0x7fffu) >= 0x7B80u;
-                    }
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) b[8 * j + e] = t[e] << 16;
+                    for (int e = 0; e < 32; ++e) wide |= (a[e] & 0x7fffu) >= 0x7B80u;
                 }
+                if (!epilogue32_lut_bits<128>(p, b, xs_r, vs + 32, lut_sm)) {
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) wide |= (b[e] & 0x7fffu) >= 0x7B80u;
+                }
+#pragma unroll
+                for (int e = 0; e < 32; ++e) a[e] <<= 16, b[e] <<= 16;
                 const bool ex = __any_sync(0xffffffffu, wide);
                 big |= ex;
                 rotate_block64(a, b, ex);
