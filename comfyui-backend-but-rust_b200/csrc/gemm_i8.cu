@@ -487,28 +487,31 @@ template <typename OutT> __device__ __forceinline__ float2 unpack2(uint32_t w) {
     if constexpr (std::is_same<OutT, bf16>::value) return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
     else return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
-// A warp's per-column vectors of a tile, and the row scale of its lanes: fetched a tile ahead, kept in shared memory while in use
+// A warp's per-column vectors of a tile, and the row scale of its lanes: fetched a tile ahead, kept in shared memory while in use. The 2-byte
+// ones stay as they are loaded until then: widened at once, they made the warp wait for the loads it had just issued, 1500 cycles a tile.
 struct DrainVecs {
-    float ws[4], b[4], rs[4], xs;
+    float ws[4], xs;
+    uint16_t b[4], rs[4];
     template <typename OutT, int EPI>
     __device__ __forceinline__ void fetch(const GemmParams& p, int row, int col0, int chunks, int lane) {
         xs = p.xs ? gload(p.xs + min(row, p.M - 1)) : 1.f;
+        constexpr uint16_t kOne = std::is_same<OutT, bf16>::value ? 0x3F80 : 0x3C00;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int n = col0 + 32 * k + lane;
             const bool in = k < chunks && n < p.N;
             ws[k] = in ? gload(p.ws + n) : 0.f;
-            b[k] = in && p.bias ? to_f<OutT>(gload(reinterpret_cast<const OutT*>(p.bias) + n)) : 0.f;
-            if (EPI == EPI_RESID) rs[k] = !in ? 0.f : p.rscale ? to_f<OutT>(gload(reinterpret_cast<const OutT*>(p.rscale) + n)) : 1.f;
+            b[k] = in && p.bias ? gload(reinterpret_cast<const uint16_t*>(p.bias) + n) : (uint16_t)0;
+            if (EPI == EPI_RESID) rs[k] = !in ? (uint16_t)0 : p.rscale ? gload(reinterpret_cast<const uint16_t*>(p.rscale) + n) : kOne;
         }
     }
-    template <int EPI> __device__ __forceinline__ void stage(float* vec, int lane) const {
+    template <typename OutT, int EPI> __device__ __forceinline__ void stage(float* vec, int lane) const {
         __syncwarp();
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             vec[32 * k + lane] = ws[k];
-            vec[128 + 32 * k + lane] = b[k];
-            if (EPI == EPI_RESID) vec[256 + 32 * k + lane] = rs[k];
+            vec[128 + 32 * k + lane] = to_f<OutT>(*reinterpret_cast<const OutT*>(b + k));
+            if (EPI == EPI_RESID) vec[256 + 32 * k + lane] = to_f<OutT>(*reinterpret_cast<const OutT*>(rs + k));
         }
         __syncwarp();
     }
@@ -638,7 +641,7 @@ __device__ __forceinline__ void epilogue_wide(const GemmParams& p, uint8_t* stag
     for (int w = cluster_id; w < p.num_items; w += nclusters) {
         place(w, row, col0);
         const float xs = next.xs;
-        next.stage<EPI>(vec, lane);
+        next.stage<OutT, EPI>(vec, lane);
         if (w + nclusters < p.num_items) {
             int nrow, ncol;
             place(w + nclusters, nrow, ncol);
@@ -708,7 +711,7 @@ __device__ __forceinline__ void epilogue_staged(const GemmParams& p, const CUten
     for (int w = cluster_id; w < p.num_items; w += nclusters) {
         place(w, row, col0);
         const float xs = next.xs;
-        next.stage<EPI>(vec, lane);
+        next.stage<OutT, EPI>(vec, lane);
         int nrow = 0, ncol = 0;
         const bool more = w + nclusters < p.num_items;
         if (more) {
@@ -830,7 +833,8 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
     uint32_t tphase = 0;
 
     // this warp's columns of ws / bias and this lane's row scale, for the tile `w`
-    float nx_ws[4], nx_b[4], nx_xs = 1.f;
+    float nx_ws[4], nx_xs = 1.f;
+    uint16_t nx_b[4];                         // bf16 bits: widened when used, not while the load is under way
     auto fetch = [&](int w) {
         int tm, tn;
         tile_coords(w, p.tiles_m, p.tiles_n, tm, tn, p.group_m ? p.group_m : 8);
@@ -840,7 +844,7 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
         for (int k = 0; k < 4; ++k) {
             const int n = tn * 256 + (4 * half + k) * 32 + lane;
             nx_ws[k] = gload(p.ws + n);
-            nx_b[k] = bias ? __bfloat162float(bias[n]) : 0.f;
+            nx_b[k] = bias ? gload(reinterpret_cast<const uint16_t*>(bias) + n) : (uint16_t)0;
         }
     };
     if (cluster_id < p.num_items) fetch(cluster_id);
@@ -856,7 +860,7 @@ __device__ __forceinline__ void epilogue_rot(const GemmParams& p, const CUtensor
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             my_vec[32 * k + lane] = nx_ws[k];
-            my_vec[128 + 32 * k + lane] = nx_b[k];
+            my_vec[128 + 32 * k + lane] = __uint_as_float((uint32_t)nx_b[k] << 16);
         }
         __syncwarp();
         if (w + nclusters < p.num_items) fetch(w + nclusters);      // in flight while this tile is processed
@@ -1394,7 +1398,7 @@ gemm_i8_small_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                     for (int c = 0; c < 4; ++c)
                         if (c < chunks) drain_resid<OutT>(p, rq[c], row, col0 + 32 * c);
                 }
-                v.stage<EPI>(vec, lane);
+                v.stage<OutT, EPI>(vec, lane);
                 bool ok = true;
                 if (lane == 0) ok = mbar_wait(bar_tfull, 0, abort_s, ST_TIMEOUT_TMEM_FULL);
                 if (__shfl_sync(0xffffffffu, (int)ok, 0)) {
