@@ -89,7 +89,7 @@ struct QuantArgs {
     int8_t* digits;
     int* zero;
     int nzero;
-    int early;              // the stream's next kernel may start as soon as this one has (see early_trigger)
+    int early;              // the stream's next kernel may start as soon as the rows are in (see early_trigger)
 };
 
 template <int PRO> __host__ __device__ constexpr bool is_ln() { return PRO == PRO_LAYERNORM || PRO == PRO_LN_MOD || PRO == PRO_LN_AFFINE; }
@@ -393,6 +393,7 @@ struct DirectLane {
 // From a lane's values to stored codes; false when something in the CTA's rows is not finite.
 template <typename T, bool DIGITS>
 __device__ __forceinline__ bool direct_first(const QuantArgs& p, const DirectLane& l, const float (&v)[32]) {
+    if (p.early) pdl_trigger();      // the row is in
     float2 P[16];
     rotate_lane<false>(P, v, l.tbuf_w, l.t8, l.tsw, l.wmask);
     unsigned b = __float_as_uint(max32_abs_nan(P));      // non-negative floats order as integers, infinities and NaNs above
@@ -522,6 +523,7 @@ __device__ __forceinline__ void direct_values(const QuantArgs& p, const DirectLa
         const T* x = reinterpret_cast<const T*>(p.x) + l.m * p.x_stride + l.col;
         load32<T, false>(x, v);
         if (has_aux<PRO>()) load32<T, false>(x + p.up_offset, u);
+        if (p.early) pdl_trigger();
         elementwise_prologue<T, PRO>(v, u, p.lut >= 0 ? g_act_lut[p.lut] : nullptr);
     }
 }
@@ -549,7 +551,6 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel
     const DirectLane l = direct_lane(p, smem);
     direct_clear(p, l.bits);
     pdl_wait();
-    if (p.early) pdl_trigger();
     if (DIGITS) clear_counters(p);
     __syncthreads();
     bool done;
@@ -722,7 +723,6 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) quant_norm_kernel(c
     const DirectLane l = norm_lane(p, smem);
     direct_clear(p, l.bits);
     pdl_wait();
-    if (p.early) pdl_trigger();
     if (DIGITS) clear_counters(p);
     __syncthreads();
     bool done;
@@ -1268,7 +1268,6 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
     unsigned* amax_s = reinterpret_cast<unsigned*>(smem + off_amax);
     for (int i = threadIdx.x; i < rows; i += blockDim.x) amax_s[i] = 0u;
     pdl_wait();
-    if (early) pdl_trigger();
     // rows of this CTA; GroupNorm's belong to one image (blockIdx.y), so that one set of statistics serves the CTA
     const int64_t limit = SRC == SDQ_GN ? (int64_t)(blockIdx.y + 1) * s.P : M;
     const int64_t m0 = (SRC == SDQ_GN ? (int64_t)blockIdx.y * s.P : 0) + (int64_t)blockIdx.x * rows;
@@ -1293,6 +1292,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
 #pragma unroll
         for (int c = 0; c < 4; ++c) unpack_half8(r[sd_piece(4 * tin + c)], *reinterpret_cast<float(*)[8]>(v + 8 * c));
     }
+    if (early) pdl_trigger();
     float2 P[16];
     if (ROT) {
 #pragma unroll
@@ -1475,9 +1475,11 @@ int sm_count_of(int dev) {
     return c;
 }
 
-// A quantizer of few CTAs, each on an SM of its own, lets its successor in at once: the other SMs are idle, the successor's setup and
-// whatever it may do ahead (the few-rows GEMM brings its weights to L2) run beside it, and no CTA of the quantizer is left that could
-// land badly. The adaLN linear 1 x 3072 -> 18432 with its quantizer: 17.2 us, now 16.3.
+// A quantizer of few CTAs, each on an SM of its own, lets its successor in as soon as its rows are in (elementwise prologues: requested), before
+// their rotation: the other SMs are idle, the successor's setup and whatever it may do ahead (the few-rows GEMM brings its weights to
+// L2) run beside the rest, and no CTA of the quantizer is left that could land badly. The adaLN linear 1 x 3072 -> 18432 with its
+// quantizer: 17.2 us, now 16.4. Right behind the wait the successor's CTAs and their prefetches compete with the quantizer's own loads: the
+// W6A8 block of 64 rows (four quantizers of 64 CTAs) takes 121.5 us that way, 116.4 this.
 int early_trigger(int64_t ctas) {
     int dev = 0;
     cudaGetDevice(&dev);

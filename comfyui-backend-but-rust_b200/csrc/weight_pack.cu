@@ -269,10 +269,9 @@ __global__ void __launch_bounds__(256) sd_group_sums_kernel(const half* x, doubl
         atomicAdd(&sums[ng * 2 + 1], (double)ss);
     }
 }
-// As a kernel of the chain, unlike a memset, it starts beside the end of its predecessor and lets the next one in.
+// As a kernel of the chain, unlike a memset, it starts beside the end of its predecessor and the next one beside its own.
 __global__ void __launch_bounds__(256) sd_zero_sums_kernel(double* sums, int n) {
     pdl_wait();
-    pdl_trigger();
     for (int i = threadIdx.x; i < n; i += 256) sums[i] = 0.0;
 }
 // The quantizer over a row that another of the reference's kernels would have written in half first (csrc/sd.cu:611-724), for what
