@@ -16,8 +16,9 @@
 //     one of two tensor-memory accumulators; a commit releases a stage in both CTAs, another hands the finished
 //     accumulator to both epilogues
 //   - warps 2-9 of each CTA drain that CTA's 128 accumulator rows (two warps per TMEM lane quarter, splitting the
-//     32-column chunks), apply scales / bias / activation or residual, round, and write through shared memory with
-//     TMA stores (full-line writes; a direct-store path serves outputs that TMA cannot address)
+//     32-column chunks), apply scales / bias / activation or residual, round, and write: 2-byte
+//     outputs 32 bytes a lane straight from registers, or, where K is short, through shared memory with TMA stores; 4-byte ones
+//     and the rotating epilogue's through shared memory; a direct-store path serves outputs that neither can address
 //   - the persistent grid walks the tiles round-robin; bn is chosen per shape so the last round is not mostly idle
 // Every wait is bounded; a wait that runs out records a code in g_kernel_status and the CTA pair unwinds.
 #include <algorithm>
@@ -48,7 +49,7 @@ constexpr int kRotEpiWarps = 8;                      // epilogue warps of the ro
 constexpr int kRotThreads = 64 + 32 * kRotEpiWarps;
 constexpr int kMaxStages = 8;
 constexpr int kSmemBytes = 232448;            // the per-CTA maximum (227 KB)
-// Epilogue staging, 32 KB. 4-byte outputs: per warp 32 rows x 128 B. 2-byte outputs: per warp a 2 KB chunk buffer (32 rows x
+// Epilogue staging, 32 KB (the staged drain of short K has a size of its own, GemmParams::staging). 4-byte outputs: per warp 32 rows x 128 B. 2-byte outputs: per warp a 2 KB chunk buffer (32 rows x
 // 64 B), then per warp the staged per-column vectors (ws | bias [| rscale], 128 floats each), and, for the activation
 // epilogue, the shared-memory part of the activation table behind them (16 + 8 + 8 KB).
 constexpr int kStagingBytes = kEpiWarps * 4096;
