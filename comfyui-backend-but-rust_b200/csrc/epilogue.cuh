@@ -56,9 +56,13 @@ int act_lut_ptr(int act, cudaStream_t st, const uint16_t** out);
 // quant_rows.cu: the quantizer's status word (non-zero after a staging wait ran out), read and cleared
 int quant_status_read_clear(int* out);
 // quant_rows.cu: gpu_rotate_rows_f32's prologue + rotation with the rows written as three signed 8-bit digits [3][M, K] and a factor
-// per row; zeroes nzero words at `zero`
+// per row, negative for a spread row, whose groups of 256 have the factor |f| 2^-shift with shifts [K / 256][M] (written for spread
+// rows only); zeroes nzero words at `zero`
 int rotate_rows_digits(int prologue, const float* x, int64_t x_stride, int64_t up_offset, const float* norm_w, float eps, int8_t* digits,
-                       float* factors, int* zero, int nzero, int M, int K, cudaStream_t st);
+                       float* factors, uint8_t* shifts, int* zero, int nzero, int M, int K, cudaStream_t st);
+// The largest shift. A spread row's sums are kept in units of |f| 2^-40 where the row's maximum is at least 1 (and of |f| below: no group lies
+// more than 149 under such a maximum), which lets 2^-shift end at f32's 2^-149 without a sum of 2^43 units ending beyond 2^127.
+constexpr int kWo8MaxShift = 189, kWo8Lift = 40;
 // quant_rows.cu: the fp16 row quantizers on the register kernel; false when the shape is outside what it takes
 bool sd_quant_fast(int src, const SdSrc& s, int8_t* q, float* scales, int M, int K, int rotate, cudaStream_t st, int* rc);
 bool skinny_gemm_applies(int64_t M, int64_t N, int64_t K);

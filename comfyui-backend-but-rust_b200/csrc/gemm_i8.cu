@@ -1913,12 +1913,13 @@ GPU_API int gpu_wo8_linear(int prologue, const float* x, int64_t x_stride, int64
     const Wo8Plan plan = plan_wo8(M, N, K, clusters);
     int8_t* digits = reinterpret_cast<int8_t*>(a_scratch);
     float* factors = reinterpret_cast<float*>(digits + (size_t)3 * M * K);
-    if (int rc = rotate_rows_digits(prologue, x, x_stride, up_offset, norm_w, eps, digits, factors, reinterpret_cast<int*>(w_scratch),
+    uint8_t* shifts = reinterpret_cast<uint8_t*>(factors + M);
+    if (int rc = rotate_rows_digits(prologue, x, x_stride, up_offset, norm_w, eps, digits, factors, shifts, reinterpret_cast<int*>(w_scratch),
                                     plan.whole ? 0 : plan.clusters * kWo8Counters, M, K, st))
         return rc;
     if (M > INT32_MAX / 3 || plan.tiles == 0) return -200;
     if ((uintptr_t)out & 15) return -202;
-    return run_wo8(beta == 1.f, plan, digits, factors, Wq, ws, out, w_scratch, M, N, K, st);
+    return run_wo8(beta == 1.f, plan, digits, factors, shifts, Wq, ws, out, w_scratch, M, N, K, st);
 }
 
 // D[M,N] = (A[M,K] . W[N,K]^T) * xs[m] * ws[n] + bias[n]; replaces the reference's csrc/gemm.cu:123-129.

@@ -1,8 +1,12 @@
 // The weight-only int8 linear's product (included by gemm_i8.cu): D[M,N] (f32) = [D +] x[M,K] . (Wq[N,K] * ws[n])^T on the int8
 // tensor cores. The f32 rows arrive as fixed-point numbers of 22 bits and sign, a power of two per row, cut into three signed 8-bit
 // digits: x = (d0 2^16 + d1 2^8 + d2) xs[m], planes [3][M, K] int8 (quant_rows.cu). W is int8 as it lies, so the three products are
-// exact int32 sums, and what is lost is the row's rounding to 2^-22 of its maximum (two bf16 terms leave 2^-18 of each value) and
-// a few f32 roundings at the end.
+// exact int32 sums, and what is lost is the row's rounding to 2^-22 of its maximum, at most 2^-20 of the maximum of the value's rotation
+// group (two bf16 terms leave 2^-18 of each value), and a few f32 roundings at the end.
+//
+// Rows whose groups lie further apart (xs[m] negative) have a power of two per group of 256. A token tile with such a row is
+// drained after every group, two K boxes, and the groups meet in f32: the price is the drain between each two boxes' MMAs, which is why ordinary
+// tiles do not go this way. SPREAD_FIGURES
 //
 // Three int8 products take three quarters of the time of the two bf16 ones they replace, W goes to the SMs in one byte
 // instead of two, and the pass that widened W is gone: bound by the tensor core from a few hundred tokens up, by W's bytes below.
@@ -20,7 +24,8 @@ constexpr int kWo8Threads = 320;          // warp 0 loads, warp 1 issues the MMA
 constexpr int kWo8MaxTokens = 160;
 constexpr int kWo8Counters = 16;          // per shared tile: CTA of the pair x lane quarter x half of the tokens
 struct Wo8Params {
-    const float* xs;     // [M] row factors
+    const float* xs;     // [M] row factors, negative: a spread row, with
+    const uint8_t* shifts;      // [K / 256][M]: the factor of group g is |xs[m]| 2^-shifts[g][m]
     const float* ws;     // [N]
     float* D;            // [M, N]
     int M, N, add;
@@ -79,6 +84,21 @@ gemm_wo8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
     pdl_wait();
     const uint32_t tmem_base = *tmem_ptr_s;
     const int64_t u0 = wo8_start(p, cluster_id), u1 = wo8_start(p, cluster_id + 1);
+    // Whether a tile's tokens hold a spread row, in two steps: the loads, and the warp's answer
+    struct Factors { float v[NCH]; };
+    auto tile_factors = [&](int tile) {
+        Factors f;
+        const int t0 = tile % p.tiles_m * T + lane;
+#pragma unroll
+        for (int i = 0; i < NCH; ++i) f.v[i] = t0 + 32 * i < p.M ? gload(p.xs + t0 + 32 * i) : 0.f;
+        return f;
+    };
+    auto any_spread = [](const Factors& f) {
+        int s = 0;
+#pragma unroll
+        for (int i = 0; i < NCH; ++i) s |= __float_as_int(f.v[i]);
+        return __any_sync(0xffffffffu, s < 0) != 0;
+    };
 
     if (warp == 0) {
         if (lane == 0) {
@@ -101,8 +121,9 @@ gemm_wo8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             const bool one = elect_one();
             int stage = 0;
             uint32_t phase = 0, tphase = 0;
-            int kb = (int)(u0 % p.k_iters);
-            bool fresh = true;
+            int tile = (int)(u0 / p.k_iters), kb = (int)(u0 - (int64_t)tile * p.k_iters);
+            bool fresh = true, spread = any_spread(tile_factors(tile));
+            Factors next = tile_factors(tile + 1);      // requested a tile ahead
             for (int64_t u = u0; u < u1; ++u) {
                 if (fresh && !__all_sync(0xffffffffu, mbar_wait(bar_tempty, tphase ^ 1u, abort_s, ST_TIMEOUT_TMEM_EMPTY))) break;
                 if (fresh) tc_fence_after();
@@ -118,12 +139,17 @@ gemm_wo8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
                 }
                 __syncwarp();
                 if (++stage == S) stage = 0, phase ^= 1u;
-                fresh = ++kb == p.k_iters || u + 1 == u1;
+                ++kb;
+                fresh = kb == p.k_iters || u + 1 == u1 || (spread && (kb & 1) == 0);
                 if (fresh) {
                     if (one) umma_commit_pair(bar_tfull);
                     __syncwarp();
                     tphase ^= 1u;
-                    if (kb == p.k_iters) kb = 0;
+                    if (kb == p.k_iters) {
+                        kb = 0, ++tile;
+                        spread = any_spread(next);
+                        next = tile_factors(tile + 1);
+                    }
                 }
             }
         }
@@ -141,33 +167,79 @@ gemm_wo8_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constan
             const int n = tn * 2 * BM + (int)rank * BM + quad * 32 + lane;
             const bool n_ok = n < p.N;
             const float ws = n_ok ? gload(p.ws + n) : 0.f;
-            float xs[(NCH + 1) / 2];                   // lane l: factors of tokens t0 + l, t0 + 32 + l, ...
+            constexpr int kRegs = (NCH + 1) / 2;       // lane l: factors of tokens t0 + l, t0 + 32 + l, ...
+            float xs[kRegs];
 #pragma unroll
-            for (int i = 0; i < (NCH + 1) / 2; ++i) xs[i] = t0 + 32 * i + lane < p.M ? gload(p.xs + t0 + 32 * i + lane) : 0.f;
-            if (!mbar_wait_warp_relaxed(bar_tfull, tphase, abort_s, ST_TIMEOUT_TMEM_FULL)) break;
-            tphase ^= 1u;
-            tc_fence_after();
+            for (int i = 0; i < kRegs; ++i) xs[i] = t0 + 32 * i + lane < p.M ? gload(p.xs + t0 + 32 * i + lane) : 0.f;
+            const bool spread = any_spread(tile_factors(tile));
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16);
             auto column = [&](int d, int c) {          // of digit d, tokens 16 c .. 16 c + 15 of this warp's half
                 const int r = d * kTok + 16 * c;
                 return (uint32_t)(r < r0 ? half * r0 + r : 2 * r0 + half * r1 + r - r0);
             };
-            // out of tensor memory first: the next tile's MMAs wait for it, not for the stores
+            auto hand_back = [&]() {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_remote(mapa_shared(bar_tempty, 0));
+            };
             float f[kTok];
+            if (!spread) {
+                if (!mbar_wait_warp_relaxed(bar_tfull, tphase, abort_s, ST_TIMEOUT_TMEM_FULL)) break;
+                tphase ^= 1u;
+                tc_fence_after();
+                // out of tensor memory first: the next tile's MMAs wait for it, not for the stores
 #pragma unroll
-            for (int c = 0; c < NCH; ++c) {
-                uint32_t a[16], b[16], d[16];
-                tmem_ld16(taddr + column(0, c), a);
-                tmem_ld16(taddr + column(1, c), b);
-                tmem_ld16(taddr + column(2, c), d);
-                tmem_ld_wait();
+                for (int c = 0; c < NCH; ++c) {
+                    uint32_t a[16], b[16], d[16];
+                    tmem_ld16(taddr + column(0, c), a);
+                    tmem_ld16(taddr + column(1, c), b);
+                    tmem_ld16(taddr + column(2, c), d);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    f[16 * c + i] = __fmaf_rn(__int2float_rn((int)a[i]), 65536.f, __fmaf_rn(__int2float_rn((int)b[i]), 256.f, __int2float_rn((int)d[i])));
+                    for (int i = 0; i < 16; ++i)
+                        f[16 * c + i] = __fmaf_rn(__int2float_rn((int)a[i]), 65536.f, __fmaf_rn(__int2float_rn((int)b[i]), 256.f, __int2float_rn((int)d[i])));
+                }
+                hand_back();
+            } else {
+                // Group by group. The sums of 256 products of a digit stay below 2^22: the lower two digits join as integers.
+#pragma unroll
+                for (int i = 0; i < kTok; ++i) f[i] = 0.f;
+                bool ok = true;
+                for (int64_t v = u; v < end;) {
+                    const int kb = (int)(v - (int64_t)tile * p.k_iters);
+                    v = min(v + 2 - (kb & 1), end);
+                    float rel[kRegs];                  // 2^-shift, as two factors (the product may be subnormal)
+#pragma unroll
+                    for (int i = 0; i < kRegs; ++i) {
+                        rel[i] = 1.f;
+                        if (__float_as_int(xs[i]) < 0) {
+                            const int s = gload(p.shifts + (int64_t)(kb >> 1) * p.M + t0 + 32 * i + lane), h = s >> 1;
+                            rel[i] = __uint_as_float((uint32_t)(127 + (xs[i] <= -0x1p-21f ? kWo8Lift : 0) - h) << 23) * __uint_as_float((uint32_t)(127 - (s - h)) << 23);
+                        }
+                    }
+                    if (!mbar_wait_warp_relaxed(bar_tfull, tphase, abort_s, ST_TIMEOUT_TMEM_FULL)) { ok = false; break; }
+                    tphase ^= 1u;
+                    tc_fence_after();
+#pragma unroll
+                    for (int c = 0; c < NCH; ++c) {
+                        uint32_t a[16], b[16], d[16];
+                        tmem_ld16(taddr + column(0, c), a);
+                        tmem_ld16(taddr + column(1, c), b);
+                        tmem_ld16(taddr + column(2, c), d);
+                        tmem_ld_wait();
+                        if (c + 1 == NCH) hand_back();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float lower = __int2float_rn((int)(b[i] * 256u + d[i]));
+                            f[16 * c + i] = __fmaf_rn(__fmaf_rn(__int2float_rn((int)a[i]), 65536.f, lower), __shfl_sync(0xffffffffu, rel[c >> 1], 16 * (c & 1) + i), f[16 * c + i]);
+                        }
+                    }
+                }
+                if (!ok) break;
+#pragma unroll
+                for (int i = 0; i < kRegs; ++i)
+                    if (__float_as_int(xs[i]) < 0) xs[i] = xs[i] <= -0x1p-21f ? xs[i] * -0x1p-40f : -xs[i];
             }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(mapa_shared(bar_tempty, 0));
             u = end;
             if (!whole) {
                 // this cluster's share of the tile into its slot; the last to arrive at the tile's counter adds the slots up
@@ -265,8 +337,8 @@ int launch_wo8(const CUtensorMap& tw, const CUtensorMap& tx, const Wo8Params& p,
     return launch_pdl(kern, dim3(2 * clusters), kWo8Threads, kSmemBytes, st, tw, tx, p);
 }
 
-// How a call is cut, and what it leaves in the caller's scratch: the digits [3][M, K] and the row factors [M] in a_scratch (4 M K
-// bytes, K >= 256), the counters and the shared tiles' values in w_scratch (2 N K bytes).
+// How a call is cut, and what it leaves in the caller's scratch: the digits [3][M, K], the row factors [M] and the groups' shifts
+// [K / 256][M] in a_scratch (4 M K bytes, K >= 256), the counters and the shared tiles' values in w_scratch (2 N K bytes).
 struct Wo8Plan {
     int tokens, tiles_m, tiles, clusters;
     bool whole;
@@ -296,10 +368,10 @@ Wo8Plan plan_wo8(int64_t M, int64_t N, int64_t K, int max_clusters) {
     r.clusters = r.whole && tiles < max_clusters ? (int)tiles : max_clusters;
     return r;
 }
-int run_wo8(bool add, const Wo8Plan& r, const int8_t* digits, const float* xs, const int8_t* W, const float* ws, float* D, void* w_scratch,
+int run_wo8(bool add, const Wo8Plan& r, const int8_t* digits, const float* xs, const uint8_t* shifts, const int8_t* W, const float* ws, float* D, void* w_scratch,
             int64_t M, int64_t N, int64_t K, cudaStream_t st) {
     Wo8Params p{};
-    p.xs = xs, p.ws = ws, p.D = D;
+    p.xs = xs, p.shifts = shifts, p.ws = ws, p.D = D;
     p.M = (int)M, p.N = (int)N, p.add = add;
     p.tiles_m = r.tiles_m;
     p.k_iters = (int)(K / BK);

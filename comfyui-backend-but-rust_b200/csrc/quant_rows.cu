@@ -85,8 +85,10 @@ struct QuantArgs {
     int staged;             // rows arrive through the staging buffer (bulk copies) instead of direct loads
     uint32_t off_amax, off_norm, off_stage, off_bar;
     // when set (f32 rows, with q and out_f unset): the rotated rows leave as fixed-point numbers in three signed 8-bit digits, planes
-    // [3][M, K], the row's factor in `scales`; the first CTA zeroes nzero words at `zero` for the kernel that follows
+    // [3][M, K], the row's factor in `scales`, the groups' shifts [K / 256][M] of spread rows in `shifts` (see store_digits); the first
+    // CTA zeroes nzero words at `zero` for the kernel that follows
     int8_t* digits;
+    uint8_t* shifts;
     int* zero;
     int nzero;
     int early;              // the stream's next kernel may start as soon as the rows are in (see early_trigger)
@@ -211,24 +213,40 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 }
 
 // The rotated values of a lane ((2 t8, 2 t8 + 1) + 16 r, pairs swapped when tsw) as the weight-only linear takes them:
-// x = (d0 2^16 + d1 2^8 + d2) f with signed 8-bit digits and one power of two f per row, chosen so that the row's maximum lies in
-// [2^21, 2^22): what rounds away is at most 2^-22 of the row's maximum. The product with the power of two is exact and rint comes with the
-// addition of 1.5 * 2^23. A row holding an infinity or a NaN gets the factor NaN.
-// P and amax come in units of `unit` (1/16 without the rotation's halvings).
-__device__ __forceinline__ void store_digits(float2 (&P)[16], float amax, float unit, const QuantArgs& p, bool live, int64_t m, int col, bool first,
+// x = (d0 2^16 + d1 2^8 + d2) f with signed 8-bit digits and a power of two f, chosen so that a maximum lies in [2^21, 2^22): what rounds
+// away is at most 2^-22 of that maximum. The product with the power of two is exact and rint comes with the addition of 1.5 * 2^23.
+// The maximum is the row's as long as every group of 256 that is not all zero reaches 2^19 with it, so that no value loses more than 2^-20 of its
+// group's maximum, about what the rotation's own f32 sums leave (two bf16 terms kept 2^-18 of each value). A row spread
+// wider (a massive activation beside ordinary ones) has a power of two per group instead: the row's factor is stored negative, and
+// f_group = f_row 2^-shift. A row holding an infinity or a NaN gets the factor NaN.
+// P and the maxima come in units of `unit` (1/16 without the rotation's halvings).
+constexpr int kDigitSpread = 3;           // binary orders of magnitude between the row's and a group's maximum that make a spread row
+// floor(log2 v) of a positive v; a subnormal one's is found too, through a product
+__device__ __forceinline__ int exponent_of(float v) {
+    const bool low = v < 0x1p-90f;
+    return (int)(__float_as_uint(low ? v * 0x1p64f : v) >> 23) - (low ? 127 + 64 : 127);
+}
+struct DigitMax { float row, least, group; };      // maxima: the row's, the smallest of its groups' that are not zero, this lane's group's
+__device__ __forceinline__ void store_digits(float2 (&P)[16], DigitMax mx, float unit, const QuantArgs& p, bool live, int64_t m, int col, bool first,
                                              int tsw, int t8, float* tbuf, unsigned wmask) {
     float inv = 0.f, f = 0.f;
-    if (!(amax <= FLT_MAX)) f = __int_as_float(0x7fc00000);
-    else if (amax > 0.f) {
-        float back = unit;
-        if (amax < 0x1p-90f) {                      // the power of two would leave f32's range
-            amax *= 0x1p64f, back *= 0x1p-64f;
+    if (!(mx.row <= FLT_MAX)) f = __int_as_float(0x7fc00000);
+    else if (mx.row > 0.f) {
+        const int kr = max(exponent_of(mx.row), -124);      // f ends at 2^-149
+        int k = kr;
+        if (kr - exponent_of(mx.least) >= kDigitSpread) {
+            unit = -unit;
+            if (mx.group > 0.f) k = max(exponent_of(mx.group), max(kr - kWo8MaxShift, -124));
+            if (live && t8 == 0) p.shifts[(int64_t)(col >> 8) * p.M + m] = (uint8_t)(kr - k);
+        }
+        // f as a product of two, it may be subnormal; k + 64 where 2^(21 - k) would leave f32's range
+        f = __uint_as_float((uint32_t)(127 - 21 + kr + (kr < -90 ? 64 : 0)) << 23) * (kr < -90 ? unit * 0x1p-64f : unit);
+        if (k < -90) {
+            k += 64;
 #pragma unroll
             for (int r = 0; r < 16; ++r) P[r] = __fmul2_rn(P[r], make_float2(0x1p64f, 0x1p64f));
         }
-        const int k = (int)(__float_as_uint(amax) >> 23) - 127;
         inv = __uint_as_float((uint32_t)(127 + 21 - k) << 23);
-        f = __uint_as_float((uint32_t)(127 - 21 + k) << 23) * back;
     }
     if (live && first) p.scales[m] = f;
     uint32_t w[32];
@@ -381,7 +399,8 @@ template <typename T> __device__ __forceinline__ float row_scale(float amax) {
     return fmaxf(fminf(amax, finite_max<T>()) * (1.f / 127.f), 1.0e-30f);
 }
 // A lane's place in both kernels. `bits` in shared memory, zero before: [rows] maxima of the first pass, [rows] of the second, one word that
-// is set when something is not finite or nearly so.
+// is set when something is not finite or nearly so; for the digits then [rows] and [rows] complements of the groups' least maxima.
+__host__ __device__ constexpr int direct_words(int rows, bool digits) { return (digits ? 4 : 2) * rows + 1; }
 struct DirectLane {
     float *tbuf, *tbuf_w;     // the team's transposition buffer, and where the transposition starts in it
     unsigned* bits;
@@ -402,13 +421,15 @@ __device__ __forceinline__ bool direct_first(const QuantArgs& p, const DirectLan
     b = max(b, __shfl_xor_sync(l.wmask, b, 4));
     if (l.t8 == 0) {
         atomicMax(l.bits + l.rloc, b);
+        if (DIGITS && b) atomicMax(l.bits + 2 * p.rows_per_cta + 1 + l.rloc, ~b);
         if (b >= 0x7f000000u) l.bits[2 * p.rows_per_cta] = 1u;     // 2^127: short of what rounds to an infinity of bf16
     }
     __syncthreads();
     if (l.bits[2 * p.rows_per_cta] != 0u) return false;
     pdl_trigger();
     if constexpr (DIGITS) {
-        store_digits(P, __uint_as_float(l.bits[l.rloc]), 0.0625f, p, l.live, l.m, l.col, l.first, l.tsw, l.t8, l.tbuf, l.wmask);
+        const DigitMax mx = {__uint_as_float(l.bits[l.rloc]), __uint_as_float(~l.bits[2 * p.rows_per_cta + 1 + l.rloc]), __uint_as_float(b)};
+        store_digits(P, mx, 0.0625f, p, l.live, l.m, l.col, l.first, l.tsw, l.t8, l.tbuf, l.wmask);
     } else {
         const float amax = __uint_as_float(l.bits[l.rloc]) * 0.0625f, scale = row_scale<T>(amax);
         if (l.live && l.first) p.scales[l.m] = scale;
@@ -425,12 +446,22 @@ __device__ __forceinline__ void direct_second(const QuantArgs& p, const DirectLa
     float amax = 0.f;                                    // without NaNs, which the reference's fmaxf drops
 #pragma unroll
     for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fmaxf(fabsf(P[i].x), fabsf(P[i].y)));
-    if (DIGITS) amax = max32_abs_nan(P);                 // with them: the row's factor becomes one
+    if constexpr (DIGITS) {
+        amax = max32_abs_nan(P);                         // with them: the row's factor becomes one
+        unsigned b = __float_as_uint(amax);
+        b = max(b, __shfl_xor_sync(l.wmask, b, 1));
+        b = max(b, __shfl_xor_sync(l.wmask, b, 2));
+        b = max(b, __shfl_xor_sync(l.wmask, b, 4));
+        amax = __uint_as_float(b);
+        if (b) atomicMax(l.bits + 3 * p.rows_per_cta + 1 + l.rloc, ~b);
+    }
     atomicMax(l.bits + p.rows_per_cta + l.rloc, __float_as_uint(amax));
     __syncthreads();
+    const float group = amax;
     amax = __uint_as_float(l.bits[p.rows_per_cta + l.rloc]);
     if constexpr (DIGITS) {
-        store_digits(P, amax, 1.f, p, l.live, l.m, l.col, l.first, l.tsw, l.t8, l.tbuf, l.wmask);
+        const DigitMax mx = {amax, __uint_as_float(~l.bits[3 * p.rows_per_cta + 1 + l.rloc]), group};
+        store_digits(P, mx, 1.f, p, l.live, l.m, l.col, l.first, l.tsw, l.t8, l.tbuf, l.wmask);
     } else {
         const float scale = row_scale<T>(amax), st = rnd<T>(scale);
         if (l.live && l.first) p.scales[l.m] = scale;
@@ -441,8 +472,8 @@ __device__ __forceinline__ void direct_second(const QuantArgs& p, const DirectLa
         store_codes(c16, p.q + l.m * (int64_t)p.K + l.col, l.live, l.tbuf, l.t8, l.wmask);
     }
 }
-__device__ __forceinline__ void direct_clear(const QuantArgs& p, unsigned* bits) {
-    for (int i = threadIdx.x; i <= 2 * p.rows_per_cta; i += blockDim.x) bits[i] = 0u;
+template <bool DIGITS> __device__ __forceinline__ void direct_clear(const QuantArgs& p, unsigned* bits) {
+    for (int i = threadIdx.x; i < direct_words(p.rows_per_cta, DIGITS); i += blockDim.x) bits[i] = 0u;
 }
 // for the kernel that follows the digits
 __device__ __forceinline__ void clear_counters(const QuantArgs& p) {
@@ -549,7 +580,7 @@ template <typename T, int PRO, int MAXT, bool DIGITS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const DirectLane l = direct_lane(p, smem);
-    direct_clear(p, l.bits);
+    direct_clear<DIGITS>(p, l.bits);
     pdl_wait();
     if (DIGITS) clear_counters(p);
     __syncthreads();
@@ -721,7 +752,7 @@ template <typename T, int PRO, int MAXT, bool DIGITS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) quant_norm_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const DirectLane l = norm_lane(p, smem);
-    direct_clear(p, l.bits);
+    direct_clear<DIGITS>(p, l.bits);
     pdl_wait();
     if (DIGITS) clear_counters(p);
     __syncthreads();
@@ -1653,7 +1684,7 @@ template <typename T, int PRO, bool DIGITS = false> int launch_norm(QuantArgs p,
     p.off_norm = (uint32_t)(warps * kWarpWords * 4);
     p.off_amax = p.off_norm + rows * 64 * 4;
     p.early = early_trigger(p.nblocks);
-    const size_t smem = p.off_amax + (2 * rows + 1) * 4;
+    const size_t smem = p.off_amax + direct_words(rows, DIGITS) * 4;
     return warps <= 8 ? launch_norm_cfg<T, PRO, 256, DIGITS>(p, 32 * warps, smem, st) : launch_norm_cfg<T, PRO, 1024, DIGITS>(p, 32 * warps, smem, st);
 }
 
@@ -1727,7 +1758,7 @@ int launch_quant(QuantArgs& p, cudaStream_t st) {
     const int threads = rows * p.tpr;
     auto up = [](size_t v, size_t a) { return (v + a - 1) / a * a; };
     size_t off = (size_t)((threads + 31) / 32) * kWarpWords * 4;
-    p.off_amax = (uint32_t)off, off += (size_t)3 * rows * 4;
+    p.off_amax = (uint32_t)off, off += (size_t)(p.digits ? direct_words(rows, true) : 3 * rows) * 4;
     p.off_norm = (uint32_t)off, off += is_norm<PRO>() ? (size_t)rows * norm_words(p.K) * 4 : 0;
     off = up(off, 16);
     off = up(off, 8);
@@ -1821,14 +1852,14 @@ GPU_API int gpu_rotate_rows_f32(int prologue, const float* x, int64_t x_stride, 
     }
 }
 
-// The same with the rotated rows written as three 8-bit digits [3][M, K] and a factor per row: the activation side of the
-// weight-only linear on the int8 tensor cores. The first CTA zeroes `nzero` words at `zero`.
+// The same with the rotated rows written as three 8-bit digits [3][M, K], a factor per row and, for spread rows, a shift per group
+// [K / 256][M]: the activation side of the weight-only linear on the int8 tensor cores. The first CTA zeroes `nzero` words at `zero`.
 int b200q::rotate_rows_digits(int prologue, const float* x, int64_t x_stride, int64_t up_offset, const float* norm_w, float eps,
-                              int8_t* digits, float* factors, int* zero, int nzero, int M, int K, cudaStream_t st) {
+                              int8_t* digits, float* factors, uint8_t* shifts, int* zero, int nzero, int M, int K, cudaStream_t st) {
     if ((K % 256) != 0) return -1;
     QuantArgs p{x, x_stride, nullptr, 0, up_offset, nullptr, factors, nullptr, M, K, 1, 0, 0, 0, -1, nullptr, nullptr,
                 norm_w, nullptr, eps, nullptr, nullptr};
-    p.digits = digits, p.zero = zero, p.nzero = nzero;
+    p.digits = digits, p.shifts = shifts, p.zero = zero, p.nzero = nzero;
     switch (prologue) {
         case PRO_PLAIN: return launch_quant<float, PRO_PLAIN>(p, st);
         case PRO_RMS: return launch_quant<float, PRO_RMS>(p, st);

@@ -124,6 +124,64 @@ def test_rows_without_a_maximum(pkg, dev):
         assert (out[m].double() - exact[m]).abs().max().item() <= 2e-6 * exact[m].abs().max().item(), m
 
 
+def _keeps_what_a_group_holds(got, xr, wf, what):
+    """Per output: a value is off by at most 2^-20 of the maximum of its rotation group (of 256); the sums of the groups are rounded to f32
+    a few times each and added, one rounding per group. Where the products of 16 significant bits of each value would be closer, not
+    further off than those either."""
+    M, K = xr.shape
+    err = (got.double() - xr @ wf.t()).abs()
+    terms = xr.abs() @ wf.abs().t()
+    groups = xr.abs().view(M, K // 256, 256).amax(2) @ wf.abs().view(-1, K // 256, 256).sum(2).t()
+    bound = 2.0 ** -20 * groups + (K // 256 + 8) * 2.0 ** -24 * terms
+    ok = err <= torch.minimum(bound, 2.0 ** -18 * terms)
+    assert bool(ok.all()), (what, int((~ok).sum()), (err / terms).max().item() * 2.0 ** 18, (err / bound).max().item())
+
+
+# Rows whose groups lie far apart (a massive activation beside ordinary ones), and weight rows that do not read the large group: what the small
+# groups hold must not be lost beside it. Gaps around the line between one power of two per row and one per group (2 to 4 binary orders of
+# magnitude), ordinary, and absurd ones; every row spread, every seventh, one row of a thousand; token tiles of every width, K boxes shared between
+# clusters in the middle of a group, several tiles a cluster; rows of infinity, NaN and zeros and groups of zeros beside them.
+@pytest.mark.parametrize("M,N,K,gap,every,limit,pro", [(1, 8, 512, 12, 1, 0, PLAIN), (20, 520, 9728, 8, 1, 0, PLAIN), (33, 1000, 2560, 20, 1, 0, PLAIN),
+                                                       (64, 300, 512, 2, 1, 0, PLAIN), (64, 300, 512, 3, 1, 0, PLAIN), (64, 300, 512, 4, 1, 0, PLAIN),
+                                                       (160, 257, 768, 16, 1, 0, PLAIN), (330, 255, 4096, 40, 7, 0, PLAIN), (1024, 3584, 1280, 10, 1024, 0, PLAIN),
+                                                       (513, 5120, 768, 11, 5, 3, PLAIN), (96, 700, 2048, 140, 2, 0, PLAIN), (128, 512, 1536, 9, 3, 5, RMS),
+                                                       (257, 1030, 2816, 13, 4, 0, SWIGLU)])
+def test_small_groups_beside_large_ones(pkg, dev, M, N, K, gap, every, limit, pro):
+    g = torch.Generator().manual_seed(M + N + K + gap)
+    L = pkg.linear
+    x = torch.randn(M, 2 * K if pro == SWIGLU else K, generator=g)
+    far = torch.arange(M) % every == every // 2
+    x[far, :256] *= 2.0 ** min(gap, 100)
+    x[far, 256:K] *= 2.0 ** min(100 - gap, 0)
+    odd = {}
+    if M > 16:
+        odd = {1: float("nan"), 4: float("inf"), 8: 0.0}
+        for m, v in odd.items():
+            x[m] = v if v == 0.0 else x[m].index_fill(0, torch.tensor([300]), v)
+        x[far & (torch.arange(M) % 3 == 0), 256:512] = 0.0
+    x = x.to(dev)
+    kw = dict(K=K, up_offset=K if pro == SWIGLU else 0, norm_w=(torch.randn(K, generator=g) * 0.1 + 1.0).to(dev) if pro == RMS else None, eps=1e-6)
+    Wq, ws = L.convrot_requant((torch.randn(N, K, generator=g) * 0.03).to(dev), 0)
+    Wq[N // 2:, :256] = 0
+    xr, wf = L.rotate_rows_f32(x, pro, **kw).double(), L.dequant_i8(Wq, ws).double()
+    out = torch.full((M + 1, N), 7.0, device=dev)
+    base = torch.randn(M, N, generator=g).to(dev)
+    acc, again = base.clone(), torch.empty(M, N, device=dev)
+    was = L.set_gemm_cluster_limit(limit)
+    try:
+        L.wo8_linear(x, Wq, ws, pro, out=out[:M], **kw)
+        L.wo8_linear(x, Wq, ws, pro, out=again, **kw)
+        L.wo8_linear(x, Wq, ws, pro, out=acc, beta=1.0, **kw)
+    finally:
+        L.set_gemm_cluster_limit(was)
+    rows = [m for m in range(M) if m not in odd]
+    _keeps_what_a_group_holds(out[rows], xr[rows], wf, f"{int(far.sum())} spread rows")
+    for m, v in odd.items():
+        assert bool((out[m] == 0).all() if v == 0.0 else out[m].isnan().all()), m
+    assert bool((out[M] == 7.0).all()) and torch.equal(again[rows], out[rows]) and torch.equal(acc[rows], out[rows] + base[rows])
+    assert L.kernel_status() == 0
+
+
 def test_argument_checks(pkg, dev):
     L = pkg.linear
     x = torch.zeros(4, 300, device=dev)
