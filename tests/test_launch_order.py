@@ -73,3 +73,93 @@ def test_no_read_only_loads_in_kernels_that_start_early():
     for name in _launched_early():
         params, body = kernels[name]
         assert "__restrict__" not in params + body, name
+
+
+# ---- the same rules through the functions that kernels call ----------------------------------------------------------------------
+
+def _device_functions():
+    """name -> [(qualifiers, parameter list, body)] of every __device__ function; overloads and specialisations side by side."""
+    out = {}
+    for _, text in _sources():
+        for m in re.finditer(r"((?:__noinline__\s+)?__device__[^;{}()]*?)\b(\w+)\s*\(((?:[^(){}]|\((?:[^()]|\([^()]*\))*\))*)\)\s*(?:const\s*)?\{", text):
+            depth, i = 1, m.end()
+            while depth:
+                depth += (text[i] == "{") - (text[i] == "}")
+                i += 1
+            out.setdefault(m.group(2), []).append((m.group(1), m.group(3), text[m.end():i]))
+    return out
+
+
+def _followed(body, functions, out_of_line=False, stack=()):
+    """A body with the bodies of the functions it calls in place of the calls, in the order of the text; those of functions out of line
+    only on demand (what they do, they do beside the kernel's common path)."""
+    def put(m):
+        name = m.group(1)
+        if name not in functions or name in stack:
+            return m.group(0)
+        inner = [_followed(b, functions, out_of_line, stack + (name,)) for q, _, b in functions[name] if out_of_line or "__noinline__" not in q]
+        return m.group(2) + "( {" + " ".join(inner) + "} "
+    return re.sub(r"\b(\w+)((?:\s*<[^;(){}<>]*(?:<[^;(){}<>]*>[^;(){}<>]*)*>)?\s*)\(", put, body)
+
+
+_NAMES = ("pdl_wait", "pdl_trigger", "gload")      # stay as they are in the text
+
+
+def _order_of(kernels, functions):
+    """What breaks the rules for kernels that start early or let a successor in, and the kernels that have a trigger."""
+    functions = {n: f for n, f in functions.items() if n not in _NAMES}
+    wrong, with_trigger = [], []
+    for name in sorted(_launched_early()):
+        params, body = kernels[name]
+        text = _followed(body, functions)
+        whole = _followed(body, functions, out_of_line=True)
+        if "__restrict__" in whole or "__ldg(" in whole:
+            wrong.append((name, "a read through the read-only path"))
+        loads = [m.start() for m in re.finditer(r"\bgload\(|\bload32<", text)]
+        if "pdl_wait()" not in text or (loads and loads[0] < text.index("pdl_wait()")):
+            wrong.append((name, "a load before the wait"))
+        if "pdl_trigger()" not in text:
+            continue
+        with_trigger.append(name)
+        if "gemm" in name:
+            wrong.append((name, "a GEMM with a trigger"))
+        at = text.index("pdl_trigger()")
+        if at < text.index("pdl_wait()") or not loads or loads[0] > at:
+            wrong.append((name, "a trigger before the wait and the rows"))
+        if re.search(r"\bload32<|\bgload\(reinterpret_cast<const (?:uint4|float4)\*>\(x|\bgload\((?:x|up|aux|in)\b", text[at:]):
+            wrong.append((name, "rows requested behind the trigger"))
+    return wrong, with_trigger
+
+
+def test_successors_are_let_in_behind_the_loads_of_called_functions_too():
+    """The rules above hold for what a kernel does in the functions it calls: the row quantizers wait in the kernel, load in one function and let
+    their successor in from there or from the next."""
+    kernels, functions = _kernels(), _device_functions()
+    wrong, with_trigger = _order_of(kernels, functions)
+    assert not wrong, wrong
+    assert {"quant_direct_kernel", "quant_norm_kernel", "sd_quant_fast_kernel", "w6_decode32_kernel"} <= set(with_trigger), with_trigger
+
+
+def test_a_trigger_out_of_order_is_noticed():
+    """The check above on sources with a mistake in them: it looks at the functions that matter."""
+    def planted(name, change, kernel=False):
+        kernels, functions = _kernels(), _device_functions()
+        if kernel:
+            params, body = kernels[name]
+            assert change(body) != body
+            kernels[name] = (params, change(body))
+        else:
+            before = functions[name]
+            functions[name] = [(q, p, change(b)) for q, p, b in before]
+            assert functions[name] != before, name
+        return {n for n, _ in _order_of(kernels, functions)[0]}
+    first = lambda b: " pdl_trigger(); " + b
+    assert "quant_direct_kernel" in planted("direct_values", first)
+    assert "quant_norm_kernel" in planted("norm_values", first)
+    for k in ("quant_direct_kernel", "quant_norm_kernel"):
+        assert k in planted(k, first, kernel=True)
+        assert k in planted(k, lambda b: b.replace("pdl_wait();", "pdl_trigger(); pdl_wait();", 1), kernel=True)
+    assert "quant_direct_kernel" in planted("direct_values", lambda b: b.replace("elementwise_prologue<", "gload(x); elementwise_prologue<"))
+    assert "gemm_i8_pair_kernel" in planted("drain_values", first)
+    assert "quant_direct_kernel" in planted("load32", lambda b: "const T* __restrict__ y = x; " + b)
+    assert "quant_norm_kernel" in planted("norm_lane", lambda b: "gload(x); " + b)
