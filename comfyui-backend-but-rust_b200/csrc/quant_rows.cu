@@ -558,20 +558,21 @@ __device__ __forceinline__ void direct_values(const QuantArgs& p, const DirectLa
         elementwise_prologue<T, PRO>(v, u, p.lut >= 0 ? g_act_lut[p.lut] : nullptr);
     }
 }
-__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem) {
+__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem, unsigned wmask) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = lane >> 3;
     const int rloc = threadIdx.x / p.tpr, tin = threadIdx.x - rloc * p.tpr;
     const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
     float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
     // idle rows compute on the last row and store nothing; the last warp of a CTA may be partial (threads = rows * K / 32)
     return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc, tin << 5, tin & 7, team & 1,
-            m < p.M, tin == 0, __activemask()};
+            m < p.M, tin == 0, wmask};
 }
-// The second pass, out of line: what it holds would take registers from the first.
+// The second pass, out of line: what it holds would take registers from the first. The warp's mask is the kernel's: it says which lanes there are,
+// and is read where all of them are together.
 template <typename T, int PRO, bool DIGITS>
-__device__ __noinline__ void direct_again(const QuantArgs& p) {
+__device__ __noinline__ void direct_again(const QuantArgs& p, unsigned wmask) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = direct_lane(p, smem);
+    const DirectLane l = direct_lane(p, smem, wmask);
     float v[32];
     direct_values<T, PRO>(p, l, v);
     direct_second<T, DIGITS>(p, l, v);
@@ -579,7 +580,7 @@ __device__ __noinline__ void direct_again(const QuantArgs& p) {
 template <typename T, int PRO, int MAXT, bool DIGITS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = direct_lane(p, smem);
+    const DirectLane l = direct_lane(p, smem, __activemask());
     direct_clear<DIGITS>(p, l.bits);
     pdl_wait();
     if (DIGITS) clear_counters(p);
@@ -590,7 +591,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel
         direct_values<T, PRO>(p, l, v);
         done = direct_first<T, DIGITS>(p, l, v);
     }
-    if (!done) direct_again<T, PRO, DIGITS>(p);
+    if (!done) direct_again<T, PRO, DIGITS>(p, l.wmask);
 }
 
 // Normalising prologues on bf16 rows. The row sums are added in the reference's order (csrc/kernels.cu:113-147, csrc/common.cuh:30-55), so

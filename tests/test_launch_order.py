@@ -163,3 +163,12 @@ def test_a_trigger_out_of_order_is_noticed():
     assert "gemm_i8_pair_kernel" in planted("drain_values", first)
     assert "quant_direct_kernel" in planted("load32", lambda b: "const T* __restrict__ y = x; " + b)
     assert "quant_norm_kernel" in planted("norm_lane", lambda b: "gload(x); " + b)
+
+
+def test_functions_out_of_line_are_given_their_warp_mask():
+    """Which lanes a partial warp has is read once, at a kernel's start. Read again in a called function it would be whichever lanes the
+    compiler happens to have there together."""
+    functions = _device_functions()
+    inside = {n: _followed(b, functions, out_of_line=True) for n, forms in functions.items() for q, _, b in forms if "__noinline__" in q}
+    assert {"direct_again", "norm_again"} <= set(inside)
+    assert [n for n, text in inside.items() if "__activemask(" in text] == []
