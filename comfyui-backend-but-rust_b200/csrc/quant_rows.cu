@@ -353,7 +353,7 @@ __device__ __forceinline__ void store_codes(const uint32_t (&c16)[16], int8_t* q
 }
 // P = 16 x the rotated values, all finite; amax = the row's maximum
 template <typename T>
-__device__ __forceinline__ void codes_fast(float2 (&P)[16], uint32_t (&c16)[16], float amax, float scale, int tsw) {
+__device__ __forceinline__ void codes_fast(float2 (&P)[16], uint32_t (&c16)[16], float amax, float scale, int tsw, unsigned wmask) {
     const float2 magic = make_float2(12582912.f, 12582912.f);       // rint: the integer's low byte is the sum's
     const uint32_t pick = tsw ? 0x0004u : 0x0040u;                   // the two low bytes in element order
     const float st = rnd<T>(scale);
@@ -365,8 +365,9 @@ __device__ __forceinline__ void codes_fast(float2 (&P)[16], uint32_t (&c16)[16],
             const float2 t = __fmul2_rn(bf16x2_f(a), rcp2);
             return bf16x2_f(__floats2bfloat162_rn(t.x, t.y));
         };
-        // 128 needs the clamp. Quotients grow with their dividends, so the maximum's tells for the row (about one row in eight).
-        if (rnd<T>(rnd<T>(amax) * rcp) < 127.5f) {
+        // 128 needs the clamp. Quotients grow with their dividends, so the maximum's tells for the row (about one row in eight). One form for the warp:
+        // with rows of 256 its teams have four, and each would wait for the others' form (16896 x 256 6.7 us, 6.2 with one).
+        if (!__any_sync(wmask, !(rnd<T>(rnd<T>(amax) * rcp) < 127.5f))) {
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const float2 u = __fadd2_rn(quotient(P[i]), magic);
@@ -434,7 +435,7 @@ __device__ __forceinline__ bool direct_first(const QuantArgs& p, const DirectLan
         const float amax = __uint_as_float(l.bits[l.rloc]) * 0.0625f, scale = row_scale<T>(amax);
         if (l.live && l.first) p.scales[l.m] = scale;
         uint32_t c16[16];
-        codes_fast<T>(P, c16, amax, scale, l.tsw);
+        codes_fast<T>(P, c16, amax, scale, l.tsw, l.wmask);
         store_codes(c16, p.q + l.m * (int64_t)p.K + l.col, l.live, l.tbuf, l.t8, l.wmask);
     }
     return true;
@@ -555,24 +556,34 @@ __device__ __forceinline__ void direct_values(const QuantArgs& p, const DirectLa
         load32<T, false>(x, v);
         if (has_aux<PRO>()) load32<T, false>(x + p.up_offset, u);
         if (p.early) pdl_trigger();
-        elementwise_prologue<T, PRO>(v, u, p.lut >= 0 ? g_act_lut[p.lut] : nullptr);
+        elementwise_prologue<T, PRO>(v, u, PRO != PRO_GELU && p.lut >= 0 ? g_act_lut[p.lut] : nullptr);      // GELU's table: see launch_quant
     }
 }
-__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem, unsigned wmask) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = lane >> 3;
-    const int rloc = threadIdx.x / p.tpr, tin = threadIdx.x - rloc * p.tpr;
+// A warp's lanes: all of them but in a partial last warp (threads = rows * K / 32)
+__device__ __forceinline__ unsigned warp_lanes(unsigned tid) {
+    const unsigned left = blockDim.x - (tid & ~31u);
+    return left >= 32 ? 0xffffffffu : (1u << left) - 1;
+}
+__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem, unsigned tid) {
+    const int warp = tid >> 5, lane = tid & 31, team = lane >> 3;
+    const int rloc = tid / (unsigned)p.tpr, tin = tid - rloc * p.tpr;
     const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
     float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
-    // idle rows compute on the last row and store nothing; the last warp of a CTA may be partial (threads = rows * K / 32)
+    // idle rows compute on the last row and store nothing
     return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc, tin << 5, tin & 7, team & 1,
-            m < p.M, tin == 0, wmask};
+            m < p.M, tin == 0, warp_lanes(tid)};
 }
-// The second pass, out of line: what it holds would take registers from the first. The warp's mask is the kernel's: it says which lanes there are,
-// and is read where all of them are together.
+// The thread's index, read anew: what is worked out from it need not stay in registers while a row's 32 values and their look-ups fill them
+__device__ __forceinline__ unsigned tid_anew() {
+    unsigned t;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+    return t;
+}
+// The second pass, out of line: what it holds would take registers from the first.
 template <typename T, int PRO, bool DIGITS>
-__device__ __noinline__ void direct_again(const QuantArgs& p, unsigned wmask) {
+__device__ __noinline__ void direct_again(const QuantArgs& p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = direct_lane(p, smem, wmask);
+    const DirectLane l = direct_lane(p, smem, threadIdx.x);
     float v[32];
     direct_values<T, PRO>(p, l, v);
     direct_second<T, DIGITS>(p, l, v);
@@ -580,7 +591,8 @@ __device__ __noinline__ void direct_again(const QuantArgs& p, unsigned wmask) {
 template <typename T, int PRO, int MAXT, bool DIGITS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = direct_lane(p, smem, __activemask());
+    constexpr bool kAnew = sizeof(T) == 2 && (PRO == PRO_SILU || PRO == PRO_GELU || PRO == PRO_GELU_TANH);
+    const DirectLane l = direct_lane(p, smem, threadIdx.x);
     direct_clear<DIGITS>(p, l.bits);
     pdl_wait();
     if (DIGITS) clear_counters(p);
@@ -589,9 +601,10 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel
     {
         float v[32];
         direct_values<T, PRO>(p, l, v);
-        done = direct_first<T, DIGITS>(p, l, v);
+        if constexpr (kAnew) done = direct_first<T, DIGITS>(p, direct_lane(p, smem, tid_anew()), v);
+        else done = direct_first<T, DIGITS>(p, l, v);
     }
-    if (!done) direct_again<T, PRO, DIGITS>(p, l.wmask);
+    if (!done) direct_again<T, PRO, DIGITS>(p);
 }
 
 // Normalising prologues on bf16 rows. The row sums are added in the reference's order (csrc/kernels.cu:113-147, csrc/common.cuh:30-55), so
@@ -1781,7 +1794,10 @@ int launch_quant(QuantArgs& p, cudaStream_t st) {
     }
     const bool codes = p.rotate && !p.out_f && !p.digits && !p.amax_in && !p.amax_out;
     if constexpr (direct_threads<T, PRO>() > 0) {
-        if (codes && threads <= direct_threads<T, PRO>()) return launch_direct<T, PRO, direct_threads<T, PRO>()>(p, threads, smem, st);
+        // Tabulated, GELU is SILU's kernel on another table; its own computes it. Both forms in one, erff beside the look-ups, spilled.
+        constexpr int kPro = sizeof(T) == 2 && PRO == PRO_GELU ? PRO_SILU : PRO;
+        if (codes && threads <= direct_threads<T, PRO>())
+            return p.lut >= 0 ? launch_direct<T, kPro, direct_threads<T, PRO>()>(p, threads, smem, st) : launch_direct<T, PRO, direct_threads<T, PRO>()>(p, threads, smem, st);
     }
     if constexpr (sizeof(T) == 2 && is_norm<PRO>()) {
         if (codes) return launch_norm<T, PRO>(p, st);

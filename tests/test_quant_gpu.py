@@ -236,3 +236,24 @@ def test_misaligned_rows_are_refused(pkg, dev):
     x = torch.zeros(4, 520, device=dev, dtype=torch.bfloat16)
     with pytest.raises(pkg.GpuKernelError, match="-5"):
         pkg.linear.quant_rows(x[:, 4:], PLAIN, 0, K=512)          # rows start 8 bytes off a 16-byte boundary
+
+
+@pytest.mark.parametrize("pro", [SILU, GELU, GELU_TANH])
+@pytest.mark.parametrize("M,K", [(45, 768), (4352, 256), (2100, 512), (1100, 1024), (120, 9216)])
+def test_unary_prologues_with_and_without_a_table(pkg, dev, pro, M, K):
+    """Both sides of the line between computed and tabulated activations (2^20 values), warps whose four teams hold rows of their own and warps inside one
+    row: in one kernel against the maxima and the quantization as two. Every bf16 pattern is among the values; infinities and NaNs take CTAs of
+    several rows through the second pass, ordinary rows beside them."""
+    g = torch.Generator().manual_seed(K + pro)
+    x = (torch.randn(M, K, generator=g) * torch.exp2(torch.randint(-6, 7, (M, 1), generator=g).float())).bfloat16()
+    every = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    rows = min(M // 2, 65536 // K)
+    x[: 2 * rows : 2] = every[torch.randperm(65536, generator=g)][: rows * K].view(rows, K)
+    finite = every[every.isfinite() & (every.float().abs() < 2.0 ** 100)]
+    x[1 : 2 * rows : 6, :256] = finite[torch.randint(0, finite.numel(), (len(range(1, 2 * rows, 6)), 256), generator=g)]
+    x = x.to(dev)
+    q, s = pkg.linear.quant_rows(x, pro, 1)
+    q2, s2 = pkg.linear.quant_rows_scaled(x, pkg.linear.quant_rows_amax(x, pro, 1), pro, 1)
+    assert_bits_equal(q, q2, "codes")
+    assert_bits_equal(s, s2, "scales")
+    assert pkg.linear.kernel_status() == 0
