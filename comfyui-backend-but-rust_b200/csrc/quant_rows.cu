@@ -1301,7 +1301,7 @@ __device__ __forceinline__ void sd_source_rows(const SdSrc& s, uint4* row_s, int
 // six: 8192 rows of 640 values are 1024 such CTAs, which six per SM take in two rounds, the second an eighth full.
 // In a chain of launches 8192 x 640: rows as they lie 7.6 -> 6.0 us.
 constexpr int kSdThreads = 288;
-template <int ROT, int SRC, int MAXT>
+template <int ROT, int SRC, int MAXT, bool EARLY>
 __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fast_kernel(const SdSrc s, int8_t* q, float* scales, int M,
                                                             int K, int tpr, int rows, uint32_t off_amax, uint32_t off_rows, int early) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -1337,7 +1337,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= kSdThreads ? 4 : 1) sd_quant_fas
 #pragma unroll
         for (int c = 0; c < 4; ++c) unpack_half8(r[sd_piece(4 * tin + c)], *reinterpret_cast<float(*)[8]>(v + 8 * c));
     }
-    if (early) pdl_trigger();
+    if (EARLY && early) pdl_trigger();      // a kernel of its own where the rows are values at once: the branch there cost the others 3 %
     float2 P[16];
     if (ROT) {
 #pragma unroll
@@ -1530,10 +1530,13 @@ int early_trigger(int64_t ctas) {
     cudaGetDevice(&dev);
     return ctas <= sm_count_of(dev);
 }
-template <int ROT, int SRC, int MAXT>
+template <int ROT, int SRC, int MAXT, bool EARLY = true>
 int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 grid, int threads, int rows, uint32_t smem, uint32_t off_amax,
                   uint32_t off_rows, cudaStream_t st) {
-    auto kern = sd_quant_fast_kernel<ROT, SRC, MAXT>;
+    const int early = early_trigger((int64_t)grid.x * grid.y);
+    if constexpr (SRC == SDQ_ROWS && EARLY)
+        if (!early) return launch_sd_cfg<ROT, SRC, MAXT, false>(s, q, scales, M, K, grid, threads, rows, smem, off_amax, off_rows, st);
+    auto kern = sd_quant_fast_kernel<ROT, SRC, MAXT, EARLY>;
     if (smem > 48 * 1024) {
         static std::atomic<uint64_t> configured{0};
         int dev = 0;
@@ -1545,7 +1548,7 @@ int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 g
             configured.fetch_or(bit, std::memory_order_release);
         }
     }
-    return launch_pdl(kern, grid, threads, smem, st, s, q, scales, M, K, K / 32, rows, off_amax, off_rows, early_trigger((int64_t)grid.x * grid.y));
+    return launch_pdl(kern, grid, threads, smem, st, s, q, scales, M, K, K / 32, rows, off_amax, off_rows, early);
 }
 template <int ROT, int SRC>
 int launch_sd_fast(const SdSrc& s, int8_t* q, float* scales, int M, int K, cudaStream_t st) {
