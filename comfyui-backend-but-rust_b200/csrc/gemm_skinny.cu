@@ -22,11 +22,13 @@ __global__ void __launch_bounds__(kWarps * 32) skinny_gemm_kernel(const SkinnyPa
     const int K = p.K;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nblocks = (p.N + kRowsPerWarp - 1) / kRowsPerWarp;
-    // This warp's first weight rows on their way to L2 while the predecessor, as a rule the quantizer of these few rows, still runs.
-    // Nothing is read here: whatever the predecessor writes is seen by the loads behind the wait.
+    // The head of this warp's first weight rows on its way to L2 while the predecessor, as a rule the quantizer of these few rows, still runs.
+    // Nothing is read here: whatever the predecessor writes is seen by the loads behind the wait. 4 KB a warp, 19 MB in all: of the whole
+    // rows the loads overtake most, and they get in one another's way. Quantizer and GEMM, none | 4 KB | whole rows: 1 x 3072 -> 18432 17.0 | 15.8 | 16.7 us,
+    // 1 x 5120 -> 15360 19.8 | 18.6 | 19.6, 2 x 5120 -> 30720 33.6 | 32.4 | 32.6; the GEMM alone 8 x 5120 -> 30720 41.2 | 40.7 | 43.4.
     if (lane == 0) {
         const int n0 = (blockIdx.x * kWarps + warp) * kRowsPerWarp, rows = min(kRowsPerWarp, p.N - n0);
-        if (rows > 0) prefetch_l2(p.W + (int64_t)n0 * K, (uint32_t)rows * K);
+        if (rows > 0) prefetch_l2(p.W + (int64_t)n0 * K, min((uint32_t)rows * K, 4096u));
     }
     pdl_wait();
     for (int i = threadIdx.x; i < p.M * K / 16; i += blockDim.x)
