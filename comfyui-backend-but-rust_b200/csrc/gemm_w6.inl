@@ -240,14 +240,14 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
                         uint8_t* out = sm + (sB - base) + sb * b_bytes + rr * 128;
                         const uint4 h0 = *reinterpret_cast<const uint4*>(hi + ((hf ^ sw_hi) << 4));
                         const uint32_t hw[4] = {h0.x, h0.y, h0.z, h0.w};
-                        const int mode = w6_mode(sr);      // the other thread's half with it: the row's scales of the box
+                        const int mode = w6_mode<false>(sr);      // the other thread's half with it: the row's scales of the box
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {      // 32 elements = one scale group per 16-byte piece of nibbles
                             if ((c >> 1) != hf) continue;  // the other thread of the row (the same for the whole warp)
                             const int hi_w = 2 * (c & 1);
                             const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
                             uint32_t o[8];
-                            w6_group(mode, l, hw[hi_w], hw[hi_w + 1], (sr >> (8 * c)) & 0xffu, o);
+                            w6_group_of<false>(mode, l, hw[hi_w], hw[hi_w + 1], (sr >> (8 * c)) & 0xffu, o);
                             if (has_row) {
                                 *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
                                 *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);

@@ -26,12 +26,15 @@
 // merged before the permute that pairs them.
 enum { W6_UNIT = 0, W6_SMALL = 1, W6_ANY = 2, W6_MID = 3 };
 // The form for the four scale bytes of a lane and those of its warp's other lanes (absent ones filled with 0x38, a scale of 1)
+// MID: whether the caller has the W6_MID form. The pair kernel has not: what bounds it is not its arithmetic, and a fourth form of eight groups
+// beside the others took 234 us where three take 195 (2048 x 5120 -> 15360; 600 rows 132 and 116).
+template <bool MID = true>
 __device__ __forceinline__ int w6_mode(uint32_t sb4) {
     // bytes up to 0x48 (4.0), sign clear: adding 0x37 carries into bit 7 from 0x49 on
     const bool small = (((sb4 & 0x7f7f7f7fu) + 0x37373737u) & 0x80808080u) == 0u && (sb4 & 0x80808080u) == 0u;
     if (!__all_sync(0xffffffffu, small)) return W6_ANY;
-    if (!__all_sync(0xffffffffu, (((sb4 | 0x80808080u) - 0x28282828u) & 0x80808080u) == 0x80808080u)) return W6_SMALL;      // from 0x28 (1/4) on
-    return __all_sync(0xffffffffu, sb4 == 0x38383838u) ? W6_UNIT : W6_MID;
+    if (__all_sync(0xffffffffu, sb4 == 0x38383838u)) return W6_UNIT;
+    return MID && __all_sync(0xffffffffu, (((sb4 | 0x80808080u) - 0x28282828u) & 0x80808080u) == 0x80808080u) ? W6_MID : W6_SMALL;      // from 0x28 (1/4) on
 }
 template <int MODE>
 __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
@@ -96,8 +99,9 @@ __device__ __forceinline__ void w6_group(const uint4 l, uint32_t ha, uint32_t hb
     }
 }
 // with the mode in a variable (the same in the whole warp)
-__device__ __forceinline__ void w6_group(int mode, const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
-    if (mode == W6_MID) w6_group<W6_MID>(l, ha, hb, sb, o);
+template <bool MID = true>
+__device__ __forceinline__ void w6_group_of(int mode, const uint4 l, uint32_t ha, uint32_t hb, uint32_t sb, uint32_t (&o)[8]) {
+    if (MID && mode == W6_MID) w6_group<W6_MID>(l, ha, hb, sb, o);
     else if (mode == W6_SMALL) w6_group<W6_SMALL>(l, ha, hb, sb, o);
     else if (mode == W6_UNIT) w6_group<W6_UNIT>(l, ha, hb, sb, o);
     else w6_group<W6_ANY>(l, ha, hb, sb, o);

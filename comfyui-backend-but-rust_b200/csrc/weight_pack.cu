@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(256) w6_decode32_kernel(const uint8_t* q, cons
     const uint32_t sb = s_rel[n * (K / G) + c * 32 / G];
     pdl_trigger();
     uint32_t o[8];
-    w6_group(w6_mode(sb | 0x38383800u), lo, hi.x, hi.y, sb, o);
+    w6_group_of(w6_mode(sb | 0x38383800u), lo, hi.x, hi.y, sb, o);
     if (live) {
         uint4* d = reinterpret_cast<uint4*>(out + n * (int64_t)K + c * 32);
         d[0] = make_uint4(o[0], o[1], o[2], o[3]);
