@@ -621,17 +621,25 @@ __device__ __forceinline__ void row_barrier(int rloc, int warps) {
     else named_bar_sync(1 + rloc, 32 * warps);
 }
 // f32 rows (RMS without modulation, the weight-only linear's): the same with 1 KB a group.
-template <typename T, int PRO>
+// ROWS: rows a warp holds, more than one for rows of 256 (four) and 512 (two) values: a group each in the same four places. With a row a warp three of its four
+// teams had nothing to rotate: 16896 x 256 RMS 19.9 us, 8.3 with four rows; 16896 x 512 21.6 and 13.6 with two.
+template <typename T, int PRO, int ROWS>
 __device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane& l, uint8_t* smem, float (&v)[32]) {
-    static_assert(sizeof(T) == 2 || PRO == PRO_RMS, "f32 rows: RMS only");
-    const int lane = threadIdx.x & 31, nwr = p.tpr, w = (threadIdx.x >> 5) - l.rloc * nwr, ngroups = p.K >> 8, grp = l.col >> 8;
-    float* slice0 = reinterpret_cast<float*>(smem) + l.rloc * nwr * kWarpWords;       // the row's first warp's buffer
+    static_assert((sizeof(T) == 2 || PRO == PRO_RMS) && (sizeof(T) == 2 || ROWS == 1), "f32 rows: RMS only, a row a warp or more");
+    constexpr int kPer = 4 / ROWS;              // places of a row
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwr = ROWS > 1 ? 1 : p.tpr, row0 = ROWS > 1 ? warp * ROWS : l.rloc;
+    const int w = ROWS > 1 ? 0 : warp - l.rloc * nwr, ngroups = ROWS > 1 ? kPer : p.K >> 8, grp = l.col >> 8;
+    float* slice0 = reinterpret_cast<float*>(smem) + (ROWS > 1 ? warp : l.rloc * nwr) * kWarpWords;       // the row's first warp's buffer
     float* sums = reinterpret_cast<float*>(smem + p.off_norm) + l.rloc * 64;          // [2][32]
-    const T* x = reinterpret_cast<const T*>(p.x) + l.m * p.x_stride + 8 * lane;
+    auto group_of = [&](int i) { return ROWS > 1 ? i % kPer : w + nwr * i; };         // in place i
+    const T* x = reinterpret_cast<const T*>(p.x) + (ROWS > 1 ? 0 : l.m * p.x_stride) + 8 * lane;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int g = w + nwr * i;
-        if constexpr (sizeof(T) == 2) {
+        const int g = group_of(i);
+        if constexpr (ROWS > 1) {
+            const int64_t m = min((int64_t)blockIdx.x * p.rows_per_cta + row0 + i / kPer, (int64_t)p.M - 1);
+            unpack_bf16x8(gload(reinterpret_cast<const uint4*>(x + m * p.x_stride + (g << 8))), v + 8 * i);
+        } else if constexpr (sizeof(T) == 2) {
             unpack_bf16x8(g < ngroups ? gload(reinterpret_cast<const uint4*>(x + (g << 8))) : make_uint4(0, 0, 0, 0), v + 8 * i);
         } else {
 #pragma unroll
@@ -641,12 +649,13 @@ __device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane
             }
         }
     }
-    auto row_sum = [&](bool squares, float* slot) -> float {
+    auto row_sum = [&](int r, bool squares, float* slot) -> float {      // r: the warp's row
         float s = 0.f;                             // the zeros of missing groups come last and change nothing
 #pragma unroll
-        for (int i = 0; i < 32; ++i) s = squares ? __fmaf_rn(v[i], v[i], s) : __fadd_rn(s, v[i]);
+        for (int i = 0; i < 8 * kPer; ++i) s = squares ? __fmaf_rn(v[8 * kPer * r + i], v[8 * kPer * r + i], s) : __fadd_rn(s, v[8 * kPer * r + i]);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        if constexpr (ROWS > 1) return __fadd_rn(s, 0.f);      // the tree over one warp adds zeros
         if (lane == 0) slot[w] = s;
         row_barrier(l.rloc, nwr);
         s = lane < nwr ? slot[lane] : 0.f;
@@ -655,10 +664,12 @@ __device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane
         return s;
     };
     if constexpr (is_ln<PRO>()) {
-        const float mean = __fdiv_rn(row_sum(false, sums), (float)p.K);
+        float mean[ROWS];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) mean[r] = __fdiv_rn(row_sum(r, false, sums), (float)p.K);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float sub = w + nwr * i < ngroups ? mean : 0.f;
+            const float sub = group_of(i) < ngroups ? mean[i / kPer] : 0.f;
 #pragma unroll
             for (int j = 0; j < 8; j += 2) {
                 const float2 d = __fadd2_rn(make_float2(v[8 * i + j], v[8 * i + j + 1]), make_float2(-sub, -sub));
@@ -666,14 +677,16 @@ __device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane
             }
         }
     }
-    const float rstd = rsqrtf(__fadd_rn(__fdiv_rn(row_sum(true, sums + 32), (float)p.K), p.eps));
+    float rstd[ROWS];
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) rstd[r] = rsqrtf(__fadd_rn(__fdiv_rn(row_sum(r, true, sums + 32), (float)p.K), p.eps));
     const bf16* ms_p = reinterpret_cast<const bf16*>(p.mod_scale);
     const bf16* sh_p = reinterpret_cast<const bf16*>(p.mod_shift);
-    const float2 rstd2 = make_float2(rstd, rstd);
     if constexpr (sizeof(T) == 4) {
+        const float2 rstd2 = make_float2(rstd[0], rstd[0]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int g = w + nwr * i;
+            const int g = group_of(i);
             if (g >= ngroups) break;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -698,8 +711,9 @@ __device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane
     } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int g = w + nwr * i;
+            const int g = group_of(i);
             if (g >= ngroups) break;
+            const float2 rstd2 = make_float2(rstd[i / kPer], rstd[i / kPer]);
             const int c0 = (g << 8) + 8 * lane;
             uint4 mw = make_uint4(0, 0, 0, 0), sw = mw;
             float nw[8], nb[8];
@@ -735,17 +749,27 @@ __device__ __forceinline__ void norm_values(const QuantArgs& p, const DirectLane
                 o[j] = *reinterpret_cast<const uint32_t*>(&h);
             }
             // piece (g & 3) * 32 + lane of the slice, its low bits mixed with the next ones: free of bank conflicts both ways
-            const int c = ((g & 3) << 5) + lane;
-            reinterpret_cast<uint4*>(slice0 + (g >> 2) * kWarpWords)[c ^ ((c >> 2) & 7)] = make_uint4(o[0], o[1], o[2], o[3]);
+            const int c = ((ROWS > 1 ? i : g & 3) << 5) + lane;
+            reinterpret_cast<uint4*>(slice0 + (ROWS > 1 ? 0 : g >> 2) * kWarpWords)[c ^ ((c >> 2) & 7)] = make_uint4(o[0], o[1], o[2], o[3]);
         }
         row_barrier(l.rloc, nwr);
         const uint4* mine = reinterpret_cast<const uint4*>(slice0 + w * kWarpWords);
+        const int place = ROWS > 1 ? lane >> 3 : grp - 4 * w;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) unpack_bf16x8(mine[((grp - 4 * w) * 32 + 4 * l.t8 + k) ^ l.t8], v + 8 * k);
+        for (int k = 0; k < 4; ++k) unpack_bf16x8(mine[(place * 32 + 4 * l.t8 + k) ^ l.t8], v + 8 * k);
         __syncwarp();                                  // the slice is the transposition buffer from here on
     }
 }
+template <int ROWS>
 __device__ __forceinline__ DirectLane norm_lane(const QuantArgs& p, uint8_t* smem) {
+    if constexpr (ROWS > 1) {
+        constexpr int kPer = 4 / ROWS;
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = lane >> 3, rloc = warp * ROWS + team / kPer;
+        const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
+        float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
+        return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc,
+                (team % kPer << 8) + ((lane & 7) << 5), lane & 7, team & 1, m < p.M, team % kPer == 0 && (lane & 7) == 0, 0xffffffffu};
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, team = lane >> 3, nwr = p.tpr;      // nwr: warps per row
     const int rloc = warp / nwr, w = warp - rloc * nwr, ngroups = p.K >> 8, grp = min(4 * w + team, ngroups - 1);
     const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
@@ -754,18 +778,18 @@ __device__ __forceinline__ DirectLane norm_lane(const QuantArgs& p, uint8_t* sme
     return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc,
             (grp << 8) + ((lane & 7) << 5), lane & 7, team & 1, m < p.M && 4 * w + team < ngroups, w == 0 && lane == 0, 0xffffffffu};
 }
-template <typename T, int PRO, bool DIGITS>
+template <typename T, int PRO, bool DIGITS, int ROWS>
 __device__ __noinline__ void norm_again(const QuantArgs& p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = norm_lane(p, smem);
+    const DirectLane l = norm_lane<ROWS>(p, smem);
     float v[32];
-    norm_values<T, PRO>(p, l, smem, v);
+    norm_values<T, PRO, ROWS>(p, l, smem, v);
     direct_second<T, DIGITS>(p, l, v);
 }
-template <typename T, int PRO, int MAXT, bool DIGITS>
+template <typename T, int PRO, int MAXT, bool DIGITS, int ROWS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) quant_norm_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = norm_lane(p, smem);
+    const DirectLane l = norm_lane<ROWS>(p, smem);
     direct_clear<DIGITS>(p, l.bits);
     pdl_wait();
     if (DIGITS) clear_counters(p);
@@ -773,10 +797,10 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 4 : 1) quant_norm_kernel(c
     bool done;
     {
         float v[32];
-        norm_values<T, PRO>(p, l, smem, v);
+        norm_values<T, PRO, ROWS>(p, l, smem, v);
         done = direct_first<T, DIGITS>(p, l, v);
     }
-    if (!done) norm_again<T, PRO, DIGITS>(p);
+    if (!done) norm_again<T, PRO, DIGITS, ROWS>(p);
 }
 
 // MAXT = 384 asks for two CTAs per SM (at most 80 registers: 768 threads with the next block's rows in flight);
@@ -1687,21 +1711,29 @@ int launch_direct(QuantArgs& p, int threads, size_t smem, cudaStream_t st) {
     if (int rc = raise_smem(kern, configured, smem)) return rc;
     return launch_pdl(kern, dim3(p.nblocks), threads, smem, st, p);
 }
-template <typename T, int PRO, int MAXT, bool DIGITS>
+template <typename T, int PRO, int MAXT, bool DIGITS, int ROWS = 1>
 int launch_norm_cfg(const QuantArgs& p, int threads, size_t smem, cudaStream_t st) {
     static std::atomic<uint64_t> configured{0};
-    auto kern = quant_norm_kernel<T, PRO, MAXT, DIGITS>;
+    auto kern = quant_norm_kernel<T, PRO, MAXT, DIGITS, ROWS>;
     if (int rc = raise_smem(kern, configured, smem)) return rc;
     return launch_pdl(kern, dim3(p.nblocks), threads, smem, st, p);
 }
-// Rows of ceil(K / 1024) warps, about eight warps per CTA
+// Rows of ceil(K / 1024) warps, about eight warps per CTA. Warps of four rows of 256 values or two of 512 from two CTAs an SM on: 2368 x 256 RMS takes
+// 5.6 us with a row a warp, 2369 4.5 with four, 4736 6.6 and 5.3. On fewer rows more warps hide one another's latencies (1111 x 256: 4.0).
 template <typename T, int PRO, bool DIGITS = false> int launch_norm(QuantArgs p, cudaStream_t st) {
-    const int nwr = ((p.K >> 8) + 3) >> 2, rows = nwr >= 8 ? 1 : 8 / nwr, warps = rows * nwr;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const int nwr = ((p.K >> 8) + 3) >> 2, per_warp = sizeof(T) == 2 && p.K <= 512 && p.M > 8 * 2 * sm_count_of(dev) ? 1024 / p.K : 1;
+    const int rows = per_warp * (nwr >= 8 ? 1 : 8 / nwr), warps = rows / per_warp * nwr;
     p.tpr = nwr, p.rows_per_cta = rows, p.nblocks = (p.M + rows - 1) / rows;
     p.off_norm = (uint32_t)(warps * kWarpWords * 4);
-    p.off_amax = p.off_norm + rows * 64 * 4;
+    p.off_amax = p.off_norm + (per_warp > 1 ? 0 : rows * 64 * 4);
     p.early = early_trigger(p.nblocks);
     const size_t smem = p.off_amax + direct_words(rows, DIGITS) * 4;
+    if constexpr (sizeof(T) == 2) {
+        if (per_warp == 4) return launch_norm_cfg<T, PRO, 256, DIGITS, 4>(p, 32 * warps, smem, st);
+        if (per_warp == 2) return launch_norm_cfg<T, PRO, 256, DIGITS, 2>(p, 32 * warps, smem, st);
+    }
     return warps <= 8 ? launch_norm_cfg<T, PRO, 256, DIGITS>(p, 32 * warps, smem, st) : launch_norm_cfg<T, PRO, 1024, DIGITS>(p, 32 * warps, smem, st);
 }
 

@@ -150,3 +150,59 @@ def test_bf16_norm_prologues_for_every_row_length(pkg, ref, dev, pro, variant):
         qr, sr = ref.quant_rows(c["x"].to(dev), pro, 1, **kw)
         assert_bits_equal(s, sr, f"scales K={K}")
         assert_bits_equal(q, qr, f"codes K={K}")
+
+
+FORMS = [(RMS, 1), (RMS, 3), (LAYERNORM, 3), (ADALN, 0), (LN_MOD, 2), (LN_AFFINE, 0)]
+
+
+@pytest.mark.parametrize("pro,variant", FORMS)
+@pytest.mark.parametrize("M,K", [(2369, 256), (4800, 512), (9999, 256)])
+def test_rows_of_one_and_two_groups_several_to_a_warp(pkg, dev, pro, variant, M, K):
+    """Many rows of 256 or 512 values share warps, few have one each: the same codes and scales, at the line between the two (2368 rows on 148 SMs),
+    with a last CTA and a last warp that are not full, a row stride, and infinities and NaNs beside ordinary rows (the second pass)."""
+    c = _case(M, K, 7 * pro + variant + K)
+    c["x"][[5, M // 2, M - 1], [0, 100, K - 1]] = torch.tensor([float("inf"), float("nan"), -float("inf")], dtype=torch.bfloat16)
+    wide = torch.zeros(M, K + 64, dtype=torch.bfloat16)
+    wide[:, :K] = c["x"]
+    x, kw = wide.to(dev)[:, :K], _to(dev, _kwargs(pro, c, variant))
+    q, s = pkg.linear.quant_rows(x, pro, 1, **kw)
+    for m in range(0, M, 1500):
+        q1, s1 = pkg.linear.quant_rows(x[m : m + 1500], pro, 1, **kw)
+        assert_bits_equal(q[m : m + 1500], q1, f"codes from row {m}")
+        assert_bits_equal(s[m : m + 1500], s1, f"scales from row {m}")
+    assert pkg.linear.kernel_status() == 0
+
+
+@pytest.mark.parametrize("pro,variant", FORMS)
+@pytest.mark.parametrize("M,K", [(37, 256), (4760, 256), (4760, 512), (37, 2560), (11, 9216)])
+def test_second_pass_of_the_norm_prologues(pkg, oracle, dev, pro, variant, M, K):
+    """A row with an infinity, a NaN or values near the end of the range sends its whole CTA through the pass with the halvings: its ordinary neighbours keep
+    the codes and scales that they have without it, and rows that are finite after the norm agree with the oracle."""
+    c = _case(M, K, 13 * pro + variant + K)
+    kw = _kwargs(pro, c, variant)
+    special = {1: float("inf"), 6: float("nan"), M - 2: -float("inf")}
+    plain, odd = c["x"].clone(), c["x"].clone()
+    for m, v in special.items():
+        odd[m, (17 * m) % K] = v
+    d = _to(dev, kw)
+    q0, s0 = pkg.linear.quant_rows(plain.to(dev), pro, 1, **d)
+    q1, s1 = pkg.linear.quant_rows(odd.to(dev), pro, 1, **d)
+    keep = torch.tensor([m for m in range(M) if m not in special])
+    assert_bits_equal(q1.cpu()[keep], q0.cpu()[keep], "codes of ordinary rows")
+    assert_bits_equal(s1.cpu()[keep], s0.cpu()[keep], "scales of ordinary rows")
+    for m in special:                                  # the same alone in a CTA of one row
+        qa, sa = pkg.linear.quant_rows(odd[m : m + 1].to(dev), pro, 1, **d)
+        assert_bits_equal(q1[m : m + 1], qa, f"codes of row {m}")
+        assert_bits_equal(s1[m : m + 1], sa, f"scales of row {m}")
+    # every row through it: weights or modulation that take the normalised values past 2^123
+    big = {k: v.clone() if torch.is_tensor(v) else v for k, v in kw.items()}
+    for k in ("norm_w", "mod_scale"):
+        if torch.is_tensor(big.get(k)):
+            big[k][: K // 2] = 2.0 ** 121
+            break
+    qo, so = oracle.quant_rows(plain, pro, 1, **big)
+    qb, sb = pkg.linear.quant_rows(plain.to(dev), pro, 1, **_to(dev, big))
+    diff = (qb.cpu().int() - qo.int()).abs()
+    assert int(diff.max()) <= 1 and float((diff != 0).float().mean()) <= 2e-3      # as against the oracle above
+    assert torch.allclose(sb.cpu(), so, rtol=2e-2)
+    assert pkg.linear.kernel_status() == 0
