@@ -195,3 +195,22 @@ def test_argument_checks(pkg, dev):
         L.wo8_linear(x, Wq, ws, beta=0.5)
     with pytest.raises(pkg.GpuKernelError, match="-3"):
         L.wo8_linear(x, Wq, ws, 11)                                 # a prologue gpu_rotate_rows_f32 does not take
+
+
+@pytest.mark.parametrize("pro,K", [(RMS, 512), (RMS, 2560), (SWIGLU, 512), (SWIGLU, 9728)])
+def test_rows_without_a_maximum_behind_a_prologue(pkg, dev, pro, K):
+    """The digits' second pass behind RMS and SWIGLU: a row with an infinity or a NaN becomes NaN, its ordinary neighbours in the same CTA keep their bits."""
+    g = torch.Generator().manual_seed(K + pro)
+    L = pkg.linear
+    N, M = 264, 37
+    x = torch.randn(M, 2 * K if pro == SWIGLU else K, generator=g)
+    kw = dict(K=K, up_offset=K) if pro == SWIGLU else dict(norm_w=(torch.randn(K, generator=g) * 0.1 + 1.0).to(dev), eps=1e-6)
+    odd = x.clone()
+    odd[1, 7], odd[2, 300], odd[M - 1, K - 1] = float("inf"), float("nan"), float("inf")
+    odd[5] = 0.0
+    Wq, ws = L.convrot_requant((torch.randn(N, K, generator=g) * 0.03).to(dev), 0)
+    plain, out = L.wo8_linear(x.to(dev), Wq, ws, pro, **kw), L.wo8_linear(odd.to(dev), Wq, ws, pro, **kw)
+    keep = [m for m in range(M) if m not in (1, 2, 5, M - 1)]
+    assert torch.equal(plain[keep], out[keep])
+    assert bool(out[[1, 2, M - 1]].isnan().all()) and bool((out[5] == 0).all())
+    assert L.kernel_status() == 0
