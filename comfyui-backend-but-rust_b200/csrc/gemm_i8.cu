@@ -32,6 +32,7 @@
 
 #include "common.cuh"
 #include "epilogue.cuh"
+#include "w6_rows_plan.h"
 #include "w6_decode.cuh"
 
 __device__ int g_kernel_status = 0;

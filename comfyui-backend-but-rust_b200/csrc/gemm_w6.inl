@@ -370,9 +370,10 @@ gemm_w6a8_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 // of four warps take K boxes in turn (the expansion is what bounds the kernel, a few instructions per code; three groups left the
 // issue slots idle two cycles in five). A lane expands one scale group of one row at a time, eight rows of a box to a warp's step, so
 // that a tile need not have 128 rows: the host side picks the height (a multiple of eight; the MMA's other rows are never read) that
-// spreads the weight's rows evenly over the SMs. 15360 rows are 120 tiles of 128 for 148 SMs, or 148 of 104. All of them run the epilogue:
-// a lane owns an output column. Tiles of 128 rows and one row a lane -> this, at 64 tokens: 5120 -> 15360 34.0 -> 31.8 us, 5120 -> 13824 34.4 -> 30.4;
-// 5120 -> 5120 (40 tiles in either form) 18.6 -> 18.9, 13824 -> 5120 30.8 -> 31.4.
+// spreads the weight's rows evenly over the SMs. 15360 rows are 120 tiles of 128 for 148 SMs, or 148 of 104. Many tokens beside whole tiles have a row a lane
+// (w6_row_a_lane()). All warps run the epilogue: a lane owns an output column.
+// Back to back, us, tiles of 128 rows with a row a lane and one lane issuing | this: 64 tokens 5120 -> 15360 31.6 | 26.6, 5120 -> 5120 17.1 | 16.0, 5120 -> 13824
+// 31.3 | 25.2, 13824 -> 5120 29.7 | 26.3; 200 tokens 38.1 | 38.7, 20.9 | 20.6, 37.7 | 37.0, 34.0 | 33.8; 64 x 1024 -> 64 7.2 | 7.3.
 constexpr int kW6RowsWarps = 20;
 constexpr int kW6RowsThreads = 32 * (2 + kW6RowsWarps);
 constexpr int kW6RowsMaxTokens = 256;
@@ -392,7 +393,7 @@ __device__ __forceinline__ int ld_shared_cluster(uint32_t addr) {
 }
 
 // TILED: several tiles of tokens. With one the offsets are left out: computed, they cost the epilogue of the activation form 0.4 us.
-template <typename OutT, int EPI, bool TILED>
+template <typename OutT, int EPI, bool TILED, bool ROW_A_LANE>
 __global__ void __launch_bounds__(kW6RowsThreads, 1)
 gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_lo,
                       const __grid_constant__ CUtensorMap tmap_hi, const GemmParams p, const W6RowsParams x6) {
@@ -474,60 +475,146 @@ gemm_w6a8_rows_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (ok && one) umma_commit(bar_tfull);
     } else {
         const int uw = warp - 2, grp = uw >> 2;
-        // Step i of a box: its rows 8 i .. 8 i + 7; lane = (row, scale group). Warp j of a group takes every fourth step, counted from
-        // where its last box left off, so that all four do as much.
-        const int steps = R / 8, c = lane & 3;
-        auto row_of = [&](int i) { return 8 * i + (lane >> 2); };
-        auto first = [&](int kb) { return ((uw & 3) + 4 - (kb / x6.groups * steps & 3)) & 3; };
-        auto fetch = [&](int kb) -> uint32_t {                     // the steps' scale bytes of box kb, a turn ahead of their use
-            uint32_t b[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int i = first(kb) + 4 * j;
-                b[j] = i < steps && kb < k1 ? gload(x6.s_rel + (size_t)min(n0 + row_of(i), p.N - 1) * x6.srel_pitch + 4 * kb + c) : 0x38u;
-            }
-            return b[0] | b[1] << 8 | b[2] << 16 | b[3] << 24;
-        };
-        const int g = x6.groups;
-        int sa = grp, sb = grp;                                    // a group beyond the boxes has none
-        uint32_t pa = 0, pb = 0;
         bool ok = true;
-        uint32_t sc_next = fetch(k0 + grp);
-        for (int kb = grp < g ? k0 + grp : k1; kb < k1; kb += g) {
-            const uint32_t sc = sc_next;
-            sc_next = fetch(kb + g);
-            // the expanded slot first, as above: groups <= sb <= sa keeps every awaited phase the current or the last one
-            if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
-                !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
-            if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
-                !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
-            const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes;
-            const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes;
-            uint8_t* out = sm + sb * w_bytes;
-            auto expand = [&](auto mode) {
-#pragma unroll 1
-                for (int i = first(kb), s4 = (int)sc; i < steps; i += 4, s4 = (int)((uint32_t)s4 >> 8)) {
-                    const int r = row_of(i);
-                    const uint4 l = *reinterpret_cast<const uint4*>(lo + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
-                    const uint2 h = *reinterpret_cast<const uint2*>(hi + r * 32 + (((c >> 1) ^ ((r >> 2) & 1)) << 4) + ((c & 1) << 3));
-                    uint32_t o[8];
-                    w6_group<decltype(mode)::value>(l, h.x, h.y, (uint32_t)s4 & 0xffu, o);
-                    uint8_t* row = out + r * 128;
-                    *reinterpret_cast<uint4*>(row + (((2 * c) ^ (r & 7)) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
-                    *reinterpret_cast<uint4*>(row + (((2 * c + 1) ^ (r & 7)) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+        if constexpr (ROW_A_LANE) {
+            const int r = 32 * (uw & 3) + lane;                        // weight row of the tile
+            const uint8_t* srow = x6.s_rel + (size_t)min(n0 + r, p.N - 1) * x6.srel_pitch;
+            const bool wide = (x6.srel_pitch & 15) == 0 && ((uintptr_t)x6.s_rel & 15) == 0;   // scale rows readable 16 bytes at a time
+            auto fetch = [&](int kb4) -> uint4 {                       // scales of boxes 4 kb4 .. 4 kb4 + 3
+                if (wide) return gload(reinterpret_cast<const uint4*>(srow) + kb4);
+                uint4 v = make_uint4(0, 0, 0, 0);
+                const uint32_t* s32 = reinterpret_cast<const uint32_t*>(srow) + 4 * kb4;
+                const int left = p.k_iters - 4 * kb4;
+                if (left > 0) v.x = gload(s32);
+                if (left > 1) v.y = gload(s32 + 1);
+                if (left > 2) v.z = gload(s32 + 2);
+                if (left > 3) v.w = gload(s32 + 3);
+                return v;
+            };
+            const int sw_lo = (r >> 1) & 3, sw_hi = (r >> 2) & 1, sw_out = r & 7;
+            int sa = 0, sb = 0, turn = 0;
+            uint32_t pa = 0, pb = 0;
+            uint4 sc_cur = make_uint4(0, 0, 0, 0), sc_next = fetch(k0 >> 2);
+            for (int kb = grp < x6.groups ? k0 : k1; kb < k1; ++kb) {
+                if ((kb & 3) == 0 || kb == k0) {
+                    sc_cur = sc_next;
+                    if ((kb & ~3) + 4 < k1) sc_next = fetch((kb >> 2) + 1);
+                }
+                if (turn == grp) {
+                    const int q = kb & 3;
+                    const uint32_t sr = q == 0 ? sc_cur.x : q == 1 ? sc_cur.y : q == 2 ? sc_cur.z : sc_cur.w;
+                    // the expanded slot first, as above: groups <= sb <= sa keeps every awaited phase the current or the last one
+                    if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
+                        !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                    if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
+                        !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                    const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + r * 64;
+                    const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + r * 32;
+                    uint8_t* out = sm + sb * w_bytes + r * 128;
+                    const uint4 h0 = *reinterpret_cast<const uint4*>(hi + (sw_hi << 4)), h1 = *reinterpret_cast<const uint4*>(hi + ((1 ^ sw_hi) << 4));
+                    const uint32_t hw[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                    auto expand = [&](auto mode) {
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {                  // 32 codes = one scale group per 16-byte piece of nibbles
+                            const uint4 l = *reinterpret_cast<const uint4*>(lo + ((c ^ sw_lo) << 4));
+                            uint32_t o[8];
+                            w6_group<decltype(mode)::value>(l, hw[2 * c], hw[2 * c + 1], (sr >> (8 * c)) & 0xffu, o);
+                            *reinterpret_cast<uint4*>(out + (((2 * c) ^ sw_out) << 4)) = make_uint4(o[0], o[1], o[2], o[3]);
+                            *reinterpret_cast<uint4*>(out + (((2 * c + 1) ^ sw_out) << 4)) = make_uint4(o[4], o[5], o[6], o[7]);
+                        }
+                    };
+                    const int mode = w6_mode(sr);
+                    if (mode == W6_MID) expand(std::integral_constant<int, W6_MID>());
+                    else if (mode == W6_SMALL) expand(std::integral_constant<int, W6_SMALL>());
+                    else if (mode == W6_UNIT) expand(std::integral_constant<int, W6_UNIT>());
+                    else expand(std::integral_constant<int, W6_ANY>());
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
+                }
+                if (++turn == x6.groups) turn = 0;
+                if (++sa == SA) sa = 0, pa ^= 1u;
+                if (++sb == SB) sb = 0, pb ^= 1u;
+            }
+        } else {
+            // Step i of a box: its rows 8 i .. 8 i + 7; lane = (row, scale group). Warp j of a group takes every fourth step, counted from
+            // where its last box left off, so that all four do as much.
+            const int steps = R / 8, c = lane & 3;
+            auto row_of = [&](int i) { return 8 * i + (lane >> 2); };
+            // where a lane's pieces lie among a step's rows: the swizzles look at the row's low three bits, which are the lane's
+            const uint32_t l8 = lane >> 2, lo_at = l8 * 64 + ((c ^ ((l8 >> 1) & 3)) << 4), hi_at = l8 * 32 + (((c >> 1) ^ (l8 >> 2)) << 4) + ((c & 1) << 3),
+                           out_at = l8 * 128 + (((2 * c) ^ l8) << 4);
+            const int out_next = (int)((out_at ^ 16u) - out_at);
+            auto first = [&](int kb) { return ((uw & 3) + 4 - (kb / x6.groups * steps & 3)) & 3; };
+            const int g = x6.groups;
+            // The scales of four turns at a time, a word (a row's four groups) a load: lane (row, c) requests those of its rows for the c-th of the turns and
+            // the lanes of a row hand them round. The first turn's come by themselves, before what can wait.
+            uint32_t sc_cur[4], sc_next[4];
+            const uint32_t pick = (uint32_t)(c | (c + 4) << 4);        // byte c of two words
+            auto fetch = [&](uint32_t (&w)[4], int k) {                // of box k
+                const int i0 = first(k);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    w[j] = 0x38383838u;
+                    if (i0 + 4 * j < steps && k < k1) w[j] = gload(reinterpret_cast<const uint32_t*>(x6.s_rel + (size_t)min(n0 + row_of(i0 + 4 * j), p.N - 1) * x6.srel_pitch) + k);
                 }
             };
-            const int mode = w6_mode(sc);
-            if (mode == W6_MID) expand(std::integral_constant<int, W6_MID>());
-            else if (mode == W6_SMALL) expand(std::integral_constant<int, W6_SMALL>());
-            else if (mode == W6_UNIT) expand(std::integral_constant<int, W6_UNIT>());
-            else expand(std::integral_constant<int, W6_ANY>());
-            fence_proxy_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
-            sa += g, sb += g;
-            if (sa >= SA) sa -= SA, pa ^= 1u;
-            if (sb >= SB) sb -= SB, pb ^= 1u;
+            int sa = grp, sb = grp;                                    // a group beyond the boxes has none
+            uint32_t pa = 0, pb = 0;
+            fetch(sc_cur, k0 + grp);
+            fetch(sc_next, k0 + grp + (c + 1) * g);
+            for (int kb = grp < g ? k0 + grp : k1, turn = 0; kb < k1; kb += g, ++turn) {
+                if ((turn & 3) == 1) {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) sc_cur[j] = sc_next[j];
+                    fetch(sc_next, kb + (c + 4) * g);
+                }
+                uint32_t w[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = __shfl_sync(0xffffffffu, sc_cur[j], (lane & 28) | ((turn + 3) & 3));
+                const uint32_t sc = __byte_perm(__byte_perm(w[0], w[1], pick), __byte_perm(w[2], w[3], pick), 0x5410);
+                // the expanded slot first, as above: groups <= sb <= sa keeps every awaited phase the current or the last one
+                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_wempty + 8 * sb, pb ^ 1u)) &&
+                    !mbar_wait_warp(bar_wempty + 8 * sb, pb ^ 1u, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                if (!__all_sync(0xffffffffu, mbar_try_wait(bar_full + 8 * sa, pa)) &&
+                    !mbar_wait_warp(bar_full + 8 * sa, pa, abort_s, ST_TIMEOUT_UNPACK)) { ok = false; break; }
+                const int i0 = first(kb);
+                const uint8_t* lo = sm + (sLo - base) + sa * lo_bytes + i0 * 512 + lo_at;
+                const uint8_t* hi = sm + (sHi - base) + sa * hi_bytes + i0 * 256 + hi_at;
+                uint8_t* out = sm + sb * w_bytes + i0 * 1024 + out_at;
+                // Up to four steps in a straight line: one by one, a warp waits for each (64 x 5120 -> 15360 27.5 us, 26.5 with the next line's scales).
+                uint32_t s4 = sc;
+                auto expand = [&](auto mode) {
+                    auto lines = [&](auto count) {
+                        constexpr int kN = decltype(count)::value;
+                        uint4 l[kN];
+                        uint2 h[kN];
+#pragma unroll
+                        for (int j = 0; j < kN; ++j) l[j] = *reinterpret_cast<const uint4*>(lo + 2048 * j), h[j] = *reinterpret_cast<const uint2*>(hi + 1024 * j);
+#pragma unroll
+                        for (int j = 0; j < kN; ++j) {
+                            uint32_t o[8];
+                            w6_group<decltype(mode)::value>(l[j], h[j].x, h[j].y, (s4 >> (8 * j)) & 0xffu, o);
+                            *reinterpret_cast<uint4*>(out + 4096 * j) = make_uint4(o[0], o[1], o[2], o[3]);
+                            *reinterpret_cast<uint4*>(out + 4096 * j + out_next) = make_uint4(o[4], o[5], o[6], o[7]);
+                        }
+                    };
+                    if (i0 + 12 < steps) lines(std::integral_constant<int, 4>());
+                    else if (i0 + 8 < steps) lines(std::integral_constant<int, 3>());
+                    else lines(std::integral_constant<int, 2>());      // tiles have eight steps or more
+                };
+                const int mode = w6_mode(sc);
+                if (mode == W6_MID) expand(std::integral_constant<int, W6_MID>());
+                else if (mode == W6_SMALL) expand(std::integral_constant<int, W6_SMALL>());
+                else if (mode == W6_UNIT) expand(std::integral_constant<int, W6_UNIT>());
+                else expand(std::integral_constant<int, W6_ANY>());
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bar_wfull + 8 * sb);
+                sa += g, sb += g;
+                if (sa >= SA) sa -= SA, pa ^= 1u;
+                if (sb >= SB) sb -= SB, pb ^= 1u;
+            }
         }
         // accumulators to shared memory, [token][weight row] int32, over the rings (all copies have landed and all MMAs have
         // read them when the accumulator is complete)
@@ -636,10 +723,10 @@ int launch_w6(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& 
                    : launch_w6_mh<OutT, EPI, 1>(ta, tlo, thi, td, p, x6, grid, st);
 }
 
-template <typename OutT, int EPI, bool TILED>
+template <typename OutT, int EPI, bool TILED, bool ROW_A_LANE>
 int launch_w6_rows_tiled(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const GemmParams& p, const W6RowsParams& x6,
                          size_t smem, cudaStream_t st) {
-    auto kern = gemm_w6a8_rows_kernel<OutT, EPI, TILED>;
+    auto kern = gemm_w6a8_rows_kernel<OutT, EPI, TILED, ROW_A_LANE>;
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
     cudaGetDevice(&dev);
@@ -655,12 +742,12 @@ int launch_w6_rows_tiled(const CUtensorMap& ta, const CUtensorMap& tlo, const CU
 template <typename OutT, int EPI>
 int launch_w6_rows(const CUtensorMap& ta, const CUtensorMap& tlo, const CUtensorMap& thi, const GemmParams& p, const W6RowsParams& x6,
                    size_t smem, cudaStream_t st) {
-    return p.tiles_m > 1 ? launch_w6_rows_tiled<OutT, EPI, true>(ta, tlo, thi, p, x6, smem, st)
-                         : launch_w6_rows_tiled<OutT, EPI, false>(ta, tlo, thi, p, x6, smem, st);
+    return p.tiles_m > 1 ? launch_w6_rows_tiled<OutT, EPI, true, false>(ta, tlo, thi, p, x6, smem, st)
+           : w6_row_a_lane(x6.tokens, x6.height, true) ? launch_w6_rows_tiled<OutT, EPI, false, true>(ta, tlo, thi, p, x6, smem, st)
+                                                 : launch_w6_rows_tiled<OutT, EPI, false, false>(ta, tlo, thi, p, x6, smem, st);
 }
 
 // Clusters of 1 .. 8 CTAs of the kernel above that the current device holds at once ([0] unused): asked of the runtime once per device.
-constexpr int kW6RowsMaxSplits = 8;
 const int* w6_rows_clusters() {
     static int count[64][kW6RowsMaxSplits + 1];
     static std::mutex mu;
@@ -669,7 +756,7 @@ const int* w6_rows_clusters() {
     std::lock_guard<std::mutex> lk(mu);
     int* c = count[dev & 63];
     if (c[0] == 0) {
-        auto kern = gemm_w6a8_rows_kernel<bf16, EPI_PLAIN, false>;
+        auto kern = gemm_w6a8_rows_kernel<bf16, EPI_PLAIN, false, false>;
         c[1] = device_sm_count(dev);
         if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes) == cudaSuccess) {
             for (int i = 2; i <= kW6RowsMaxSplits; ++i) {
@@ -691,33 +778,8 @@ const int* w6_rows_clusters() {
 int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, cudaStream_t st) {
     const int64_t M = p.M, N = p.N, K = p.K;
     W6RowsParams x6{s_rel, (int)(K / 32), 0, 1, p.k_iters, 0, 0, 0, BM};
-    // Token tiles and K slices: rounds of clusters times the cost of one, in K boxes (0.56 us of expansion each). A CTA's rings take
-    // a whole SM and a cluster has to lie in one GPC, so the device holds fewer clusters than SMs / s (148, 74, 45, 33, 26, 22, 15,
-    // 15 of 1 to 8 CTAs); a second round costs as much as the first. Start, end and the tokens' share of epilogue and exchange as
-    // measured at 16, 64, 128 and 256 tokens for 25 sizes of N and K (64 x 1024 to 20480 x 5120): the slices chosen are within
-    // 3.5 % of the best of all eight. Narrower token tiles expand the weight once more each, which pays where SMs would idle
-    // (256 x 120 x 1024 in four: 7.9 us, 10.9 in one); they have to promise 5 %.
-    const int* clusters = w6_rows_clusters();
-    double best = 1e30;
-    int last = 0;
-    for (const int width : {256, 192, 128, 96, 64}) {
-        const int tiles_m = (int)((M + width - 1) / width);
-        const int tokens = (int)(((M + tiles_m - 1) / tiles_m + 15) / 16 * 16);      // equal shares, at most 256
-        if (tokens == last) continue;
-        last = tokens;
-        double cost = 1e30;
-        int splits = 1, kps = p.k_iters;
-        int height = BM;
-        for (int h = BM; h >= 64; h -= 8)
-            for (int s = 1; s <= kW6RowsMaxSplits && s <= p.k_iters; ++s) {
-                const int k = (p.k_iters + s - 1) / s, room = clusters[s];
-                if ((p.k_iters + k - 1) / k != s || room < 1) continue;          // a slice would be empty; no such cluster fits
-                const double rounds = (double)(((N + h - 1) / h * tiles_m + room - 1) / room);
-                const double c = rounds * (k * (h / 8 + 2) / 18.0 + (s == 1 ? 8 + tokens / 28.0 : 10.5 + tokens / (s <= 4 ? 40.0 : 26.0)));
-                if (c < cost) cost = c, splits = s, kps = k, height = h;
-            }
-        if (cost < 0.95 * best) best = cost, x6.tokens = tokens, x6.splits = splits, x6.kps = kps, x6.height = height;
-    }
+    const W6RowsPlan plan = w6_rows_search(M, N, p.k_iters, w6_rows_clusters());
+    x6.tokens = plan.tokens, x6.splits = plan.splits, x6.kps = plan.kps, x6.height = plan.height;
     p.tiles_m = (int)((M + x6.tokens - 1) / x6.tokens);
     p.tiles_n = (int)((N + x6.height - 1) / x6.height);
     p.idesc = umma_idesc_i8(BM, x6.tokens);

@@ -209,3 +209,18 @@ def test_argument_checks(pkg, dev):
     packed = torch.zeros((16, 192), dtype=torch.uint8, device=dev)
     with pytest.raises(RuntimeError, match="-206"):
         L.w6a8_gemm_acc_i32(A, packed, torch.zeros((16, 4), dtype=torch.uint8, device=dev), G=64)
+
+
+# One tile of more than 112 tokens beside weight tiles of whole height: a lane has a row of a box. Slices that begin inside a block of four boxes, scale rows
+# that cannot be read 16 bytes at a time, a last tile of 20 and of 1 rows, rings of three, four and five slots.
+@pytest.mark.parametrize("M,N,K", [(113, 5121, 3456), (129, 5120, 2560), (200, 9217, 896), (200, 18900, 640), (256, 18900, 128), (256, 5120, 3584), (256, 9300, 2048)])
+def test_few_rows_whole_tiles_and_many_tokens(pkg, oracle, dev, M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    packed = torch.randint(0, 256, (N, K // 4 * 3), dtype=torch.uint8, generator=g).to(dev)
+    A = torch.randint(-127, 128, (M, K), dtype=torch.int8, generator=g).to(dev)
+    for scales in (torch.randint(0x28, 0x49, (N, K // 32), generator=g), torch.randint(0, 0x7f, (N, K // 32), generator=g), torch.full((N, K // 32), 0x38)):
+        s_rel = scales.to(torch.uint8).to(dev)
+        acc = pkg.linear.w6a8_gemm_acc_i32(A, packed, s_rel)
+        want = pkg.linear.int8_gemm_acc_i32(A, pkg.linear.w6_decode(packed, s_rel, K))
+        assert_bits_equal(acc, want, "accumulators")
+    assert pkg.linear.kernel_status() == 0
