@@ -778,7 +778,9 @@ const int* w6_rows_clusters() {
 int run_w6_rows(int epi, const int8_t* A, const uint8_t* Wq6, const uint8_t* s_rel, GemmParams& p, int out_dt, cudaStream_t st) {
     const int64_t M = p.M, N = p.N, K = p.K;
     W6RowsParams x6{s_rel, (int)(K / 32), 0, 1, p.k_iters, 0, 0, 0, BM};
-    const W6RowsPlan plan = w6_rows_search(M, N, p.k_iters, w6_rows_clusters());
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const W6RowsPlan plan = w6_rows_plan(dev, M, N, p.k_iters, w6_rows_clusters());
     x6.tokens = plan.tokens, x6.splits = plan.splits, x6.kps = plan.kps, x6.height = plan.height;
     p.tiles_m = (int)((M + x6.tokens - 1) / x6.tokens);
     p.tiles_n = (int)((N + x6.height - 1) / x6.height);
