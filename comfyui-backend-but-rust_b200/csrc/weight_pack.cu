@@ -669,6 +669,7 @@ __global__ void __launch_bounds__(256) w6_requant_kernel(const bf16* __restrict_
 __device__ __forceinline__ float rint_clamped(float x, float bound) {
     return __fsub_rn(__fadd_rn(fminf(bound, fmaxf(-bound, x)), 12582912.f), 12582912.f);
 }
+template <bool LONG>
 __global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* w, uint8_t* packed, uint8_t* s_rel,
                                                               float* s_channel, int64_t N, int K, int rows, uint64_t seed) {
     extern __shared__ __align__(128) float smem_f[];
@@ -729,18 +730,19 @@ __global__ void __launch_bounds__(512) w6_requant_regs_kernel(const bf16* w, uin
     const uint32_t e0 = (uint32_t)(n * (int64_t)K + g * 32);
     auto level = [&](float f) { return rint_clamped(__fmul_rn(f, s), 127.f); };       // w6_level(i) at f = i - 31
     // Eight values at a time, from the buffer they came back through: unrolled over all 32 the search alone is 30 KB of instructions, and
-    // waiting for those was the largest stall (5120 x 5120: 126 us, now 106).
+    // waiting for those was the largest stall (5120 x 5120: 126 us, now 106). LONG: rows of more than 288 threads, whose warps go through it side by side and wait
+    // less than the loop costs (3072 x 12288 unrolled 148 us, in the loop 157).
     const float* re = l.tbuf_w + tpad(l.t8 << 5) + l.tsw;
     const float* ro = l.tbuf_w + tpad(l.t8 << 5) - l.tsw;
     uint4 lo = make_uint4(0u, 0u, 0u, 0u);
     uint2 hi = make_uint2(0u, 0u);
-#pragma unroll 1
+#pragma unroll (LONG ? 4 : 1)
     for (int q = 0; q < 4; ++q) {
         uint32_t lw8 = 0u, hw8 = 0u;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int i = 8 * q + j;
-            const float t = __fmul_rn(((j & 1) ? ro : re)[i], inv_sc);
+            const float t = __fmul_rn(LONG ? v[i] : ((j & 1) ? ro : re)[i], inv_sc);
             int pos = min(max(__float2int_ru(__fmul_rn(__fsub_rn(ceilf(t), 0.5f), inv_s)), -31), 32) + 31;
             float f = (float)(pos - 31), below = level(f - 1.f), at = level(f);
             while (pos > 0 && below >= t) --pos, f -= 1.f, at = below, below = level(f - 1.f);
@@ -1043,8 +1045,9 @@ GPU_API int gpu_w6_requant(const void* weight, void* packed, void* s_rel, void* 
     if (N <= 0) return 0;
     if (K <= kRegRowsMaxK && (((uintptr_t)weight & 15) == 0)) {
         const RegRows g = reg_rows(K);
-        if (int rc = set_smem((const void*)w6_requant_regs_kernel, g.smem)) return rc;
-        return launch_pdl(w6_requant_regs_kernel, dim3((unsigned)((N + g.rows - 1) / g.rows)), g.threads, g.smem, (cudaStream_t)stream,
+        auto kern = g.threads > 288 ? w6_requant_regs_kernel<true> : w6_requant_regs_kernel<false>;
+        if (int rc = set_smem((const void*)kern, g.smem)) return rc;
+        return launch_pdl(kern, dim3((unsigned)((N + g.rows - 1) / g.rows)), g.threads, g.smem, (cudaStream_t)stream,
                           (const bf16*)weight, (uint8_t*)packed, (uint8_t*)s_rel, (float*)s_channel, N, K, g.rows, seed);
     }
     const size_t smem = (size_t)(padded_words(K) + K / 32) * sizeof(float);

@@ -406,3 +406,14 @@ def test_loader_threads_with_rows_of_different_length(pkg, dev, call):
         t.join()
     torch.cuda.synchronize()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("N,K", [(7, 8192), (5, 9216), (6, 9472), (3, 12288), (2, 16384)])
+def test_w6_requant_rows_on_either_side_of_288_threads(pkg, oracle, dev, N, K):
+    """The search for the codes is a loop in CTAs of up to 288 threads and unrolled in longer ones: the same codes and scales."""
+    g = torch.Generator().manual_seed(N + K)
+    w = (torch.randn(N, K, generator=g) * torch.exp2(torch.randint(-4, 5, (N, K // 32), generator=g).float()).repeat_interleave(32, 1) * 0.02).bfloat16()
+    w[0, :256] = 0.0
+    for seed in (0, 5):
+        for a, b, what in zip(pkg.linear.w6_requant(w.to(dev), seed), oracle.w6_requant(w, seed), ("codes", "group scales", "channel scales")):
+            assert_bits_equal(a, b, what)
