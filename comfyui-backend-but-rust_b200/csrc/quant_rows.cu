@@ -1548,11 +1548,12 @@ int sm_count_of(int dev) {
 // their rotation: the other SMs are idle, the successor's setup and whatever it may do ahead (the few-rows GEMM brings its weights to
 // L2) run beside the rest, and no CTA of the quantizer is left that could land badly. The adaLN linear 1 x 3072 -> 18432 with its
 // quantizer: 17.2 us, now 16.4. Right behind the wait the successor's CTAs and their prefetches compete with the quantizer's own loads: the
-// W6A8 block of 64 rows (four quantizers of 64 CTAs) takes 121.5 us that way, 116.4 this.
+// W6A8 block of 64 rows (four quantizers of 64 CTAs) takes 121.5 us that way, 116.4 this. Up to seven SMs in eight: 125 CTAs and a GEMM (250 x 3072 -> 3072)
+// 12.8 us, 12.9 without; 139 (1111 x 1024 -> 3072) 12.5 and 12.1, 140 (140 x 8192 -> 3072) 19.9 and 19.5, for what starts early finds no SM idle.
 int early_trigger(int64_t ctas) {
     int dev = 0;
     cudaGetDevice(&dev);
-    return ctas <= sm_count_of(dev);
+    return ctas * 8 <= (int64_t)sm_count_of(dev) * 7;
 }
 template <int ROT, int SRC, int MAXT, bool EARLY = true>
 int launch_sd_cfg(const SdSrc& s, int8_t* q, float* scales, int M, int K, dim3 grid, int threads, int rows, uint32_t smem, uint32_t off_amax,
