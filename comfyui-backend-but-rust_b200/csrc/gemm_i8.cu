@@ -46,6 +46,7 @@ constexpr int kThreads = 320;  // warp 0 producer, warp 1 MMA, warps 2-9 epilogu
 constexpr int kEpiWarps = 8;
 constexpr int64_t kResidentOperandBytes = 32ll << 20;   // an A this small stays in L2 while W and D stream past it
 constexpr double kSmallProblemOps = 2.0e9;           // below this many int8 operations a GEMM takes the one-CTA-per-tile kernel
+constexpr int64_t kSmallProblemK = 5120;             // ... and up to this K
 constexpr int kRotEpiWarps = 8;                      // epilogue warps of the rotating epilogue (two per tensor-memory lane quarter)
 constexpr int kRotThreads = 64 + 32 * kRotEpiWarps;
 constexpr int kMaxStages = 8;
@@ -1745,11 +1746,13 @@ int run_gemm(int epi, const int8_t* A, const int8_t* W, const float* xs, const f
     while (small_bn > 32 && (int64_t)small_tm * ((N + small_bn - 1) / small_bn) < 96) small_bn >>= 1;
     const int64_t small_tiles = (int64_t)small_tm * ((N + small_bn - 1) / small_bn);
     const double ops = 2.0 * (double)M * (double)N * (double)K;
-    // measured on the SDXL shapes: below 2 Gop always (154 x 2048 x 640: 10.2 against 13.5 us in kernel); up to 8 Gop when
-    // the tiles fit the SMs in little more than one wave (2048 x 1280 x 1280, 160 tiles: 14.9 against 16.5 us; 8192 x 640 x
-    // 640, 320 tiles: 21.7 against 18.8, so not there)
-    const bool small = !rot && ((ops < kSmallProblemOps && (K <= 4096 || small_tiles >= 64)) ||
-                                (ops < 4.0 * kSmallProblemOps && K <= 4096 && small_tiles * 5 <= (int64_t)device_sm_count(dev) * 6));
+    // Back to back, us, this kernel | the pair kernel, fp16 without a residual and with one. Below 2 Gop: 154 x 2048 -> 1280 6.0 | 7.2 and 6.1 | 9.2, 2048 x 640 -> 640 4.9 | 6.1 and
+    // 5.2 | 6.8. Up to 8 Gop when the tiles fit the SMs in little more than one wave: 2048 x 1280 -> 1280 (160 tiles) 7.8 | 7.6 and 8.9 | 9.0, 4096 x 640 -> 640 6.4 | 6.9;
+    // 8192 x 640 -> 640 (320 tiles) 9.8 | 8.9, so not there. (Some beyond that line still gain, 333 x 1280 -> 3840 6.2 | 7.2 and 6.6 | 8.5: 180 tiles.) A longer K is cut
+    // over all SMs by the pair kernel: 333 x 5120 -> 1280 10.8 | 11.5 and 11.0 | 12.4, 13 x 5120 -> 1280 10.7 | 11.6 and 10.7 | 13.5, 154 x 6144 -> 1280 12.2 | 11.2
+    // and 12.4 | 13.0, 154 x 8192 -> 640 15.3 | 12.5 with a residual.
+    const bool small = !rot && ((ops < kSmallProblemOps && (K <= kSmallProblemK || small_tiles >= 64)) ||
+                                (ops < 4.0 * kSmallProblemOps && K <= kSmallProblemK && small_tiles * 5 <= (int64_t)device_sm_count(dev) * 6));
     if (small) {
         const int tiles_m = small_tm;
         const int bn = small_bn;

@@ -357,3 +357,21 @@ def test_bias_residual_add_and_cluster_limit(pkg, oracle, dev):
     finally:
         L.set_gemm_cluster_limit(0)
     assert L.kernel_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(13, 1280, 5120), (13, 1280, 5136), (77, 320, 4112), (333, 1272, 5104), (154, 648, 5248)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+def test_few_tiles_and_a_long_k_on_either_kernel(pkg, oracle, dev, M, N, K, dtype):
+    """Few tiles with a K at the line between one CTA per tile and the pair kernel's K slices: accumulators, the plain and the residual form."""
+    g, A, W, xs, ws = _operands(M, N, K, M + N + K)
+    bias, rscale, resid = (torch.randn(*s, generator=g).to(dtype) for s in ((N,), (N,), (M, N)))
+    d = lambda t: t.to(dev)
+    L = pkg.linear
+    acc = L.int8_gemm_acc_i32(d(A), d(W))
+    assert_bits_equal(acc, (d(A).double() @ d(W).double().t()).to(torch.int32), "accumulators")
+    a = (d(A), d(W), d(xs), d(ws), d(bias))
+    assert_bits_equal(L.int8_gemm(*a, out_dtype=dtype), L.int8_epilogue(acc, *a[2:], out_dtype=dtype), "plain")
+    out = d(resid).clone()
+    assert_bits_equal(L.int8_gemm(*a, out_dtype=dtype, rscale=d(rscale), resid=out, out=out),
+                      L.int8_epilogue(acc, *a[2:], out_dtype=dtype, rscale=d(rscale), resid=d(resid)), "residual in place")
+    assert L.kernel_status() == 0
