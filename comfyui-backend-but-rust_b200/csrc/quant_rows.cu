@@ -559,19 +559,14 @@ __device__ __forceinline__ void direct_values(const QuantArgs& p, const DirectLa
         elementwise_prologue<T, PRO>(v, u, PRO != PRO_GELU && p.lut >= 0 ? g_act_lut[p.lut] : nullptr);      // GELU's table: see launch_quant
     }
 }
-// A warp's lanes: all of them but in a partial last warp (threads = rows * K / 32)
-__device__ __forceinline__ unsigned warp_lanes(unsigned tid) {
-    const unsigned left = blockDim.x - (tid & ~31u);
-    return left >= 32 ? 0xffffffffu : (1u << left) - 1;
-}
-__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem, unsigned tid) {
+__device__ __forceinline__ DirectLane direct_lane(const QuantArgs& p, uint8_t* smem, unsigned tid, unsigned wmask) {
     const int warp = tid >> 5, lane = tid & 31, team = lane >> 3;
     const int rloc = tid / (unsigned)p.tpr, tin = tid - rloc * p.tpr;
     const int64_t m = (int64_t)blockIdx.x * p.rows_per_cta + rloc;
     float* tbuf = reinterpret_cast<float*>(smem) + warp * kWarpWords + team * kGroupWords + 4 * (team >> 1);
-    // idle rows compute on the last row and store nothing
+    // idle rows compute on the last row and store nothing; the last warp of a CTA may be partial (threads = rows * K / 32)
     return {tbuf, tbuf - 2 * (team >> 1), reinterpret_cast<unsigned*>(smem + p.off_amax), m < p.M ? m : p.M - 1, rloc, tin << 5, tin & 7, team & 1,
-            m < p.M, tin == 0, warp_lanes(tid)};
+            m < p.M, tin == 0, wmask};
 }
 // The thread's index, read anew: what is worked out from it need not stay in registers while a row's 32 values and their look-ups fill them
 __device__ __forceinline__ unsigned tid_anew() {
@@ -579,11 +574,12 @@ __device__ __forceinline__ unsigned tid_anew() {
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
     return t;
 }
-// The second pass, out of line: what it holds would take registers from the first.
+// The second pass, out of line: what it holds would take registers from the first. The warp's mask is the kernel's: it says which lanes there are,
+// and is read where all of them are together.
 template <typename T, int PRO, bool DIGITS>
-__device__ __noinline__ void direct_again(const QuantArgs& p) {
+__device__ __noinline__ void direct_again(const QuantArgs& p, unsigned wmask) {
     extern __shared__ __align__(128) uint8_t smem[];
-    const DirectLane l = direct_lane(p, smem, threadIdx.x);
+    const DirectLane l = direct_lane(p, smem, threadIdx.x, wmask);
     float v[32];
     direct_values<T, PRO>(p, l, v);
     direct_second<T, DIGITS>(p, l, v);
@@ -592,7 +588,7 @@ template <typename T, int PRO, int MAXT, bool DIGITS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr bool kAnew = sizeof(T) == 2 && (PRO == PRO_SILU || PRO == PRO_GELU || PRO == PRO_GELU_TANH);
-    const DirectLane l = direct_lane(p, smem, threadIdx.x);
+    const DirectLane l = direct_lane(p, smem, threadIdx.x, __activemask());
     direct_clear<DIGITS>(p, l.bits);
     pdl_wait();
     if (DIGITS) clear_counters(p);
@@ -601,10 +597,10 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel
     {
         float v[32];
         direct_values<T, PRO>(p, l, v);
-        if constexpr (kAnew) done = direct_first<T, DIGITS>(p, direct_lane(p, smem, tid_anew()), v);
+        if constexpr (kAnew) done = direct_first<T, DIGITS>(p, direct_lane(p, smem, tid_anew(), l.wmask), v);
         else done = direct_first<T, DIGITS>(p, l, v);
     }
-    if (!done) direct_again<T, PRO, DIGITS>(p);
+    if (!done) direct_again<T, PRO, DIGITS>(p, l.wmask);
 }
 
 // Normalising prologues on bf16 rows. The row sums are added in the reference's order (csrc/kernels.cu:113-147, csrc/common.cuh:30-55), so
