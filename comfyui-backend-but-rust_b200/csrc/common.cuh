@@ -29,8 +29,8 @@ typedef __nv_bfloat16 bf16;
 //     stream has ended and its writes are visible. Every thread that touches such memory waits, so an order that held
 //     between whole kernels (results, buffers used again, the zeros of the split scratch) holds as before;
 //   - in the quantizers and the W6 decoder pdl_trigger(), when a CTA has its rows and little but the codes and their stores is
-//     left: the stream's next kernel may be brought onto the SMs once every CTA has got there or ended. The others, the GEMMs
-//     among them, leave it at the end of their CTAs. A trigger at a kernel's start loses more than it hides: the successor's
+//     left, or as soon as its rows are in where the CTAs leave SMs idle (early_trigger() in quant_rows.cu): the stream's next kernel may be
+//     brought onto the SMs once every CTA has got there or ended. The others, the GEMMs among them, leave it at the end of their CTAs. A trigger at a kernel's start loses more than it hides: the successor's
 //     CTAs then go where there is room beside the running kernel, and a small quantizer after a GEMM on 64 of 74 cluster pairs
 //     lands on the twenty idle SMs, all of it. As CUDA graphs, with the trigger at the start | here | ordinary launches: DiT block
 //     512 x 1536 105 | 85 | 90 us, SwiGLU block 512 x 1536 90 | 70 | 75, linear 333 x 3072 x 3072 18.3 | 15.4 | 16.9, two

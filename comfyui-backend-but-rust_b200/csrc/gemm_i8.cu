@@ -466,8 +466,9 @@ template <int N> __device__ __forceinline__ void bulk_wait_read() {
 // contiguous bytes per lane and store (whole sectors: no staging in shared memory, no fence, nothing to wait for). With a short K
 // this is what sets a tile's pace, so nothing of it is waited for in the drain itself: the per-column vectors, the row scale and
 // the residual of the whole tile are requested before the accumulator is awaited, and the accumulator is handed back as soon as
-// the last chunk is out of tensor memory. In a chain of launches, us, before | now: 8192 x 640 -> 5120 52 | 38, 8192 x 640 -> 640 14.8 | 9.8 and with a
-// residual 17.2 | 14.1, 2048 x 1280 -> 1280 (one CTA per tile) 14.5 | 9.8, 4352 x 3072 -> 3072 with a residual 46.7 | 38.6.
+// the last chunk is out of tensor memory. In a chain of launches, us, staged and read back chunk by chunk | this: 4352 x 3072 -> 3072 with a residual 46.7 | 38.6,
+// 2048 x 1280 -> 1280 (one CTA per tile) 14.5 | 9.8; alone, back to back, the latter takes 7.8 and 8.9 with a residual. A pair's tiles of shorter K go through
+// shared memory all the same (epilogue_staged below).
 __device__ __forceinline__ void st_global_v8(void* p, const uint32_t (&v)[8]) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -1682,6 +1683,10 @@ int* split_workspace(int dev, cudaStream_t st, size_t need) {
 // the last round nearly empty at 256 takes a narrower tile instead; narrower tiles read A from L2 once more per column
 // tile, and on large shapes the L2 -> SM path, not the tensor core, is what the kernel waits for (up-projection: 113 us
 // at 256 against 118 at 224 and 124 at 192, although 224 has the smaller product), hence the mild penalty on width lost.
+// The constant of 32 columns a tile is the time of a drain that has since changed three ways, and the short ring of the staged one is not in it. With the
+// present drains, 100 shapes of 77 to 8192 rows, K and N 320 to 10240, fp16 with and without a residual: the width chosen is 1.8 % from the best on
+// average; from 5 % up are 8192 x 1280 -> 3840 with a residual (49.0 us, 42.5 at 256), 8192 x 2048 -> 1280 (23.1, 20.5 at 224), 2048 x 4096 -> 1024 with one
+// (14.6, 13.3 at 128), 8192 x 5120 -> 1280 (47.7, 43.6 at 224).
 // (Launching only as many CTA pairs as the round count needs, 68 instead of 74 for 816 tiles in 12 rounds, leaves SMs idle
 // and raises the power-capped clock by about 1 %, but the step was 0.7 % slower: not done.)
 int choose_bn(int64_t M, int64_t N, int clusters) {
@@ -1898,12 +1903,13 @@ GPU_API int gpu_w6a8_gemm_acc_i32(const int8_t* A, const uint8_t* Wq6, const uin
 // New: the weight-only int8 linear of the text encoders in one call. The reference rotates the f32 activation rows
 // (gpu_rotate_rows_f32, csrc/kernels.cu:316-327), dequantizes the whole int8 weight to f32 (gpu_dequant_i8, :330-343) and runs
 // an fp32 GEMM with beta 0 or 1 (src/te.rs:493-511). Here: out[M,N] = beta * out + R256(prologue(x)) . (Wq * ws[n])^T with the
-// product on the int8 tensor cores: Wq as it is, the rotated rows as fixed-point numbers of 22 bits and sign in three 8-bit digits, one
-// power of two per row, so a value is within 2^-22 of its row's maximum and the rest is exact up to the f32 roundings at the end.
+// product on the int8 tensor cores: Wq as it is, the rotated rows as fixed-point numbers of 22 bits and sign in three 8-bit digits. One power of two
+// per row, or per rotation group of 256 in rows whose groups lie three binary orders or more apart: a value is within 2^-20 of the maximum of its group, the
+// products are exact and the rest is f32 roundings at the end.
 //   prologue   PRO_PLAIN, PRO_RMS (norm_w, eps) or PRO_SWIGLU (up_offset) as gpu_rotate_rows_f32 takes them
 //   a_scratch  >= 4 * M * K bytes (the reference's rotated-rows buffer has that size), w_scratch >= 2 * N * K bytes
 //              (half of the reference's dequantized-weight buffer); both 16-byte aligned
-//   beta       0 or 1 (-207 otherwise); K % 256 == 0 (-1); N * 4 bytes a multiple of 16 for the fast store path
+//   beta       0 or 1 (-207 otherwise); K % 256 == 0 (-1)
 GPU_API int gpu_wo8_linear(int prologue, const float* x, int64_t x_stride, int64_t up_offset, const float* norm_w, float eps,
                            const int8_t* Wq, const float* ws, float* out, float beta, void* a_scratch, void* w_scratch, int M,
                            int N, int K, void* stream) {
