@@ -587,7 +587,7 @@ __device__ __noinline__ void direct_again(const QuantArgs& p, unsigned wmask) {
 template <typename T, int PRO, int MAXT, bool DIGITS>
 __global__ void __launch_bounds__(MAXT, MAXT <= 288 ? 4 : 1) quant_direct_kernel(const __grid_constant__ QuantArgs p) {
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr bool kAnew = sizeof(T) == 2 && (PRO == PRO_SILU || PRO == PRO_GELU || PRO == PRO_GELU_TANH);
+    constexpr bool kAnew = sizeof(T) == 2 && (PRO == PRO_SILU || PRO == PRO_GELU || PRO == PRO_GELU_TANH || PRO == PRO_SWIGLU);
     const DirectLane l = direct_lane(p, smem, threadIdx.x, __activemask());
     direct_clear<DIGITS>(p, l.bits);
     pdl_wait();

@@ -161,7 +161,8 @@ int gpu_int8_epilogue(const int32_t* acc, const float* xs, const float* ws, cons
  * or 1 (src/te.rs:493-511); this computes out[M,N] = beta * out + R256(prologue(x)) . (Wq * ws[n])^T on the int8 tensor
  * cores: Wq [N,K] as it is, the rotated f32 rows as fixed-point numbers of 22 bits and sign in three 8-bit digits with exact
  * int32 sums, a power of two per row or, where a row's rotation groups of 256 lie far apart, per group: a value keeps 2^-20 of the
- * maximum of its group, whatever lies beside it (a value far below its own group's maximum keeps fewer bits of its own). prologue PLAIN, RMS (norm_w, eps) or SWIGLU (up_offset) as for gpu_rotate_rows_f32 (-3).
+ * maximum of its group, whatever lies beside it (a value far below its own group's maximum keeps fewer bits of its own).
+ * prologue PLAIN, RMS (norm_w, eps) or SWIGLU (up_offset) as for gpu_rotate_rows_f32 (-3).
  * a_scratch >= 4*M*K bytes, w_scratch >= 2*N*K bytes, 16-byte aligned (-202); beta 0 or 1 (-207); K % 256 == 0 (-1).
  * Result: within 1e-5 of the largest output of the fp32 flow, and each output within 2^-20 of the maxima of the groups that its
  * weights read, summed over them (tests state the bounds). */
